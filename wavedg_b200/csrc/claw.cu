@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "claw_model.cuh"
+#include "exact_line.cuh"
 #include "wave_impl.hpp"
 
 using namespace wdg;
@@ -22,8 +23,8 @@ struct wdg_claw
     wdg_wave *w = nullptr;
     int n = 0, nv = 4;
     double *d_buf[4] = {nullptr, nullptr, nullptr, nullptr}; // stepping: RK4 B, C, register; SSPRK3 y1, y2
-    // approx_quad = false: the exact operators' geometry and M^{-1} (an internal exact handle,
-    // whose collocation handle is w), the volume rule (q points) and the face rule (qf points)
+    // approx_quad = false: the exact operators' geometry (an internal exact handle, whose
+    // collocation handle is w), the volume rule (q points) and the face rule (qf points)
     wdg_waveq *exact = nullptr;
     int q = 0, qf = 0;
     double *d_xv = nullptr, *d_wv = nullptr, *d_Pv = nullptr, *d_Dv = nullptr, *d_wf = nullptr, *d_Pf = nullptr;
@@ -101,26 +102,90 @@ namespace
 {
     // ------------------------------------------------------------------ approx_quad = false
     // The Euler operators of examples/cl2d.cpp as shipped (DivF2D<false>, EdgeFluxF2D<false>,
-    // MassMatrix<false>; wavedg/DivF.hpp:262-394, wavedg/EdgeFluxF.hpp:182-254) fused per
-    // element, a warp each: u interpolated to the q x q volume points (P), the physical flux
-    // there, its contravariant form with the Jacobian at the points and the weights, the D and
-    // P contractions back to the nodes; per side the element's own nodal trace and its
-    // neighbour's (partner table; boundary: the own trace, exterior = interior) interpolated
-    // to the qf face points, the local Lax-Friedrichs flux with the element's own normal times
-    // w_i |E|/2, projected back and subtracted; then the dense inverse mass matrix, and the RHS
-    // or one RK4 / SSPRK3 stage.
+    // MassMatrix<false>; wavedg/DivF.hpp:262-394, wavedg/EdgeFluxF.hpp:182-254).  The RHS and the
+    // time-stepping stages are exact_line.cuh's fused kernel with this model: the physical flux at
+    // the 2n x 2n points made contravariant, the local Lax-Friedrichs flux at the 2n points of each
+    // side with the element's own normal (boundary: exterior = interior).
+    struct EulerX
+    {
+        static constexpr int NV = 4;
+        static constexpr bool LEG = false, FORCE = false;
+        __host__ __device__ static constexpr int q(int n) { return 2 * n; }
+        __host__ __device__ static constexpr int qf(int n) { return 2 * n; }
+        template <int N>
+        __device__ static const XTab<N, 2 * N, 2 * N> &table();
+        __device__ static void exterior(int, const double *, const double *own, double *x)
+        {
+#pragma unroll
+            for (int d = 0; d < 4; ++d)
+                x[d] = own[d];
+        }
+        // velocities and pressure over density with one reciprocal
+        __device__ static void primitive(const double *q, double &ir, double &u, double &v, double &p)
+        {
+            ir = 1.0 / q[0];
+            u = q[1] * ir;
+            v = q[2] * ir;
+            p = (ClawEuler::gamma - 1.0) * (q[3] - 0.5 * q[0] * (u * u + v * v));
+        }
+        template <int Q>
+        __device__ static void point(const XArgs &, int, int, int, double Xx, double Yx, double Xe, double Ye,
+                                     const double *U, double *F, double *G)
+        {
+            // contravariant components: momenta (Ye, -Xe) . m and (-Yx, Xx) . m carry the state,
+            // the pressure acts along the same vectors
+            double ir, u, v, p;
+            primitive(U, ir, u, v, p);
+            const double a = Ye * u - Xe * v, b = Xx * v - Yx * u, H = U[3] + p;
+            F[0] = U[0] * a;
+            F[1] = U[1] * a + Ye * p;
+            F[2] = U[2] * a - Xe * p;
+            F[3] = H * a;
+            G[0] = U[0] * b;
+            G[1] = U[1] * b - Yx * p;
+            G[2] = U[2] * b + Xx * p;
+            G[3] = H * b;
+        }
+        template <int N>
+        __device__ static void face(const XArgs &, int, int, int, const double *sn, double wf, const double *qL,
+                                    const double *qR, double *uf)
+        {
+            const double nx = sn[0], ny = sn[1], w = -0.5 * wf * sn[2];
+            double iL, uL, vL, pL, iR, uR, vR, pR;
+            primitive(qL, iL, uL, vL, pL);
+            primitive(qR, iR, uR, vR, pR);
+            const double c = fmax(sqrt(uL * uL + vL * vL) + sqrt(ClawEuler::gamma * pL * iL),
+                                  sqrt(uR * uR + vR * vR) + sqrt(ClawEuler::gamma * pR * iR));
+            const double nL = nx * uL + ny * vL, nR = nx * uR + ny * vR, ps = pL + pR;
+            uf[0] = w * (qL[0] * nL + qR[0] * nR + c * (qL[0] - qR[0]));
+            uf[1] = w * (qL[1] * nL + qR[1] * nR + nx * ps + c * (qL[1] - qR[1]));
+            uf[2] = w * (qL[2] * nL + qR[2] * nR + ny * ps + c * (qL[2] - qR[2]));
+            uf[3] = w * ((qL[3] + pL) * nL + (qR[3] + pR) * nR + c * (qL[3] - qR[3]));
+        }
+        template <int VP>
+        __device__ static void store(const XArgs &A, size_t el0, int at, const double *u, const double *p, const double *y)
+        {
+            x_store<VP>(A.c, el0, at, u, p, y);
+        }
+    };
+    __constant__ XTabs<EulerX> c_euler_x;
+    template <int N>
+    __device__ const XTab<N, 2 * N, 2 * N> &EulerX::table() { return xtab<N>(c_euler_x); }
+
+    // DivF2D<false>::action alone (the volume term against the nodal basis, added to the output):
+    // one warp per element, generic loops over shared memory
     struct QEArgs
     {
         ClawArgs c;
-        const double *xv, *wv, *Pv, *Dv, *wf, *Pf, *Minv;
-        int n, q, qf;
+        const double *xv, *wv, *Pv, *Dv;
+        int n, q;
     };
     constexpr int kQENV = 4;
 
-    __host__ __device__ inline int qe_warp_doubles(int n, int q, int qf)
+    __host__ __device__ inline int qe_warp_doubles(int n, int q)
     {
-        // su r (4 n^2 each) | Pu (4 n q) | Uq (4 q^2) | Fq (8 q^2) | Df Pg (4 q n each) | T1 (4 n 4) | UF (4 qf 4)
-        return 8 * n * n + 4 * n * q + 12 * q * q + 8 * q * n + 16 * n + 16 * qf;
+        // su (4 n^2) | Pu (4 n q) | Uq (4 q^2) | Fq (8 q^2) | Df Pg (4 q n each)
+        return 4 * n * n + 4 * n * q + 12 * q * q + 8 * q * n;
     }
 
     __device__ inline void qe_jac(const double *c, double xi, double eta, double J[4])
@@ -130,35 +195,23 @@ namespace
         J[2] = 0.25 * ((1.0 - xi) * (c[6] - c[0]) + (1.0 + xi) * (c[4] - c[2]));
         J[3] = 0.25 * ((1.0 - xi) * (c[7] - c[1]) + (1.0 + xi) * (c[5] - c[3]));
     }
-    __device__ inline int qe_node(int n, int s, int k)
-    {
-        const int i = (s == 0 || s == 2) ? k : (s == 1 ? n - 1 : 0);
-        const int j = (s == 1 || s == 3) ? k : (s == 2 ? n - 1 : 0);
-        return i + n * j;
-    }
     __global__ void qeuler_kernel(const QEArgs A, int warps)
     {
         extern __shared__ double esm[];
         const ClawArgs &a = A.c;
-        const int n = A.n, q = A.q, qf = A.qf, nn = n * n, qq = q * q, NV = kQENV;
+        const int n = A.n, q = A.q, nn = n * n, qq = q * q, NV = kQENV;
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        double *su = esm + (size_t)warp * qe_warp_doubles(n, q, qf);
-        double *r = su + NV * nn, *Pu = r + NV * nn, *Uq = Pu + NV * n * q, *Fq = Uq + NV * qq, *Df = Fq + 2 * NV * qq;
-        double *Pg = Df + NV * q * n, *T1 = Pg + NV * q * n, *UF = T1 + 4 * n * NV;
-        const long long limit = (long long)nn * a.nel;
+        double *su = esm + (size_t)warp * qe_warp_doubles(n, q);
+        double *Pu = su + NV * nn, *Uq = Pu + NV * n * q, *Fq = Uq + NV * qq, *Df = Fq + 2 * NV * qq;
+        double *Pg = Df + NV * q * n;
         for (int el = blockIdx.x * warps + warp; el < a.nel; el += gridDim.x * warps)
         {
             const double *xe = a.x + (size_t)NV * nn * el;
             for (int k = lane; k < NV * nn; k += 32)
-            {
                 su[k] = xe[k];
-                r[k] = 0.0;
-            }
             double c[8];
             for (int k = 0; k < 8; ++k)
                 c[k] = __ldg(a.corners + 8 * (size_t)el + k);
-            const uint32_t codes = __ldg(a.fcode + el);
-            const int4 fb = __ldg(a.fbase + el);
             __syncwarp();
             // Pu(l, d, i) = sum_k P(i, k) u(d, k, l)
             for (int o = lane; o < NV * n * q; o += 32)
@@ -210,127 +263,14 @@ namespace
                 Df[o] = df;
                 Pg[o] = pg;
             }
-            // neighbour nodal traces T1(s, k, d); boundary: the own trace
-            for (int o = lane; o < 4 * n; o += 32)
-            {
-                const int s = o / n, k = o - s * n;
-                const uint32_t byte = (codes >> (8 * s)) & 0xffu;
-                const double *own = su + NV * qe_node(n, s, k);
-                double *t1 = T1 + NV * o;
-                bool copy = (byte & 0x80u) != 0;
-                if (!copy)
-                {
-                    const int off = (s == 0) ? fb.x : (s == 1) ? fb.y : (s == 2) ? fb.z : fb.w;
-                    const uint32_t sc = byte & 3u;
-                    const int stride = (sc == 0) ? 1 : (sc == 1) ? -1 : (sc == 2) ? n : -n; // in nodes
-                    const long long pn = (long long)(off / 3) + (long long)k * stride;
-                    if (off < 0 || pn < 0 || pn >= limit)
-                    {
-                        atomicOr(a.err, 2u);
-                        copy = true;
-                    }
-                    else
-                        for (int d = 0; d < NV; ++d)
-                            t1[d] = __ldg(a.x + (size_t)NV * pn + d);
-                }
-                if (copy)
-                    for (int d = 0; d < NV; ++d)
-                        t1[d] = own[d];
-            }
             __syncwarp();
-            // volume result
             for (int o = lane; o < NV * nn; o += 32)
             {
                 const int d = o % NV, k = (o / NV) % n, l = o / (NV * n);
                 double t = 0.0;
                 for (int j = 0; j < q; ++j)
                     t += A.Pv[j + q * l] * Df[j + q * (d + NV * k)] + A.Dv[j + q * l] * Pg[j + q * (d + NV * k)];
-                r[o] = t;
-            }
-            // face points: UF(s, i, d) = w_i |E|/2 fh(n, own, neighbour)
-            for (int o = lane; o < 4 * qf; o += 32)
-            {
-                const int s = o / qf, i = o - s * qf;
-                double nx, ny, meas, qL[4] = {0, 0, 0, 0}, qR[4] = {0, 0, 0, 0};
-                claw_side(c, s, nx, ny, meas);
-                for (int j = 0; j < n; ++j)
-                {
-                    const double pw = A.Pf[i + qf * j];
-                    const double *own = su + NV * qe_node(n, s, j), *nb = T1 + NV * (s * n + j);
-                    for (int d = 0; d < NV; ++d)
-                    {
-                        qL[d] += own[d] * pw;
-                        qR[d] += nb[d] * pw;
-                    }
-                }
-                double fh[4];
-                ClawEuler::numflux<4>(a, el, s, nx, ny, qL, qR, fh);
-                const double ds = A.wf[i] * meas;
-                for (int d = 0; d < NV; ++d)
-                    UF[NV * o + d] = fh[d] * ds;
-            }
-            __syncwarp();
-            if (a.mode == CLAW_DIV)
-            {
-                for (int o = lane; o < NV * nn; o += 32)
-                    a.out[(size_t)NV * nn * el + o] += r[o];
-                __syncwarp();
-                continue;
-            }
-            // back to the face nodes, subtracted: sides 0 and 2, then 1 and 3
-            for (int pass = 0; pass < 2; ++pass)
-            {
-                for (int o = lane; o < 2 * n; o += 32)
-                {
-                    const int s = pass + 2 * (o / n), k = o % n, node = qe_node(n, s, k);
-                    for (int d = 0; d < NV; ++d)
-                    {
-                        double f = 0.0;
-                        for (int i = 0; i < qf; ++i)
-                            f += UF[NV * (s * qf + i) + d] * A.Pf[i + qf * k];
-                        r[NV * node + d] -= f;
-                    }
-                }
-                __syncwarp();
-            }
-            // M^{-1} (dense, per field) and the output: lane per row
-            const double *Me = A.Minv + (size_t)nn * nn * el;
-            for (int row = lane; row < nn; row += 32)
-            {
-                double y[4] = {0, 0, 0, 0};
-                for (int j = 0; j < nn; ++j)
-                {
-                    const double m = __ldg(Me + row + (size_t)nn * j);
-                    for (int d = 0; d < NV; ++d)
-                        y[d] += m * r[NV * j + d];
-                }
-                const size_t g0 = (size_t)NV * (nn * (size_t)el + row);
-                for (int d = 0; d < NV; ++d)
-                {
-                    const double qd = su[NV * row + d];
-                    switch (a.mode)
-                    {
-                    case CLAW_RHS:
-                        a.out[g0 + d] = y[d];
-                        break;
-                    case CLAW_RK4:
-                    {
-                        const double kd = (a.rk_a == 0.0) ? a.dt * y[d] : a.rk_a * a.du[g0 + d] + a.dt * y[d];
-                        a.du[g0 + d] = kd;
-                        a.out[g0 + d] = qd + a.rk_b * kd;
-                        break;
-                    }
-                    case CLAW_SSP0:
-                        a.out[g0 + d] = qd + a.dt * y[d];
-                        break;
-                    case CLAW_SSP1:
-                        a.out[g0 + d] = 0.25 * (qd + 3.0 * a.base[g0 + d] + a.dt * y[d]);
-                        break;
-                    default:
-                        a.out[g0 + d] = (a.base[g0 + d] + 2.0 * qd + 2.0 * a.dt * y[d]) / 3.0;
-                        break;
-                    }
-                }
+                a.out[(size_t)NV * nn * el + o] += t;
             }
             __syncwarp();
         }
@@ -381,26 +321,29 @@ namespace
 
     int qe_warps(const wdg_claw *h)
     {
-        const size_t per = sizeof(double) * (size_t)qe_warp_doubles(h->n, h->q, h->qf);
+        const size_t per = sizeof(double) * (size_t)qe_warp_doubles(h->n, h->q);
         return (int)std::max<size_t>(1, std::min<size_t>(4, (size_t)(200 * 1024) / per));
     }
 
     int qe_launch(wdg_claw *h, const ClawArgs &c)
     {
+        if (c.mode != CLAW_DIV)
+        {
+            XArgs X{};
+            X.c = c;
+            WDG_CUDA(xline_launch<EulerX>(h->n, X, h->w->stream));
+            return WDG_OK;
+        }
         QEArgs A{};
         A.c = c;
         A.xv = h->d_xv;
         A.wv = h->d_wv;
         A.Pv = h->d_Pv;
         A.Dv = h->d_Dv;
-        A.wf = h->d_wf;
-        A.Pf = h->d_Pf;
-        A.Minv = waveq_minv(h->exact);
         A.n = h->n;
         A.q = h->q;
-        A.qf = h->qf;
         const int warps = qe_warps(h);
-        const size_t smem = sizeof(double) * (size_t)qe_warp_doubles(h->n, h->q, h->qf) * warps;
+        const size_t smem = sizeof(double) * (size_t)qe_warp_doubles(h->n, h->q) * warps;
         const unsigned blocks = (unsigned)std::max(1, std::min((c.nel + warps - 1) / warps, 148 * 16));
         qeuler_kernel<<<blocks, 32 * warps, smem, h->w->stream>>>(A, warps);
         WDG_CUDA(cudaGetLastError());
@@ -495,8 +438,12 @@ namespace
         if (!(set & (1ull << dev)))
         {
             WDG_CUDA(cudaFuncSetAttribute(qeuler_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+            std::vector<XTabs<EulerX>> t(1);
+            xtabs_fill(t[0], false);
+            WDG_CUDA(cudaMemcpyToSymbol(c_euler_x, t.data(), sizeof(XTabs<EulerX>)));
             set |= 1ull << dev;
         }
+        WDG_CUDA(xline_prepare<EulerX>(n));
         return WDG_OK;
     }
 } // namespace

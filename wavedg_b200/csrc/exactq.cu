@@ -13,12 +13,12 @@
 // the argument staging are the collocation handle's (an internal wdg_wave, FP64).
 //
 // FP64 only.  The accuracy path for callers that set approx_quad = false.  The RHS and every
-// RK4 stage (WaveHoltz periods included) are one fused launch, a warp per element
-// (qfused_kernel: volume term, the four faces through the partner table, forcing, the dense
-// inverse mass matrix formed at set-up from the block Cholesky factors, the stage update);
-// the operator entry points (Div, EdgeFlux, the mass matrix and its inverse) keep component
-// kernels in the reference layouts: one CTA per element for the volume term, one thread per
-// edge for the face term, one warp per element for the dense mass products.
+// RK4 stage (WaveHoltz periods included) are one fused launch (xline_kernel of
+// exact_line.cuh: volume term, the four sides through the partner table, forcing, the inverse mass
+// matrix as two one-dimensional contractions around a diagonal, the stage update); the operator
+// entry points (Div, EdgeFlux, the mass matrix and its inverse) keep component kernels in the
+// reference layouts: one CTA per element for the volume term, one thread per edge for the face
+// term, one warp per element for the mass matrix.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -26,6 +26,7 @@
 #include <mutex>
 #include <vector>
 
+#include "exact_line.cuh"
 #include "wave_bc.cuh"
 #include "wave_impl.hpp"
 
@@ -38,7 +39,7 @@ struct wdg_waveq
     double *d_xd = nullptr, *d_wd = nullptr, *d_Pd = nullptr, *d_Dd = nullptr; // Div rule, P(i,k), D(i,k)
     double *d_wf = nullptr, *d_Pf = nullptr;                                   // face rule, P(i,k)
     double *d_nI = nullptr, *d_nB = nullptr; // per edge (n_x, n_y, |E| / 2)
-    double *d_M = nullptr, *d_Minv = nullptr; // element mass matrices and their inverses (n^2, n^2, nel)
+    MassTables mass;
     double *d_uf = nullptr, *d_uB = nullptr; // face traces
 };
 
@@ -91,87 +92,67 @@ namespace wdg
             }
     }
 
-    const double *waveq_minv(const wdg_waveq *h) { return h->d_Minv; }
-
-    // MassMatrix<false> (source/MassMatrix.cpp:84-227) on the basis with nodes x: the element
-    // mass matrices M(i, j) = sum_p w_p det J_p phi_i phi_j on the qm x qm Gauss-Legendre rule
-    // (lower triangle, Cholesky in place; chol, linalg.cpp:5-30) and their inverses, solved
-    // column by column (solve_chol, linalg.cpp:32-66); (n^2, n^2, nel) each
-    int exact_mass(const wdg_mesh &mesh, int n, const double *x, int qm, std::vector<double> &Mf,
-                   std::vector<double> &Mi)
+    // a warp per element, wpb warps of 2 nv n^2 doubles
+    __global__ void x_mass_kernel(int n, int nel, int nv, int inverse, const double *__restrict__ A,
+                                  const double *__restrict__ xg, const double *__restrict__ wg,
+                                  const double *__restrict__ corners, const double *x, double *y)
     {
-        const int c = n * n, q2 = qm * qm;
-        std::vector<double> xm(qm), wm(qm), Bm((size_t)qm * n), L((size_t)c * c, 0.0), detJ(q2);
-        Mf.assign((size_t)c * c * mesh.nel, 0.0);
-        Mi.assign((size_t)c * c * mesh.nel, 0.0);
-        gauss_legendre(qm, xm.data(), wm.data());
-        interp_matrix(n, x, qm, xm.data(), Bm.data());
-        int st = WDG_OK;
-        for (int el = 0; el < mesh.nel && st == WDG_OK; ++el)
+        extern __shared__ double sx[];
+        const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5, m = nv * n * n;
+        double *xs = sx + (size_t)wib * 2 * m;
+        for (int el = blockIdx.x * wpb + wib; el < nel; el += gridDim.x * wpb)
         {
-            const double *cr = &mesh.corners[8 * (size_t)el];
-            for (int p = 0; p < q2; ++p)
-            {
-                double J[4];
-                quad_jacobian(cr, xm[p % qm], xm[p / qm], J);
-                detJ[p] = J[0] * J[3] - J[2] * J[1];
-            }
-            double *M = L.data();
-            std::fill(L.begin(), L.end(), 0.0);
-            for (int j = 0; j < c; ++j)
-                for (int i = j; i < c; ++i)
-                {
-                    double mij = 0.0;
-                    for (int p = 0; p < q2; ++p)
-                    {
-                        const double bi = Bm[p % qm + qm * (i % n)] * Bm[p / qm + qm * (i / n)];
-                        const double bj = Bm[p % qm + qm * (j % n)] * Bm[p / qm + qm * (j / n)];
-                        mij += bi * bj * detJ[p] * wm[p % qm] * wm[p / qm];
-                    }
-                    M[i + c * j] = mij;
-                    Mf[(size_t)c * c * el + i + c * j] = mij;
-                    Mf[(size_t)c * c * el + j + c * i] = mij;
-                }
-            for (int k = 0; k < c && st == WDG_OK; ++k)
-            {
-                for (int j = k + 1; j < c; ++j)
-                {
-                    const double sc = M[j + c * k] / M[k + c * k];
-                    for (int i = j; i < c; ++i)
-                        M[i + c * j] -= sc * M[i + c * k];
-                }
-                if (!(M[k + c * k] > 0.0))
-                    st = fail(WDG_ERR_ARG, "an element mass matrix is not positive definite");
-                else
-                {
-                    const double sc = 1.0 / std::sqrt(M[k + c * k]);
-                    for (int i = k; i < c; ++i)
-                        M[i + c * k] *= sc;
-                }
-            }
-            // M^{-1} column by column: solve_chol on the unit vectors (linalg.cpp:32-66)
-            for (int col = 0; col < c && st == WDG_OK; ++col)
-            {
-                double *X = &Mi[(size_t)c * c * el + (size_t)c * col];
-                for (int i = 0; i < c; ++i)
-                    X[i] = (i == col) ? 1.0 : 0.0;
-                for (int j = 0; j < c; ++j)
-                {
-                    X[j] /= M[j + c * j];
-                    for (int i = j + 1; i < c; ++i)
-                        X[i] -= M[i + c * j] * X[j];
-                }
-                for (int j = c - 1; j >= 0; --j)
-                {
-                    X[j] /= M[j + c * j];
-                    for (int i = 0; i < j; ++i)
-                        X[i] -= M[j + c * i] * X[j];
-                }
-            }
+            for (int o = lane; o < m; o += 32)
+                xs[o] = x[(size_t)m * el + o];
+            __syncwarp();
+            x_mass(n, nv, inverse != 0, A, xg, wg, corners + 8 * (size_t)el, xs, xs + m, lane);
+            for (int o = lane; o < m; o += 32)
+                y[(size_t)m * el + o] = xs[o];
+            __syncwarp();
         }
-        return st;
     }
 
+    int mass_tables(int n, const double *x, MassTables &t)
+    {
+        std::vector<double> g(n), w(n), C((size_t)n * n), R((size_t)n * n);
+        gauss_legendre(n, g.data(), w.data());
+        auto put = [&](double **d, const std::vector<double> &v) -> int
+        {
+            WDG_TRY(device_alloc(d, v.size()));
+            return device_put(*d, v);
+        };
+        auto rows = [&]() // column-major -> row-major
+        {
+            for (int r = 0; r < n; ++r)
+                for (int c = 0; c < n; ++c)
+                    R[r * n + c] = C[r + (size_t)n * c];
+        };
+        interp_matrix(n, g.data(), n, x, C.data());
+        rows();
+        WDG_TRY(put(&t.T, R));
+        interp_matrix(n, x, n, g.data(), C.data());
+        rows();
+        WDG_TRY(put(&t.B, R));
+        WDG_TRY(put(&t.xg, g));
+        return put(&t.wg, w);
+    }
+    void mass_tables_free(MassTables &t)
+    {
+        for (double *p : {t.T, t.B, t.xg, t.wg})
+            if (p)
+                cudaFree(p);
+        t = MassTables{};
+    }
+    int mass_launch(const MassTables &t, int n, int nel, int nv, bool inverse, const double *corners, const double *x,
+                    double *y, cudaStream_t s)
+    {
+        const size_t per = sizeof(double) * 2 * nv * n * n; // at most 20.3 KB (nv <= 16, n <= 9)
+        const int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (48 * 1024) / per));
+        x_mass_kernel<<<(unsigned)std::max(1, std::min((nel + wpb - 1) / wpb, 148 * 32)), 32 * wpb, per * wpb, s>>>(
+            n, nel, nv, inverse ? 1 : 0, inverse ? t.T : t.B, t.xg, t.wg, corners, x, y);
+        WDG_CUDA(cudaGetLastError());
+        return WDG_OK;
+    }
 } // namespace wdg
 
 namespace
@@ -326,324 +307,67 @@ namespace
             }
     }
 
-    // ---------------------------------------------------------------- MassMatrix<false>
-    // x <- A x per element for a dense n^2 x n^2 matrix A (the element mass matrix, or its
-    // inverse formed at set-up from the Cholesky factors), nv interleaved right-hand sides,
-    // in place: one warp per element, the element's x staged in shared memory; lanes take
-    // consecutive rows, so each column of A is read coalesced.
-    __global__ void qdense_kernel(int c, int nel, int nv, const double *__restrict__ A, double *x)
-    {
-        extern __shared__ double sx[];
-        const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-        double *xs = sx + (size_t)wib * nv * c;
-        const int m = nv * c;
-        for (int el = blockIdx.x * wpb + wib; el < nel; el += gridDim.x * wpb)
-        {
-            double *xe = x + (size_t)m * el;
-            const double *Ae = A + (size_t)c * c * el;
-            for (int o = lane; o < m; o += 32)
-                xs[o] = xe[o];
-            __syncwarp();
-            for (int o = lane; o < m; o += 32)
-            {
-                const int i = o / nv, d = o - i * nv;
-                double y = 0.0;
-                for (int j = 0; j < c; ++j)
-                    y += Ae[i + (size_t)c * j] * xs[d + nv * j];
-                xe[o] = y;
-            }
-            __syncwarp();
-        }
-    }
-
     // ---------------------------------------------------------------- fused RHS / RK4 stage
-    // One warp per element does what rhs_dev's chain of launches does, in one pass over the
-    // element: the Gauss-point volume term of Div<false> (as qdiv_kernel), the four faces of
-    // EdgeFlux<false> / WaveBC (the element's own nodal trace and its neighbour's, read through
-    // the fused kernels' partner table, or the exterior state of the boundary code at the
-    // nodes, both interpolated to the face rule; the closed-form upwind flux of qflux_kernel
-    // with the element's own outward normal, which makes the two elements of an edge add
-    // exactly opposite terms; projected back to the face nodes), the forcing s F, the dense
-    // inverse mass matrix, then the RHS or the RK4 stage update (with the WaveHoltz filter on
-    // the last stage).
-    struct QFusedArgs
+    // The model of exact_line.cuh: what rhs_dev's operators add up to, with the boundary codes'
+    // exterior states at the nodes, the closed-form upwind flux with the element's own outward
+    // normal (so the two elements of an edge add exactly opposite terms), the forcing s F, and the
+    // WaveHoltz filter on the last stage.
+    struct WaveX
     {
-        const double *x;      // state the RHS is evaluated at
-        double *out;          // RHS: dudt; RK4: u'
-        double *du;           // RK4 register
-        const double *F;      // forcing (nullable) times fs
-        double fs;
-        double *acc;          // FP64 filter (stage 4, nullable) += acc_c u'
-        double acc_c;
-        const double *corners, *xd, *wd, *Pd, *Dd, *wf, *Pf, *Minv;
-        const int4 *fbase;
-        const uint32_t *fcode;
-        unsigned *err;
-        int n, q, qf, nel, rk; // rk: 0 RHS, 1 RK4 stage (rk_a == 0 on the first)
-        double rk_a, rk_b, dt;
-    };
-    constexpr int kQWarps = 4;
-
-    __host__ __device__ inline int qfused_warp_doubles(int n, int q, int qf)
-    {
-        // su r (3 n^2 each) | Pu (3 n q) | Uq (3 q^2) | Fq (7 q^2: six fluxes per point at an odd
-        // stride, which spreads a warp's accesses over the shared-memory banks) | Df Pg (3 q n
-        // each) | T1 (4 n 3) | UF (4 qf 3)
-        return 6 * n * n + 3 * n * q + 10 * q * q + 6 * q * n + 12 * n + 12 * qf;
-    }
-
-    // outward unit normal and measure (length / 2) of side s (StraightEdge, wavedg/Edge.hpp:107-122);
-    // side s runs from corner p0 to p1: 0: 0 -> 1, 1: 1 -> 2, 2: 3 -> 2, 3: 0 -> 3
-    __device__ inline void qside(const double *c, int s, double &nx, double &ny, double &meas)
-    {
-        const int p0 = (s == 0 || s == 3) ? 0 : (s == 1 ? 1 : 3), p1 = (s == 0) ? 1 : (s == 3 ? 3 : 2);
-        const double dx = c[2 * p1] - c[2 * p0], dy = c[2 * p1 + 1] - c[2 * p0 + 1];
-        const double len = sqrt(dx * dx + dy * dy), sgn = (s >= 2) ? -1.0 : 1.0;
-        nx = sgn * dy / len;
-        ny = -sgn * dx / len;
-        meas = 0.5 * len;
-    }
-    // partner walk of a side code (bits 0-1): +3, -3, +3n, -3n values per face node
-    __device__ inline int qstride(int n, uint32_t byte)
-    {
-        const uint32_t c = byte & 3u;
-        return (c == 0) ? 3 : (c == 1) ? -3 : (c == 2) ? 3 * n : -3 * n;
-    }
-
-    __device__ inline int qface_node(int n, int s, int k)
-    {
-        const int i = (s == 0 || s == 2) ? k : (s == 1 ? n - 1 : 0);
-        const int j = (s == 1 || s == 3) ? k : (s == 2 ? n - 1 : 0);
-        return i + n * j;
-    }
-
-    __global__ void __launch_bounds__(32 * kQWarps) qfused_kernel(const QFusedArgs a)
-    {
-        extern __shared__ double qsm[];
-        const int n = a.n, q = a.q, qf = a.qf, nn = n * n, qq = q * q;
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        double *su = qsm + (size_t)warp * qfused_warp_doubles(n, q, qf);
-        double *r = su + 3 * nn, *Pu = r + 3 * nn, *Uq = Pu + 3 * n * q, *Fq = Uq + 3 * qq, *Df = Fq + 7 * qq;
-        double *Pg = Df + 3 * q * n, *T1 = Pg + 3 * q * n, *UF = T1 + 12 * n;
-        const long long limit = 3LL * nn * a.nel;
-        for (int el = blockIdx.x * kQWarps + warp; el < a.nel; el += gridDim.x * kQWarps)
+        static constexpr int NV = 3;
+        static constexpr bool LEG = false, FORCE = true;
+        __host__ __device__ static constexpr int q(int n) { return n; }
+        __host__ __device__ static constexpr int qf(int n) { return n + 1; }
+        template <int N>
+        __device__ static const XTab<N, N, N + 1> &table();
+        __device__ static void exterior(int code, const double *sn, const double *own, double *x)
         {
-            const double *ue = a.x + (size_t)3 * nn * el;
-            for (int k = lane; k < 3 * nn; k += 32)
-            {
-                su[k] = ue[k];
-                r[k] = 0.0;
-            }
-            double c[8];
-            for (int k = 0; k < 8; ++k)
-                c[k] = __ldg(a.corners + 8 * (size_t)el + k);
-            const uint32_t codes = __ldg(a.fcode + el);
-            const int4 fb = __ldg(a.fbase + el);
-            __syncwarp();
-            // ---- volume (Div<false>): Pu, U at the points, fluxes, half contractions, back
-            for (int o = lane; o < 3 * n * q; o += 32)
-            {
-                const int l = o % n, d = (o / n) % 3, i = o / (3 * n);
-                double s = 0.0;
-                for (int k = 0; k < n; ++k)
-                    s += a.Pd[i + q * k] * su[d + 3 * (k + n * l)];
-                Pu[o] = s;
-            }
-            __syncwarp();
-            for (int o = lane; o < 3 * qq; o += 32)
-            {
-                const int d = o % 3, i = (o / 3) % q, j = o / (3 * q);
-                double s = 0.0;
-                for (int l = 0; l < n; ++l)
-                    s += a.Pd[j + q * l] * Pu[l + n * (d + 3 * i)];
-                Uq[o] = s;
-            }
-            __syncwarp();
-            for (int o = lane; o < qq; o += 32)
-            {
-                const int i = o % q, j = o / q;
-                double J[4];
-                jac(c, a.xd[i], a.xd[j], J);
-                const double W = a.wd[i] * a.wd[j];
-                const double Xxi = J[0] * W, Yxi = J[1] * W, Xeta = J[2] * W, Yeta = J[3] * W;
-                const double *U = Uq + 3 * o;
-                double *Fo = Fq + 7 * o;
-                Fo[0] = Yeta * U[1] - Xeta * U[2];
-                Fo[1] = -Yxi * U[1] + Xxi * U[2];
-                Fo[2] = Yeta * U[0];
-                Fo[3] = -Yxi * U[0];
-                Fo[4] = -Xeta * U[0];
-                Fo[5] = Xxi * U[0];
-            }
-            __syncwarp();
-            for (int o = lane; o < 3 * q * n; o += 32)
-            {
-                const int j = o % q, d = (o / q) % 3, k = o / (3 * q);
-                double df = 0.0, pg = 0.0;
-                for (int i = 0; i < q; ++i)
-                {
-                    df += a.Dd[i + q * k] * Fq[2 * d + 7 * (i + q * j)];
-                    pg += a.Pd[i + q * k] * Fq[2 * d + 1 + 7 * (i + q * j)];
-                }
-                Df[o] = df;
-                Pg[o] = pg;
-            }
-            // ---- neighbour / exterior nodal traces of the four sides, face-node order: T1(s, k, d)
-            for (int o = lane; o < 4 * n; o += 32)
-            {
-                const int s = o / n, k = o - s * n;
-                const uint32_t byte = (codes >> (8 * s)) & 0xffu;
-                const double *own = su + 3 * qface_node(n, s, k);
-                double *t1 = T1 + 3 * o;
-                if (byte & 0x80u)
-                {
-                    double nx, ny, meas;
-                    qside(c, s, nx, ny, meas);
-                    const double qv[3] = {own[0], own[1], own[2]};
-                    exterior<double>((int)((byte >> 3) & 3u), nx, ny, qv, t1);
-                }
-                else
-                {
-                    const int off = (s == 0) ? fb.x : (s == 1) ? fb.y : (s == 2) ? fb.z : fb.w;
-                    const long long pos = (long long)off + (long long)k * qstride(n, byte);
-                    if (off < 0 || pos < 0 || pos + 3 > limit)
-                    {
-                        atomicOr(a.err, 2u);
-                        t1[0] = own[0];
-                        t1[1] = own[1];
-                        t1[2] = own[2];
-                    }
-                    else
-                    {
-                        t1[0] = __ldg(a.x + pos);
-                        t1[1] = __ldg(a.x + pos + 1);
-                        t1[2] = __ldg(a.x + pos + 2);
-                    }
-                }
-            }
-            __syncwarp();
-            // volume result into r
-            for (int o = lane; o < 3 * nn; o += 32)
-            {
-                const int d = o % 3, k = (o / 3) % n, l = o / (3 * n);
-                double s = 0.0;
-                for (int j = 0; j < q; ++j)
-                    s += a.Pd[j + q * l] * Df[j + q * (d + 3 * k)] + a.Dd[j + q * l] * Pg[j + q * (d + 3 * k)];
-                r[o] = s;
-            }
-            // ---- face points: both traces to the face rule, upwind flux: UF(s, i, d)
-            for (int o = lane; o < 4 * qf; o += 32)
-            {
-                const int s = o / qf, i = o - s * qf;
-                double nx, ny, meas;
-                qside(c, s, nx, ny, meas);
-                double U0[3] = {0.0, 0.0, 0.0}, U1[3] = {0.0, 0.0, 0.0};
-                for (int j = 0; j < n; ++j)
-                {
-                    const double p = a.Pf[i + qf * j];
-                    const double *own = su + 3 * qface_node(n, s, j), *nb = T1 + 3 * (s * n + j);
-                    for (int d = 0; d < 3; ++d)
-                    {
-                        U0[d] += own[d] * p;
-                        U1[d] += nb[d] * p;
-                    }
-                }
-                const double w = a.wf[i] * meas;
-                const double s0 = -0.5 * w * (U0[0] + nx * U0[1] + ny * U0[2]);
-                const double s1 = 0.5 * w * (U1[0] - nx * U1[1] - ny * U1[2]);
-                UF[3 * o] = s0 + s1;
-                UF[3 * o + 1] = nx * (s0 - s1);
-                UF[3 * o + 2] = ny * (s0 - s1);
-            }
-            __syncwarp();
-            // back to the face nodes: sides 0 and 2, then 1 and 3 (corner nodes are shared only
-            // by neighbouring sides)
-            for (int pass = 0; pass < 2; ++pass)
-            {
-                for (int o = lane; o < 2 * n; o += 32)
-                {
-                    const int s = pass + 2 * (o / n), k = o % n;
-                    const int node = qface_node(n, s, k);
-                    for (int d = 0; d < 3; ++d)
-                    {
-                        double f = 0.0;
-                        for (int j = 0; j < qf; ++j)
-                            f += UF[3 * (s * qf + j) + d] * a.Pf[j + qf * k];
-                        r[3 * node + d] += f;
-                    }
-                }
-                __syncwarp();
-            }
-            // ---- forcing, then M^{-1} and the output: lane per row of the element's matrix
-            if (a.F)
-            {
-                for (int o = lane; o < 3 * nn; o += 32)
-                    r[o] += a.fs * __ldg(a.F + (size_t)3 * nn * el + o);
-                __syncwarp();
-            }
-            const double *Me = a.Minv + (size_t)nn * nn * el;
-            for (int row = lane; row < nn; row += 32)
-            {
-                double y[3] = {0.0, 0.0, 0.0};
-                for (int j = 0; j < nn; ++j)
-                {
-                    const double m = __ldg(Me + row + (size_t)nn * j);
-                    y[0] += m * r[3 * j];
-                    y[1] += m * r[3 * j + 1];
-                    y[2] += m * r[3 * j + 2];
-                }
-                const size_t g = (size_t)3 * (nn * (size_t)el + row);
-                for (int d = 0; d < 3; ++d)
-                {
-                    if (!a.rk)
-                    {
-                        a.out[g + d] = y[d];
-                        continue;
-                    }
-                    const double kd = (a.rk_a == 0.0) ? a.dt * y[d] : a.rk_a * a.du[g + d] + a.dt * y[d];
-                    a.du[g + d] = kd;
-                    const double un = su[3 * row + d] + a.rk_b * kd;
-                    a.out[g + d] = un;
-                    if (a.acc)
-                        a.acc[g + d] += a.acc_c * un;
-                }
-            }
-            __syncwarp();
+            const double o[3] = {own[0], own[1], own[2]};
+            wdg::exterior<double>(code, sn[0], sn[1], o, x);
         }
-    }
-
-
-
+        template <int Q>
+        __device__ static void point(const XArgs &, int, int, int, double Xx, double Yx, double Xe, double Ye,
+                                     const double *U, double *F, double *G)
+        {
+            F[0] = Ye * U[1] - Xe * U[2];
+            G[0] = -Yx * U[1] + Xx * U[2];
+            F[1] = Ye * U[0];
+            G[1] = -Yx * U[0];
+            F[2] = -Xe * U[0];
+            G[2] = Xx * U[0];
+        }
+        template <int N>
+        __device__ static void face(const XArgs &, int, int, int, const double *sn, double wf, const double *U0,
+                                    const double *U1, double *uf)
+        {
+            const double nx = sn[0], ny = sn[1], w = 0.5 * wf * sn[2];
+            const double s0 = -w * (U0[0] + nx * U0[1] + ny * U0[2]), s1 = w * (U1[0] - nx * U1[1] - ny * U1[2]);
+            uf[0] = s0 + s1;
+            uf[1] = nx * (s0 - s1);
+            uf[2] = ny * (s0 - s1);
+        }
+        template <int VP>
+        __device__ static void store(const XArgs &A, size_t el0, int at, const double *u, const double *p, const double *y)
+        {
+            x_store<VP>(A.c, el0, at, u, p, y);
+            if (A.acc)
+#pragma unroll
+                for (int d = 0; d < VP; ++d)
+                    A.acc[el0 + at + d] += A.acc_c * A.c.out[el0 + at + d];
+        }
+    };
+    __constant__ XTabs<WaveX> c_wave_x;
+    template <int N>
+    __device__ const XTab<N, N, N + 1> &WaveX::table() { return xtab<N>(c_wave_x); }
 
     size_t face_count(const wdg_waveq *h, int type)
     {
         return (size_t)h->n * 3 * 2 * (type == 0 ? h->w->nI : h->w->nB);
     }
 
-    // one launch of the fused kernel on the handle's tables (shared memory above 48 KB is opted
-    // in once per device when the handle is created)
-    int qfused_launch(wdg_waveq *h, QFusedArgs &a)
+    int qfused_launch(wdg_waveq *h, const XArgs &a)
     {
-        wdg_wave *w = h->w;
-        a.corners = w->d_corners;
-        a.xd = h->d_xd;
-        a.wd = h->d_wd;
-        a.Pd = h->d_Pd;
-        a.Dd = h->d_Dd;
-        a.wf = h->d_wf;
-        a.Pf = h->d_Pf;
-        a.Minv = h->d_Minv;
-        a.fbase = w->d_fbase;
-        a.fcode = w->d_fcode;
-        a.err = w->d_err;
-        a.n = h->n;
-        a.q = h->nqd;
-        a.qf = h->nqf;
-        a.nel = w->nel;
-        const size_t smem = sizeof(double) * kQWarps * qfused_warp_doubles(h->n, h->nqd, h->nqf);
-        const unsigned blocks = (unsigned)std::max(1, std::min((w->nel + kQWarps - 1) / kQWarps, 148 * 16));
-        qfused_kernel<<<blocks, 32 * kQWarps, smem, w->stream>>>(a);
-        WDG_CUDA(cudaGetLastError());
+        WDG_CUDA(xline_launch<WaveX>(h->n, a, h->w->stream));
         return WDG_OK;
     }
 
@@ -656,10 +380,11 @@ namespace
         wdg_wave *w = h->w;
         WDG_TRY(ensure_states(w));
         double *B = static_cast<double *>(w->d_state[1]), *Cb = static_cast<double *>(w->d_state[2]);
-        QFusedArgs a{};
-        a.du = static_cast<double *>(w->d_du);
-        a.rk = 1;
-        a.dt = dt;
+        XArgs a{};
+        a.c = claw_args(w, u, nullptr);
+        a.c.du = static_cast<double *>(w->d_du);
+        a.c.mode = CLAW_RK4;
+        a.c.dt = dt;
         a.F = F;
         for (int step = 0; step < nsteps; ++step)
         {
@@ -667,10 +392,10 @@ namespace
             for (int st = 0; st < 5; ++st)
             {
                 double *dst = (st == 4) ? u : ((st % 2 == 0) ? B : Cb);
-                a.x = src;
-                a.out = dst;
-                a.rk_a = rk4a[st];
-                a.rk_b = rk4b[st];
+                a.c.x = src;
+                a.c.out = dst;
+                a.c.rk_a = rk4a[st];
+                a.c.rk_b = rk4b[st];
                 a.fs = F ? -std::sin(omega * (t + rk4c[st] * dt)) / omega : 0.0;
                 a.acc = (st == 4) ? acc : nullptr;
                 a.acc_c = (st == 4 && acc) ? c_filter[step] : 0.0;
@@ -704,16 +429,9 @@ namespace
         WDG_CUDA(cudaGetLastError());
         return WDG_OK;
     }
-    int mass_dev(wdg_waveq *h, int nv, double *x, bool inverse)
+    int mass_dev(wdg_waveq *h, int nv, const double *x, double *y, bool inverse)
     {
-        wdg_wave *w = h->w;
-        const int c = h->n * h->n;
-        const int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (48 * 1024) / (sizeof(double) * nv * c)));
-        const size_t smem = sizeof(double) * wpb * nv * c; // at most 48 KB (nv <= 16, c <= 81: 10.4 KB a warp)
-        qdense_kernel<<<(unsigned)std::min((w->nel + wpb - 1) / wpb, 148 * 32), 32 * wpb, smem, w->stream>>>(
-            c, w->nel, nv, inverse ? h->d_Minv : h->d_M, x);
-        WDG_CUDA(cudaGetLastError());
-        return WDG_OK;
+        return mass_launch(h->mass, h->n, h->w->nel, nv, inverse, h->w->d_corners, x, y, h->w->stream);
     }
     // du += Div u + Prol_I^T Flux_I Prol_I u
     int wave_dev(wdg_waveq *h, const double *u, double *du)
@@ -743,9 +461,9 @@ namespace
     // dudt = M^{-1} (A u + B u + s F), one fused launch
     int rhs_dev(wdg_waveq *h, const double *u, double *dudt, const double *F, double s)
     {
-        QFusedArgs a{};
-        a.x = u;
-        a.out = dudt;
+        XArgs a{};
+        a.c = claw_args(h->w, u, dudt);
+        a.c.mode = CLAW_RHS;
         a.F = F;
         a.fs = s;
         return qfused_launch(h, a);
@@ -809,22 +527,27 @@ extern "C"
         h->nqm = qface(n_colloc);
         DeviceScope g(w->device);
         {
-            // the fused kernel's shared memory (70.4 KiB at n = 9), opted in once per device and
-            // before any period is captured into a graph
+            // the fused kernel's matrices (once per device) and its shared memory, before any period
+            // is captured into a graph
             static std::mutex mu;
             static uint64_t set = 0;
             std::lock_guard<std::mutex> lock(mu);
+            cudaError_t e = cudaSuccess;
             if (!(set & (1ull << (w->device & 63))))
             {
-                const cudaError_t e = cudaFuncSetAttribute(qfused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                           100 * 1024);
-                if (e != cudaSuccess)
-                {
-                    wdg_wave_destroy(w);
-                    delete h;
-                    return cuda_fail(e, "cudaFuncSetAttribute(qfused_kernel)");
-                }
-                set |= 1ull << (w->device & 63);
+                std::vector<XTabs<WaveX>> t(1);
+                xtabs_fill(t[0], false);
+                e = cudaMemcpyToSymbol(c_wave_x, t.data(), sizeof(XTabs<WaveX>));
+                if (e == cudaSuccess)
+                    set |= 1ull << (w->device & 63);
+            }
+            if (e == cudaSuccess)
+                e = xline_prepare<WaveX>(n_colloc);
+            if (e != cudaSuccess)
+            {
+                wdg_wave_destroy(w);
+                delete h;
+                return cuda_fail(e, "wdg_waveq_create: fused kernel");
             }
         }
         const int n = n_colloc, c = n * n;
@@ -857,8 +580,7 @@ extern "C"
             return nr;
         };
         const std::vector<double> nI = normals(mesh->interior), nB = normals(mesh->boundary);
-        std::vector<double> Mf, Mi;
-        int st = exact_mass(*mesh, n, x.data(), h->nqm, Mf, Mi);
+        int st = exact_mass_check(*mesh, n);
         auto chk = [&](int r)
         {
             if (st == WDG_OK)
@@ -872,8 +594,6 @@ extern "C"
         chk(device_alloc(&h->d_Pf, Pf.size()));
         chk(device_alloc(&h->d_nI, nI.size()));
         chk(device_alloc(&h->d_nB, nB.size()));
-        chk(device_alloc(&h->d_M, Mf.size()));
-        chk(device_alloc(&h->d_Minv, Mi.size()));
         chk(device_alloc(&h->d_uf, face_count(h, 0)));
         chk(device_alloc(&h->d_uB, face_count(h, 1)));
         if (st == WDG_OK)
@@ -886,8 +606,7 @@ extern "C"
             chk(device_put(h->d_Pf, Pf));
             chk(device_put(h->d_nI, nI));
             chk(device_put(h->d_nB, nB));
-            chk(device_put(h->d_M, Mf));
-            chk(device_put(h->d_Minv, Mi));
+            chk(mass_tables(n, x.data(), h->mass));
         }
         if (st == WDG_OK)
         {
@@ -914,10 +633,10 @@ extern "C"
             return;
         {
             DeviceScope g(h->w ? h->w->device : 0);
-            for (double *p : {h->d_xd, h->d_wd, h->d_Pd, h->d_Dd, h->d_wf, h->d_Pf, h->d_nI, h->d_nB, h->d_M, h->d_Minv, h->d_uf,
-                              h->d_uB})
+            for (double *p : {h->d_xd, h->d_wd, h->d_Pd, h->d_Dd, h->d_wf, h->d_Pf, h->d_nI, h->d_nB, h->d_uf, h->d_uB})
                 if (p)
                     cudaFree(p);
+            mass_tables_free(h->mass);
         }
         if (h->w)
             wdg_wave_destroy(h->w);
@@ -975,7 +694,7 @@ extern "C"
         DeviceScope g(h->w->device);
         HostArg a;
         WDG_TRY(bind_arg(h->w, 0, x, (size_t)n_var * h->n * h->n * h->w->nel, true, true, a));
-        WDG_TRY(mass_dev(h, n_var, a.dev, true));
+        WDG_TRY(mass_dev(h, n_var, a.dev, a.dev, true));
         return finish_args(h->w, &a, 1);
     }
 
@@ -988,9 +707,7 @@ extern "C"
         HostArg a[2];
         WDG_TRY(bind_arg(h->w, 0, x, cnt, true, false, a[0]));
         WDG_TRY(bind_arg(h->w, 1, y, cnt, false, true, a[1]));
-        if (a[1].dev != a[0].dev)
-            WDG_CUDA(cudaMemcpyAsync(a[1].dev, a[0].dev, sizeof(double) * cnt, cudaMemcpyDeviceToDevice, h->w->stream));
-        WDG_TRY(mass_dev(h, n_var, a[1].dev, false));
+        WDG_TRY(mass_dev(h, n_var, a[0].dev, a[1].dev, false));
         return finish_args(h->w, a, 2);
     }
 

@@ -5,8 +5,9 @@
 // M^{-1} (f, phi)).
 //
 //   approx_quad = true    M = diag(w_i w_j det J) at the basis nodes (MassMatrix<true>)
-//   approx_quad = false   the element matrices on the (n + 1)-point Gauss-Legendre rule and their
-//                         inverses (MassMatrix<false>), applied per element by one warp
+//   approx_quad = false   the element matrices of the (n + 1)-point Gauss-Legendre rule and their
+//                         inverses (MassMatrix<false>) in factored form (exact_line.cuh: one-
+//                         dimensional contractions around a diagonal), one warp per element
 //   load                  (f, phi) from f's values at the default n-point Gauss-Legendre points:
 //                         f w_k w_l det J there, projected along y, then along x
 //                         (LinearFunctional<2>::action), on the host, once per call
@@ -16,6 +17,7 @@
 #include <cmath>
 #include <vector>
 
+#include "exact_line.cuh"
 #include "wave_impl.hpp"
 
 using namespace wdg;
@@ -29,7 +31,7 @@ struct wdg_massmatrix
     std::vector<double> corners;                 // (8, nel), for the load vector's geometry
     std::vector<double> xq, wq, B;               // the load vector's n-point rule, B(q, basis node)
     double *d_m = nullptr;                       // approx: w_i w_j det J per node
-    double *d_M = nullptr, *d_Minv = nullptr;    // exact: element matrices and inverses (c, c, nel)
+    MassTables mass;                             // exact: the factors' matrices
 };
 
 namespace
@@ -42,32 +44,6 @@ namespace
             return;
         const double mi = m[t / nv];
         y[t] = inverse ? x[t] / mi : mi * x[t];
-    }
-
-    // y(d, i) = sum_j A(i, j) x(d, j) per element (A column-major, c x c); x and y may alias
-    __global__ void dense_kernel(const double *__restrict__ A, int c, int nv, int nel, const double *x, double *y,
-                                 int warps)
-    {
-        extern __shared__ double xs_all[];
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = nv * c;
-        double *xs = xs_all + (size_t)warp * m;
-        for (int el = blockIdx.x * warps + warp; el < nel; el += gridDim.x * warps)
-        {
-            const double *xe = x + (size_t)m * el;
-            const double *Ae = A + (size_t)c * c * el;
-            for (int o = lane; o < m; o += 32)
-                xs[o] = xe[o];
-            __syncwarp();
-            for (int o = lane; o < m; o += 32)
-            {
-                const int i = o / nv, d = o - i * nv;
-                double s = 0.0;
-                for (int j = 0; j < c; ++j)
-                    s += __ldg(Ae + i + (size_t)c * j) * xs[d + nv * j];
-                y[(size_t)m * el + o] = s;
-            }
-            __syncwarp();
-        }
     }
 
     int check(const wdg_massmatrix *h) { return h ? WDG_OK : fail(WDG_ERR_ARG, "null mass-matrix handle"); }
@@ -84,13 +60,9 @@ namespace
         }
         else
         {
-            const int warps = 4;
-            const size_t smem = sizeof(double) * (size_t)warps * nv * c;
-            if (smem > 48 * 1024)
+            if (sizeof(double) * 4 * (size_t)nv * c > 48 * 1024)
                 return fail(WDG_ERR_UNSUPPORTED, "mass matrix: n_var too large for one element in shared memory");
-            const unsigned blocks = (unsigned)std::max(1, std::min((h->nel + warps - 1) / warps, 148 * 16));
-            dense_kernel<<<blocks, 32 * warps, smem, h->w->stream>>>(inverse ? h->d_Minv : h->d_M, c, nv, h->nel, x, y,
-                                                                      warps);
+            return mass_launch(h->mass, h->n, h->nel, nv, inverse, h->w->d_corners, x, y, h->w->stream);
         }
         WDG_CUDA(cudaGetLastError());
         return WDG_OK;
@@ -146,16 +118,9 @@ extern "C"
             }
             else
             {
-                std::vector<double> Mf, Mi;
-                st = exact_mass(*mesh, n, xb.data(), 1 + (2 * (n - 1) + 2) / 2, Mf, Mi);
+                st = exact_mass_check(*mesh, n);
                 if (st == WDG_OK)
-                    st = device_alloc(&h->d_M, Mf.size());
-                if (st == WDG_OK)
-                    st = device_put(h->d_M, Mf);
-                if (st == WDG_OK)
-                    st = device_alloc(&h->d_Minv, Mi.size());
-                if (st == WDG_OK)
-                    st = device_put(h->d_Minv, Mi);
+                    st = mass_tables(n, xb.data(), h->mass);
             }
         }
         if (st != WDG_OK)
@@ -174,9 +139,9 @@ extern "C"
         if (h->w)
         {
             DeviceScope g(h->w->device);
-            for (double *p : {h->d_m, h->d_M, h->d_Minv})
-                if (p)
-                    cudaFree(p);
+            if (h->d_m)
+                cudaFree(h->d_m);
+            mass_tables_free(h->mass);
             wdg_wave_destroy(h->w);
         }
         delete h;

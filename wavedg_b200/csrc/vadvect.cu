@@ -16,7 +16,9 @@
 //           source/EdgeFlux.cpp:31-88, 140-190, 430-494), + for the edge's first element and -
 //           for its second (fb(side 1) = -fb(side 0)), the neighbour's matrix 0 on the boundary
 //           (exterior state 0).
-// The kernel (one warp per element, the element staged in shared memory) forms u at the volume
+// With approx_quad = false and one variable the RHS and the stages run exact_line.cuh's kernel on
+// these tables.  Everything else -- the operators' actions, collocation, systems -- runs the
+// table-driven kernel below (one warp per element, the element staged in shared memory): it forms u at the volume
 // points, the flux sum_c op(comp, c, d) u_c and its D / P contractions back to the nodes
 // (div_2d_c and div_2d_q, source/Div.cpp:131-180, 469-589); per side the own trace and the
 // neighbour's at the face points (Lobatto: nodal values, through the partner table of the
@@ -34,6 +36,7 @@
 #include <mutex>
 #include <vector>
 
+#include "exact_line.cuh"
 #include "wave_impl.hpp"
 
 using namespace wdg;
@@ -46,7 +49,7 @@ struct wdg_vadvect
     double *d_Pv = nullptr, *d_Dv = nullptr, *d_Pf = nullptr;  // the rules' matrices (Q x n, Qf x n)
     double *d_xg = nullptr, *d_wg = nullptr, *d_e = nullptr;   // basis nodes, weights, phi(-1)
     double *d_op = nullptr, *d_G = nullptr;                    // volume and face tables
-    double *d_Minv = nullptr;                                  // approx_quad = false: MassMatrix<false>^{-1}
+    MassTables mass;                                           // approx_quad = false: MassMatrix<false>'s factors
     int *d_nb = nullptr; // Gauss-Legendre: per side (neighbour element * 4 + its side) * 2 + reversed, -1 boundary
     double *d_buf[3] = {nullptr, nullptr, nullptr};
 };
@@ -62,10 +65,56 @@ namespace
     struct VArgs
     {
         ClawArgs c; // state, output, stage coefficients, geometry, partner table, error word
-        const double *op, *G, *Pv, *Dv, *Pf, *xg, *wg, *e, *Minv;
+        const double *op, *G, *Pv, *Dv, *Pf, *xg, *wg, *e;
+        MassTables mass;
         const int *nb;
         int n, nv, Q, Qf, approx, legendre;
     };
+
+    // one variable, approx_quad = false: exact_line.cuh's model on the handle's tables
+    template <bool LEGENDRE>
+    struct AdvectX
+    {
+        static constexpr int NV = 1;
+        static constexpr bool LEG = LEGENDRE, FORCE = false;
+        // the rules of Div<false> and EdgeFlux<false> for a coefficient of the basis's degree
+        __host__ __device__ static constexpr int q(int n) { return 1 + (3 * n - 3) / 2; }
+        __host__ __device__ static constexpr int qf(int n) { return 1 + (3 * n - 1) / 2; }
+        template <int N>
+        __device__ static const XTab<N, 1 + (3 * N - 3) / 2, 1 + (3 * N - 1) / 2> &table();
+        __device__ static void exterior(int, const double *, const double *, double *x) { x[0] = 0.0; }
+        template <int Q>
+        __device__ static void point(const XArgs &A, int el, int i, int j, double, double, double, double, const double *U,
+                                     double *F, double *G)
+        {
+            const double2 t = __ldg(reinterpret_cast<const double2 *>(A.op) + ((size_t)el * Q * Q + i + Q * j));
+            F[0] = t.x * U[0];
+            G[0] = t.y * U[0];
+        }
+        template <int N>
+        __device__ static void face(const XArgs &A, int el, int s, int q_, const double *, double, const double *U0,
+                                    const double *U1, double *uf)
+        {
+            const double2 t = __ldg(reinterpret_cast<const double2 *>(A.G) + (((size_t)el * 4 + s) * qf(N) + q_));
+            uf[0] = t.x * U0[0] + t.y * U1[0];
+        }
+        template <int VP>
+        __device__ static void store(const XArgs &A, size_t el0, int at, const double *u, const double *p, const double *y)
+        {
+            x_store<VP>(A.c, el0, at, u, p, y);
+        }
+    };
+    __constant__ XTabs<AdvectX<false>> c_advect_gll;
+    __constant__ XTabs<AdvectX<true>> c_advect_gl;
+    template <bool LEGENDRE>
+    template <int N>
+    __device__ const XTab<N, 1 + (3 * N - 3) / 2, 1 + (3 * N - 1) / 2> &AdvectX<LEGENDRE>::table()
+    {
+        if constexpr (LEGENDRE)
+            return xtab<N>(c_advect_gl);
+        else
+            return xtab<N>(c_advect_gll);
+    }
 
     __host__ __device__ inline int va_warp_doubles(int n, int nv, int Q, int Qf)
     {
@@ -356,22 +405,16 @@ namespace
                 __syncwarp();
                 continue;
             }
-            // M^{-1} and the output: lane per node
+            // M^{-1} and the output: lane per node.  The volume term's half contractions are done with
+            // Df, which holds at least nv n^2 values (Q >= n)
+            if (ex)
+                x_mass(n, nv, true, A.mass.T, A.mass.xg, A.mass.wg, a.corners + 8 * (size_t)el, r, Df, lane);
             for (int row = lane; row < nn; row += 32)
             {
                 double y[kJacobiMax];
                 if (ex)
-                {
-                    const double *Me = A.Minv + (size_t)nn * nn * el;
                     for (int d = 0; d < nv; ++d)
-                        y[d] = 0.0;
-                    for (int j = 0; j < nn; ++j)
-                    {
-                        const double m = __ldg(Me + row + (size_t)nn * j);
-                        for (int d = 0; d < nv; ++d)
-                            y[d] += m * r[nv * j + d];
-                    }
-                }
+                        y[d] = r[nv * row + d];
                 else
                 {
                     // MassMatrix<true>: w_i w_j det J at the basis node
@@ -647,6 +690,17 @@ namespace
 
     int va_launch(wdg_vadvect *h, const ClawArgs &c)
     {
+        if (!h->approx && h->nv == 1 && c.mode != VA_ACT && c.mode != VA_BC)
+        {
+            XArgs X{};
+            X.c = c;
+            X.op = h->d_op;
+            X.G = h->d_G;
+            X.nb = h->d_nb;
+            WDG_CUDA(h->legendre ? xline_launch<AdvectX<true>>(h->n, X, h->w->stream)
+                                 : xline_launch<AdvectX<false>>(h->n, X, h->w->stream));
+            return WDG_OK;
+        }
         VArgs A{};
         A.c = c;
         A.op = h->d_op;
@@ -658,7 +712,7 @@ namespace
         A.wg = h->d_wg;
         A.e = h->d_e;
         A.nb = h->d_nb;
-        A.Minv = h->d_Minv;
+        A.mass = h->mass;
         A.n = h->n;
         A.nv = h->nv;
         A.Q = h->Q;
@@ -710,7 +764,7 @@ extern "C"
         const int Q = approx ? n : 1 + ((n - 2) + (n - 1) + 1 + (n - 1)) / 2;
         const int Qf = approx ? n : 1 + (2 * (n - 1) + 2 + (n - 1)) / 2;
         std::vector<double> xg(n), wg(n), xv(Q), wv(Q), xf(Qf), wf(Qf), P((size_t)Q * n), D((size_t)Q * n),
-            Pf((size_t)Qf * n), e(n), op, G, Mf, Mi;
+            Pf((size_t)Qf * n), e(n), op, G;
         if (legendre)
             gauss_legendre(n, xg.data(), wg.data());
         else
@@ -735,7 +789,7 @@ extern "C"
         volume_table(*mesh, n, nv, Q, approx, a, xg, wg, xv, wv, P, op);
         WDG_TRY(face_table(*mesh, n, nv, Qf, approx, legendre, a, e, wg, wf, Pf, G));
         if (!approx)
-            WDG_TRY(exact_mass(*mesh, n, xg.data(), 1 + (2 * (n - 1) + 2) / 2, Mf, Mi));
+            WDG_TRY(exact_mass_check(*mesh, n));
         // Legendre: each side's neighbour and its side, and whether the edge runs against it
         std::vector<int> nb;
         if (legendre)
@@ -777,7 +831,7 @@ extern "C"
         chk(upload(G, &h->d_G));
         chk(upload(e, &h->d_e));
         if (!approx)
-            chk(upload(Mi, &h->d_Minv));
+            chk(mass_tables(n, xg.data(), h->mass));
         if (legendre)
         {
             chk(device_alloc(&h->d_nb, nb.size()));
@@ -792,12 +846,26 @@ extern "C"
             const int dev = h->w->device & 63;
             if (!(set & (1ull << dev)))
             {
-                const cudaError_t e =
+                cudaError_t e =
                     cudaFuncSetAttribute(vadv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+                std::vector<XTabs<AdvectX<false>>> t0(1);
+                std::vector<XTabs<AdvectX<true>>> t1(1);
+                xtabs_fill(t0[0], false);
+                xtabs_fill(t1[0], true);
+                if (e == cudaSuccess)
+                    e = cudaMemcpyToSymbol(c_advect_gll, t0.data(), sizeof(t0[0]));
+                if (e == cudaSuccess)
+                    e = cudaMemcpyToSymbol(c_advect_gl, t1.data(), sizeof(t1[0]));
                 if (e != cudaSuccess)
-                    st = cuda_fail(e, "cudaFuncSetAttribute(vadv_kernel)");
+                    st = cuda_fail(e, "wdg_vadvect_create: kernel set-up");
                 else
                     set |= 1ull << dev;
+            }
+            if (st == WDG_OK && !approx && nv == 1)
+            {
+                const cudaError_t e = legendre ? xline_prepare<AdvectX<true>>(n) : xline_prepare<AdvectX<false>>(n);
+                if (e != cudaSuccess)
+                    st = cuda_fail(e, "wdg_vadvect_create: fused kernel");
             }
         }
         if (st != WDG_OK)
@@ -816,10 +884,11 @@ extern "C"
         if (h->w)
         {
             DeviceScope g(h->w->device);
-            for (double *p : {h->d_Pv, h->d_Dv, h->d_Pf, h->d_xg, h->d_wg, h->d_e, h->d_op, h->d_G, h->d_Minv,
+            for (double *p : {h->d_Pv, h->d_Dv, h->d_Pf, h->d_xg, h->d_wg, h->d_e, h->d_op, h->d_G,
                               h->d_buf[0], h->d_buf[1], h->d_buf[2]})
                 if (p)
                     cudaFree(p);
+            mass_tables_free(h->mass);
             if (h->d_nb)
                 cudaFree(h->d_nb);
         }

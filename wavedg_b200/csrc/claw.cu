@@ -109,7 +109,7 @@ namespace
     struct EulerX
     {
         static constexpr int NV = 4;
-        static constexpr bool LEG = false, FORCE = false;
+        static constexpr bool LEG = false, FORCE = false, LINEAR = false, WEIGHTED = true;
         __host__ __device__ static constexpr int q(int n) { return 2 * n; }
         __host__ __device__ static constexpr int qf(int n) { return 2 * n; }
         template <int N>
@@ -147,10 +147,10 @@ namespace
             G[3] = H * b;
         }
         template <int N>
-        __device__ static void face(const XArgs &, int, int, int, const double *sn, double wf, const double *qL,
-                                    const double *qR, double *uf)
+        __device__ static void face(const XArgs &, int, int, int, const double *sn, const double *qL, const double *qR,
+                                    double *uf)
         {
-            const double nx = sn[0], ny = sn[1], w = -0.5 * wf * sn[2];
+            const double nx = sn[0], ny = sn[1], w = -0.5 * sn[2];
             double iL, uL, vL, pL, iR, uR, vR, pR;
             primitive(qL, iL, uL, vL, pL);
             primitive(qR, iR, uR, vR, pR);
@@ -161,11 +161,6 @@ namespace
             uf[1] = w * (qL[1] * nL + qR[1] * nR + nx * ps + c * (qL[1] - qR[1]));
             uf[2] = w * (qL[2] * nL + qR[2] * nR + ny * ps + c * (qL[2] - qR[2]));
             uf[3] = w * ((qL[3] + pL) * nL + (qR[3] + pR) * nR + c * (qL[3] - qR[3]));
-        }
-        template <int VP>
-        __device__ static void store(const XArgs &A, size_t el0, int at, const double *u, const double *p, const double *y)
-        {
-            x_store<VP>(A.c, el0, at, u, p, y);
         }
     };
     __constant__ XTabs<EulerX> c_euler_x;

@@ -51,9 +51,11 @@ namespace wdg
     struct XTab
     {
         double P[Q][N], Pt[Q][N], Dt[Q][N]; // phi, psi, psi' at the volume points
-        double Pf[QF][N], Pft[QF][N];       // phi, psi at the face points
+        double Pf[QF][N], Pft[QF][N];       // phi, psi at the face points (psi times the weights where
+                                            // the model's flux does not hold them)
+        double R[N][N];                     // Pft^T Pf: a side's trace to its projection
         double T[N][N];                     // psi at the basis nodes
-        double xq[Q], wq[Q], wf[QF];
+        double xq[Q], wq[Q];
         double xg[N], wg[N], sm[N], sp[N];  // Gauss points and weights, psi(-1), psi(+1)
         double e[N];                        // phi(-1) (Gauss-Legendre bases' traces)
     };
@@ -86,16 +88,16 @@ namespace wdg
     }
 
     template <int N, int Q, int QF>
-    inline void xtab_fill(XTab<N, Q, QF> &t, bool legendre)
+    inline void xtab_fill(XTab<N, Q, QF> &t, bool legendre, bool weighted)
     {
-        double x[N], w[N], xf[QF];
+        double x[N], w[N], xf[QF], wf[QF];
         if (legendre)
             gauss_legendre(N, x, w);
         else
             gauss_lobatto(N, x, w);
         gauss_legendre(N, t.xg, t.wg);
         gauss_legendre(Q, t.xq, t.wq);
-        gauss_legendre(QF, xf, t.wf);
+        gauss_legendre(QF, xf, wf);
         std::vector<double> B((size_t)(Q > QF ? Q : QF) * N);
         auto put = [&](int rows, double *dst) // column-major (rows x N) -> row-major
         {
@@ -113,6 +115,16 @@ namespace wdg
         put(QF, &t.Pf[0][0]);
         interp_matrix(N, t.xg, QF, xf, B.data());
         put(QF, &t.Pft[0][0]);
+        for (int q = 0; q < QF && weighted; ++q)
+            for (int m = 0; m < N; ++m)
+                t.Pft[q][m] *= wf[q];
+        for (int m = 0; m < N; ++m)
+            for (int k = 0; k < N; ++k)
+            {
+                t.R[m][k] = 0.0;
+                for (int q = 0; q < QF; ++q)
+                    t.R[m][k] += t.Pft[q][m] * t.Pf[q][k];
+            }
         interp_matrix(N, t.xg, N, x, B.data());
         put(N, &t.T[0][0]);
         const double ends[2] = {-1.0, 1.0};
@@ -123,14 +135,14 @@ namespace wdg
     template <class M>
     inline void xtabs_fill(XTabs<M> &t, bool legendre)
     {
-        xtab_fill(t.t2, legendre);
-        xtab_fill(t.t3, legendre);
-        xtab_fill(t.t4, legendre);
-        xtab_fill(t.t5, legendre);
-        xtab_fill(t.t6, legendre);
-        xtab_fill(t.t7, legendre);
-        xtab_fill(t.t8, legendre);
-        xtab_fill(t.t9, legendre);
+        xtab_fill(t.t2, legendre, M::WEIGHTED);
+        xtab_fill(t.t3, legendre, M::WEIGHTED);
+        xtab_fill(t.t4, legendre, M::WEIGHTED);
+        xtab_fill(t.t5, legendre, M::WEIGHTED);
+        xtab_fill(t.t6, legendre, M::WEIGHTED);
+        xtab_fill(t.t7, legendre, M::WEIGHTED);
+        xtab_fill(t.t8, legendre, M::WEIGHTED);
+        xtab_fill(t.t9, legendre, M::WEIGHTED);
     }
 
     // Every det J at the n x n Gauss points positive: exactly when M is positive definite (M is
@@ -223,26 +235,93 @@ namespace wdg
         const int *nb;        // Gauss-Legendre bases: the sides' neighbours
     };
 
+    // Shared-memory strides.  A warp's 64-bit accesses go out in halves of 16 lanes, conflict-free when
+    // the 16 addresses differ modulo 16.  Lanes are (element, column i) at i * sp and (element, row l,
+    // part) at l * nv + part, elements e (mod 16) apart; of all strides the pair with the fewest
+    // wavefronts is taken (odd variable counts: none above two per access), then su, the stride of the
+    // nodal rows, likewise.
+    struct XStride
+    {
+        int sp, su, e;
+    };
+    constexpr int x_waves(int lanes, int q, int parts, int n, int a, int b, int e)
+    {
+        int waves = 0;
+        for (int h = 0; h < 2; ++h)
+        {
+            int cnt[16] = {}, most = 0;
+            for (int i = 16 * h; i < 16 * h + 16 && i < lanes; ++i)
+            {
+                const int el = i / q, ln = i % q;
+                if (ln >= n * parts)
+                    continue;
+                const int at = (el * e + (ln % n) * a + (ln / n) * b) & 15;
+                if (++cnt[at] > most)
+                    most = cnt[at];
+            }
+            waves += most;
+        }
+        return waves;
+    }
+    constexpr XStride x_strides(int n, int nv, int q, int parts)
+    {
+        XStride best{n * nv, n * nv, 0};
+        int cost = 1 << 30;
+        const int lanes = (32 / q) * q;
+        for (int sp = n * nv; sp < n * nv + 16; ++sp)
+            for (int e = 0; e < 16; ++e)
+            {
+                const int c = 64 * (3 * x_waves(lanes, q, 1, q, sp, 0, e) + 4 * x_waves(lanes, q, parts, n, nv, 1, e)) +
+                              sp - n * nv;
+                if (c < cost)
+                {
+                    cost = c;
+                    best.sp = sp;
+                    best.e = e;
+                }
+            }
+        cost = 1 << 30;
+        for (int su = n * nv; su < n * nv + 16; ++su)
+        {
+            const int c = 64 * x_waves(lanes, q, parts, n, su, 1, best.e) + su;
+            if (c < cost)
+            {
+                cost = c;
+                best.su = su;
+            }
+        }
+        return best;
+    }
+
     template <int N, class M>
     struct XShape
     {
         static constexpr int NV = M::NV, Q = M::q(N), QF = M::qf(N), NN = N * N, ND = NV * NN;
         static constexpr int EW = 32 / Q;          // elements per warp
         static constexpr bool COLLOC = Q == N;     // the volume points are the Gauss points: psi = identity
-        static constexpr int PARTS = (Q >= 2 * N && NV % 2 == 0) ? 2 : 1; // row lanes per row: variable halves
+        // row lanes per row: two, with every other variable each, where the lanes are there
+        static constexpr int PARTS = (Q >= 2 * N && NV % 2 == 0) ? 2 : 1;
         static constexpr int VP = NV / PARTS;
-        static constexpr int SP = (N * NV) | 1;    // doubles per column of points, odd: lanes on different banks
-        static constexpr int HALF = (Q * SP > 4 * QF * NV) ? Q * SP : 4 * QF * NV;
-        static constexpr int TN = 4 * N * NV;      // a trace array
-        // per element: nodal values | two half-contracted arrays (first the interpolated columns and
-        // the side fluxes) | neighbour traces, later the projected side fluxes | own traces
-        // (Gauss-Legendre bases) | forcing | side normals and measures | corners; odd in total
-        static constexpr int oH = ND, oT = oH + 2 * HALF, oT0 = oT + TN, oF = oT0 + (M::LEG ? TN : 0),
-                             oS = oF + (M::FORCE ? N * SP : 0), oC = oS + 12, ES = (oC + 8) | 1;
-        static constexpr size_t smem = sizeof(double) * (size_t)(QF * N + kXWarps * EW * ES);
+        static constexpr XStride ST = x_strides(N, NV, Q, PARTS);
+        static constexpr int SP = ST.sp, SU = ST.su; // doubles per column of points, per nodal row
+        static constexpr int H1 = Q * SP;
+        // both traces at the face points, the flux over the first
+        static constexpr int TQ = 4 * QF * NV;
+        static constexpr int H2 = (H1 > 2 * TQ || M::LINEAR) ? H1 : 2 * TQ;
+        static constexpr int TN = 4 * N * NV; // a trace array
+        // per element: nodal values | two half-contracted arrays (the first also the interpolated
+        // columns, the second the face points) | neighbour traces, later the projected side fluxes | own
+        // traces (Gauss-Legendre bases) | side normals and measures | corners
+        static constexpr int oH = N * SU, oH2 = oH + H1, oT = oH2 + H2, oT0 = oT + TN, oS = oT0 + (M::LEG ? TN : 0),
+                             oC = oS + 12;
+        static constexpr int ES = oC + 8 + ((ST.e - (oC + 8)) & 15);
+        static constexpr size_t smem = sizeof(double) * (size_t)(kXWarps * EW * ES);
         // columns of points kept in registers while the accumulators leave room for them
         static constexpr bool REG = COLLOC || 3 * N * NV <= 64;
+        static_assert(smem <= 227 * 1024, "a CTA's elements fit shared memory");
         static constexpr int MINB = N <= 5 ? 3 : 2;
+        // shared-memory place of value v (of ND) of an element's nodal data
+        __device__ static __forceinline__ int node(int v) { return (v / (N * NV)) * SU + v % (N * NV); }
     };
 
     // outward unit normal and measure (length / 2) of side s (StraightEdge, wavedg/Edge.hpp:107-122)
@@ -255,20 +334,22 @@ namespace wdg
         ny = -sgn * dx / len;
         meas = 0.5 * len;
     }
-    // face-node k of side s: k-th of base + k * stride (source/FaceProlongator.cpp:508-514)
-    template <int N>
-    __device__ __forceinline__ int x_face_base(int s) { return s == 1 ? N - 1 : s == 2 ? N * (N - 1) : 0; }
-    template <int N>
-    __device__ __forceinline__ int x_face_stride(int s) { return (s & 1) ? N : 1; }
-
+    // face-node k of side s in the staged rows: base + k * stride (source/FaceProlongator.cpp:508-514)
+    template <int N, class S>
+    __device__ __forceinline__ int x_face_base(int s)
+    {
+        return s == 1 ? S::NV * (N - 1) : s == 2 ? S::SU * (N - 1) : 0;
+    }
+    template <class S>
+    __device__ __forceinline__ int x_face_stride(int s) { return (s & 1) ? S::SU : S::NV; }
     // LegendreFaceProlongator's node map (source/FaceProlongator.cpp:716-737): the node at distance m
-    // from side s at position i along it
+    // from side s at position i along it, rows `su` apart
     template <int N>
-    __device__ __forceinline__ int x_line(int s, int i, int m)
+    __device__ __forceinline__ int x_line(int s, int i, int m, int su)
     {
         const int x = (s == 0 || s == 2) ? i : (s == 1 ? N - 1 - m : m);
         const int y = (s == 1 || s == 3) ? i : (s == 2 ? N - 1 - m : m);
-        return x + N * y;
+        return x + su * y;
     }
     // asynchronous 8-byte copies to shared memory, in groups
     __device__ __forceinline__ void x_copy8(double *dst, const double *src)
@@ -289,57 +370,48 @@ namespace wdg
         return (a.mode == CLAW_RK4) ? (a.rk_a == 0.0 ? nullptr : a.du) : (a.mode == CLAW_SSP1 || a.mode == CLAW_SSP2) ? a.base
                                                                                                                  : nullptr;
     }
-    // the RHS or one stage of ode::RungeKutta4 / ode::SSPRK3 (wavedg/ode.hpp:66-93, 145-186) at VP
-    // consecutive values; el0: the element's first value, at: the value within it, u: the staged
-    // element, p: x_prev's values
-    template <int VP>
-    __device__ __forceinline__ void x_store(const ClawArgs &a, size_t el0, int at, const double *u, const double *p,
-                                            const double *y)
+    // the RHS or one stage of ode::RungeKutta4 / ode::SSPRK3 (wavedg/ode.hpp:66-93, 145-186) of one
+    // value: g its place, q the staged state, p x_prev's value, y the RHS; the new state where there is one
+    __device__ __forceinline__ double x_stage(const ClawArgs &a, size_t g, double q, double p, double y)
     {
-        const size_t g = el0 + at;
-#pragma unroll
-        for (int d = 0; d < VP; ++d)
+        double v;
+        switch (a.mode)
         {
-            const double q = u[at + d];
-            switch (a.mode)
-            {
-            case CLAW_RHS:
-                a.out[g + d] = y[d];
-                break;
-            case CLAW_RK4:
-            {
-                const double kd = (a.rk_a == 0.0) ? a.dt * y[d] : a.rk_a * p[d] + a.dt * y[d];
-                a.du[g + d] = kd;
-                a.out[g + d] = q + a.rk_b * kd;
-                break;
-            }
-            case CLAW_SSP0:
-                a.out[g + d] = q + a.dt * y[d];
-                break;
-            case CLAW_SSP1:
-                a.out[g + d] = 0.25 * (q + 3.0 * p[d] + a.dt * y[d]);
-                break;
-            default: // CLAW_SSP2
-                a.out[g + d] = (p[d] + 2.0 * q + 2.0 * a.dt * y[d]) / 3.0;
-                break;
-            }
+        case CLAW_RHS:
+            v = y;
+            break;
+        case CLAW_RK4:
+        {
+            const double kd = (a.rk_a == 0.0) ? a.dt * y : a.rk_a * p + a.dt * y;
+            a.du[g] = kd;
+            v = q + a.rk_b * kd;
+            break;
         }
+        case CLAW_SSP0:
+            v = q + a.dt * y;
+            break;
+        case CLAW_SSP1:
+            v = 0.25 * (q + 3.0 * p + a.dt * y);
+            break;
+        default: // CLAW_SSP2
+            v = (p + 2.0 * q + 2.0 * a.dt * y) / 3.0;
+            break;
+        }
+        a.out[g] = v;
+        return v;
     }
 
     template <int N, class M>
     __global__ void __launch_bounds__(32 * kXWarps, XShape<N, M>::MINB) xline_kernel(const XArgs A)
     {
         using S = XShape<N, M>;
-        constexpr int NV = S::NV, Q = S::Q, QF = S::QF, NN = S::NN, ND = S::ND, EW = S::EW, SP = S::SP, VP = S::VP;
-        constexpr int TN = S::TN;
+        constexpr int NV = S::NV, Q = S::Q, QF = S::QF, NN = S::NN, ND = S::ND, EW = S::EW, SP = S::SP, SU = S::SU;
+        constexpr int VP = S::VP, PT = S::PARTS;
         extern __shared__ double xsm[];
         const ClawArgs &a = A.c;
         const auto &tab = M::template table<N>();
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        double *sPf = xsm, *base = xsm + QF * N + (size_t)warp * EW * S::ES;
-        for (int k = threadIdx.x; k < QF * N; k += blockDim.x)
-            sPf[k] = (&tab.Pf[0][0])[k];
-        __syncthreads();
+        double *base = xsm + (size_t)warp * EW * S::ES;
         const long long limit = (long long)a.nel * NN; // nodes a neighbour index may name
         const int le = lane / Q, ln = lane - le * Q;   // element of the warp, line
         double *E = base + le * S::ES;                 // this lane's element
@@ -348,11 +420,14 @@ namespace wdg
         {
             const int e0 = g * EW, ne = min(EW, a.nel - e0);
             const bool on = le < ne;
+            // row lanes: row l, variables part, part + PT, ...
+            const bool row = on && ln < N * PT;
+            const int l = ln % N, part = ln / N;
             // ---- nodal values and corners by asynchronous copies; meanwhile the side codes and partner
             // offsets of this lane's face nodes, all in flight together, then (second copy group) the
-            // traces T1(s, k, d) of the sides' neighbours
+            // traces T(s, k, d) of the sides' neighbours
             for (int o = lane; o < ne * ND; o += 32)
-                x_copy8(base + (o / ND) * S::ES + o % ND, a.x + (size_t)e0 * ND + o);
+                x_copy8(base + (o / ND) * S::ES + S::node(o % ND), a.x + (size_t)e0 * ND + o);
             for (int o = lane; o < ne * 8; o += 32)
                 x_copy8(base + (o >> 3) * S::ES + S::oC + (o & 7), a.corners + 8 * (size_t)e0 + o);
             x_copy_commit();
@@ -390,7 +465,7 @@ namespace wdg
                     else
 #pragma unroll
                         for (int m = 0; m < N; ++m)
-                            w += __ldg(a.x + (size_t)NN * nel + x_line<N>(ns, kk, m)) * tab.e[m];
+                            w += __ldg(a.x + (size_t)NN * nel + x_line<N>(ns, kk, m, N)) * tab.e[m];
                     t1[0] = w;
                 }
                 else
@@ -422,46 +497,15 @@ namespace wdg
                 sn[1] = ny;
                 sn[2] = meas;
             }
-            __syncwarp();
-            // the sides without a neighbour, and the own traces of Gauss-Legendre bases
-#pragma unroll
-            for (int t = 0; t < IT; ++t)
-            {
-                const int o = lane + 32 * t, s = (o / N) & 3, k = o % N;
-                double *Eo = base + (o / (4 * N)) * S::ES, *t1 = Eo + S::oT + NV * (s * N + k);
-                if (byte[t] & 0x100u)
-                    continue;
-                if constexpr (M::LEG)
-                {
-                    double v = 0.0;
-#pragma unroll
-                    for (int m = 0; m < N; ++m)
-                        v += Eo[x_line<N>(s, k, m)] * tab.e[m];
-                    Eo[S::oT0 + s * N + k] = v;
-                    if (byte[t] & 0x80u)
-                        t1[0] = 0.0;
-                }
-                else
-                {
-                    const double *own = Eo + NV * (x_face_base<N>(s) + k * x_face_stride<N>(s));
-                    if (byte[t] & 0x80u)
-                        M::exterior((int)((byte[t] >> 3) & 3u), Eo + S::oS + 3 * s, own, t1);
-                    else if (byte[t] & 0x200u)
-#pragma unroll
-                        for (int d = 0; d < NV; ++d)
-                            t1[d] = own[d];
-                }
-            }
             // ---- 1: rows to the points along xi; H[i][l][d], column-of-points major
-            if (on && ln < N * S::PARTS)
+            if (row)
             {
-                const int l = ln % N, d0 = (ln / N) * VP;
                 double v[N][VP];
 #pragma unroll
                 for (int k = 0; k < N; ++k)
 #pragma unroll
                     for (int d = 0; d < VP; ++d)
-                        v[k][d] = E[NV * (l * N + k) + d0 + d];
+                        v[k][d] = E[SU * l + NV * k + part + PT * d];
 #pragma unroll
                 for (int i = 0; i < Q; ++i)
                 {
@@ -476,90 +520,178 @@ namespace wdg
                             s[d] += tab.P[i][k] * v[k][d];
 #pragma unroll
                     for (int d = 0; d < VP; ++d)
-                        E[S::oH + i * SP + l * NV + d0 + d] = s[d];
+                        E[S::oH + i * SP + l * NV + part + PT * d] = s[d];
                 }
             }
             if constexpr (M::FORCE)
-                if (A.F && on && ln < N)
+            {
+                static_assert(S::COLLOC && PT == 1, "the forcing's columns wait where phase 2 puts its own");
+                if (A.F && row)
                 {
-                    // the forcing's load vector against psi along eta: lane = node column k
-                    const double *Fe = A.F + (size_t)(e0 + le) * ND + NV * ln;
+                    // the forcing's load vector against psi along xi
+                    const double *Fe = A.F + (size_t)(e0 + le) * ND + NV * N * l;
                     double f[N][NV];
 #pragma unroll
-                    for (int l = 0; l < N; ++l)
+                    for (int k = 0; k < N; ++k)
 #pragma unroll
                         for (int d = 0; d < NV; ++d)
-                            f[l][d] = __ldg(Fe + NV * N * l + d);
+                            f[k][d] = __ldg(Fe + NV * k + d);
 #pragma unroll
-                    for (int m = 0; m < N; ++m)
+                    for (int i = 0; i < N; ++i)
 #pragma unroll
                         for (int d = 0; d < NV; ++d)
                         {
                             double s = 0.0;
 #pragma unroll
-                            for (int l = 0; l < N; ++l)
-                                s += tab.T[l][m] * f[l][d];
-                            E[S::oF + ln * SP + m * NV + d] = A.fs * s;
+                            for (int k = 0; k < N; ++k)
+                                s += tab.T[k][i] * f[k][d];
+                            E[S::oH2 + i * SP + l * NV + d] = A.fs * s;
                         }
                 }
+            }
             x_copy_wait<0>();
             __syncwarp();
-            // ---- sides: both traces at the face points, the numerical flux there (what the element
-            // adds, weights included), in the second half of H
-            for (int o = lane; o < ne * 4 * QF; o += 32)
+            // ---- sides.  Exterior states (and the own traces of Gauss-Legendre bases)
+#pragma unroll
+            for (int t = 0; t < IT; ++t)
             {
-                const int eo = o / (4 * QF), s = (o / QF) & 3, q = o % QF;
-                double *Eo = base + eo * S::ES;
-                const double *own = M::LEG ? Eo + S::oT0 + s * N : Eo + NV * x_face_base<N>(s);
-                const int os = M::LEG ? 1 : NV * x_face_stride<N>(s);
-                const double *nb = Eo + S::oT + NV * s * N;
-                double qL[NV], qR[NV];
-#pragma unroll
-                for (int d = 0; d < NV; ++d)
-                    qL[d] = qR[d] = 0.0;
-#pragma unroll
-                for (int j = 0; j < N; ++j)
+                const int o = lane + 32 * t, s = (o / N) & 3, k = o % N;
+                double *Eo = base + (o / (4 * N)) * S::ES, *t1 = Eo + S::oT + NV * (s * N + k);
+                if (byte[t] & 0x100u)
+                    continue;
+                if constexpr (M::LEG)
                 {
-                    const double p = sPf[q * N + j];
+                    double v = 0.0;
+#pragma unroll
+                    for (int m = 0; m < N; ++m)
+                        v += Eo[x_line<N>(s, k, m, SU)] * tab.e[m];
+                    Eo[S::oT0 + s * N + k] = v;
+                    if (byte[t] & 0x80u)
+                        t1[0] = 0.0;
+                }
+                else
+                {
+                    const double *own = Eo + x_face_base<N, S>(s) + k * x_face_stride<S>(s);
+                    if (byte[t] & 0x80u)
+                        M::exterior((int)((byte[t] >> 3) & 3u), Eo + S::oS + 3 * s, own, t1);
+                    else if (byte[t] & 0x200u)
+#pragma unroll
+                        for (int d = 0; d < NV; ++d)
+                            t1[d] = own[d];
+                    if constexpr (M::LINEAR)
+                        M::combine(Eo + S::oS + 3 * s, own, t1);
+                }
+            }
+            __syncwarp();
+            if constexpr (M::LINEAR)
+            {
+                // the flux is linear with coefficients constant along the side: it is the nodal
+                // combinations' two scalars through R
+#pragma unroll
+                for (int o = lane; o < ((EW * 8 + 31) & ~31); o += 32)
+                {
+                    const bool act = o < ne * 8;
+                    const int s = (o >> 1) & 3, which = o & 1;
+                    double *Eo = base + (act ? o >> 3 : 0) * S::ES, *t1 = Eo + S::oT + NV * s * N;
+                    double v[N], m[N];
+#pragma unroll
+                    for (int k = 0; k < N; ++k)
+                    {
+                        v[k] = t1[NV * k + which];
+                        m[k] = 0.0;
+                    }
+                    __syncwarp(); // both of the side's lanes have read it
+#pragma unroll
+                    for (int k = 0; k < N; ++k)
+#pragma unroll
+                        for (int j = 0; j < N; ++j)
+                            m[j] += tab.R[j][k] * v[k];
+                    if (act)
+#pragma unroll
+                        for (int k = 0; k < N; ++k)
+                            M::spread(Eo + S::oS + 3 * s, which, m[k], t1 + NV * k);
+                }
+            }
+            else
+            {
+                // both traces to the face points, lane per (element, side, variable); in the face array
+                // point p = s QF + q of variable d is at d 4 QF + p
+                for (int o = lane; o < ne * 4 * NV; o += 32)
+                {
+                    const int s = (o / NV) & 3, d = o % NV;
+                    double *Eo = base + (o / (4 * NV)) * S::ES, *qp = Eo + S::oH2 + d * 4 * QF + s * QF;
+                    const double *own = M::LEG ? Eo + S::oT0 + s * N : Eo + x_face_base<N, S>(s) + d;
+                    const int os = M::LEG ? 1 : x_face_stride<S>(s);
+                    const double *nb = Eo + S::oT + NV * s * N + d;
+                    double v[N], w[N];
+#pragma unroll
+                    for (int k = 0; k < N; ++k)
+                    {
+                        v[k] = own[k * os];
+                        w[k] = nb[NV * k];
+                    }
+#pragma unroll
+                    for (int q = 0; q < QF; ++q)
+                    {
+                        double x = 0.0, y = 0.0;
+#pragma unroll
+                        for (int k = 0; k < N; ++k)
+                        {
+                            x += tab.Pf[q][k] * v[k];
+                            y += tab.Pf[q][k] * w[k];
+                        }
+                        qp[q] = x;
+                        qp[S::TQ + q] = y;
+                    }
+                }
+                __syncwarp();
+                // the numerical flux: what the element adds
+                for (int o = lane; o < ne * 4 * QF; o += 32)
+                {
+                    const int eo = o / (4 * QF), pt = o % (4 * QF), s = pt / QF;
+                    double *Eo = base + eo * S::ES, *qp = Eo + S::oH2 + pt;
+                    double qL[NV], qR[NV], uf[NV];
 #pragma unroll
                     for (int d = 0; d < NV; ++d)
                     {
-                        qL[d] += p * own[j * os + d];
-                        qR[d] += p * nb[NV * j + d];
+                        qL[d] = qp[d * 4 * QF];
+                        qR[d] = qp[S::TQ + d * 4 * QF];
                     }
+                    M::template face<N>(A, e0 + eo, s, pt - s * QF, Eo + S::oS + 3 * s, qL, qR, uf);
+#pragma unroll
+                    for (int d = 0; d < NV; ++d)
+                        qp[d * 4 * QF] = uf[d];
                 }
-                M::template face<N>(A, e0 + eo, s, q, Eo + S::oS + 3 * s, tab.wf[q], qL, qR,
-                                    Eo + S::oH + S::HALF + NV * (s * QF + q));
-            }
-            __syncwarp();
-            // the side fluxes against psi along the side: lane per (element, side, variable)
-            for (int o = lane; o < ne * 4 * NV; o += 32)
-            {
-                const int eo = o / (4 * NV), s = (o / NV) & 3, d = o % NV;
-                double *Eo = base + eo * S::ES;
-                const double *uf = Eo + S::oH + S::HALF + NV * s * QF + d;
-                double m[N];
-#pragma unroll
-                for (int k = 0; k < N; ++k)
-                    m[k] = 0.0;
-#pragma unroll
-                for (int q = 0; q < QF; ++q)
+                __syncwarp();
+                // against psi along the side
+                for (int o = lane; o < ne * 4 * NV; o += 32)
                 {
-                    const double f = uf[NV * q];
+                    const int s = (o / NV) & 3, d = o % NV;
+                    double *Eo = base + (o / (4 * NV)) * S::ES;
+                    const double *uf = Eo + S::oH2 + d * 4 * QF + s * QF;
+                    double m[N];
 #pragma unroll
                     for (int k = 0; k < N; ++k)
-                        m[k] += tab.Pft[q][k] * f;
-                }
+                        m[k] = 0.0;
 #pragma unroll
-                for (int k = 0; k < N; ++k)
-                    Eo[S::oT + NV * (s * N + k) + d] = m[k];
+                    for (int q = 0; q < QF; ++q)
+                    {
+                        const double f = uf[q];
+#pragma unroll
+                        for (int k = 0; k < N; ++k)
+                            m[k] += tab.Pft[q][k] * f;
+                    }
+#pragma unroll
+                    for (int k = 0; k < N; ++k)
+                        Eo[S::oT + NV * (s * N + k) + d] = m[k];
+                }
             }
             __syncwarp();
             // ---- 2: column i of points
             if (on)
             {
                 const int i = ln;
-                double *H = E + S::oH + i * SP, *H2 = H + S::HALF;
+                double *H = E + S::oH + i * SP, *H2 = E + S::oH2 + i * SP;
                 const double *c = E + S::oC;
                 const double xi = tab.xq[i], wi = tab.wq[i];
                 const double Xe = 0.25 * ((1.0 - xi) * (c[6] - c[0]) + (1.0 + xi) * (c[4] - c[2]));
@@ -569,19 +701,33 @@ namespace wdg
                 if constexpr (S::REG)
                 {
 #pragma unroll
-                    for (int l = 0; l < N; ++l)
+                    for (int j = 0; j < N; ++j)
 #pragma unroll
                         for (int d = 0; d < NV; ++d)
-                            v[l][d] = H[l * NV + d];
+                            v[j][d] = H[j * NV + d];
                 }
 #pragma unroll
-                for (int l = 0; l < N; ++l)
+                for (int j = 0; j < N; ++j)
 #pragma unroll
                     for (int d = 0; d < NV; ++d)
                     {
-                        ga[l][d] = 0.0;
+                        ga[j][d] = 0.0;
                         if constexpr (!S::COLLOC)
-                            fa[l][d] = 0.0;
+                            fa[j][d] = 0.0;
+                    }
+                if constexpr (M::FORCE)
+                    if (A.F)
+                    {
+                        // + the forcing's column against psi along eta
+                        for (int k = 0; k < N; ++k)
+#pragma unroll
+                            for (int d = 0; d < NV; ++d)
+                            {
+                                const double f = H2[k * NV + d];
+#pragma unroll
+                                for (int j = 0; j < N; ++j)
+                                    ga[j][d] += tab.T[k][j] * f;
+                            }
                     }
                 // a collocated column's F goes straight to its row slot, over the interpolated column
                 // it no longer needs once that is in registers (REG holds for every collocated shape)
@@ -593,22 +739,22 @@ namespace wdg
                     for (int d = 0; d < NV; ++d)
                         U[d] = 0.0;
 #pragma unroll
-                    for (int l = 0; l < N; ++l)
+                    for (int m = 0; m < N; ++m)
 #pragma unroll
                         for (int d = 0; d < NV; ++d)
-                            U[d] += tab.P[j][l] * (S::REG ? v[S::REG ? l : 0][d] : H[l * NV + d]);
+                            U[d] += tab.P[j][m] * (S::REG ? v[S::REG ? m : 0][d] : H[m * NV + d]);
                     const double eta = tab.xq[j], W = wi * tab.wq[j];
                     const double Xx = 0.25 * ((1.0 - eta) * dx0 + (1.0 + eta) * dx1);
                     const double Yx = 0.25 * ((1.0 - eta) * dy0 + (1.0 + eta) * dy1);
                     M::template point<Q>(A, e0 + le, i, j, W * Xx, W * Yx, W * Xe, W * Ye, U, F, G);
 #pragma unroll
-                    for (int l = 0; l < N; ++l)
+                    for (int m = 0; m < N; ++m)
 #pragma unroll
                         for (int d = 0; d < NV; ++d)
                         {
-                            ga[l][d] += tab.Dt[j][l] * G[d];
+                            ga[m][d] += tab.Dt[j][m] * G[d];
                             if constexpr (!S::COLLOC)
-                                fa[l][d] += tab.Pt[j][l] * F[d];
+                                fa[m][d] += tab.Pt[j][m] * F[d];
                         }
                     if constexpr (S::COLLOC)
 #pragma unroll
@@ -628,35 +774,40 @@ namespace wdg
                         point(j);
                 }
 #pragma unroll
-                for (int l = 0; l < N; ++l)
+                for (int j = 0; j < N; ++j)
 #pragma unroll
                     for (int d = 0; d < NV; ++d)
                     {
-                        H2[l * NV + d] = ga[l][d];
+                        H2[j * NV + d] = ga[j][d];
                         if constexpr (!S::COLLOC)
-                            H[l * NV + d] = fa[l][d];
+                            H[j * NV + d] = fa[j][d];
                     }
             }
             __syncwarp();
-            // ---- 3: row l of Gauss points
-            const bool row = on && ln < N * S::PARTS;
-            const int l = ln % N, d0 = (ln / N) * VP;
-            double r[N][VP];
+            // ---- 3: row l of Gauss points.  What the stage reads beside its input is asked for first
+            double r[N][VP], p[N][VP];
+            const size_t ge = (size_t)(e0 + le) * ND;
+            const double *prev = x_prev(a);
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+#pragma unroll
+                for (int d = 0; d < VP; ++d)
+                    p[k][d] = (row && prev) ? prev[ge + NV * (M::LEG ? l * N + k : k * N + l) + part + PT * d] : 0.0;
             if (row)
             {
-                const double *H = E + S::oH + l * NV + d0, *H2 = H + S::HALF, *Sf = E + S::oT + d0;
+                const double *H = E + S::oH + l * NV + part, *H2 = E + S::oH2 + l * NV + part, *Sf = E + S::oT + part;
                 const double *c = E + S::oC;
 #pragma unroll
                 for (int k = 0; k < N; ++k)
 #pragma unroll
                     for (int d = 0; d < VP; ++d)
-                        r[k][d] = S::COLLOC ? H2[k * SP + d] : 0.0;
+                        r[k][d] = S::COLLOC ? H2[k * SP + PT * d] : 0.0;
 #pragma unroll
                 for (int i = 0; i < Q; ++i)
 #pragma unroll
                     for (int d = 0; d < VP; ++d)
                     {
-                        const double f = H[i * SP + d], gg = S::COLLOC ? 0.0 : H2[i * SP + d];
+                        const double f = H[i * SP + PT * d], gg = S::COLLOC ? 0.0 : H2[i * SP + PT * d];
 #pragma unroll
                         for (int k = 0; k < N; ++k)
                         {
@@ -665,23 +816,16 @@ namespace wdg
                                 r[k][d] += tab.Pt[i][k] * gg;
                         }
                     }
-                if constexpr (M::FORCE)
-                    if (A.F)
-                    {
-#pragma unroll
-                        for (int m = 0; m < N; ++m)
-#pragma unroll
-                            for (int d = 0; d < VP; ++d)
-                            {
-                                const double f = E[S::oF + m * SP + l * NV + d0 + d];
-#pragma unroll
-                                for (int k = 0; k < N; ++k)
-                                    r[k][d] += tab.T[m][k] * f;
-                            }
-                    }
                 const double el = tab.xg[l], wl = tab.wg[l], sml = tab.sm[l], spl = tab.sp[l];
                 const double Xx = 0.25 * ((1.0 - el) * (c[2] - c[0]) + (1.0 + el) * (c[4] - c[6]));
                 const double Yx = 0.25 * ((1.0 - el) * (c[3] - c[1]) + (1.0 + el) * (c[5] - c[7]));
+                double s1[VP], s3[VP];
+#pragma unroll
+                for (int d = 0; d < VP; ++d)
+                {
+                    s1[d] = Sf[NV * (N + l) + PT * d];
+                    s3[d] = Sf[NV * (3 * N + l) + PT * d];
+                }
 #pragma unroll
                 for (int k = 0; k < N; ++k)
                 {
@@ -691,26 +835,30 @@ namespace wdg
                     const double mi = 1.0 / (wl * tab.wg[k] * (Xx * Ye - Yx * Xe));
 #pragma unroll
                     for (int d = 0; d < VP; ++d)
-                        r[k][d] = mi * (r[k][d] + sml * Sf[NV * k + d] + spl * Sf[NV * (2 * N + k) + d] +
-                                        tab.sm[k] * Sf[NV * (3 * N + l) + d] + tab.sp[k] * Sf[NV * (N + l) + d]);
+                        r[k][d] = mi * (r[k][d] + sml * Sf[NV * k + PT * d] + spl * Sf[NV * (2 * N + k) + PT * d] +
+                                        tab.sm[k] * s3[d] + tab.sp[k] * s1[d]);
                 }
             }
-            // ---- 4: to the basis nodes (Gauss-Legendre bases are there), output.  The register or the
-            // step's first state comes from global memory: all of this lane's values are asked for first
-            const int ge = e0 + le;
-            double p[N][VP];
-            const double *prev = x_prev(a);
-#pragma unroll
-            for (int k = 0; k < N; ++k)
+            // ---- 4: to the basis nodes (Gauss-Legendre bases are there), output
+            auto finish = [&](int i, int j, const double *pv, const double *y)
+            {
+                const size_t gn = ge + NV * (j * N + i) + part;
+                const double *u = E + SU * j + NV * i + part;
 #pragma unroll
                 for (int d = 0; d < VP; ++d)
-                    p[k][d] = (row && prev) ? prev[(size_t)ge * ND + NV * (M::LEG ? l * N + k : k * N + l) + d0 + d] : 0.0;
+                {
+                    const double v = x_stage(a, gn + PT * d, u[PT * d], pv[d], y[d]);
+                    if constexpr (M::FORCE) // the WaveHoltz filter of a step's last stage
+                        if (A.acc)
+                            A.acc[gn + PT * d] += A.acc_c * v;
+                }
+            };
             if constexpr (M::LEG)
             {
                 if (row)
 #pragma unroll
                     for (int k = 0; k < N; ++k)
-                        M::template store<VP>(A, (size_t)ge * ND, NV * (l * N + k) + d0, E, p[k], r[k]);
+                        finish(k, l, p[k], r[k]);
             }
             else
             {
@@ -726,19 +874,19 @@ namespace wdg
 #pragma unroll
                             for (int m = 0; m < N; ++m)
                                 s += tab.T[k][m] * r[m][d];
-                            E[S::oH + k * SP + l * NV + d0 + d] = s;
+                            E[S::oH + k * SP + l * NV + part + PT * d] = s;
                         }
                 }
                 __syncwarp();
                 if (row)
                 {
-                    // lane = node column k = l
+                    // lane = node column l
                     double v[N][VP];
 #pragma unroll
                     for (int m = 0; m < N; ++m)
 #pragma unroll
                         for (int d = 0; d < VP; ++d)
-                            v[m][d] = E[S::oH + l * SP + m * NV + d0 + d];
+                            v[m][d] = E[S::oH + l * SP + m * NV + part + PT * d];
 #pragma unroll
                     for (int j = 0; j < N; ++j)
                     {
@@ -751,7 +899,7 @@ namespace wdg
                             for (int m = 0; m < N; ++m)
                                 y[d] += tab.T[j][m] * v[m][d];
                         }
-                        M::template store<VP>(A, (size_t)ge * ND, NV * (j * N + l) + d0, E, p[j], y);
+                        finish(l, j, p[j], y);
                     }
                 }
             }

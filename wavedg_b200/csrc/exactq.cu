@@ -315,7 +315,7 @@ namespace
     struct WaveX
     {
         static constexpr int NV = 3;
-        static constexpr bool LEG = false, FORCE = true;
+        static constexpr bool LEG = false, FORCE = true, LINEAR = true, WEIGHTED = true;
         __host__ __device__ static constexpr int q(int n) { return n; }
         __host__ __device__ static constexpr int qf(int n) { return n + 1; }
         template <int N>
@@ -336,24 +336,25 @@ namespace
             F[2] = -Xe * U[0];
             G[2] = Xx * U[0];
         }
-        template <int N>
-        __device__ static void face(const XArgs &, int, int, int, const double *sn, double wf, const double *U0,
-                                    const double *U1, double *uf)
+        // The upwind flux of side 0 is -1/2 v (v . U0), v = (1, n_x, n_y), of side 1 +1/2 w (w . U1),
+        // w = (1, -n_x, -n_y) (as qflux_kernel): with s0, s1 those scalars at a face node, t becomes
+        // (s0 + s1, s0 - s1), which spread turns into the side's three projected fluxes
+        __device__ static void combine(const double *sn, const double *o, double *t)
         {
-            const double nx = sn[0], ny = sn[1], w = 0.5 * wf * sn[2];
-            const double s0 = -w * (U0[0] + nx * U0[1] + ny * U0[2]), s1 = w * (U1[0] - nx * U1[1] - ny * U1[2]);
-            uf[0] = s0 + s1;
-            uf[1] = nx * (s0 - s1);
-            uf[2] = ny * (s0 - s1);
+            const double h = 0.5 * sn[2];
+            const double s0 = -h * (o[0] + sn[0] * o[1] + sn[1] * o[2]), s1 = h * (t[0] - sn[0] * t[1] - sn[1] * t[2]);
+            t[0] = s0 + s1;
+            t[1] = s0 - s1;
         }
-        template <int VP>
-        __device__ static void store(const XArgs &A, size_t el0, int at, const double *u, const double *p, const double *y)
+        __device__ static void spread(const double *sn, int which, double v, double *t)
         {
-            x_store<VP>(A.c, el0, at, u, p, y);
-            if (A.acc)
-#pragma unroll
-                for (int d = 0; d < VP; ++d)
-                    A.acc[el0 + at + d] += A.acc_c * A.c.out[el0 + at + d];
+            if (which == 0)
+                t[0] = v;
+            else
+            {
+                t[1] = sn[0] * v;
+                t[2] = sn[1] * v;
+            }
         }
     };
     __constant__ XTabs<WaveX> c_wave_x;

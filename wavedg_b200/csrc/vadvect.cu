@@ -76,7 +76,7 @@ namespace
     struct AdvectX
     {
         static constexpr int NV = 1;
-        static constexpr bool LEG = LEGENDRE, FORCE = false;
+        static constexpr bool LEG = LEGENDRE, FORCE = false, LINEAR = false, WEIGHTED = false;
         // the rules of Div<false> and EdgeFlux<false> for a coefficient of the basis's degree
         __host__ __device__ static constexpr int q(int n) { return 1 + (3 * n - 3) / 2; }
         __host__ __device__ static constexpr int qf(int n) { return 1 + (3 * n - 1) / 2; }
@@ -92,16 +92,11 @@ namespace
             G[0] = t.y * U[0];
         }
         template <int N>
-        __device__ static void face(const XArgs &A, int el, int s, int q_, const double *, double, const double *U0,
-                                    const double *U1, double *uf)
+        __device__ static void face(const XArgs &A, int el, int s, int q_, const double *, const double *U0, const double *U1,
+                                    double *uf)
         {
             const double2 t = __ldg(reinterpret_cast<const double2 *>(A.G) + (((size_t)el * 4 + s) * qf(N) + q_));
             uf[0] = t.x * U0[0] + t.y * U1[0];
-        }
-        template <int VP>
-        __device__ static void store(const XArgs &A, size_t el0, int at, const double *u, const double *p, const double *y)
-        {
-            x_store<VP>(A.c, el0, at, u, p, y);
         }
     };
     __constant__ XTabs<AdvectX<false>> c_advect_gll;

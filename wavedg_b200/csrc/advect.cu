@@ -10,7 +10,7 @@
 // a holds A_0 and A_1 as a(d, c, k) = a[d + nv (c + nv k)].  The upwind flux needs |n . A|;
 // it is formed per edge on the host from a Jacobi eigen-decomposition, so A_0 and A_1 must
 // be symmetric (the reference's general eigen-solver path for non-symmetric A is not built).
-// FP64.  The RHS and RK4 run as one fused launch per evaluation or stage (claw_kernels.cuh:
+// FP64.  The RHS and RK4 run as one fused launch per evaluation or stage (claw_line.cu:
 // volume, both face terms with the upwind flux 1/2 (n.A)(a + b) + 1/2 |n.A| (a - b), mass
 // inverse, RK update); the operator entry points (action, bc_action) keep component kernels in
 // the reference layouts (u(d, i, j, el), face traces (i, d, side, edge)).  Geometry, edge and
@@ -30,7 +30,8 @@ struct wdg_advect
 {
     wdg_wave *w = nullptr;
     int n = 0, nv = 0;
-    double *d_a = nullptr;              // 2 nv^2
+    std::vector<double> a;              // 2 nv^2, for the fused kernel's launches
+    double *d_a = nullptr;
     double *d_x = nullptr, *d_wt = nullptr, *d_D = nullptr; // GLL nodes, weights, D(l, j)
     double *d_FI = nullptr, *d_FB = nullptr; // per edge and side: |E|/2 Fs(c, d), (nv, nv, 2, edges)
     double *d_uf = nullptr, *d_uB = nullptr;
@@ -347,12 +348,12 @@ namespace
     }
     int bc_dev(wdg_advect *h, const double *u, double *du) { return faces_dev(h, 1, u, du); }
     // dudt = M^{-1} (A u + B u): one fused launch (volume, both face terms with the upwind flux,
-    // mass inverse; claw_kernels.cuh)
+    // mass inverse; claw_line.cu)
     int rhs_dev(wdg_advect *h, const double *u, double *dudt)
     {
         wdg_wave *w = h->w;
         ClawArgs c = claw_args(w, u, dudt);
-        c.A = h->d_a;
+        c.A = h->a.data();
         c.absA = h->d_absA;
         c.mode = CLAW_RHS;
         WDG_CUDA(launch_claw(1, h->n, h->nv, c, w->stream));
@@ -397,6 +398,11 @@ extern "C"
                                     "uses a symmetric eigen-decomposition)");
         wdg_wave *w = nullptr;
         WDG_TRY(wdg_wave_create(mesh, n_colloc, nullptr, WDG_FP64, device, &w));
+        if (const int s = claw_prepare(w->device); s != WDG_OK)
+        {
+            wdg_wave_destroy(w);
+            return s;
+        }
         wdg_advect *h = new wdg_advect;
         h->w = w;
         h->n = n_colloc;
@@ -415,6 +421,7 @@ extern "C"
             if (st == WDG_OK)
                 st = r;
         };
+        h->a = av;
         chk(device_alloc(&h->d_a, av.size()));
         chk(device_alloc(&h->d_x, x.size()));
         chk(device_alloc(&h->d_wt, wt.size()));
@@ -474,8 +481,8 @@ extern "C"
         double *bufs[3] = {h->d_rk, h->d_rk + nd, h->d_rk + 2 * nd};
         HostArg a;
         WDG_TRY(bind_arg(w, 0, u, (size_t)nd, true, true, a));
-        // fused stage kernels (claw_kernels.cuh), the buffer rotation of the wave path
-        WDG_TRY(claw_steps(w, 1, h->nv, h->d_a, h->d_absA, bufs, 0, a.dev, dt, t, nsteps));
+        // fused stage kernels (claw_line.cu), the buffer rotation of the wave path
+        WDG_TRY(claw_steps(w, 1, h->nv, h->a.data(), h->d_absA, bufs, 0, a.dev, dt, t, nsteps));
         return finish_args(w, &a, 1);
     }
 }

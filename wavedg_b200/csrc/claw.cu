@@ -1,7 +1,7 @@
 // C-ABI: the nonlinear conservation-law path for the compressible Euler system of
 // examples/cl2d.cpp (DivF2D<true>, EdgeFluxF2D<true>, the Lobatto prolongators and
 // MassMatrix<true> with the example's flux and local Lax-Friedrichs numerical flux), and the
-// fused RHS / time stepping it shares with linear advection (claw_kernels.cuh).
+// fused RHS / time stepping it shares with linear advection (claw_line.cu).
 //
 // State layout: the reference's u(d, i, j, el) with d = density, x-momentum, y-momentum,
 // energy (4 values per node).  FP64.  Geometry, partner tables and argument staging are those
@@ -120,47 +120,21 @@ namespace
             for (int d = 0; d < 4; ++d)
                 x[d] = own[d];
         }
-        // velocities and pressure over density with one reciprocal
-        __device__ static void primitive(const double *q, double &ir, double &u, double &v, double &p)
-        {
-            ir = 1.0 / q[0];
-            u = q[1] * ir;
-            v = q[2] * ir;
-            p = (ClawEuler::gamma - 1.0) * (q[3] - 0.5 * q[0] * (u * u + v * v));
-        }
         template <int Q>
         __device__ static void point(const XArgs &, int, int, int, double Xx, double Yx, double Xe, double Ye,
                                      const double *U, double *F, double *G)
         {
-            // contravariant components: momenta (Ye, -Xe) . m and (-Yx, Xx) . m carry the state,
-            // the pressure acts along the same vectors
             double ir, u, v, p;
-            primitive(U, ir, u, v, p);
-            const double a = Ye * u - Xe * v, b = Xx * v - Yx * u, H = U[3] + p;
-            F[0] = U[0] * a;
-            F[1] = U[1] * a + Ye * p;
-            F[2] = U[2] * a - Xe * p;
-            F[3] = H * a;
-            G[0] = U[0] * b;
-            G[1] = U[1] * b - Yx * p;
-            G[2] = U[2] * b + Xx * p;
-            G[3] = H * b;
+            ClawEuler::primitive(U, ir, u, v, p);
+            ClawEuler::carry(Ye, -Xe, u, v, p, U, F);
+            ClawEuler::carry(-Yx, Xx, u, v, p, U, G);
         }
         template <int N>
         __device__ static void face(const XArgs &, int, int, int, const double *sn, const double *qL, const double *qR,
                                     double *uf)
         {
-            const double nx = sn[0], ny = sn[1], w = -0.5 * sn[2];
-            double iL, uL, vL, pL, iR, uR, vR, pR;
-            primitive(qL, iL, uL, vL, pL);
-            primitive(qR, iR, uR, vR, pR);
-            const double c = fmax(sqrt(uL * uL + vL * vL) + sqrt(ClawEuler::gamma * pL * iL),
-                                  sqrt(uR * uR + vR * vR) + sqrt(ClawEuler::gamma * pR * iR));
-            const double nL = nx * uL + ny * vL, nR = nx * uR + ny * vR, ps = pL + pR;
-            uf[0] = w * (qL[0] * nL + qR[0] * nR + c * (qL[0] - qR[0]));
-            uf[1] = w * (qL[1] * nL + qR[1] * nR + nx * ps + c * (qL[1] - qR[1]));
-            uf[2] = w * (qL[2] * nL + qR[2] * nR + ny * ps + c * (qL[2] - qR[2]));
-            uf[3] = w * ((qL[3] + pL) * nL + (qR[3] + pR) * nR + c * (qL[3] - qR[3]));
+            uf[0] = uf[1] = uf[2] = uf[3] = 0.0;
+            ClawEuler::face<4>(nullptr, nullptr, sn[0], sn[1], -0.5 * sn[2], qL, qR, uf);
         }
     };
     __constant__ XTabs<EulerX> c_euler_x;
@@ -235,13 +209,13 @@ namespace
                 double J[4], f[4], g[4];
                 qe_jac(c, A.xv[i], A.xv[j], J);
                 const double W = A.wv[i] * A.wv[j];
-                const double Ye = J[3] * W, Xe = J[2] * W, Yx = J[1] * W, Xx = J[0] * W;
-                ClawEuler::flux(a, Uq + NV * o, f, g);
+                ClawEuler::flux<4>(nullptr, J[3] * W, -(J[2] * W), Uq + NV * o, f);
+                ClawEuler::flux<4>(nullptr, -(J[1] * W), J[0] * W, Uq + NV * o, g);
                 double *Fo = Fq + 2 * NV * o;
                 for (int d = 0; d < NV; ++d)
                 {
-                    Fo[2 * d] = Ye * f[d] - Xe * g[d];
-                    Fo[2 * d + 1] = -Yx * f[d] + Xx * g[d];
+                    Fo[2 * d] = f[d];
+                    Fo[2 * d + 1] = g[d];
                 }
             }
             __syncwarp();
@@ -299,12 +273,11 @@ namespace
                     qL[d] += ub[j + n * (d + 4 * (0 + 2 * (size_t)e))] * Pf[i + qf * j];
                     qR[d] += ub[j + n * (d + 4 * (1 + 2 * (size_t)e))] * Pf[i + qf * j];
                 }
-            double fh[4];
-            ClawEuler::numflux<4>(ClawArgs{}, e, s, nx, ny, qL, qR, fh);
-            const double ds = wf[i] * meas;
+            double fh[4] = {0.0, 0.0, 0.0, 0.0};
+            ClawEuler::face<4>(nullptr, nullptr, nx, ny, 0.5 * wf[i] * meas, qL, qR, fh);
             for (int d = 0; d < 4; ++d)
                 for (int k = 0; k < n; ++k)
-                    acc[k][d] += fh[d] * Pf[i + qf * k] * ds;
+                    acc[k][d] += fh[d] * Pf[i + qf * k];
         }
         for (int k = 0; k < n; ++k)
             for (int d = 0; d < 4; ++d)
@@ -452,6 +425,11 @@ extern "C"
         *out = nullptr;
         wdg_wave *w = nullptr;
         WDG_TRY(wdg_wave_create(mesh, n_colloc, nullptr, WDG_FP64, device, &w));
+        if (const int s = claw_prepare(w->device); s != WDG_OK)
+        {
+            wdg_wave_destroy(w);
+            return s;
+        }
         wdg_claw *h = new wdg_claw;
         h->w = w;
         h->n = n_colloc;

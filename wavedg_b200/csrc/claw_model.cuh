@@ -1,11 +1,15 @@
 // Flux models and face geometry of the conservation-law path, shared by the fused collocation
-// kernels (claw_kernels.cuh) and the exact-quadrature Euler kernels (claw.cu).
+// kernel (claw_line.cu) and the exact-quadrature Euler kernels (claw.cu).
 //
 //   ClawEuler    the compressible Euler system of examples/cl2d.cpp:67-126 (gamma 1.4) with its
 //                local Lax-Friedrichs flux; exterior boundary state = interior state.
 //   ClawLinear   f = A_0 u, g = A_1 u (Advection<true>), upwind flux
 //                fh = 1/2 (n.A)(a + b) + 1/2 |n.A| (a - b), |n.A| per element side from a table
 //                formed at set-up; exterior boundary state 0 (AdvectionHomogeneousBC<true>).
+//
+// flux: r = a f(q) + b g(q), a contravariant component with the vector (a, b).
+// face: r += 2 w fh(n, qL, qR), exactly antisymmetric (n, qL, qR) -> (-n, qR, qL): the products of
+// the two states are rounded before they are added.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -16,51 +20,67 @@ namespace wdg
 {
     struct ClawEuler
     {
+        static constexpr bool LINEAR = false;
         static constexpr double gamma = 1.4;
-        __device__ static void flux(const ClawArgs &, const double *q, double *f, double *g)
+        // velocities and pressure over density with one reciprocal
+        __device__ __forceinline__ static void primitive(const double *q, double &ir, double &u, double &v, double &p)
         {
-            const double rho = q[0], u = q[1] / q[0], v = q[2] / q[0], E = q[3];
-            const double p = (gamma - 1.0) * (E - 0.5 * rho * (u * u + v * v));
-            f[0] = rho * u;
-            f[1] = rho * u * u + p;
-            f[2] = rho * u * v;
-            f[3] = u * (E + p);
-            g[0] = rho * v;
-            g[1] = rho * u * v;
-            g[2] = rho * v * v + p;
-            g[3] = v * (E + p);
+            ir = 1.0 / q[0];
+            u = q[1] * ir;
+            v = q[2] * ir;
+            p = (gamma - 1.0) * (q[3] - 0.5 * q[0] * (u * u + v * v));
         }
-        __device__ static double speed(const double *q)
+        // the state carried along (a, b) and the pressure acting along it
+        __device__ __forceinline__ static void carry(double a, double b, double u, double v, double p, const double *q,
+                                                     double *f)
         {
-            const double rho = q[0], u = q[1] / q[0], v = q[2] / q[0], E = q[3];
-            const double p = (gamma - 1.0) * (E - 0.5 * rho * (u * u + v * v));
-            return hypot(u, v) + sqrt(gamma * p / rho);
+            const double s = a * u + b * v;
+            f[0] = q[0] * s;
+            f[1] = q[1] * s + a * p;
+            f[2] = q[2] * s + b * p;
+            f[3] = (q[3] + p) * s;
         }
         template <int NV>
-        __device__ static void exterior(const double *q, double *x)
+        __device__ __forceinline__ static void flux(const double *, double a, double b, const double *q, double *f)
+        {
+            double ir, u, v, p;
+            primitive(q, ir, u, v, p);
+            carry(a, b, u, v, p, q, f);
+        }
+        template <int NV>
+        __device__ __forceinline__ static void exterior(const double *q, double *x)
         {
 #pragma unroll
             for (int d = 0; d < NV; ++d)
                 x[d] = q[d];
         }
         template <int NV>
-        __device__ static void numflux(const ClawArgs &a, int, int, double nx, double ny, const double *qL,
-                                       const double *qR, double *fh)
+        __device__ __forceinline__ static void face(const double *, const double *, double nx, double ny, double w,
+                                                    const double *qL, const double *qR, double *r)
         {
-            double fL[4], gL[4], fR[4], gR[4];
-            flux(a, qL, fL, gL);
-            flux(a, qR, fR, gR);
-            const double c = fmax(speed(qL), speed(qR));
-#pragma unroll
-            for (int d = 0; d < 4; ++d)
-                fh[d] = 0.5 * nx * (fL[d] + fR[d]) + 0.5 * ny * (gL[d] + gR[d]) + 0.5 * c * (qL[d] - qR[d]);
+            double iL, uL, vL, pL, iR, uR, vR, pR;
+            primitive(qL, iL, uL, vL, pL);
+            primitive(qR, iR, uR, vR, pR);
+            const double c = fmax(sqrt(uL * uL + vL * vL) + sqrt(gamma * pL * iL),
+                                  sqrt(uR * uR + vR * vR) + sqrt(gamma * pR * iR));
+            const double nL = nx * uL + ny * vL, nR = nx * uR + ny * vR, ps = pL + pR;
+            const double s0 = __dadd_rn(__dmul_rn(qL[0], nL), __dmul_rn(qR[0], nR));
+            const double s1 = __dadd_rn(__dmul_rn(qL[1], nL), __dmul_rn(qR[1], nR)) + nx * ps;
+            const double s2 = __dadd_rn(__dmul_rn(qL[2], nL), __dmul_rn(qR[2], nR)) + ny * ps;
+            const double s3 = __dadd_rn(__dmul_rn(qL[3] + pL, nL), __dmul_rn(qR[3] + pR, nR));
+            r[0] += w * (s0 + c * (qL[0] - qR[0]));
+            r[1] += w * (s1 + c * (qL[1] - qR[1]));
+            r[2] += w * (s2 + c * (qL[2] - qR[2]));
+            r[3] += w * (s3 + c * (qL[3] - qR[3]));
         }
     };
 
     struct ClawLinear
     {
+        static constexpr bool LINEAR = true;
+        // A_0, A_1 as A(d, c, k) = A[d + nv (c + nv k)]
         template <int NV>
-        __device__ static void flux_n(const ClawArgs &a, const double *q, double *f, double *g)
+        __device__ __forceinline__ static void flux(const double *A, double a, double b, const double *q, double *f)
         {
 #pragma unroll
             for (int d = 0; d < NV; ++d)
@@ -69,25 +89,24 @@ namespace wdg
 #pragma unroll
                 for (int c = 0; c < NV; ++c)
                 {
-                    s0 += a.A[d + NV * c] * q[c];
-                    s1 += a.A[d + NV * c + NV * NV] * q[c];
+                    s0 += A[d + NV * c] * q[c];
+                    s1 += A[d + NV * c + NV * NV] * q[c];
                 }
-                f[d] = s0;
-                g[d] = s1;
+                f[d] = a * s0 + b * s1;
             }
         }
         template <int NV>
-        __device__ static void exterior(const double *, double *x)
+        __device__ __forceinline__ static void exterior(const double *, double *x)
         {
 #pragma unroll
             for (int d = 0; d < NV; ++d)
                 x[d] = 0.0;
         }
+        // absA: |n.A| of the side
         template <int NV>
-        __device__ static void numflux(const ClawArgs &a, int el, int side, double nx, double ny, const double *qL,
-                                       const double *qR, double *fh)
+        __device__ __forceinline__ static void face(const double *A, const double *absA, double nx, double ny, double w,
+                                                    const double *qL, const double *qR, double *r)
         {
-            const double *T = a.absA + (size_t)NV * NV * (4 * (size_t)el + side);
 #pragma unroll
             for (int d = 0; d < NV; ++d)
             {
@@ -95,11 +114,11 @@ namespace wdg
 #pragma unroll
                 for (int k = 0; k < NV; ++k)
                 {
-                    const double nA = nx * a.A[d + NV * k] + ny * a.A[d + NV * k + NV * NV];
+                    const double nA = nx * A[d + NV * k] + ny * A[d + NV * k + NV * NV];
                     c += nA * (qL[k] + qR[k]);
-                    u += T[d + NV * k] * (qL[k] - qR[k]);
+                    u += absA[d + NV * k] * (qL[k] - qR[k]);
                 }
-                fh[d] = 0.5 * c + 0.5 * u;
+                r[d] += w * (c + u);
             }
         }
     };

@@ -39,6 +39,7 @@
 
 #include "common.hpp"
 #include "launch.hpp"
+#include "ptx.cuh"
 #include "wave_bc.cuh"
 
 namespace wdg
@@ -126,82 +127,6 @@ namespace wdg
     __constant__ int c_from[4] = {0, 1, 3, 0};
     __constant__ int c_to[4] = {1, 2, 2, 3};
 
-    // --------------------------------------------------------- PTX helpers
-    __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-    __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
-    {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-    }
-    __device__ __forceinline__ void fence_mbar_init()
-    {
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes)
-    {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                     : "memory");
-    }
-    // 1-D bulk copy global -> shared through the TMA unit; dst, src and bytes
-    // are multiples of 16 (checked by the host before use_tma is set)
-    __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
-    {
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                smem_u32(dst)),
-            "l"(src), "r"(bytes), "r"(smem_u32(bar))
-            : "memory");
-    }
-    __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
-    {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-        return ok != 0;
-    }
-    // try_wait with a suspend-time hint: the thread sleeps until the phase
-    // completes or the hint (ns) runs out, instead of spinning on the issue port
-    __device__ __forceinline__ bool mbar_try_wait_sleep(uint64_t *bar, uint32_t parity)
-    {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity), "r"(100000u)
-            : "memory");
-        return ok != 0;
-    }
-    __device__ __forceinline__ uint64_t globaltimer_ns()
-    {
-        uint64_t t;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-        return t;
-    }
-    // bounded wait: gives up after limit_ns of wall time (the copies it waits for take
-    // microseconds; the limit only guards against a lost completion).  Stage launches pass the
-    // handle's limit (StageArgs::wait_ns, 2 s unless set); other kernels use the default.
-    __device__ __forceinline__ uint64_t wait_limit(unsigned long long ns) { return ns ? ns : kWaitLimitNs; }
-    __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64_t limit_ns = kWaitLimitNs)
-    {
-        if (mbar_try_wait(bar, parity))
-            return true;
-        const uint64_t t0 = globaltimer_ns();
-        for (;;)
-        {
-            if (mbar_try_wait_sleep(bar, parity))
-                return true;
-            if (globaltimer_ns() - t0 > limit_ns)
-                return false;
-        }
-    }
-
     // ------------------------------------------------------------- geometry
     // QuadElement::jacobian (source/Element.cpp:21-27) at (xi, eta):
     // J = [x_xi, y_xi, x_eta, y_eta]; corners c = (x0,y0, x1,y1, x2,y2, x3,y3)
@@ -250,33 +175,6 @@ namespace wdg
     }
 
     // ------------------------------------------------------- stage kernel
-    // per-thread asynchronous global -> shared copies (LDGSTS); used for the
-    // neighbour traces, which are scattered 8-byte pieces unsuited to TMA
-    template <int BYTES>
-    __device__ __forceinline__ void cp_async(void *dst, const void *src)
-    {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES)
-                     : "memory");
-    }
-    __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-    template <int PENDING>
-    __device__ __forceinline__ void cp_async_wait()
-    {
-        asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
-    }
-
-    __device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes)
-    {
-        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)),
-                     "r"(bytes)
-                     : "memory");
-    }
-    __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-    __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-    __device__ __forceinline__ void bulk_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
-    __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-    __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
     template <int N>
     __device__ __forceinline__ int partner_stride(uint32_t byte)
     {
@@ -980,25 +878,11 @@ namespace wdg
 
 #include "stage_ws.cuh"
 #include "stage_ws_batch.cuh"
-#include "claw_kernels.cuh"
 
 namespace wdg
 {
     int ws_chunk_unit(int n) { return kWsConsumers * ws_epw(n); }
 
-    cudaError_t launch_claw(int model, int n, int nv, const ClawArgs &a, cudaStream_t s)
-    {
-        return model == 0 ? launch_claw_m<ClawEuler>(n, nv, a, s) : launch_claw_m<ClawLinear>(n, nv, a, s);
-    }
-    cudaError_t launch_euler_face_flux(int n, int ne, const int *edges, const double *corners, const double *ub,
-                                       double *fb, cudaStream_t s)
-    {
-        if (ne == 0)
-            return cudaSuccess;
-        const long long tot = (long long)n * ne;
-        euler_face_flux_kernel<<<(unsigned)((tot + 127) / 128), 128, 0, s>>>(n, ne, edges, corners, ub, fb);
-        return cudaGetLastError();
-    }
     int ws_slot_bytes(int n, bool fp32, int chunk, bool extra, bool filter)
     {
         const bool staged = extra && (fp32 ? WsStage<float, true>::value : WsStage<double, true>::value);

@@ -83,7 +83,7 @@ namespace wdg
     constexpr int kWsDefaultRing = 2;
     int ws_default_chunk(int n, bool fp32);   // most rounds (<= 4) whose default ring fits 3 CTAs per SM
 
-    // one launch of the fused conservation-law kernels (claw_kernels.cuh)
+    // one launch of a fused conservation-law kernel (claw_line.cu, exact_line.cuh)
     struct ClawArgs
     {
         const double *x;      // state the RHS is evaluated at (neighbour traces come from it)
@@ -93,11 +93,12 @@ namespace wdg
         const double *corners;
         const int4 *fbase;    // partner tables of the wave kernels (3 values per node): /3 gives nodes
         const uint32_t *fcode;
-        const double *A;      // ClawLinear: A_0, A_1 as a(d, c, k) = A[d + nv (c + nv k)]
+        const double *A;      // ClawLinear: A_0, A_1 as a(d, c, k) = A[d + nv (c + nv k)] (host memory)
         const double *absA;   // ClawLinear: |n.A| per element side, (nv, nv, 4, nel)
         unsigned *err;
         int nel, mode;
         double rk_a, rk_b, dt;
+        int aligned;          // claw_line.cu: x, out, du and base lie on 16-byte boundaries
     };
     enum
     {
@@ -109,6 +110,7 @@ namespace wdg
         CLAW_SSP2 = 5
     };
 
+    int claw_prepare(int device); // the kernel's matrices, once per device
     // model 0: compressible Euler (n_var 4), 1: linear with constant coefficients (n_var 1..8)
     cudaError_t launch_claw(int model, int n, int nv, const ClawArgs &a, cudaStream_t s);
     cudaError_t launch_euler_face_flux(int n, int ne, const int *edges, const double *corners, const double *ub,

@@ -40,19 +40,10 @@
 #include "common.hpp"
 #include "launch.hpp"
 #include "ptx.cuh"
-#include "wave_bc.cuh"
+#include "wave_line.cuh"
 
 namespace wdg
 {
-    // ------------------------------------------------------------------ tables
-    struct BasisTab
-    {
-        double x[kMaxN], w[kMaxN], D[kMaxN * kMaxN];     // GLL nodes, weights, D[l + n j] = phi_j'(x_l)
-        double gx[kMaxN], gw[kMaxN], B[kMaxN * kMaxN];   // n-point Gauss-Legendre and B[q + n j] = phi_j(gx_q)
-        float xf[kMaxN], wf[kMaxN], Df[kMaxN * kMaxN];
-    };
-    __constant__ BasisTab c_tab[kMaxN + 1];
-
     constexpr int kMaxThreads = 320; // threads per CTA of the stage kernel (launch bound)
 
     bool degree_supported(int n) { return n == 2 || n == 3 || n == 4 || n == 5 || n == 6 || n == 7 || n == 8 || n == 9; }
@@ -77,52 +68,7 @@ namespace wdg
         return 4;
     }
 
-    int upload_basis_tables(int device)
-    {
-        static std::mutex mu;
-        static uint64_t done = 0;
-        std::lock_guard<std::mutex> lock(mu);
-        if (device < 0 || device >= 64)
-            return fail(WDG_ERR_ARG, "device ordinal out of range");
-        if (done & (1ull << device))
-            return WDG_OK;
-        std::vector<BasisTab> tab(kMaxN + 1);
-        for (int n = kMinN; n <= kMaxN; ++n)
-        {
-            BasisTab &T = tab[n];
-            gauss_lobatto(n, T.x, T.w);
-            deriv_matrix(n, T.x, T.D);
-            gauss_legendre(n, T.gx, T.gw);
-            interp_matrix(n, T.x, n, T.gx, T.B);
-            for (int k = 0; k < n; ++k)
-            {
-                T.xf[k] = (float)T.x[k];
-                T.wf[k] = (float)T.w[k];
-            }
-            for (int k = 0; k < n * n; ++k)
-                T.Df[k] = (float)T.D[k];
-        }
-        WDG_CUDA(cudaMemcpyToSymbol(c_tab, tab.data(), sizeof(BasisTab) * (kMaxN + 1)));
-        done |= (1ull << device);
-        return WDG_OK;
-    }
-
-    template <typename Real>
-    struct Tab;
-    template <>
-    struct Tab<double>
-    {
-        static __device__ __forceinline__ double x(int n, int i) { return c_tab[n].x[i]; }
-        static __device__ __forceinline__ double w(int n, int i) { return c_tab[n].w[i]; }
-        static __device__ __forceinline__ double D(int n, int k) { return c_tab[n].D[k]; }
-    };
-    template <>
-    struct Tab<float>
-    {
-        static __device__ __forceinline__ float x(int n, int i) { return c_tab[n].xf[i]; }
-        static __device__ __forceinline__ float w(int n, int i) { return c_tab[n].wf[i]; }
-        static __device__ __forceinline__ float D(int n, int k) { return c_tab[n].Df[k]; }
-    };
+    int upload_basis_tables(int device) { return upload_basis_tab(device); }
 
     __constant__ int c_from[4] = {0, 1, 3, 0};
     __constant__ int c_to[4] = {1, 2, 2, 3};
@@ -152,19 +98,6 @@ namespace wdg
         meas = s / 2;
     }
 
-    // upwind numerical flux through a face with outward normal n, weight
-    // h = w_k * meas / 2:  r -= h [C (q + x) + |C| (q - x)],  |C| = C^2
-    template <typename Real>
-    __device__ __forceinline__ void upwind(Real nx, Real ny, Real h, const Real q[3], const Real x[3], Real r[3])
-    {
-        const Real sp = q[0] + x[0], su = q[1] + x[1], sv = q[2] + x[2];
-        const Real jp = q[0] - x[0], ju = q[1] - x[1], jv = q[2] - x[2];
-        const Real nj = nx * ju + ny * jv;
-        r[0] -= h * (nx * su + ny * sv + jp);
-        r[1] -= h * (nx * sp + nx * nj);
-        r[2] -= h * (ny * sp + ny * nj);
-    }
-
     // face-node k of side f -> node (i, j):  f0 (k,0)  f1 (n-1,k)  f2 (k,n-1)  f3 (0,k)
     // (the reference's mapV2E, source/FaceProlongator.cpp:508-514)
     __device__ __forceinline__ int face_node(int n, int f, int k)
@@ -175,13 +108,6 @@ namespace wdg
     }
 
     // ------------------------------------------------------- stage kernel
-    template <int N>
-    __device__ __forceinline__ int partner_stride(uint32_t byte)
-    {
-        const uint32_t c = byte & 3u;
-        return (c == 0) ? 3 : (c == 1) ? -3 : (c == 2) ? 3 * N : -3 * N;
-    }
-
     // Shared-memory layout of one CTA (E elements per tile, ND = 3 n^2 values per
     // element, NF = 4 n face nodes per element):
     //   [S <= 4 mbarriers][buffer 0 .. S-1][halo 0][halo 1][face flux][G][Rx][Ms][basis x, w]

@@ -71,58 +71,18 @@ namespace wdg
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
     }
 
-    // Upwind flux of face node k of side SIDE of one element (own trace `own`),
-    // subtracted into r: the closed form of EdgeFlux (source/EdgeFlux.cpp:7-139)
-    // with the side's outward normal and measure (StraightEdge, wavedg/Edge.hpp:107-122)
-    // and the exterior state of WaveBC for boundary sides.
+    // Face node k of side SIDE, subtracted into r; own trace `own`, the neighbour's in the slot's halo
     template <int N, typename Real, int SIDE>
     __device__ __forceinline__ void ws_face(uint32_t codes, int flags, const double2 c01, const double2 c23,
                                             const double2 c45, const double2 c67, Real wk, int k,
                                             const Real *own, const Real *halo_e, Real &r0, Real &r1, Real &r2)
     {
         const uint32_t byte = (codes >> (8 * SIDE)) & 0xffu;
-        const bool bnd = (byte & 0x80u) != 0;
-        if (bnd ? !(flags & F_BND) : !(flags & F_INT))
+        if ((byte & 0x80u) ? !(flags & F_BND) : !(flags & F_INT))
             return;
-        // side SIDE runs from corner p0 to p1: 0: 0->1, 1: 1->2, 2: 3->2, 3: 0->3
-        const double2 a0 = (SIDE == 0 || SIDE == 3) ? c01 : (SIDE == 1) ? c23 : c67;
-        const double2 a1 = (SIDE == 0) ? c23 : (SIDE == 3) ? c67 : c45;
-        Real nx, ny, h;
-        if constexpr (sizeof(Real) == 4)
-        {
-            // FP32 stepping: the side's length and normal in FP32 from FP64 corner differences
-            const float dx = (float)(a1.x - a0.x), dy = (float)(a1.y - a0.y);
-            const float s2 = dx * dx + dy * dy, rs = rsqrtf(s2);
-            const float sgn = (SIDE >= 2) ? -1.f : 1.f;
-            nx = sgn * dy * rs;
-            ny = -sgn * dx * rs;
-            h = wk * (0.25f * s2 * rs);
-        }
-        else
-        {
-            const double dx = a1.x - a0.x, dy = a1.y - a0.y;
-            const double s2 = dx * dx + dy * dy, rs = rsqrt(s2);
-            const double sgn = (SIDE >= 2) ? -1.0 : 1.0;
-            nx = (Real)(sgn * dy * rs);
-            ny = (Real)(-sgn * dx * rs);
-            h = wk * (Real)(0.25 * s2 * rs);
-        }
-        const Real q[3] = {own[0], own[1], own[2]};
-        Real x[3];
-        if (bnd)
-            exterior<Real>((int)((byte >> 3) & 3u), nx, ny, q, x);
-        else
-        {
-            const Real *hp = halo_e + 3 * (SIDE * N + k);
-            x[0] = hp[0];
-            x[1] = hp[1];
-            x[2] = hp[2];
-        }
-        Real r[3] = {r0, r1, r2};
-        upwind<Real>(nx, ny, h, q, x, r);
-        r0 = r[0];
-        r1 = r[1];
-        r2 = r[2];
+        Real nx, ny, hm;
+        line_side<Real, SIDE>(c01, c23, c45, c67, nx, ny, hm);
+        line_face<Real>(byte, nx, ny, wk * hm, own, halo_e + 3 * (SIDE * N + k), r0, r1, r2);
     }
 
     // One chunk of one RK stage as both roles see it (the single-solve kernel fills it from
@@ -361,41 +321,15 @@ namespace wdg
                     c67 = c2[3];
                     codes = fks[le];
 
-                    // ---- column pass: column i = ln.  Contravariant eta-fluxes of the wave system
-                    // (source/Div.cpp:5-53): G = W (-y_xi u + x_xi v, -y_xi p, x_xi p); along a
-                    // column x_eta, y_eta are constant and x_xi, y_xi vary linearly with eta.
+                    // ---- column pass: column i = ln
                     const int i = ln;
                     const Real wi = wm;
-                    const Real dx0 = Real(c23.x - c01.x), dx1 = Real(c45.x - c67.x);
-                    const Real dy0 = Real(c23.y - c01.y), dy1 = Real(c45.y - c67.y);
                     Real sp[N], su[N], sv[N];
 #pragma unroll
                     for (int j = 0; j < N; ++j)
                         sp[j] = su[j] = sv[j] = 0;
                     if (flags & F_VOL)
-                    {
-#pragma unroll
-                        for (int l = 0; l < N; ++l)
-                        {
-                            const Real el = Tab<Real>::x(N, l);
-                            const Real Xxi = Real(0.25) * ((Real(1) - el) * dx0 + (Real(1) + el) * dx1);
-                            const Real Yxi = Real(0.25) * ((Real(1) - el) * dy0 + (Real(1) + el) * dy1);
-                            const Real W = wi * Tab<Real>::w(N, l);
-                            const Real *nd = ue + 3 * (i + N * l);
-                            const Real p = nd[0], u = nd[1], v = nd[2];
-                            const Real WYx = W * Yxi, WXx = W * Xxi;
-                            const Real Gp = -WYx * u + WXx * v, Gu = -WYx * p, Gv = WXx * p;
-                            // du(i, j) += sum_l D(l, j) G(i, l)  (div_2d_c, source/Div.cpp:131-179)
-#pragma unroll
-                            for (int j = 0; j < N; ++j)
-                            {
-                                const Real d = Tab<Real>::D(N, l + N * j);
-                                sp[j] += d * Gp;
-                                su[j] += d * Gu;
-                                sv[j] += d * Gv;
-                            }
-                        }
-                    }
+                        line_column<N, Real>(c01, c23, c45, c67, ue, i, wi, sp, su, sv);
                     // face nodes of the column: (i, 0) on side 0, (i, n-1) on side 2, face-node index i
                     ws_face<N, Real, 0>(codes, flags, c01, c23, c45, c67, wi, i, ue + 3 * i, halo_e, sp[0], su[0], sv[0]);
                     ws_face<N, Real, 2>(codes, flags, c01, c23, c45, c67, wi, i, ue + 3 * (i + N * (N - 1)), halo_e,
@@ -412,14 +346,9 @@ namespace wdg
                 __syncwarp();
                 if (act)
                 {
-                    // ---- row pass: row j = ln.  F = W (y_eta u - x_eta v, y_eta p, -x_eta p); along a
-                    // row x_xi, y_xi are constant and x_eta, y_eta vary linearly with xi.
+                    // ---- row pass: row j = ln
                     const int j = ln;
-                    const Real eta = xm, wj = wm;
-                    const Real Xxi = Real(0.25) * ((Real(1) - eta) * Real(c23.x - c01.x) + (Real(1) + eta) * Real(c45.x - c67.x));
-                    const Real Yxi = Real(0.25) * ((Real(1) - eta) * Real(c23.y - c01.y) + (Real(1) + eta) * Real(c45.y - c67.y));
-                    const Real ex0 = Real(c67.x - c01.x), ex1 = Real(c45.x - c23.x);
-                    const Real ey0 = Real(c67.y - c01.y), ey1 = Real(c45.y - c23.y);
+                    const Real wj = wm;
                     Real *row = ue + 3 * N * j;
                     Real q0[N], q1[N], q2[N], mv[N];
                     Real ap[N], au[N], av[N];
@@ -431,33 +360,7 @@ namespace wdg
                         q2[l] = row[3 * l + 2];
                         ap[l] = au[l] = av[l] = 0;
                     }
-#pragma unroll
-                    for (int l = 0; l < N; ++l)
-                    {
-                        const Real xl = Tab<Real>::x(N, l);
-                        const Real Xeta = Real(0.25) * ((Real(1) - xl) * ex0 + (Real(1) + xl) * ex1);
-                        const Real Yeta = Real(0.25) * ((Real(1) - xl) * ey0 + (Real(1) + xl) * ey1);
-                        const Real W = Tab<Real>::w(N, l) * wj;
-                        // MassMatrix<true>: w_i w_j det J (source/MassMatrix.cpp:6-28)
-                        if constexpr (sizeof(Real) == 4)
-                            mv[l] = __frcp_rn(W * (Xxi * Yeta - Yxi * Xeta));
-                        else
-                            mv[l] = Real(1) / (W * (Xxi * Yeta - Yxi * Xeta));
-                        if (flags & F_VOL)
-                        {
-                            const Real WYe = W * Yeta, WXe = W * Xeta;
-                            const Real Fp = WYe * q1[l] - WXe * q2[l], Fu = WYe * q0[l], Fv = -WXe * q0[l];
-                            // du(i, j) += sum_l D(l, i) F(l, j)
-#pragma unroll
-                            for (int i = 0; i < N; ++i)
-                            {
-                                const Real d = Tab<Real>::D(N, l + N * i);
-                                ap[i] += d * Fp;
-                                au[i] += d * Fu;
-                                av[i] += d * Fv;
-                            }
-                        }
-                    }
+                    line_row<N, Real, true>(c01, c23, c45, c67, xm, wj, (flags & F_VOL) != 0, q0, q1, q2, ap, au, av, mv);
                     // face nodes of the row: (0, j) on side 3, (n-1, j) on side 1, face-node index j
                     ws_face<N, Real, 3>(codes, flags, c01, c23, c45, c67, wj, j, row, halo_e, ap[0], au[0], av[0]);
                     ws_face<N, Real, 1>(codes, flags, c01, c23, c45, c67, wj, j, row + 3 * (N - 1), halo_e,
@@ -485,10 +388,10 @@ namespace wdg
                             r2 *= mv[i];
                         }
                         Real *dn = drow + 3 * i;
-                        const Real d0 = has_du ? c.rk_a * dn[0] + c.dt * r0 : c.dt * r0;
-                        const Real d1 = has_du ? c.rk_a * dn[1] + c.dt * r1 : c.dt * r1;
-                        const Real d2 = has_du ? c.rk_a * dn[2] + c.dt * r2 : c.dt * r2;
-                        Real uo[3] = {q0[i] + c.rk_b * d0, q1[i] + c.rk_b * d1, q2[i] + c.rk_b * d2};
+                        const Real d0 = rk_register(has_du, c.rk_a, dn[0], c.dt, r0);
+                        const Real d1 = rk_register(has_du, c.rk_a, dn[1], c.dt, r1);
+                        const Real d2 = rk_register(has_du, c.rk_a, dn[2], c.dt, r2);
+                        Real uo[3] = {rk_state(q0[i], c.rk_b, d0), rk_state(q1[i], c.rk_b, d1), rk_state(q2[i], c.rk_b, d2)};
                         dn[0] = d0;
                         dn[1] = d1;
                         dn[2] = d2;

@@ -82,6 +82,25 @@ namespace wdg
                 return cuda_fail(e, "cudaMalloc(du)");
             }
         }
+        if (!w->d_flags && !w->halo && res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, 0).fits)
+        {
+            const size_t bytes = sizeof(unsigned long long) * res_flag_count(w->n, w->nel);
+            cudaError_t e = cudaMalloc(&w->d_trace, 2 * w->real_size() * 16 * (size_t)w->n * w->nel);
+            if (e == cudaSuccess)
+                e = cudaMalloc((void **)&w->d_flags, bytes);
+            if (e == cudaSuccess)
+                e = cudaMemset(w->d_flags, 0, bytes);
+            if (e != cudaSuccess)
+            {
+                if (w->d_trace)
+                    cudaFree(w->d_trace);
+                if (w->d_flags)
+                    cudaFree(w->d_flags);
+                w->d_trace = nullptr;
+                w->d_flags = nullptr;
+                return cuda_fail(e, "cudaMalloc(trace buffers)");
+            }
+        }
         return WDG_OK;
     }
 
@@ -136,6 +155,24 @@ namespace wdg
         Real *du = static_cast<Real *>(w->d_du);
         if (A == B || A == Cb)
             return fail(WDG_ERR_ARG, "rk4: state buffer aliases the rotation buffers");
+        // a mesh that fits the chip stays there for all steps (unless the caller chose a kernel, or the
+        // skipped-chunk test asks for the streaming one)
+        if (w->family == 2 && !w->explicit_launch && !w->test_skip && w->d_flags && nsteps > 0 && (!x.F || x.d_fscale) &&
+            (!x.acc || x.d_cfilter))
+        {
+            const ResPlan p = res_plan(w->n, sizeof(Real) == 4, w->nel, w->sms, w->max_ctas);
+            if (p.fits)
+            {
+                bool ran = false;
+                WDG_TRY(res_rk4<Real>(w, p, A, dt, nsteps, x, ran));
+                if (ran)
+                {
+                    for (int s = 0; s < nsteps; ++s)
+                        t += dt;
+                    return WDG_OK;
+                }
+            }
+        }
         StageArgs<Real> a = base_args<Real>(w);
         a.du = du;
         a.dt = (Real)dt;
@@ -458,12 +495,14 @@ extern "C"
             return fail(WDG_ERR_ARG, "wdg_wave_create: no such device");
         DeviceGuard guard(device);
         WDG_TRY(upload_basis_tables(device));
+        WDG_TRY(upload_res_tables(device));
 
         FaceTables ft;
         WDG_TRY(build_face_tables(*mesh, bc, ft));
 
         wdg_wave *w = new wdg_wave;
         w->device = device;
+        cudaDeviceGetAttribute(&w->sms, cudaDevAttrMultiProcessorCount, device);
         w->n = n_colloc;
         w->nel = mesh->nel;
         w->precision = precision;
@@ -569,7 +608,7 @@ extern "C"
         void *ptrs[] = {w->d_corners, w->d_nbr, w->d_finfo, w->d_face_edge, w->d_fbase, w->d_fcode, w->d_edgesI,
                         w->d_edgesB, w->d_codes,
                         w->d_state[0], w->d_state[1], w->d_state[2], w->d_du, w->d_stage[0], w->d_stage[1],
-                        w->d_stage[2], w->d_scratch, w->d_result, w->d_err, w->d_src};
+                        w->d_stage[2], w->d_scratch, w->d_result, w->d_err, w->d_src, w->d_flags, w->d_trace};
         for (void *p : ptrs)
             if (p)
                 cudaFree(p);
@@ -621,6 +660,7 @@ extern "C"
             return fail(WDG_ERR_ARG, "warp-specialised kernel: chunk x ring too large for shared memory");
         w->ws_chunk = chunk;
         w->ws_ring = ring;
+        w->explicit_launch = true;
         return WDG_OK;
     }
 
@@ -703,6 +743,7 @@ extern "C"
             return fail(WDG_ERR_ARG,
                         "wdg_wave_set_kernel: 0 (warp per element), 1 (tiled), 2 (warp-specialised) or -1 (default)");
         w->family = (family < 0) ? default_family(w->n) : family;
+        w->explicit_launch = family >= 0;
         return WDG_OK;
     }
 
@@ -740,6 +781,10 @@ extern "C"
             int family, a, b;
         };
         std::vector<Cand> cands;
+        // family 3 stands for family 2 with the elements resident, where they fit
+        const bool save_explicit = w->explicit_launch;
+        if (w->d_flags && res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, w->max_ctas).fits)
+            cands.push_back({3, 0, 0});
         cands.push_back({0, save_tile, save_stages});
         for (int st = 2; st <= 4; ++st)
             for (int tile = 4; tile <= max_tile(w->n); tile += 4)
@@ -752,7 +797,8 @@ extern "C"
         for (size_t ci = 0; ci < cands.size() && s == WDG_OK; ++ci)
             {
                 const Cand &cd = cands[ci];
-                w->family = cd.family;
+                w->family = std::min(cd.family, 2);
+                w->explicit_launch = cd.family != 3;
                 w->tile = (cd.family == 1) ? cd.a : save_tile;
                 w->stages = (cd.family == 1) ? cd.b : save_stages;
                 w->ws_chunk = (cd.family == 2) ? cd.a : save_chunk;
@@ -785,7 +831,7 @@ extern "C"
                     best = ms;
                     bt = w->tile;
                     bs = w->stages;
-                    bf = w->family;
+                    bf = cd.family;
                     bc = w->ws_chunk;
                     br = w->ws_ring;
                 }
@@ -794,7 +840,8 @@ extern "C"
         cudaEventDestroy(e1);
         w->tile = (s == WDG_OK) ? bt : save_tile;
         w->stages = (s == WDG_OK) ? bs : save_stages;
-        w->family = (s == WDG_OK) ? bf : save_family;
+        w->family = (s == WDG_OK) ? std::min(bf, 2) : save_family;
+        w->explicit_launch = (s == WDG_OK) ? bf != 3 : save_explicit;
         w->ws_chunk = (s == WDG_OK) ? bc : save_chunk;
         w->ws_ring = (s == WDG_OK) ? br : save_ring;
         if (s == WDG_OK)

@@ -15,6 +15,8 @@ struct wdg_wave
     int n = 0, nel = 0, precision = WDG_FP64, tile = 0, max_ctas = 0, stages = wdg::kDefaultStages;
     int family = 0; // fused-kernel family: 0 warp-per-element, 1 tiled TMA pipeline, 2 warp-specialised
     int ws_chunk = 0, ws_ring = wdg::kWsDefaultRing; // family 2 launch shape
+    bool explicit_launch = false; // the caller chose a kernel or its shape: no resident launches
+    int sms = 0;
     long long ndof = 0;
     long long halo = 0; // values of neighbour traces appended after the elements in each state
                         // buffer (a domain of a decomposed mesh; 0 otherwise)
@@ -41,6 +43,10 @@ struct wdg_wave
     double *d_result = nullptr; // 8 doubles
     double *h_result = nullptr; // pinned, 8 doubles
     unsigned *d_err = nullptr;
+    // resident launches, on handles whose mesh fits: a flag per element group, the value they count on
+    // from, and two trace buffers (with the states)
+    unsigned long long *d_flags = nullptr, flag_base = 0;
+    void *d_trace = nullptr;
     unsigned long long wait_ns = 0; // limit of the stage kernels' bounded waits (0: kWaitLimitNs)
     int test_skip = 0;              // test hook: 1 + chunk the next RK launch leaves unloaded
     double *d_src = nullptr;    // gaussian source table
@@ -67,7 +73,25 @@ namespace wdg
         double omega = 0.0;        // s(t) = -sin(omega t)/omega when F != nullptr
         double *acc = nullptr;     // FP64 filter (nullable)
         const double *c_filter = nullptr; // per-step filter weights (host array, nsteps)
+        // the same on the device: c_filter, and the forcing's scale s(t + c_st dt) per stage (5 nsteps);
+        // without those that F and acc need, the steps run as stage launches
+        const double *d_cfilter = nullptr, *d_fscale = nullptr;
     };
+
+    // Many stages in one launch with the elements resident on chip (stage_res.cu): whether a handle's
+    // mesh fits, and the launch shape
+    struct ResPlan
+    {
+        bool fits = false;
+        int ngroups = 0, ctas = 0, warps = 0;
+        size_t smem = 0;
+    };
+    ResPlan res_plan(int n, bool fp32, int nel, int sms, int max_ctas);
+    size_t res_flag_count(int n, int nel);
+    int upload_res_tables(int device); // once per device
+    // nsteps of RK4 on A; ran = false (and nothing done) where the device cannot hold the launch
+    template <typename Real>
+    int res_rk4(wdg_wave *w, const ResPlan &p, Real *A, double dt, int nsteps, const RKExtras &x, bool &ran);
     template <typename Real>
     int rk4_run(wdg_wave *w, Real *A, double dt, double &t, int nsteps, const RKExtras &x);
     // stage st of the RK4 step that starts at time t; with F, forcing F * s(t + c_st dt),

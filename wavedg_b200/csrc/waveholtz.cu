@@ -22,6 +22,7 @@ struct wdg_waveholtz
     int nt = 0;
     std::vector<double> c_filter; // c_it, it = 1..nt
     double c0 = 0;                // 0.5 dt K(0)
+    double *d_cfilter = nullptr, *d_fscale = nullptr; // c_filter, and the forcing's scale per stage (5 nt)
     cudaStream_t cs = nullptr;    // private capture stream
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
     double *d_W = nullptr, *d_acc = nullptr, *d_pi0 = nullptr;
@@ -65,6 +66,8 @@ namespace
         RKExtras x;
         x.acc = h->d_acc;
         x.c_filter = h->c_filter.data();
+        x.d_cfilter = h->d_cfilter;
+        x.d_fscale = h->d_fscale;
         if (forced)
         {
             x.F = h->d_F;
@@ -183,6 +186,11 @@ extern "C"
             t += h->dt;
             h->c_filter[it - 1] = ((it == h->nt) ? 0.5 : 1.0) * h->dt * K(h, t);
         }
+        std::vector<double> fscale(5 * (size_t)h->nt);
+        t = 0.0;
+        for (int it = 0; it < h->nt; ++it, t += h->dt)
+            for (int st = 0; st < 5; ++st)
+                fscale[5 * (size_t)it + st] = -1.0 / omega * std::sin(omega * (t + rk4c[st] * h->dt));
         int dev_prev = 0;
         cudaGetDevice(&dev_prev);
         cudaSetDevice(w->device);
@@ -202,6 +210,14 @@ extern "C"
             e = cudaMalloc(&h->d_pi0, sizeof(double) * nd + 64);
         if (e == cudaSuccess)
             e = cudaMalloc(&h->d_F, w->real_size() * nd + 64);
+        if (e == cudaSuccess)
+            e = cudaMalloc(&h->d_cfilter, sizeof(double) * h->c_filter.size());
+        if (e == cudaSuccess)
+            e = cudaMemcpy(h->d_cfilter, h->c_filter.data(), sizeof(double) * h->c_filter.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess)
+            e = cudaMalloc(&h->d_fscale, sizeof(double) * fscale.size());
+        if (e == cudaSuccess)
+            e = cudaMemcpy(h->d_fscale, fscale.data(), sizeof(double) * fscale.size(), cudaMemcpyHostToDevice);
         if (s == WDG_OK && e != cudaSuccess)
             s = cuda_fail(e, "wdg_waveholtz_create");
         cudaSetDevice(dev_prev);
@@ -245,7 +261,7 @@ extern "C"
             cudaGraphExecDestroy(h->g_S);
         if (h->g_pi0)
             cudaGraphExecDestroy(h->g_pi0);
-        for (void *p : {(void *)h->d_W, (void *)h->d_acc, (void *)h->d_pi0, h->d_F})
+        for (void *p : {(void *)h->d_W, (void *)h->d_acc, (void *)h->d_pi0, h->d_F, (void *)h->d_cfilter, (void *)h->d_fscale})
             if (p)
                 cudaFree(p);
         if (h->ev_in)

@@ -164,6 +164,8 @@ SIGNATURES = {
     # learned warm start (include/wdg_fno.h)
     "wdg_fno_gemm": ([_v, _v, _v, _i, _i, _i, _ll, _ll, _ll, _ll, _ll, _ll, _i, _i, _i, C.c_float, C.c_float, _i,
                       _v], _i),
+    "wdg_fno_gemm_act": ([_v, _v, _v, _i, _i, _i, _ll, _ll, _ll, _ll, _ll, _ll, _i, _i, _i, _i, _v, _v, _v, _i, _v], _i),
+    "wdg_fno_layer": ([_v, _v, _v, _v, _v, _v, _v, _v, _i, _i, _i, _i, _i, _i, _v], _i),
     "wdg_fno_dft_y": ([_v, _v, _v, _v, _v, _i, _i, _i, _i, _i, C.c_float, _v], _i),
     "wdg_fno_mix": ([_v, _v, _v, _i, _i, _i, _i, _v], _i),
     "wdg_fno_mix_bwd": ([_v, _v, _v, _v, _v, _i, _i, _i, _i, _i, _v], _i),

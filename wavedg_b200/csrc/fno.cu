@@ -6,6 +6,8 @@
 //               cores through mma.sync.m16n8k16 (BF16): every GEMM of the network has one
 //               dimension of 32 (channels or retained modes), so these are bandwidth-bound
 //               streams, not tensor-throughput-bound tiles.
+//   layer       the two GEMMs of a Fourier layer's output (inverse DFT along x, channel mix) in one
+//               pass with what follows them, forward (bias, GELU) and backward (GELU's derivative).
 //   dft_y       the truncated DFT along y (retained wavenumbers 0..K/2-1 and -K/2..-1) and its
 //               inverse/adjoint, FP32 on CUDA cores (small: K x KX modes per channel).
 //   mix         per-mode complex channel mixing and its two adjoints.
@@ -19,6 +21,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "common.hpp"
@@ -28,7 +31,7 @@ namespace
     using bf16 = __nv_bfloat16;
 
     // ------------------------------------------------------------------ GEMM
-    constexpr int TM = 64, TN = 64, TK = 32, LDS = TK + 8; // shared tiles: [64][40] bf16
+    constexpr int TM = 64, TK = 32; // TK: K per shared-memory step (two mma steps of 16, in order)
 
     __device__ __forceinline__ void mma_bf16(float c[4], const uint32_t a[4], const uint32_t b[2])
     {
@@ -38,6 +41,145 @@ namespace
             : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
             : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
     }
+    __device__ __forceinline__ uint32_t smem_at(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+    // four 8 x 8 tiles, lane l giving the row l & 7 of tile l >> 3; TRANS: each tile transposed
+    template <bool TRANS>
+    __device__ __forceinline__ void ldmatrix4(uint32_t r[4], const bf16 *p)
+    {
+        if constexpr (TRANS)
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                         : "r"(smem_at(p)));
+        else
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                         : "r"(smem_at(p)));
+    }
+
+    // A ROWS x COLS tile (COLS contiguous in memory, rows ld apart) to shared memory, rows COLS + 8
+    // apart (ldmatrix then reads eight rows from different banks); values past (rows, cols) are 0.
+    // vec: whole 16-byte pieces by cp.async (cols a multiple of 8, everything aligned)
+    template <int ROWS, int COLS>
+    __device__ __forceinline__ void load_tile(bf16 *sm, const bf16 *g, long long ld, int rows, int cols, bool vec, int t)
+    {
+        constexpr int LD = COLS + 8;
+        if (vec)
+        {
+#pragma unroll
+            for (int i = 0; i < ROWS * COLS / 8; i += 128)
+            {
+                const int q = i + t, r = q / (COLS / 8), c = q % (COLS / 8) * 8;
+                if (ROWS * COLS / 8 % 128 != 0 && q >= ROWS * COLS / 8)
+                    break;
+                const bool in = r < rows && c < cols;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_at(sm + r * LD + c)),
+                             "l"(in ? g + r * ld + c : g), "r"(in ? 16 : 0)
+                             : "memory");
+            }
+        }
+        else
+            for (int q = t; q < ROWS * COLS; q += 128)
+            {
+                const int r = q / COLS, c = q % COLS;
+                sm[r * LD + c] = (r < rows && c < cols) ? g[r * ld + c] : __float2bfloat16(0.f);
+            }
+    }
+    // acc (a warp's 32 x 32) += op(A) op(B) over one shared-memory step, K ascending; A at row m0, B at
+    // column n0 of their tiles.  TA: A stored (k, m), else (m, k); TB: B stored (n, k), else (k, n)
+    template <bool TA, bool TB, int LDA, int LDB>
+    __device__ __forceinline__ void tile_mma(float acc[2][4][4], const bf16 *As, const bf16 *Bs, int m0, int n0, int lane)
+    {
+        const int r8 = lane & 7, q = lane >> 3; // row within a tile, tile
+#pragma unroll
+        for (int kk = 0; kk < TK; kk += 16)
+        {
+            uint32_t af[2][4], bfr[2][4];
+#pragma unroll
+            for (int mi = 0; mi < 2; ++mi)
+            {
+                // tiles: (m, k), (m + 8, k), (m, k + 8), (m + 8, k + 8)
+                const int m = m0 + 16 * mi + 8 * (q & 1), k = kk + 8 * (q >> 1);
+                ldmatrix4<TA>(af[mi], TA ? As + (k + r8) * LDA + m : As + (m + r8) * LDA + k);
+            }
+#pragma unroll
+            for (int ni = 0; ni < 2; ++ni)
+            {
+                // tiles: (k, n), (k + 8, n), (k, n + 8), (k + 8, n + 8)
+                const int n = n0 + 16 * ni + 8 * (q >> 1), k = kk + 8 * (q & 1);
+                ldmatrix4<!TB>(bfr[ni], TB ? Bs + (n + r8) * LDB + k : Bs + (k + r8) * LDB + n);
+            }
+#pragma unroll
+            for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni)
+                    mma_bf16(acc[mi][ni], af[mi], bfr[ni >> 1] + 2 * (ni & 1));
+        }
+    }
+
+    __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
+    __device__ __forceinline__ float gelu_grad(float z)
+    {
+        const float cdf = 0.5f * (1.f + erff(z * 0.70710678118654752f));
+        const float pdf = 0.39894228040143268f * expf(-0.5f * z * z);
+        return cdf + z * pdf;
+    }
+
+    // what a GEMM does with its result besides, or instead of, storing it
+    enum
+    {
+        EPI_STORE = 0,    // C = alpha acc + beta C
+        EPI_BIAS_ACT = 1, // v = acc + bias[row]: C = v (nullable), y = act ? gelu(v) : v in BF16 (nullable)
+        EPI_ACT_BWD = 2   // v = act ? acc gelu'(z) : acc: C = v (nullable), y = v in BF16 (nullable)
+    };
+    struct Epilogue
+    {
+        const float *bias, *z;
+        bf16 *y;
+        int act;
+    };
+    // two neighbouring columns of one row; i: their place in C, z and y
+    __device__ __forceinline__ void epilogue(int mode, const Epilogue &e, float *C, long long i, float bias, float v0, float v1,
+                                             bool two, bool pair)
+    {
+        if (mode == EPI_BIAS_ACT)
+        {
+            v0 = v0 + bias;
+            v1 = v1 + bias;
+        }
+        else if (e.act)
+        {
+            v0 = v0 * gelu_grad(e.z[i]);
+            if (two)
+                v1 = v1 * gelu_grad(e.z[i + 1]);
+        }
+        if (C)
+        {
+            if (pair)
+                *reinterpret_cast<float2 *>(C + i) = make_float2(v0, v1);
+            else
+            {
+                C[i] = v0;
+                if (two)
+                    C[i + 1] = v1;
+            }
+        }
+        if (e.y)
+        {
+            if (mode == EPI_BIAS_ACT && e.act)
+            {
+                v0 = gelu(v0);
+                v1 = gelu(v1);
+            }
+            if (pair)
+                *reinterpret_cast<__nv_bfloat162 *>(e.y + i) = __floats2bfloat162_rn(v0, v1);
+            else
+            {
+                e.y[i] = __float2bfloat16(v0);
+                if (two)
+                    e.y[i + 1] = __float2bfloat16(v1);
+            }
+        }
+    }
 
     struct GemmArgs
     {
@@ -46,111 +188,233 @@ namespace
         int M, N, K;
         long long lda, ldb, ldc;       // leading dimensions of the stored matrices
         long long sA, sB, sC;          // batch strides (elements)
-        int transA, transB;            // op(A)[m][k] = transA ? A[k*lda + m] : A[m*lda + k]
         float alpha, beta;
         int ksplit;                    // K range per split (multiple of TK)
         int atomic;                    // accumulate with atomics (split K, or batches sharing C)
+        int vecA, vecB, pairC;         // 16-byte loads of A, B; 8-byte stores of C
+        Epilogue e;
     };
 
-    // 64 x 64 output tile per CTA, 4 warps of 32 x 32, K in steps of 32 through shared memory
+    // BM x BN output tile per CTA of four warps (32 x 32 each), K in steps of 32 through ST shared-memory
+    // stages filled by cp.async.  These GEMMs stream one operand with hundreds of thousands of rows past
+    // a matrix of at most 64 x 64: the tile shape follows the narrow side (32 x 128, 128 x 32, 64 x 64), so
+    // that no half of it is padding.  Bound by HBM.
+    template <int BM, int BN, int ST, bool TA, bool TB, int EPI>
     __global__ void __launch_bounds__(128) gemm_bf16_kernel(const GemmArgs g)
     {
-        __shared__ __align__(16) bf16 As[TM][LDS]; // (m, k)
-        __shared__ __align__(16) bf16 Bs[TN][LDS]; // (n, k)
+        constexpr int LDA = (TA ? BM : TK) + 8, LDB = (TB ? TK : BN) + 8;
+        constexpr int SA = (TA ? TK : BM) * LDA, SB = (TB ? BN : TK) * LDB;
+        extern __shared__ __align__(16) bf16 gsm[];
         const int bz = blockIdx.z;
         const int nsplit = (g.K + g.ksplit - 1) / g.ksplit;
         const int batch = bz / nsplit, split = bz - batch * nsplit;
         const bf16 *A = g.A + batch * g.sA;
         const bf16 *B = g.B + batch * g.sB;
-        float *C = g.C + batch * g.sC;
-        const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+        const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
         const int k_begin = split * g.ksplit, k_end = min(g.K, k_begin + g.ksplit);
         const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-        const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+        constexpr int WN = BN / 32;
+        const int wm = warp / WN * 32, wn = warp % WN * 32;
         const int gid = lane >> 2, tig = lane & 3;
         float acc[2][4][4] = {};
-        const bf16 zero = __float2bfloat16(0.f);
-
-        for (int k0 = k_begin; k0 < k_end; k0 += TK)
+        const int nk = (k_end - k_begin + TK - 1) / TK;
+        auto load = [&](int it)
         {
-            // stage A tile (m, k) and B tile (n, k); the stored layout decides which index runs
-            // fastest across threads so the global reads stay coalesced
-            for (int i = t; i < TM * TK; i += 128)
-            {
-                int m, k;
-                if (g.transA) { k = i / TM; m = i - k * TM; }
-                else { m = i / TK; k = i - m * TK; }
-                const int gm = m0 + m, gk = k0 + k;
-                bf16 v = zero;
-                if (gm < g.M && gk < k_end)
-                    v = g.transA ? A[(long long)gk * g.lda + gm] : A[(long long)gm * g.lda + gk];
-                As[m][k] = v;
-            }
-            for (int i = t; i < TN * TK; i += 128)
-            {
-                int n, k;
-                if (g.transB) { n = i / TK; k = i - n * TK; }
-                else { k = i / TN; n = i - k * TN; }
-                const int gn = n0 + n, gk = k0 + k;
-                bf16 v = zero;
-                if (gn < g.N && gk < k_end)
-                    v = g.transB ? B[(long long)gn * g.ldb + gk] : B[(long long)gk * g.ldb + gn];
-                Bs[n][k] = v;
-            }
-            __syncthreads();
+            bf16 *As = gsm + (it % ST) * (SA + SB), *Bs = As + SA;
+            const int k0 = k_begin + it * TK, kr = k_end - k0;
+            if constexpr (TA)
+                load_tile<TK, BM>(As, A + (long long)k0 * g.lda + m0, g.lda, kr, g.M - m0, g.vecA, t);
+            else
+                load_tile<BM, TK>(As, A + (long long)m0 * g.lda + k0, g.lda, g.M - m0, kr, g.vecA, t);
+            if constexpr (TB)
+                load_tile<BN, TK>(Bs, B + (long long)n0 * g.ldb + k0, g.ldb, g.N - n0, kr, g.vecB, t);
+            else
+                load_tile<TK, BN>(Bs, B + (long long)k0 * g.ldb + n0, g.ldb, kr, g.N - n0, g.vecB, t);
+        };
 #pragma unroll
-            for (int kk = 0; kk < TK; kk += 16)
-            {
-                uint32_t af[2][4], bfr[4][2];
-#pragma unroll
-                for (int mi = 0; mi < 2; ++mi)
-                {
-                    const int r = wm + 16 * mi + gid;
-                    af[mi][0] = *reinterpret_cast<const uint32_t *>(&As[r][kk + 2 * tig]);
-                    af[mi][1] = *reinterpret_cast<const uint32_t *>(&As[r + 8][kk + 2 * tig]);
-                    af[mi][2] = *reinterpret_cast<const uint32_t *>(&As[r][kk + 2 * tig + 8]);
-                    af[mi][3] = *reinterpret_cast<const uint32_t *>(&As[r + 8][kk + 2 * tig + 8]);
-                }
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-                {
-                    const int c = wn + 8 * ni + gid;
-                    bfr[ni][0] = *reinterpret_cast<const uint32_t *>(&Bs[c][kk + 2 * tig]);
-                    bfr[ni][1] = *reinterpret_cast<const uint32_t *>(&Bs[c][kk + 2 * tig + 8]);
-                }
-#pragma unroll
-                for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                    for (int ni = 0; ni < 4; ++ni)
-                        mma_bf16(acc[mi][ni], af[mi], bfr[ni]);
-            }
-            __syncthreads();
+        for (int q = 0; q < (ST > 1 ? ST - 1 : 1); ++q)
+        {
+            if (q < nk)
+                load(q);
+            asm volatile("cp.async.commit_group;" ::: "memory");
         }
-        // epilogue: C = alpha acc + beta C (split-K: atomic accumulation, beta applied by split 0)
+        for (int it = 0; it < nk; ++it)
+        {
+            asm volatile("cp.async.wait_group %0;" ::"n"(ST > 1 ? ST - 2 : 0) : "memory");
+            __syncthreads(); // this step has landed; every warp is done with the one before
+            if constexpr (ST > 1)
+            {
+                if (it + ST - 1 < nk)
+                    load(it + ST - 1);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            }
+            const bf16 *As = gsm + (it % ST) * (SA + SB);
+            tile_mma<TA, TB, LDA, LDB>(acc, As, As + SA, wm, wn, lane);
+            if constexpr (ST == 1)
+                if (it + 1 < nk)
+                {
+                    __syncthreads();
+                    load(it + 1);
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                }
+        }
+        float *C = g.C ? g.C + batch * g.sC : nullptr;
+        Epilogue e = g.e;
+        if (e.z)
+            e.z += batch * g.sC;
+        if (e.y)
+            e.y += batch * g.sC;
+        // (split-K: atomic accumulation into a C that was zeroed or holds beta C)
 #pragma unroll
         for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
+            for (int hr = 0; hr < 2; ++hr)
+            {
+                const int r = m0 + wm + 16 * mi + gid + 8 * hr;
+                if (r >= g.M)
+                    continue;
+                const float bias = EPI == EPI_BIAS_ACT ? g.e.bias[r] : 0.f;
 #pragma unroll
-                for (int h = 0; h < 4; ++h)
+                for (int ni = 0; ni < 4; ++ni)
                 {
-                    const int r = m0 + wm + 16 * mi + gid + ((h >= 2) ? 8 : 0);
-                    const int c = n0 + wn + 8 * ni + 2 * tig + (h & 1);
-                    if (r >= g.M || c >= g.N)
+                    const int c = n0 + wn + 8 * ni + 2 * tig;
+                    if (c >= g.N)
                         continue;
-                    float *p = C + (long long)r * g.ldc + c;
-                    const float v = g.alpha * acc[mi][ni][h];
-                    if (!g.atomic)
-                        *p = (g.beta == 0.f) ? v : v + g.beta * *p;
+                    const bool two = c + 1 < g.N, pair = g.pairC && two;
+                    const long long i = (long long)r * g.ldc + c;
+                    float v0 = acc[mi][ni][2 * hr], v1 = acc[mi][ni][2 * hr + 1];
+                    if constexpr (EPI != EPI_STORE)
+                        epilogue(EPI, e, C, i, bias, v0, v1, two, pair);
                     else
-                        atomicAdd(p, v);
+                    {
+                        v0 = g.alpha * v0;
+                        v1 = g.alpha * v1;
+                        if (g.atomic)
+                        {
+                            atomicAdd(C + i, v0);
+                            if (two)
+                                atomicAdd(C + i + 1, v1);
+                        }
+                        else if (pair)
+                        {
+                            float2 *q = reinterpret_cast<float2 *>(C + i);
+                            if (g.beta != 0.f)
+                            {
+                                const float2 old = *q;
+                                v0 = v0 + g.beta * old.x;
+                                v1 = v1 + g.beta * old.y;
+                            }
+                            *q = make_float2(v0, v1);
+                        }
+                        else
+                        {
+                            C[i] = (g.beta == 0.f) ? v0 : v0 + g.beta * C[i];
+                            if (two)
+                                C[i + 1] = (g.beta == 0.f) ? v1 : v1 + g.beta * C[i + 1];
+                        }
+                    }
                 }
+            }
     }
 
-    __global__ void scale_kernel(float *x, long long n, float s)
+    template <int BM, int BN, int ST, int EPI>
+    void gemm_launch(const GemmArgs &g, int transA, int transB, int nz, cudaStream_t s)
     {
-        for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-            x[i] *= s;
+        const dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, nz);
+        auto run = [&](auto kern, bool ta, bool tb)
+        {
+            const int lda = (ta ? BM : TK) + 8, ldb = (tb ? TK : BN) + 8;
+            const size_t smem = sizeof(bf16) * ST * ((ta ? TK : BM) * lda + (tb ? BN : TK) * ldb); // at most 38 KB
+            kern<<<grid, 128, smem, s>>>(g);
+        };
+        if (transA)
+            transB ? run(gemm_bf16_kernel<BM, BN, ST, true, true, EPI>, true, true)
+                   : run(gemm_bf16_kernel<BM, BN, ST, true, false, EPI>, true, false);
+        else
+            transB ? run(gemm_bf16_kernel<BM, BN, ST, false, true, EPI>, false, true)
+                   : run(gemm_bf16_kernel<BM, BN, ST, false, false, EPI>, false, false);
+    }
+    template <int ST, int EPI>
+    void gemm_tiles(const GemmArgs &g, int transA, int transB, int nz, cudaStream_t s)
+    {
+        if (g.M <= 32)
+            gemm_launch<32, 128, ST, EPI>(g, transA, transB, nz, s);
+        else if (g.N <= 32)
+            gemm_launch<128, 32, ST, EPI>(g, transA, transB, nz, s);
+        else
+            gemm_launch<64, 64, ST, EPI>(g, transA, transB, nz, s);
+    }
+    template <int EPI>
+    void gemm_run(GemmArgs &g, int transA, int transB, int nz, cudaStream_t s)
+    {
+        auto whole = [](const void *p, long long ld, long long stride, int contiguous)
+        { return (((uintptr_t)p & 15u) == 0 && ld % 8 == 0 && stride % 8 == 0 && contiguous % 8 == 0) ? 1 : 0; };
+        g.vecA = whole(g.A, g.lda, g.sA, transA ? g.M : g.K);
+        g.vecB = whole(g.B, g.ldb, g.sB, transB ? g.K : g.N);
+        g.pairC = (((uintptr_t)g.C & 7u) == 0 && ((uintptr_t)g.e.y & 3u) == 0 && g.ldc % 2 == 0 && g.sC % 2 == 0) ? 1 : 0;
+        if (std::min(g.K, g.ksplit) <= TK)
+            gemm_tiles<1, EPI>(g, transA, transB, nz, s);
+        else
+            gemm_tiles<3, EPI>(g, transA, transB, nz, s);
+    }
+
+    // ------------------------------------------------------------ Fourier layer
+    // One output tile of a layer, 32 channels x 128 grid points of row y of sample b, from its two GEMMs:
+    //   forward   z = W v + U Ix  (U: the mixed spectrum after the inverse DFT along y, per channel and row;
+    //             Ix: the inverse DFT along x), then bias and activation: z, y = BF16 act(z)
+    //   backward  dv = W^T dz + U Ex^T  (U: the adjoint spectrum), then the derivative of the activation below:
+    //             dz = dv gelu'(z) and its BF16 copy
+    // In launches of their own the first result went to memory and back in FP32 and the elementwise step
+    // read and wrote it again: 800 MB a layer at 4 x 32 x 512 x 512 where 270 MB are needed.  Bound by HBM.
+    struct LayerArgs
+    {
+        const bf16 *U, *X, *W, *V;
+        float *C; // z or dz (nullable)
+        int Cn, K1, G;
+        Epilogue e;
+    };
+    template <bool BACK>
+    __global__ void __launch_bounds__(128) layer_kernel(const LayerArgs g)
+    {
+        // X: forward Ix (K1, G); backward Ex (G, K1).  W: forward (o, c), backward (c, o) read as its transpose
+        constexpr int LDX = (BACK ? TK : 128) + 8, SX = (BACK ? 128 : TK) * LDX;
+        __shared__ __align__(16) bf16 Us[32 * (TK + 8)], Ws[32 * (TK + 8)], Xs[SX], Vs[TK * 136];
+        const int t = threadIdx.x, warp = t >> 5, lane = t & 31, gid = lane >> 2, tig = lane & 3;
+        const int x0 = blockIdx.x * 128, y = blockIdx.y, b = blockIdx.z;
+        const long long P = (long long)g.G * g.G, row0 = (long long)b * g.Cn;
+        load_tile<32, TK>(Us, g.U + (row0 * g.G + y) * g.K1, (long long)g.G * g.K1, g.Cn, g.K1, true, t);
+        load_tile<32, TK>(Ws, g.W, g.Cn, g.Cn, g.Cn, true, t);
+        if constexpr (BACK)
+            load_tile<128, TK>(Xs, g.X + (long long)x0 * g.K1, g.K1, g.G - x0, g.K1, true, t);
+        else
+            load_tile<TK, 128>(Xs, g.X + x0, g.G, g.K1, g.G - x0, true, t);
+        load_tile<TK, 128>(Vs, g.V + row0 * P + (long long)y * g.G + x0, P, g.Cn, g.G - x0, true, t);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        float a1[2][4][4] = {}, a2[2][4][4] = {};
+        tile_mma<false, BACK, TK + 8, LDX>(a1, Us, Xs, 0, 32 * warp, lane);
+        tile_mma<BACK, false, TK + 8, 136>(a2, Ws, Vs, 0, 32 * warp, lane);
+#pragma unroll
+        for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+            for (int hr = 0; hr < 2; ++hr)
+            {
+                const int r = 16 * mi + gid + 8 * hr;
+                if (r >= g.Cn)
+                    continue;
+                const float bias = BACK ? 0.f : g.e.bias[r];
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni)
+                {
+                    const int x = x0 + 32 * warp + 8 * ni + 2 * tig;
+                    if (x >= g.G)
+                        continue;
+                    epilogue(BACK ? EPI_ACT_BWD : EPI_BIAS_ACT, g.e, g.C, (row0 + r) * P + (long long)y * g.G + x, bias,
+                             a2[mi][ni][2 * hr] + a1[mi][ni][2 * hr], a2[mi][ni][2 * hr + 1] + a1[mi][ni][2 * hr + 1],
+                             true, true);
+                }
+            }
     }
 
     int blocks(long long n, int threads = 256)
@@ -161,67 +425,109 @@ namespace
 
     // ------------------------------------------------------------- DFT along y
     // out[bc, k, kx] = sum_y e^{s i 2 pi ky(k) y / G} in[bc, y, kx]   (forward: s = -1)
-    // ky(k) = k for k < K/2, k - K otherwise; complex values as (re, im) pairs
-    __global__ void dft_y_fwd_kernel(const float *in, float *out, const float *cs, const float *sn, int BC, int G,
-                                     int K, int KX, float sign)
+    // ky(k) = k for k < K/2, k - K otherwise; complex values as (re, im) pairs.  A CTA takes one plane bc
+    // and kDftThreads pairs of outputs (k, kx) and (k + K/2, kx), so that a value read from shared memory
+    // serves two sums; y runs in order, whatever the chunking.  The twiddles and a chunk of `chunk` rows
+    // sit in shared memory (the twiddles of a grid too large for it stay in global memory: TAB false).
+    constexpr int kDftThreads = 128, kDftRows = 128;
+    constexpr size_t kDftSmem = 96 * 1024;
+    __device__ __forceinline__ void dft_add(float2 x, float2 cs, float sign, float &re, float &im)
     {
-        const long long total = (long long)BC * K * KX;
-        for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
+        const float c = cs.x, s = sign * cs.y;
+        // (the contraction is written out: it decides later roundings to BF16)
+        re += __fmaf_rn(c, x.x, -__fmul_rn(s, x.y));
+        im += __fmaf_rn(s, x.x, __fmul_rn(c, x.y));
+    }
+    template <bool TAB>
+    __global__ void __launch_bounds__(kDftThreads) dft_y_fwd_kernel(const float *in, float *out, const float *cs,
+                                                                    const float *sn, int G, int K, int KX, float sign,
+                                                                    int chunk)
+    {
+        extern __shared__ float2 dsm[];
+        float2 *tab = dsm, *xs = dsm + (TAB ? G : 0); // (cos, sin) of 2 pi m / G; a chunk of rows
+        auto twiddle = [&](int m) { return TAB ? tab[m] : make_float2(__ldg(cs + m), __ldg(sn + m)); };
+        const int t = threadIdx.x, half = K / 2;
+        const long long bc = blockIdx.x;
+        const int q = blockIdx.y * kDftThreads + t, kx = q % KX, k = q / KX;
+        const bool on = k < half;
+        for (int m = t; TAB && m < G; m += kDftThreads)
+            tab[m] = make_float2(cs[m], sn[m]);
+        const float2 *src = reinterpret_cast<const float2 *>(in) + bc * (long long)G * KX;
+        const int step0 = k % G, step1 = ((k - half) % G + G) % G; // ky of k, of k + K/2: k + K/2 - K
+        float re0 = 0.f, im0 = 0.f, re1 = 0.f, im1 = 0.f;
+        int p0 = 0, p1 = 0;
+        for (int y0 = 0; y0 < G; y0 += chunk)
         {
-            const int kx = (int)(i % KX);
-            const int k = (int)((i / KX) % K);
-            const long long bc = i / ((long long)KX * K);
-            const int ky = (k < K / 2) ? k : k - K;
-            const int step = ((ky % G) + G) % G;
-            const float *src = in + bc * (long long)G * KX * 2 + 2 * kx;
-            float re = 0.f, im = 0.f;
-            int ph = 0;
-            for (int y = 0; y < G; ++y)
-            {
-                const float c = cs[ph], s = sign * sn[ph];
-                const float xr = src[(long long)y * KX * 2], xi = src[(long long)y * KX * 2 + 1];
-                re += c * xr - s * xi;
-                im += c * xi + s * xr;
-                ph += step;
-                if (ph >= G)
-                    ph -= G;
-            }
-            out[2 * i] = re;
-            out[2 * i + 1] = im;
+            const int rows = min(chunk, G - y0);
+            __syncthreads();
+            for (int i = t; i < rows * KX; i += kDftThreads)
+                xs[i] = src[(long long)y0 * KX + i];
+            __syncthreads();
+            if (on)
+#pragma unroll 4
+                for (int y = 0; y < rows; ++y)
+                {
+                    const float2 x = xs[y * KX + kx];
+                    dft_add(x, twiddle(p0), sign, re0, im0);
+                    dft_add(x, twiddle(p1), sign, re1, im1);
+                    p0 += step0;
+                    p0 -= p0 >= G ? G : 0;
+                    p1 += step1;
+                    p1 -= p1 >= G ? G : 0;
+                }
+        }
+        if (on)
+        {
+            float2 *o = reinterpret_cast<float2 *>(out) + bc * (long long)K * KX;
+            o[k * KX + kx] = make_float2(re0, im0);
+            o[(k + half) * KX + kx] = make_float2(re1, im1);
         }
     }
 
-    // out[bc, y, kx] = sum_k e^{s i 2 pi ky(k) y / G} in[bc, k, kx]; FP32 and/or BF16 output
-    __global__ void dft_y_inv_kernel(const float *in, float *out, bf16 *outb, const float *cs, const float *sn, int BC,
-                                     int G, int K, int KX, float sign)
+    // out[bc, y, kx] = sum_k e^{s i 2 pi ky(k) y / G} in[bc, k, kx]; FP32 and/or BF16 output.  A CTA takes one
+    // plane and kInvRows rows; the plane's modes and the twiddles sit in shared memory (TAB) where
+    // they fit, k runs in order.
+    constexpr int kInvRows = 32;
+    template <bool TAB>
+    __global__ void __launch_bounds__(kDftThreads) dft_y_inv_kernel(const float *in, float *out, bf16 *outb, const float *cs,
+                                                                    const float *sn, int G, int K, int KX, float sign)
     {
-        const long long total = (long long)BC * G * KX;
-        for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
+        extern __shared__ float2 dsm[];
+        float2 *tab = dsm, *xs = dsm + G;
+        const int t = threadIdx.x, half = K / 2;
+        const long long bc = blockIdx.x;
+        const float2 *src = reinterpret_cast<const float2 *>(in) + bc * (long long)K * KX;
+        auto twiddle = [&](int m) { return TAB ? tab[m] : make_float2(__ldg(cs + m), __ldg(sn + m)); };
+        auto mode = [&](int m) { return TAB ? xs[m] : __ldg(src + m); };
+        const int y0 = blockIdx.y * kInvRows, rows = min(kInvRows, G - y0);
+        for (int m = t; TAB && m < G; m += kDftThreads)
+            tab[m] = make_float2(cs[m], sn[m]);
+        for (int i = t; TAB && i < K * KX; i += kDftThreads)
+            xs[i] = src[i];
+        __syncthreads();
+        for (int i = t; i < rows * KX; i += kDftThreads)
         {
-            const int kx = (int)(i % KX);
-            const int y = (int)((i / KX) % G);
-            const long long bc = i / ((long long)KX * G);
-            const float *src = in + bc * (long long)K * KX * 2 + 2 * kx;
+            const int kx = i % KX, y = y0 + i / KX;
             float re = 0.f, im = 0.f;
-            for (int k = 0; k < K; ++k)
+            int p = 0;
+            for (int k = 0; k < half; ++k)
             {
-                const int ky = (k < K / 2) ? k : k - K;
-                const int ph = (int)((((long long)ky * y) % G + G) % G);
-                const float c = cs[ph], s = sign * sn[ph];
-                const float xr = src[(long long)k * KX * 2], xi = src[(long long)k * KX * 2 + 1];
-                re += c * xr - s * xi;
-                im += c * xi + s * xr;
+                dft_add(mode(k * KX + kx), twiddle(p), sign, re, im);
+                p += y;
+                p -= p >= G ? G : 0;
             }
+            p = (G - (int)((long long)half * y % G)) % G; // ky = -K/2
+            for (int k = half; k < K; ++k)
+            {
+                dft_add(mode(k * KX + kx), twiddle(p), sign, re, im);
+                p += y;
+                p -= p >= G ? G : 0;
+            }
+            const long long o = (bc * G + y) * KX + kx;
             if (out)
-            {
-                out[2 * i] = re;
-                out[2 * i + 1] = im;
-            }
+                reinterpret_cast<float2 *>(out)[o] = make_float2(re, im);
             if (outb)
-            {
-                outb[2 * i] = __float2bfloat16(re);
-                outb[2 * i + 1] = __float2bfloat16(im);
-            }
+                reinterpret_cast<__nv_bfloat162 *>(outb)[o] = __floats2bfloat162_rn(re, im);
         }
     }
 
@@ -300,14 +606,6 @@ namespace
     }
 
     // ------------------------------------------------------------- pointwise
-    __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
-    __device__ __forceinline__ float gelu_grad(float z)
-    {
-        const float cdf = 0.5f * (1.f + erff(z * 0.70710678118654752f));
-        const float pdf = 0.39894228040143268f * expf(-0.5f * z * z);
-        return cdf + z * pdf;
-    }
-
     // z[b, c, p] += bias[c]; y = act ? gelu(z) : z (BF16 and/or FP32 copies)
     __global__ void bias_act_kernel(float *z, const float *bias, bf16 *yb, float *yf, int Bn, int Cn, long long P,
                                     int act)
@@ -544,8 +842,6 @@ extern "C"
         g.sA = strideA;
         g.sB = strideB;
         g.sC = strideC;
-        g.transA = transA;
-        g.transB = transB;
         g.alpha = alpha;
         g.beta = beta;
         g.ksplit = (ksplit > 0) ? ((ksplit + TK - 1) / TK) * TK : ((K + TK - 1) / TK) * TK;
@@ -558,16 +854,82 @@ extern "C"
                 return wdg::fail(WDG_ERR_ARG, "wdg_fno_gemm: atomic accumulation needs beta 0 or 1");
             const int nb = (strideC == 0) ? 1 : batch;
             for (int b = 0; b < nb; ++b)
-                for (int r = 0; r < M; ++r)
-                    if (cudaMemsetAsync(C + b * strideC + (long long)r * ldc, 0, sizeof(float) * N, st(stream)) !=
-                        cudaSuccess)
-                        return done("wdg_fno_gemm");
+                if (cudaMemset2DAsync(C + b * strideC, sizeof(float) * ldc, 0, sizeof(float) * N, M, st(stream)) !=
+                    cudaSuccess)
+                    return done("wdg_fno_gemm");
         }
-        dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, batch * nsplit);
-        if (grid.y > 65535 || grid.z > 65535)
+        if ((M + TM - 1) / TM > 65535 || (long long)batch * nsplit > 65535)
             return wdg::fail(WDG_ERR_ARG, "wdg_fno_gemm: problem too large for one launch");
-        gemm_bf16_kernel<<<grid, 128, 0, st(stream)>>>(g);
+        gemm_run<EPI_STORE>(g, transA, transB, batch * nsplit, st(stream));
         return done("wdg_fno_gemm");
+    }
+
+    // batch products op(A[b]) op(B[b]) with an epilogue instead of alpha and beta: mode 1 v = acc + bias[row],
+    // out = v, y = BF16 act(v); mode 2 v = acc gelu'(z) (act) or acc, out = v, y = BF16 v; out and y nullable,
+    // out, z and y of C's shape (M, ldc) per batch
+    int wdg_fno_gemm_act(const void *A, const void *B, float *out, int M, int N, int K, long long lda, long long ldb,
+                         long long ldc, long long strideA, long long strideB, long long strideC, int batch, int transA,
+                         int transB, int mode, const float *bias, const float *z, void *y, int act, void *stream)
+    {
+        if (!A || !B || (!out && !y) || M < 1 || N < 1 || K < 1 || batch < 1 || batch > 65535 ||
+            (M + TM - 1) / TM > 65535 || (mode != EPI_BIAS_ACT && mode != EPI_ACT_BWD) || (mode == EPI_BIAS_ACT && !bias) ||
+            (mode == EPI_ACT_BWD && act && !z))
+            return wdg::fail(WDG_ERR_ARG, "wdg_fno_gemm_act: bad arguments");
+        GemmArgs g{};
+        g.A = static_cast<const bf16 *>(A);
+        g.B = static_cast<const bf16 *>(B);
+        g.C = out;
+        g.M = M;
+        g.N = N;
+        g.K = K;
+        g.lda = lda;
+        g.ldb = ldb;
+        g.ldc = ldc;
+        g.sA = strideA;
+        g.sB = strideB;
+        g.sC = strideC;
+        g.alpha = 1.f;
+        g.ksplit = ((K + TK - 1) / TK) * TK;
+        g.e.bias = bias;
+        g.e.z = z;
+        g.e.y = static_cast<bf16 *>(y);
+        g.e.act = act;
+        if (mode == EPI_BIAS_ACT)
+            gemm_run<EPI_BIAS_ACT>(g, transA, transB, batch, st(stream));
+        else
+            gemm_run<EPI_ACT_BWD>(g, transA, transB, batch, st(stream));
+        return done("wdg_fno_gemm_act");
+    }
+
+    // a Fourier layer's output, forward (back = 0) or backward; see layer_kernel.  C and K1 multiples of 8, at
+    // most 32; G a multiple of 8; every array 16-byte aligned
+    int wdg_fno_layer(const void *U, const void *X, const void *W, const void *V, const float *bias, const float *z,
+                      float *out, void *y, int B, int C, int K1, int G, int act, int back, void *stream)
+    {
+        if (!U || !X || !W || !V || (!out && !y) || B < 1 || B > 65535 || C < 8 || C > 32 || C % 8 || K1 < 8 || K1 > 32 ||
+            K1 % 8 || G < 8 || G > 65535 || G % 8 || (back ? (act && !z) : !bias))
+            return wdg::fail(WDG_ERR_ARG, "wdg_fno_layer: bad arguments");
+        if ((((uintptr_t)U | (uintptr_t)X | (uintptr_t)W | (uintptr_t)V | (uintptr_t)out | (uintptr_t)y) & 15u) != 0)
+            return wdg::fail(WDG_ERR_ARG, "wdg_fno_layer: arrays must be 16-byte aligned");
+        LayerArgs g{};
+        g.U = static_cast<const bf16 *>(U);
+        g.X = static_cast<const bf16 *>(X);
+        g.W = static_cast<const bf16 *>(W);
+        g.V = static_cast<const bf16 *>(V);
+        g.C = out;
+        g.Cn = C;
+        g.K1 = K1;
+        g.G = G;
+        g.e.bias = bias;
+        g.e.z = z;
+        g.e.y = static_cast<bf16 *>(y);
+        g.e.act = act;
+        const dim3 grid((G + 127) / 128, G, B);
+        if (back)
+            layer_kernel<true><<<grid, 128, 0, st(stream)>>>(g);
+        else
+            layer_kernel<false><<<grid, 128, 0, st(stream)>>>(g);
+        return done("wdg_fno_layer");
     }
 
     int wdg_fno_dft_y(const float *in, float *out, void *out_bf16, const float *cos_tab, const float *sin_tab, int BC,
@@ -579,12 +941,28 @@ extern "C"
         {
             if (!out)
                 return wdg::fail(WDG_ERR_ARG, "wdg_fno_dft_y: the forward transform writes FP32");
-            dft_y_fwd_kernel<<<blocks((long long)BC * K * KX), 256, 0, st(stream)>>>(in, out, cos_tab, sin_tab, BC, G, K,
-                                                                                    KX, sign);
+            const bool tab = sizeof(float2) * ((size_t)G + KX) <= kDftSmem;
+            const size_t left = kDftSmem / sizeof(float2) - (tab ? G : 0);
+            const int chunk = (int)std::min<size_t>(kDftRows, left / KX);
+            if (chunk < 1)
+                return wdg::fail(WDG_ERR_ARG, "wdg_fno_dft_y: more than 12288 modes along x");
+            const size_t smem = sizeof(float2) * ((tab ? (size_t)G : 0) + (size_t)chunk * KX);
+            auto kern = tab ? dft_y_fwd_kernel<true> : dft_y_fwd_kernel<false>;
+            if (smem > 48 * 1024)
+                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDftSmem);
+            kern<<<dim3(BC, (K / 2 * KX + kDftThreads - 1) / kDftThreads), kDftThreads, smem, st(stream)>>>(
+                in, out, cos_tab, sin_tab, G, K, KX, sign, chunk);
         }
         else
-            dft_y_inv_kernel<<<blocks((long long)BC * G * KX), 256, 0, st(stream)>>>(
-                in, out, static_cast<bf16 *>(out_bf16), cos_tab, sin_tab, BC, G, K, KX, sign);
+        {
+            const size_t want = sizeof(float2) * ((size_t)G + (size_t)K * KX);
+            const bool tab = want <= kDftSmem;
+            auto kern = tab ? dft_y_inv_kernel<true> : dft_y_inv_kernel<false>;
+            if (tab && want > 48 * 1024)
+                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDftSmem);
+            kern<<<dim3(BC, (G + kInvRows - 1) / kInvRows), kDftThreads, tab ? want : 0, st(stream)>>>(
+                in, out, static_cast<bf16 *>(out_bf16), cos_tab, sin_tab, G, K, KX, sign);
+        }
         return done("wdg_fno_dft_y");
     }
 

@@ -98,6 +98,23 @@ class FNO:
         check(_fn("wdg_fno_gemm")(_p(A), _p(B), _p(Cm), M, N, K, lda, ldb, ldc, sA, sB, sC, batch, tA, tB,
                                   float(alpha), float(beta), int(ksplit), self._s()), "fno gemm")
 
+    def _gemm_act(self, A, B, out, y, mode, M, N, K, lda, ldb, ldc, sA, sB, sC, batch, tA=0, tB=0, bias=None, z=None,
+                  act=0):
+        """op(A) op(B) per sample with what follows it in the same pass: mode 1 out = acc + bias and
+        y = BF16 act(out); mode 2 out = acc gelu'(z) (act) or acc and y its BF16 copy; out, y may be None."""
+        check(_fn("wdg_fno_gemm_act")(_p(A), _p(B), _p(out), M, N, K, lda, ldb, ldc, sA, sB, sC, batch, tA, tB, mode,
+                                      _p(bias), _p(z), _p(y), act, self._s()), "fno gemm")
+
+    def _layer(self, U, X, W, V, out, y, B, act, back, bias=None, z=None):
+        """Both GEMMs of a Fourier layer's output (W V + U X, backward W^T V + U X^T) and what follows them."""
+        check(_fn("wdg_fno_layer")(_p(U), _p(X), _p(W), _p(V), _p(bias), _p(z), _p(out), _p(y), B, self.Cw, 2 * self.KX,
+                                   self.G, act, back, self._s()), "fno layer")
+
+    def _fused(self):
+        """Whether the layer kernel's tile (32 channels, 32 retained modes, whole 16-byte pieces) takes this network."""
+        return (self.Cw % 8 == 0 and 8 <= self.Cw <= 32 and self.KX % 4 == 0 and 4 <= self.KX <= 16 and self.G % 8 == 0
+                and self.G <= 65535)
+
     def _bf16(self, x):
         y = self.torch.empty(x.shape, dtype=self.torch.bfloat16, device=self.dev)
         check(_fn("wdg_fno_to_bf16")(_p(x), _p(y), x.numel(), self._s()))
@@ -115,10 +132,10 @@ class FNO:
         P = G * G
         tape = {"B": B}
         inb = self._bf16(inp)
-        z = t.empty((B, Cw, P), dtype=t.float32, device=self.dev)
-        self._gemm(self._bf["P_w"], inb, z, Cw, P, self.Cin, self.Cin, P, P, 0, self.Cin * P, Cw * P, B)
+        fused = self._fused()
         v = t.empty((B, Cw, P), dtype=t.bfloat16, device=self.dev)
-        check(_fn("wdg_fno_bias_act")(_p(z), _p(self.params["P_b"]), _p(v), None, B, Cw, P, 0, self._s()))
+        self._gemm_act(self._bf["P_w"], inb, None, v, 1, Cw, P, self.Cin, self.Cin, P, P, 0, self.Cin * P, Cw * P, B,
+                       bias=self.params["P_b"])
         if keep:
             tape["in"] = inb
         for l in range(self.L):
@@ -133,21 +150,25 @@ class FNO:
             uy = t.empty((B * Cw * G, 2 * KX), dtype=t.bfloat16, device=self.dev)
             check(_fn("wdg_fno_dft_y")(_p(wh), None, _p(uy), _p(self.cos_t), _p(self.sin_t), B * Cw, G, KY, KX, 1,
                                        1.0, self._s()))
-            zl = t.empty((B, Cw, P), dtype=t.float32, device=self.dev)
-            self._gemm(uy, self.Ix, zl, B * Cw * G, G, 2 * KX, 2 * KX, G, G)
-            self._gemm(self._bf[f"W{l}"], v, zl, Cw, P, Cw, Cw, P, P, 0, Cw * P, Cw * P, B, beta=1.0)
+            # the pre-activation is needed where its derivative is: not after the last layer
+            zl = t.empty((B, Cw, P), dtype=t.float32, device=self.dev) if not fused or (keep and act) else None
             vn = t.empty((B, Cw, P), dtype=t.bfloat16, device=self.dev)
-            check(_fn("wdg_fno_bias_act")(_p(zl), _p(self.params[f"b{l}"]), _p(vn), None, B, Cw, P, act, self._s()))
+            if fused:
+                self._layer(uy, self.Ix, self._bf[f"W{l}"], v, zl, vn, B, act, 0, bias=self.params[f"b{l}"])
+            else:
+                self._gemm(uy, self.Ix, zl, B * Cw * G, G, 2 * KX, 2 * KX, G, G)
+                self._gemm(self._bf[f"W{l}"], v, zl, Cw, P, Cw, Cw, P, P, 0, Cw * P, Cw * P, B, beta=1.0)
+                check(_fn("wdg_fno_bias_act")(_p(zl), _p(self.params[f"b{l}"]), _p(vn), None, B, Cw, P, act, self._s()))
             if keep:
                 tape[f"v{l}"], tape[f"z{l}"], tape[f"vh{l}"] = v, zl, vh
             v = vn
-        zq = t.empty((B, H, P), dtype=t.float32, device=self.dev)
-        self._gemm(self._bf["Q1_w"], v, zq, H, P, Cw, Cw, P, P, 0, Cw * P, H * P, B)
+        zq = t.empty((B, H, P), dtype=t.float32, device=self.dev) if keep else None
         hb = t.empty((B, H, P), dtype=t.bfloat16, device=self.dev)
-        check(_fn("wdg_fno_bias_act")(_p(zq), _p(self.params["Q1_b"]), _p(hb), None, B, H, P, 1, self._s()))
+        self._gemm_act(self._bf["Q1_w"], v, zq, hb, 1, H, P, Cw, Cw, P, P, 0, Cw * P, H * P, B, bias=self.params["Q1_b"],
+                       act=1)
         y = t.empty((B, self.Cout, P), dtype=t.float32, device=self.dev)
-        self._gemm(self._bf["Q2_w"], hb, y, self.Cout, P, H, H, P, P, 0, H * P, self.Cout * P, B)
-        check(_fn("wdg_fno_bias_act")(_p(y), _p(self.params["Q2_b"]), None, None, B, self.Cout, P, 0, self._s()))
+        self._gemm_act(self._bf["Q2_w"], hb, y, None, 1, self.Cout, P, H, H, P, P, 0, H * P, self.Cout * P, B,
+                       bias=self.params["Q2_b"])
         if keep:
             tape["v_last"], tape["zq"], tape["hb"] = v, zq, hb
             self.tape = tape
@@ -168,25 +189,21 @@ class FNO:
         # dQ2 = sum_b dy[b] hb[b]^T
         self._gemm(dyb, tp["hb"], gr["Q2_w"], self.Cout, H, P, P, P, H, self.Cout * P, H * P, 0, B, 0, 1,
                    beta=0.0, ksplit=ks)
-        dh = t.empty((B, H, P), dtype=t.float32, device=self.dev)
-        self._gemm(self._bf["Q2_w"], dyb, dh, H, P, self.Cout, H, P, P, 0, self.Cout * P, H * P, B, tA=1)
-        dzq = t.empty_like(dh)
+        dzq = t.empty((B, H, P), dtype=t.float32, device=self.dev)
         dzqb = t.empty((B, H, P), dtype=t.bfloat16, device=self.dev)
-        check(_fn("wdg_fno_act_bwd")(_p(dh), _p(tp["zq"]), _p(dzq), _p(dzqb), dh.numel(), 1, self._s()))
+        self._gemm_act(self._bf["Q2_w"], dyb, dzq, dzqb, 2, H, P, self.Cout, H, P, P, 0, self.Cout * P, H * P, B, tA=1,
+                       z=tp["zq"], act=1)
         check(_fn("wdg_fno_bias_grad")(_p(dzq), _p(gr["Q1_b"]), B, H, P, 0, self._s()))
         self._gemm(dzqb, tp["v_last"], gr["Q1_w"], H, Cw, P, P, P, Cw, H * P, Cw * P, 0, B, 0, 1, ksplit=ks)
-        dv = t.empty((B, Cw, P), dtype=t.float32, device=self.dev)
-        self._gemm(self._bf["Q1_w"], dzqb, dv, Cw, P, H, Cw, P, P, 0, H * P, Cw * P, B, tA=1)
+        fused = self._fused()
+        # dz, dzb: the gradient at the current layer's pre-activation (the last layer has no activation)
+        dz = t.empty((B, Cw, P), dtype=t.float32, device=self.dev)
+        dzb = t.empty((B, Cw, P), dtype=t.bfloat16, device=self.dev)
+        self._gemm_act(self._bf["Q1_w"], dzqb, dz, dzb, 2, Cw, P, H, Cw, P, P, 0, H * P, Cw * P, B, tA=1)
         for l in reversed(range(self.L)):
-            act = 1 if l < self.L - 1 else 0
-            v, zl, vh = tp[f"v{l}"], tp[f"z{l}"], tp[f"vh{l}"]
-            dz = t.empty_like(dv)
-            dzb = t.empty((B, Cw, P), dtype=t.bfloat16, device=self.dev)
-            check(_fn("wdg_fno_act_bwd")(_p(dv), _p(zl), _p(dz), _p(dzb), dv.numel(), act, self._s()))
+            v, vh = tp[f"v{l}"], tp[f"vh{l}"]
             check(_fn("wdg_fno_bias_grad")(_p(dz), _p(gr[f"b{l}"]), B, Cw, P, 0, self._s()))
             self._gemm(dzb, v, gr[f"W{l}"], Cw, Cw, P, P, P, Cw, Cw * P, Cw * P, 0, B, 0, 1, ksplit=ks)
-            dvp = t.empty((B, Cw, P), dtype=t.float32, device=self.dev)
-            self._gemm(self._bf[f"W{l}"], dzb, dvp, Cw, P, Cw, Cw, P, P, 0, Cw * P, Cw * P, B, tA=1)
             # spectral branch, adjoints in reverse order
             duy = t.empty((B * Cw * G, 2 * KX), dtype=t.float32, device=self.dev)
             self._gemm(dzb, self.Ix, duy, B * Cw * G, 2 * KX, G, G, G, 2 * KX, tB=1)
@@ -199,12 +216,19 @@ class FNO:
             dvxb = t.empty((B * Cw * G, 2 * KX), dtype=t.bfloat16, device=self.dev)
             check(_fn("wdg_fno_dft_y")(_p(dvh), None, _p(dvxb), _p(self.cos_t), _p(self.sin_t), B * Cw, G, KY, KX, 1,
                                        1.0, self._s()))
-            self._gemm(dvxb, self.Ex, dvp, B * Cw * G, G, 2 * KX, 2 * KX, 2 * KX, G, tB=1, beta=1.0)
-            dv = dvp
-        # lift: v0 = P_w in + P_b (no activation)
-        check(_fn("wdg_fno_bias_grad")(_p(dv), _p(gr["P_b"]), B, Cw, P, 0, self._s()))
-        dvb = self._bf16(dv)
-        self._gemm(dvb, tp["in"], gr["P_w"], Cw, self.Cin, P, P, P, self.Cin, Cw * P, self.Cin * P, 0, B, 0, 1,
+            # to the layer below through its activation (the lift v0 = P_w in + P_b has none)
+            act = 1 if l > 0 else 0
+            below = tp[f"z{l - 1}"] if act else None
+            dz, dzn = t.empty_like(dz), t.empty_like(dzb)
+            if fused:
+                self._layer(dvxb, self.Ex, self._bf[f"W{l}"], dzb, dz, dzn, B, act, 1, z=below)
+            else:
+                self._gemm(self._bf[f"W{l}"], dzb, dz, Cw, P, Cw, Cw, P, P, 0, Cw * P, Cw * P, B, tA=1)
+                self._gemm(dvxb, self.Ex, dz, B * Cw * G, G, 2 * KX, 2 * KX, 2 * KX, G, tB=1, beta=1.0)
+                check(_fn("wdg_fno_act_bwd")(_p(dz), _p(below), _p(dz), _p(dzn), dz.numel(), act, self._s()))
+            dzb = dzn
+        check(_fn("wdg_fno_bias_grad")(_p(dz), _p(gr["P_b"]), B, Cw, P, 0, self._s()))
+        self._gemm(dzb, tp["in"], gr["P_w"], Cw, self.Cin, P, P, P, self.Cin, Cw * P, self.Cin * P, 0, B, 0, 1,
                    ksplit=ks)
 
     def mse(self, y, target):
@@ -283,7 +307,7 @@ def step_profile(grid: int = 512, width: int = 32, modes: int = 16, layers: int 
     """Time one training step (forward, MSE, backward, Adam) and one prediction after `warmup`
     rounds of both, on seeded inputs, and list every GEMM of the timed pair in launch order with
     its shape and algorithmic bytes (BF16 operands read once; the FP32 result written, and read
-    again where beta = 1 or split-K accumulates).  The command to run under a launch-list
+    again where beta = 1 or split-K accumulates; what the epilogues read and write).  The command to run under a launch-list
     profiler: python -m wavedg_b200.fno --step-profile."""
     import torch
 
@@ -301,7 +325,24 @@ def step_profile(grid: int = 512, width: int = 32, modes: int = 16, layers: int 
                         flops=2.0 * M * N * K * batch))
         return gemm(A, B, Cm, M, N, K, lda, ldb, ldc, sA, sB, sC, batch, tA, tB, alpha, beta, ksplit)
 
-    net._gemm = logged
+    def entry(M, N, K, batch, out, out_bf16, extra, **kw):
+        log.append(dict(M=M, N=N, K=K, batch=batch, bytes=batch * (2 * (M * K + K * N) + M * N * (4 * out + 2 * out_bf16))
+                        + extra, flops=2.0 * M * N * K * batch, **kw))
+
+    gemm_act, layer = net._gemm_act, net._layer
+
+    def logged_act(A, B, out, y, mode, M, N, K, lda, ldb, ldc, sA, sB, sC, batch, **kw):
+        entry(M, N, K, batch, out is not None, y is not None, 4 * batch * M * N * (kw.get("z") is not None),
+              epilogue=("", "bias_act", "act_bwd")[mode], tA=kw.get("tA", 0))
+        return gemm_act(A, B, out, y, mode, M, N, K, lda, ldb, ldc, sA, sB, sC, batch, **kw)
+
+    def logged_layer(U, X, W, V, out, y, B, act, back, **kw):
+        entry(net.Cw, grid * grid, net.Cw, B, out is not None, True, 4 * net.Cw * B * grid * grid * (kw.get("z") is not None)
+              + 4 * net.Cw * B * grid * net.KX, epilogue="layer", back=back)
+        log[-1]["flops"] += 4.0 * net.Cw * B * grid * grid * net.KX
+        return layer(U, X, W, V, out, y, B, act, back, **kw)
+
+    net._gemm, net._gemm_act, net._layer = logged, logged_act, logged_layer
 
     def train_step():
         x = inputs(grid, rng.uniform(-0.5, 0.5, (train_batch, 2)), 0.05, 1.0)

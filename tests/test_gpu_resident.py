@@ -60,6 +60,39 @@ def test_captured(gpu_lib, precision):
     assert np.array_equal(a.download(), b.download())
 
 
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_batch(gpu_lib, precision):
+    """Batched solves as resident periods against the streaming launches (an explicit launch shape): uneven
+    meshes, degrees and frequencies, more least shares than SMs, cold, warm and with a known |pi0|."""
+    import wavedg_b200 as W
+    from wavedg_b200.dg import WaveHoltzBatch
+
+    rng = np.random.default_rng(11)
+    shapes = [(9, 4), (31, 5), (8, 7), (5, 2), (24, 9), (40, 3), (1, 4), (16, 6)]
+    meshes = [W.Mesh2D.uniform_rect(m, -1.0, 1.0, m, -1.0, 1.0) for m, _ in shapes]
+    omegas = rng.uniform(2.0, 8.0, len(shapes))
+    F = [rng.standard_normal(3 * m * m * n * n) / m for m, n in shapes]
+    W0 = [rng.standard_normal(f.size) for f in F]
+    warm = [0, 1, 0, 1, 1, 0, 1, 0]
+    got = []
+    for explicit in (False, True):
+        systems = [W.WaveSystem(mesh, n, None, precision=precision) for mesh, (_, n) in zip(meshes, shapes)]
+        systems[5].set_max_ctas(4)
+        b = WaveHoltzBatch(systems, omegas)
+        if explicit:
+            b.set_launch(1, 2)
+        runs = []
+        for kw in (dict(maxit=3), dict(maxit=2, warm=warm), dict(maxit=2, warm=warm, pi0_norm=np.where(warm, 2.0, 0.0))):
+            w, it, res, st = b.solve(F, tol=1e-12, W=[x.copy() for x in W0], **kw)
+            runs.append((w, it.copy(), res.copy(), st.copy(), b.pi0_norm.copy()))
+        got.append(runs)
+    for (wa, ia, ra, sa, pa), (wb, ib, rb, sb, pb) in zip(*got):
+        assert np.array_equal(ia, ib) and np.array_equal(sa, sb)
+        assert np.allclose(ra, rb, rtol=1e-9, atol=0) and np.allclose(pa, pb, rtol=1e-12, atol=0)
+        for x, y in zip(wa, wb):
+            assert np.linalg.norm(x - y) <= 1e-12 * np.linalg.norm(y)
+
+
 @pytest.mark.parametrize("n", [3, 5, 8])
 def test_waveholtz_period(gpu_lib, n):
     import wavedg_b200 as W

@@ -132,7 +132,7 @@ namespace wdg
         template <int N, int NV, class M>
         struct LineShape
         {
-            static constexpr int NN = N * N, ND = NV * NN, W = NV % 2 == 0 ? 2 : 1;
+            static constexpr int NN = N * N, ND = NV * NN;
             static constexpr int AB = M::LINEAR ? 4 * NV * NV : 0; // |n.A| of the four sides
             // elements per warp: a lane per line, less where the staging of many variables would leave
             // fewer than five warps on an SM

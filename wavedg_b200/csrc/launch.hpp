@@ -177,6 +177,12 @@ namespace wdg
     template <typename Real>
     cudaError_t whb_occupancy(int n, bool last, size_t smem, int *grid); // last: the fifth stage's kernel
     cudaError_t launch_whb_step_end(WhbState *state, int nsolves, cudaStream_t s);
+    // periods as resident launches: a solve's tables (5 nt and nt values), and the end of a period
+    constexpr int kWhbEndBlocks = 256; // partial sums: 2 per block
+    cudaError_t launch_whb_tables(double omega, double dt, int nt, double *fscale, double *cfilter, cudaStream_t s);
+    template <typename Real>
+    cudaError_t launch_whb_period_end(WhbState *state, Real *u, double *acc, double *W, double c0, long long n, double *part,
+                                      cudaStream_t s);
 
     // fused stage: RK = true for the time-stepping epilogue
     template <typename Real>

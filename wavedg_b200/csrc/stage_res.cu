@@ -118,7 +118,16 @@ namespace wdg
                 }
             return b;
         }
-        // a warp's scratch: the forcing, then the column sums of a group
+        // FP32 stepping adds the forcing where the streaming kernel does, to the row's finished sums, so that
+        // batches of either kind give the same bits; its values then need a place of their own.  FP64 adds it
+        // to the column's sums and lets it share the scratch: that place would cost a warp or two.
+        template <typename Real>
+        constexpr bool kLateForcing = sizeof(Real) == 4;
+        __host__ __device__ constexpr int res_forcing(int n, int real)
+        {
+            return real == 4 ? ((32 / n) * 3 * n * n * real + 15) & ~15 : 0;
+        }
+        // a warp's scratch: the forcing (FP64), then the column sums of a group
         __host__ __device__ constexpr int res_scratch(int n, int real)
         {
             return ((32 / n) * res_strides(n).el * real + 15) & ~15;
@@ -164,7 +173,10 @@ namespace wdg
             unsigned char *groups = rsm;
             constexpr int kScratch = res_scratch(N, sizeof(Real));
             constexpr ResStride RS = res_strides(N);
-            Real *Rc = reinterpret_cast<Real *>(groups + (size_t)most * L.bytes + (size_t)warp * kScratch);
+            constexpr bool LATE = kLateForcing<Real>;
+            const int scratch = kScratch + (a.F ? res_forcing(N, sizeof(Real)) : 0);
+            Real *Rc = reinterpret_cast<Real *>(groups + (size_t)most * L.bytes + (size_t)warp * scratch);
+            Real *Fc = LATE ? Rc + kScratch / (int)sizeof(Real) : Rc; // the group's forcing
             const int le = lane / N, ln = lane - le * N;
             const bool lane_on = lane < EW * N;
             const Real xm = lane_on ? Tab<Real>::x(N, ln) : Real(0), wm = lane_on ? Tab<Real>::w(N, ln) : Real(0);
@@ -328,7 +340,7 @@ namespace wdg
                     if (a.F)
                     {
                         for (int o = lane; o < ne * ND; o += 32)
-                            cp_async<sizeof(Real)>(Rc + o, a.F + (size_t)e0 * ND + o);
+                            cp_async<sizeof(Real)>(Fc + o, a.F + (size_t)e0 * ND + o);
                         cp_async_commit();
                     }
                     // column pass, volume (and forcing): needs nothing from the neighbours
@@ -347,7 +359,7 @@ namespace wdg
                             own2[d] = Ue[3 * (ln + N * (N - 1)) + d];
                         }
                     }
-                    if (a.F)
+                    if (!LATE && a.F)
                     {
                         cp_async_wait<0>();
                         __syncwarp();
@@ -356,7 +368,7 @@ namespace wdg
 #pragma unroll
                             for (int j = 0; j < N; ++j)
                             {
-                                const Real *o = Rc + ae * ND + 3 * (ln + N * j);
+                                const Real *o = Fc + ae * ND + 3 * (ln + N * j);
                                 sp[j] += fs * o[0];
                                 su[j] += fs * o[1];
                                 sv[j] += fs * o[2];
@@ -405,6 +417,8 @@ namespace wdg
                             o[2] = sv[j];
                         }
                     }
+                    if (LATE)
+                        cp_async_wait<0>();
                     __syncwarp();
                     if (act)
                     {
@@ -429,6 +443,13 @@ namespace wdg
                             const Real *cr = rc + RS.row * j + 3 * i;
                             const Real mv = Mi[N * j + i];
                             Real r0 = ap[i] + cr[0], r1 = au[i] + cr[1], r2 = av[i] + cr[2];
+                            if (LATE && a.F)
+                            {
+                                const Real *f = Fc + ae * ND + 3 * (i + N * j);
+                                r0 += fs * f[0];
+                                r1 += fs * f[1];
+                                r2 += fs * f[2];
+                            }
                             r0 *= mv;
                             r1 *= mv;
                             r2 *= mv;
@@ -452,10 +473,11 @@ namespace wdg
                         st_release(a.flags + (size_t)kFlagStride * g, a.base + stg + 2);
                     if (a.acc && st == 4)
                     {
+                        // this warp alone writes these; a reduction leaves the addition to L2
                         const Real *U = reinterpret_cast<const Real *>(gb + L.u);
                         const double cf = __ldg(a.cfilter + step);
                         for (int o = lane; o < ne * ND; o += 32)
-                            a.acc[(size_t)e0 * ND + o] += cf * (double)U[o];
+                            atomicAdd(a.acc + (size_t)e0 * ND + o, cf * (double)U[o]);
                     }
                 }
                 if (++st == 5)
@@ -504,7 +526,7 @@ namespace wdg
 
     int upload_res_tables(int device) { return upload_basis_tab(device); }
 
-    ResPlan res_plan(int n, bool fp32, int nel, int sms, int max_ctas)
+    ResPlan res_plan(int n, bool fp32, int nel, int sms, int max_ctas, bool forced)
     {
         ResPlan p;
         p.ngroups = (nel + 32 / n - 1) / (32 / n);
@@ -515,7 +537,7 @@ namespace wdg
             return p;
         const int most = (p.ngroups + p.ctas - 1) / p.ctas;
         const size_t gb = (size_t)(fp32 ? res_layout<float>(n).bytes : res_layout<double>(n).bytes);
-        const size_t sc = (size_t)res_scratch(n, fp32 ? 4 : 8);
+        const size_t sc = (size_t)res_scratch(n, fp32 ? 4 : 8) + (forced ? res_forcing(n, fp32 ? 4 : 8) : 0);
         // as few rounds of groups per warp as twelve warps allow, the warps evened out over them; fewer
         // warps where their scratch is what does not fit
         for (int rounds = (most + kResMaxWarps - 1) / kResMaxWarps; rounds <= most && rounds <= 4 * kResMaxWarps; ++rounds)
@@ -533,13 +555,13 @@ namespace wdg
     }
 
     template <typename Real>
-    int res_rk4(wdg_wave *w, const ResPlan &p, Real *A, double dt, int nsteps, const RKExtras &x, bool &ran)
+    int res_rk4(wdg_wave *w, const ResPlan &p, Real *A, double dt, int nsteps, const RKExtras &x, bool &ran, cudaStream_t stream)
     {
         ran = false;
         ResArgs<Real> a{};
         a.A = A;
-        a.T[0] = static_cast<Real *>(w->d_trace);
-        a.T[1] = a.T[0] + 16 * (size_t)w->n * w->nel;
+        a.T[0] = static_cast<Real *>(w->d_trace[0]);
+        a.T[1] = static_cast<Real *>(w->d_trace[1]);
         a.corners = w->d_corners;
         a.fbase = w->d_fbase;
         a.fcode = w->d_fcode;
@@ -557,7 +579,7 @@ namespace wdg
         a.acc = x.acc;
         a.wait_ns = w->wait_ns;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        WDG_CUDA(cudaStreamIsCapturing(w->stream, &cap));
+        WDG_CUDA(cudaStreamIsCapturing(stream, &cap));
         constexpr int kSteps = 4096; // per launch
         for (int s0 = 0; s0 < nsteps; s0 += kSteps)
         {
@@ -567,19 +589,19 @@ namespace wdg
             // A replayed graph repeats this launch with the same base, so its flags start below it again;
             // launches outside a graph count on from a base no replay has reached
             if (cap == cudaStreamCaptureStatusActive)
-                WDG_CUDA(cudaMemsetAsync(w->d_flags, 0, sizeof(unsigned long long) * kFlagStride * p.ngroups, w->stream));
+                WDG_CUDA(cudaMemsetAsync(w->d_flags, 0, sizeof(unsigned long long) * kFlagStride * p.ngroups, stream));
             a.base = w->flag_base;
             cudaError_t e = cudaErrorInvalidValue;
             switch (w->n)
             {
-            case 2: e = launch_n<2, Real>(a, p, w->stream); break;
-            case 3: e = launch_n<3, Real>(a, p, w->stream); break;
-            case 4: e = launch_n<4, Real>(a, p, w->stream); break;
-            case 5: e = launch_n<5, Real>(a, p, w->stream); break;
-            case 6: e = launch_n<6, Real>(a, p, w->stream); break;
-            case 7: e = launch_n<7, Real>(a, p, w->stream); break;
-            case 8: e = launch_n<8, Real>(a, p, w->stream); break;
-            case 9: e = launch_n<9, Real>(a, p, w->stream); break;
+            case 2: e = launch_n<2, Real>(a, p, stream); break;
+            case 3: e = launch_n<3, Real>(a, p, stream); break;
+            case 4: e = launch_n<4, Real>(a, p, stream); break;
+            case 5: e = launch_n<5, Real>(a, p, stream); break;
+            case 6: e = launch_n<6, Real>(a, p, stream); break;
+            case 7: e = launch_n<7, Real>(a, p, stream); break;
+            case 8: e = launch_n<8, Real>(a, p, stream); break;
+            case 9: e = launch_n<9, Real>(a, p, stream); break;
             default: break;
             }
             if (e == cudaErrorCooperativeLaunchTooLarge && s0 == 0)
@@ -594,8 +616,8 @@ namespace wdg
         }
         return WDG_OK;
     }
-    template int res_rk4<double>(wdg_wave *, const ResPlan &, double *, double, int, const RKExtras &, bool &);
-    template int res_rk4<float>(wdg_wave *, const ResPlan &, float *, double, int, const RKExtras &, bool &);
+    template int res_rk4<double>(wdg_wave *, const ResPlan &, double *, double, int, const RKExtras &, bool &, cudaStream_t);
+    template int res_rk4<float>(wdg_wave *, const ResPlan &, float *, double, int, const RKExtras &, bool &, cudaStream_t);
 
     size_t res_flag_count(int n, int nel) { return (size_t)kFlagStride * ((nel + 32 / n - 1) / (32 / n)); }
 } // namespace wdg

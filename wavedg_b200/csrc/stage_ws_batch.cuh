@@ -214,9 +214,47 @@ namespace wdg
         }
     }
 
+    // end of a solve's period with the sums d = sum (W' - W)^2 and nrm = sum W'^2: residual and status
+    // (examples/waveholtz2d.cpp:165-185: ||W - W_prev|| / ||pi0|| against tol, maxit)
+    __device__ __forceinline__ void whb_finish_period(WhbState &P, double d, double nrm)
+    {
+        if (P.phase == 0)
+        {
+            P.pi0sq = nrm;
+            P.phase = 1;
+            return;
+        }
+        if (P.iter == 0 && P.zero_start)
+            P.pi0sq = nrm; // the first period from zero is pi0 itself
+        const double scale = P.pi0sq > 0.0 ? sqrt(P.pi0sq) : 1.0;
+        P.residual = sqrt(d) / scale;
+        P.iter += 1;
+        if (P.residual < P.best)
+        {
+            P.best = P.residual;
+            P.stall = 0;
+        }
+        else
+            P.stall += 1;
+        if (P.residual < P.tol)
+        {
+            P.active = 0;
+            P.status = 0;
+        }
+        else if (P.iter >= P.maxit)
+        {
+            P.active = 0;
+            P.status = 1;
+        }
+        else if (P.stall_limit > 0 && P.stall >= P.stall_limit)
+        {
+            P.active = 0;
+            P.status = 2;
+        }
+    }
+
     // After the fifth stage of every step: advance each running solve's step counter; at the
-    // end of a period reduce its partial sums in a fixed order and update residual and status
-    // (examples/waveholtz2d.cpp:165-185: ||W - W_prev|| / ||pi0|| against tol, maxit).
+    // end of a period reduce its partial sums in a fixed order and update residual and status.
     __global__ void whb_step_end_kernel(WhbState *state, int nsolves)
     {
         const int s = blockIdx.x;
@@ -255,40 +293,109 @@ namespace wdg
         if (threadIdx.x != 0)
             return;
         P.k = 0;
-        if (P.phase == 0)
-        {
-            P.pi0sq = sn[0];
-            P.phase = 1;
+        whb_finish_period(P, sd[0], sn[0]);
+    }
+
+    // ---- periods as resident launches (one solve per launch)
+    // the forcing's scales and the filter's weights of every step of a solve's period, as whb_stage_kernel
+    // forms them
+    __global__ void whb_tables_kernel(double omega, double dt, int nt, double *fscale, double *cfilter)
+    {
+        const int k = blockIdx.x * blockDim.x + threadIdx.x;
+        if (k >= nt)
             return;
-        }
-        if (P.iter == 0 && P.zero_start)
-            P.pi0sq = sn[0]; // the first period from zero is pi0 itself
-        const double scale = P.pi0sq > 0.0 ? sqrt(P.pi0sq) : 1.0;
-        P.residual = sqrt(sd[0]) / scale;
-        P.iter += 1;
-        if (P.residual < P.best)
+        for (int st = 0; st < 5; ++st)
         {
-            P.best = P.residual;
-            P.stall = 0;
+            const double ts = (k + c_rk4c[st]) * dt;
+            fscale[5 * k + st] = -sin(omega * ts) / omega;
         }
-        else
-            P.stall += 1;
-        if (P.residual < P.tol)
+        const double t1 = (k + 1) * dt;
+        cfilter[k] = ((k + 1 == nt) ? 0.5 : 1.0) * dt * (omega / M_PI * (cos(omega * t1) - 0.25));
+    }
+    // end of a period whose result is in acc: W <- acc (or, after the pi0 period of a warm start, W as it
+    // is), the state and the filter restart from it; per-block partial sums of (W' - W)^2 and acc^2
+    template <typename Real>
+    __global__ void whb_period_end_kernel(const WhbState *state, Real *u, double *acc, double *W, double c0, long long n,
+                                          double *part)
+    {
+        __shared__ double sd[256], sn[256];
+        const bool pi0 = state->phase == 0;
+        double d = 0.0, nrm = 0.0;
+        for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
         {
-            P.active = 0;
-            P.status = 0;
+            const double fin = acc[q], w = W[q];
+            nrm += fin * fin;
+            double w0 = w;
+            if (!pi0)
+            {
+                const double dw = fin - w;
+                d += dw * dw;
+                W[q] = fin;
+                w0 = fin;
+            }
+            acc[q] = c0 * w0;
+            u[q] = (Real)w0;
         }
-        else if (P.iter >= P.maxit)
+        sd[threadIdx.x] = d;
+        sn[threadIdx.x] = nrm;
+        __syncthreads();
+        for (int h = blockDim.x / 2; h > 0; h >>= 1)
         {
-            P.active = 0;
-            P.status = 1;
+            if ((int)threadIdx.x < h)
+            {
+                sd[threadIdx.x] += sd[threadIdx.x + h];
+                sn[threadIdx.x] += sn[threadIdx.x + h];
+            }
+            __syncthreads();
         }
-        else if (P.stall_limit > 0 && P.stall >= P.stall_limit)
+        if (threadIdx.x == 0)
         {
-            P.active = 0;
-            P.status = 2;
+            part[2 * blockIdx.x] = sd[0];
+            part[2 * blockIdx.x + 1] = sn[0];
         }
     }
+    __global__ void whb_period_sum_kernel(WhbState *state, const double *part, int blocks)
+    {
+        __shared__ double sd[256], sn[256];
+        double d = 0.0, nrm = 0.0;
+        for (int i = threadIdx.x; i < blocks; i += blockDim.x)
+        {
+            d += part[2 * i];
+            nrm += part[2 * i + 1];
+        }
+        sd[threadIdx.x] = d;
+        sn[threadIdx.x] = nrm;
+        __syncthreads();
+        for (int h = blockDim.x / 2; h > 0; h >>= 1)
+        {
+            if ((int)threadIdx.x < h)
+            {
+                sd[threadIdx.x] += sd[threadIdx.x + h];
+                sn[threadIdx.x] += sn[threadIdx.x + h];
+            }
+            __syncthreads();
+        }
+        if (threadIdx.x == 0)
+            whb_finish_period(*state, sd[0], sn[0]);
+    }
+    cudaError_t launch_whb_tables(double omega, double dt, int nt, double *fscale, double *cfilter, cudaStream_t s)
+    {
+        whb_tables_kernel<<<(nt + 127) / 128, 128, 0, s>>>(omega, dt, nt, fscale, cfilter);
+        return cudaGetLastError();
+    }
+    template <typename Real>
+    cudaError_t launch_whb_period_end(WhbState *state, Real *u, double *acc, double *W, double c0, long long n, double *part,
+                                      cudaStream_t s)
+    {
+        const int blocks = (int)std::min<long long>(kWhbEndBlocks, (n + 255) / 256);
+        whb_period_end_kernel<Real><<<blocks, 256, 0, s>>>(state, u, acc, W, c0, n, part);
+        whb_period_sum_kernel<<<1, 256, 0, s>>>(state, part, blocks);
+        return cudaGetLastError();
+    }
+    template cudaError_t launch_whb_period_end<double>(WhbState *, double *, double *, double *, double, long long, double *,
+                                                       cudaStream_t);
+    template cudaError_t launch_whb_period_end<float>(WhbState *, float *, double *, double *, double, long long, double *,
+                                                      cudaStream_t);
 
     int whb_smem_bytes(int n, int slot_bytes, int warp_scratch, int ring, bool fp32)
     {

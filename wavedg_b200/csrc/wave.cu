@@ -58,21 +58,54 @@ namespace wdg
         return WDG_OK;
     }
 
+    // what resident launches need beside the state, where the mesh fits: flags and the two trace buffers (two
+    // allocations: the driver carves those below a megabyte out of what it has)
+    int ensure_resident(wdg_wave *w)
+    {
+        if (w->d_flags || w->halo || !res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, 0, false).fits)
+            return WDG_OK;
+        const size_t flags = (sizeof(unsigned long long) * res_flag_count(w->n, w->nel) + 255) & ~size_t(255);
+        const size_t trace = w->real_size() * 16 * (size_t)w->n * w->nel;
+        unsigned char *p = nullptr, *q = nullptr;
+        cudaError_t e = cudaMalloc((void **)&p, flags + trace);
+        if (e == cudaSuccess)
+            e = cudaMalloc((void **)&q, trace);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(p, 0, flags, w->stream);
+        if (e != cudaSuccess)
+        {
+            if (p)
+                cudaFree(p);
+            if (q)
+                cudaFree(q);
+            return cuda_fail(e, "cudaMalloc(trace buffers)");
+        }
+        w->d_flags = reinterpret_cast<unsigned long long *>(p);
+        w->d_trace[0] = p + flags;
+        w->d_trace[1] = q;
+        return WDG_OK;
+    }
+
     // the three state buffers and the RK register, allocated on first use so
     // that operator-only handles (WaveEquation, WaveBC, MassMatrix drop-ins)
     // hold geometry only
+    static int ensure_state(wdg_wave *w, int k)
+    {
+        if (!w->d_state[k])
+        {
+            cudaError_t e = cudaMalloc(&w->d_state[k], w->real_size() * (size_t)(w->ndof + w->halo) + 64);
+            if (e != cudaSuccess)
+            {
+                w->d_state[k] = nullptr;
+                return cuda_fail(e, "cudaMalloc(state)");
+            }
+        }
+        return WDG_OK;
+    }
     int ensure_states(wdg_wave *w)
     {
         for (int k = 0; k < 3; ++k)
-            if (!w->d_state[k])
-            {
-                cudaError_t e = cudaMalloc(&w->d_state[k], w->real_size() * (size_t)(w->ndof + w->halo) + 64);
-                if (e != cudaSuccess)
-                {
-                    w->d_state[k] = nullptr;
-                    return cuda_fail(e, "cudaMalloc(state)");
-                }
-            }
+            WDG_TRY(ensure_state(w, k));
         if (!w->d_du)
         {
             cudaError_t e = cudaMalloc(&w->d_du, w->real_size() * (size_t)w->ndof + 64);
@@ -82,26 +115,18 @@ namespace wdg
                 return cuda_fail(e, "cudaMalloc(du)");
             }
         }
-        if (!w->d_flags && !w->halo && res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, 0).fits)
-        {
-            const size_t bytes = sizeof(unsigned long long) * res_flag_count(w->n, w->nel);
-            cudaError_t e = cudaMalloc(&w->d_trace, 2 * w->real_size() * 16 * (size_t)w->n * w->nel);
-            if (e == cudaSuccess)
-                e = cudaMalloc((void **)&w->d_flags, bytes);
-            if (e == cudaSuccess)
-                e = cudaMemset(w->d_flags, 0, bytes);
-            if (e != cudaSuccess)
-            {
-                if (w->d_trace)
-                    cudaFree(w->d_trace);
-                if (w->d_flags)
-                    cudaFree(w->d_flags);
-                w->d_trace = nullptr;
-                w->d_flags = nullptr;
-                return cuda_fail(e, "cudaMalloc(trace buffers)");
-            }
-        }
         return WDG_OK;
+    }
+    // what WaveHoltz periods need before one is captured: the rotation buffers and the register only where
+    // they will not be resident
+    int ensure_period(wdg_wave *w)
+    {
+        auto fits = [&](bool forced)
+        { return res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, w->max_ctas, forced).fits; };
+        if (w->family != 2 || w->explicit_launch || w->halo || !fits(true) || !fits(false))
+            return ensure_states(w);
+        WDG_TRY(ensure_state(w, 0));
+        return ensure_resident(w);
     }
 
     int check_device_error(wdg_wave *w)
@@ -149,22 +174,19 @@ namespace wdg
     template <typename Real>
     int rk4_run(wdg_wave *w, Real *A, double dt, double &t, int nsteps, const RKExtras &x)
     {
-        WDG_TRY(ensure_states(w));
-        Real *B = static_cast<Real *>(w->d_state[1]);
-        Real *Cb = static_cast<Real *>(w->d_state[2]);
-        Real *du = static_cast<Real *>(w->d_du);
-        if (A == B || A == Cb)
+        if (A && (A == w->d_state[1] || A == w->d_state[2]))
             return fail(WDG_ERR_ARG, "rk4: state buffer aliases the rotation buffers");
         // a mesh that fits the chip stays there for all steps (unless the caller chose a kernel, or the
         // skipped-chunk test asks for the streaming one)
-        if (w->family == 2 && !w->explicit_launch && !w->test_skip && w->d_flags && nsteps > 0 && (!x.F || x.d_fscale) &&
+        if (w->family == 2 && !w->explicit_launch && !w->test_skip && nsteps > 0 && (!x.F || x.d_fscale) &&
             (!x.acc || x.d_cfilter))
         {
-            const ResPlan p = res_plan(w->n, sizeof(Real) == 4, w->nel, w->sms, w->max_ctas);
-            if (p.fits)
+            WDG_TRY(ensure_resident(w));
+            const ResPlan p = res_plan(w->n, sizeof(Real) == 4, w->nel, w->sms, w->max_ctas, x.F != nullptr);
+            if (p.fits && w->d_flags)
             {
                 bool ran = false;
-                WDG_TRY(res_rk4<Real>(w, p, A, dt, nsteps, x, ran));
+                WDG_TRY(res_rk4<Real>(w, p, A, dt, nsteps, x, ran, w->stream));
                 if (ran)
                 {
                     for (int s = 0; s < nsteps; ++s)
@@ -173,6 +195,10 @@ namespace wdg
                 }
             }
         }
+        WDG_TRY(ensure_states(w));
+        Real *B = static_cast<Real *>(w->d_state[1]);
+        Real *Cb = static_cast<Real *>(w->d_state[2]);
+        Real *du = static_cast<Real *>(w->d_du);
         StageArgs<Real> a = base_args<Real>(w);
         a.du = du;
         a.dt = (Real)dt;
@@ -608,7 +634,7 @@ extern "C"
         void *ptrs[] = {w->d_corners, w->d_nbr, w->d_finfo, w->d_face_edge, w->d_fbase, w->d_fcode, w->d_edgesI,
                         w->d_edgesB, w->d_codes,
                         w->d_state[0], w->d_state[1], w->d_state[2], w->d_du, w->d_stage[0], w->d_stage[1],
-                        w->d_stage[2], w->d_scratch, w->d_result, w->d_err, w->d_src, w->d_flags, w->d_trace};
+                        w->d_stage[2], w->d_scratch, w->d_result, w->d_err, w->d_src, w->d_flags, w->d_trace[1]};
         for (void *p : ptrs)
             if (p)
                 cudaFree(p);
@@ -766,6 +792,7 @@ extern "C"
             return fail(WDG_ERR_ARG, "wdg_wave_autotune: bad arguments");
         DeviceGuard g(w->device);
         WDG_TRY(ensure_states(w));
+        WDG_TRY(ensure_resident(w));
         cudaEvent_t e0, e1;
         WDG_CUDA(cudaEventCreate(&e0));
         WDG_CUDA(cudaEventCreate(&e1));
@@ -783,7 +810,7 @@ extern "C"
         std::vector<Cand> cands;
         // family 3 stands for family 2 with the elements resident, where they fit
         const bool save_explicit = w->explicit_launch;
-        if (w->d_flags && res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, w->max_ctas).fits)
+        if (w->d_flags && res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, w->max_ctas, false).fits)
             cands.push_back({3, 0, 0});
         cands.push_back({0, save_tile, save_stages});
         for (int st = 2; st <= 4; ++st)

@@ -46,7 +46,7 @@ struct wdg_wave
     // resident launches, on handles whose mesh fits: a flag per element group, the value they count on
     // from, and two trace buffers (with the states)
     unsigned long long *d_flags = nullptr, flag_base = 0;
-    void *d_trace = nullptr;
+    void *d_trace[2] = {nullptr, nullptr}; // (the first is part of d_flags' allocation)
     unsigned long long wait_ns = 0; // limit of the stage kernels' bounded waits (0: kWaitLimitNs)
     int test_skip = 0;              // test hook: 1 + chunk the next RK launch leaves unloaded
     double *d_src = nullptr;    // gaussian source table
@@ -61,6 +61,8 @@ namespace wdg
     int is_device_ptr(const wdg_wave *w, const void *p, bool &dev);
     int ensure_stage(wdg_wave *w, int k);
     int ensure_states(wdg_wave *w);
+    int ensure_resident(wdg_wave *w);
+    int ensure_period(wdg_wave *w);
     int check_device_error(wdg_wave *w);
     int sync(wdg_wave *w);
 
@@ -86,12 +88,13 @@ namespace wdg
         int ngroups = 0, ctas = 0, warps = 0;
         size_t smem = 0;
     };
-    ResPlan res_plan(int n, bool fp32, int nel, int sms, int max_ctas);
+    ResPlan res_plan(int n, bool fp32, int nel, int sms, int max_ctas, bool forced);
     size_t res_flag_count(int n, int nel);
     int upload_res_tables(int device); // once per device
-    // nsteps of RK4 on A; ran = false (and nothing done) where the device cannot hold the launch
+    // nsteps of RK4 on A, on `stream`; ran = false (and nothing done) where the device cannot hold the launch
     template <typename Real>
-    int res_rk4(wdg_wave *w, const ResPlan &p, Real *A, double dt, int nsteps, const RKExtras &x, bool &ran);
+    int res_rk4(wdg_wave *w, const ResPlan &p, Real *A, double dt, int nsteps, const RKExtras &x, bool &ran,
+                cudaStream_t stream);
     template <typename Real>
     int rk4_run(wdg_wave *w, Real *A, double dt, double &t, int nsteps, const RKExtras &x);
     // stage st of the RK4 step that starts at time t; with F, forcing F * s(t + c_st dt),

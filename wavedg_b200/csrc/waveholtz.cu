@@ -82,6 +82,8 @@ namespace
     {
         wdg_wave *w = h->w;
         const bool fp32 = w->precision == WDG_FP32;
+        if (!h->q)
+            WDG_TRY(ensure_period(w)); // the launch settings may have changed since
         WDG_CUDA(cudaStreamBeginCapture(h->cs, cudaStreamCaptureModeThreadLocal));
         int s = WDG_OK;
         cudaError_t e = cudaSuccess;
@@ -195,7 +197,7 @@ extern "C"
         cudaGetDevice(&dev_prev);
         cudaSetDevice(w->device);
         // state buffers must exist before a period is captured into a graph
-        int s = ensure_states(w);
+        int s = ensure_period(w);
         cudaError_t e = (s == WDG_OK) ? cudaStreamCreateWithFlags(&h->cs, cudaStreamNonBlocking) : cudaSuccess;
         if (e == cudaSuccess)
             e = cudaEventCreateWithFlags(&h->ev_in, cudaEventDisableTiming);

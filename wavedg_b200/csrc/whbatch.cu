@@ -6,6 +6,13 @@
 // each solve's step counter, period ends, residual and status live on the device
 // (WhbState), so a replay needs no host decision.  Iteration and residual follow the
 // reference's fixed-point loop (examples/waveholtz2d.cpp:165-185; WaveHoltz.cpp:55-121).
+//
+// Solves whose elements fit the chip beside others' run their periods as resident launches
+// (stage_res.cu) instead, several at a time, each on its share of the SMs: a round is one period of
+// every solve it holds, the shares set by the periods' work, after which the host reads the
+// records.  A stage of the listed kind -- four solves of 4096 to 16384 elements in FP32 -- takes 31 us as
+// launches of the three degrees, mostly their start and end, and about 9 us of a solve's
+// share here.  Batches with explicitly chosen launch shapes, and solves that do not fit, run as above.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -48,6 +55,12 @@ struct wdg_whbatch
     WhbState *h_state = nullptr; // pinned
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
+    // resident periods: per solve its tables, partial sums and stream (made on first use)
+    bool explicit_launch = false;
+    std::vector<double *> d_fscale, d_cfilter, d_end;
+    std::vector<cudaStream_t> rs;
+    std::vector<cudaEvent_t> rdone;
+    unsigned *h_err = nullptr; // pinned
 };
 
 namespace
@@ -189,6 +202,8 @@ namespace
     {
         const bool fp32 = b->precision == WDG_FP32;
         const bool fork = b->groups.size() > 1;
+        for (wdg_wave *w : b->w)
+            WDG_TRY(ensure_states(w));
         WDG_CUDA(cudaStreamBeginCapture(b->cs, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = cudaSuccess;
         for (int k = 0; k < kGraphSteps && e == cudaSuccess; ++k)
@@ -276,6 +291,151 @@ namespace
         S.part = b->d_part[s];
         return S;
     }
+    // the smallest number of CTAs with which solve s is resident; 0: none
+    int least_ctas(const wdg_whbatch *b, int s)
+    {
+        const wdg_wave *w = b->w[s];
+        if (!w->d_flags || w->family != 2 || w->explicit_launch)
+            return 0;
+        auto fits = [&](int c) { return res_plan(w->n, b->precision == WDG_FP32, w->nel, w->sms, c, true).fits; };
+        const int most = w->max_ctas > 0 ? std::min(w->sms, w->max_ctas) : w->sms;
+        if (!fits(most))
+            return 0;
+        int lo = 1, hi = most;
+        while (lo < hi)
+        {
+            const int mid = (lo + hi) / 2;
+            if (fits(mid))
+                hi = mid;
+            else
+                lo = mid + 1;
+        }
+        // (a share may fit a little less well than the next smaller one: rounds of groups are whole)
+        while (lo < most && !fits(lo))
+            ++lo;
+        return lo;
+    }
+
+    int resident_prepare(wdg_whbatch *b)
+    {
+        if (!b->rs.empty())
+            return WDG_OK;
+        b->d_fscale.assign(b->n, nullptr);
+        b->d_cfilter.assign(b->n, nullptr);
+        b->d_end.assign(b->n, nullptr);
+        b->rs.assign(b->n, nullptr);
+        b->rdone.assign(b->n, nullptr);
+        WDG_CUDA(cudaMallocHost(&b->h_err, sizeof(unsigned) * b->n));
+        for (int s = 0; s < b->n; ++s)
+        {
+            WDG_CUDA(cudaMalloc(&b->d_fscale[s], sizeof(double) * 5 * b->nt[s]));
+            WDG_CUDA(cudaMalloc(&b->d_cfilter[s], sizeof(double) * b->nt[s]));
+            WDG_CUDA(cudaMalloc(&b->d_end[s], sizeof(double) * 2 * kWhbEndBlocks));
+            WDG_CUDA(cudaStreamCreateWithFlags(&b->rs[s], cudaStreamNonBlocking));
+            WDG_CUDA(cudaEventCreateWithFlags(&b->rdone[s], cudaEventDisableTiming));
+            WDG_CUDA(launch_whb_tables(b->omega[s], b->dt[s], b->nt[s], b->d_fscale[s], b->d_cfilter[s], b->cs));
+        }
+        return WDG_OK;
+    }
+
+    // one period of solve s on `ctas` CTAs, on its own stream
+    template <typename Real>
+    int resident_period(wdg_whbatch *b, int s, int ctas, bool &ran)
+    {
+        wdg_wave *w = b->w[s];
+        RKExtras x;
+        x.F = b->d_F[s];
+        x.omega = b->omega[s];
+        x.acc = b->d_acc[s];
+        x.d_fscale = b->d_fscale[s];
+        x.d_cfilter = b->d_cfilter[s];
+        const ResPlan p = res_plan(w->n, sizeof(Real) == 4, w->nel, w->sms, ctas, true);
+        Real *u = static_cast<Real *>(w->d_state[0]);
+        WDG_TRY(res_rk4<Real>(w, p, u, b->dt[s], b->nt[s], x, ran, b->rs[s]));
+        if (ran)
+            WDG_CUDA(launch_whb_period_end<Real>(b->d_state + s, u, b->d_acc[s], b->d_W[s], b->c0[s], w->ndof, b->d_end[s],
+                                                 b->rs[s]));
+        return WDG_OK;
+    }
+
+    // Every solve that can be resident, to its end; the others' records stay as they are.  A round holds as
+    // many running solves as the SMs do, each on at least its least share and on two rounds of groups per warp
+    // where it has them; what is left of the SMs goes by the work of a period.
+    int resident_solves(wdg_whbatch *b)
+    {
+        std::vector<int> least(b->n, 0);
+        bool any = false;
+        int sms = b->w[0]->sms;
+        for (int s = 0; s < b->n; ++s)
+            any = (least[s] = b->explicit_launch ? 0 : least_ctas(b, s)) > 0 || any;
+        if (!any)
+            return WDG_OK;
+        WDG_TRY(resident_prepare(b));
+        std::vector<double> work(b->n);
+        for (int s = 0; s < b->n; ++s)
+            work[s] = (double)b->w[s]->ndof * b->nt[s];
+        for (;;)
+        {
+            std::vector<int> in, share;
+            int used = 0;
+            for (int s = 0; s < b->n; ++s)
+            {
+                if (!least[s] || !b->h_state[s].active)
+                    continue;
+                const ResPlan p = res_plan(b->w[s]->n, b->precision == WDG_FP32, b->w[s]->nel, sms, least[s], true);
+                const int want = std::max(least[s], std::min(sms, (p.ngroups + 23) / 24));
+                if (!in.empty() && used + want > sms)
+                    continue;
+                in.push_back(s);
+                share.push_back(want);
+                used += want;
+            }
+            if (in.empty())
+                return WDG_OK;
+            // the SMs left over, to the solve with the longest period so far
+            for (int left = sms - used; left > 0; --left)
+            {
+                int at = -1;
+                double longest = 0.0;
+                for (size_t k = 0; k < in.size(); ++k)
+                {
+                    const wdg_wave *w = b->w[in[k]];
+                    const int cap = std::min(w->max_ctas > 0 ? std::min(sms, w->max_ctas) : sms, (w->nel + 32 / w->n - 1) / (32 / w->n));
+                    if (share[k] < cap && work[in[k]] / share[k] > longest)
+                    {
+                        longest = work[in[k]] / share[k];
+                        at = (int)k;
+                    }
+                }
+                if (at < 0)
+                    break;
+                ++share[at];
+            }
+            WDG_CUDA(cudaEventRecord(b->fork, b->cs));
+            for (size_t k = 0; k < in.size(); ++k)
+            {
+                const int s = in[k];
+                // a share between two that fit may not: the next smaller one that does
+                while (share[k] > least[s] &&
+                       !res_plan(b->w[s]->n, b->precision == WDG_FP32, b->w[s]->nel, sms, share[k], true).fits)
+                    --share[k];
+                WDG_CUDA(cudaStreamWaitEvent(b->rs[s], b->fork, 0));
+                bool ran = false;
+                WDG_TRY(b->precision == WDG_FP32 ? resident_period<float>(b, s, share[k], ran)
+                                                 : resident_period<double>(b, s, share[k], ran));
+                if (!ran)
+                    least[s] = 0; // the device cannot hold it: left to the streaming launches
+                WDG_CUDA(cudaMemcpyAsync(b->h_err + s, b->w[s]->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, b->rs[s]));
+                WDG_CUDA(cudaEventRecord(b->rdone[s], b->rs[s]));
+                WDG_CUDA(cudaStreamWaitEvent(b->cs, b->rdone[s], 0));
+            }
+            WDG_CUDA(cudaMemcpyAsync(b->h_state, b->d_state, sizeof(WhbState) * b->n, cudaMemcpyDeviceToHost, b->cs));
+            WDG_CUDA(cudaStreamSynchronize(b->cs));
+            for (int s : in)
+                if (b->h_err[s])
+                    WDG_TRY(check_device_error(b->w[s]));
+        }
+    }
 } // namespace
 
 extern "C"
@@ -339,7 +499,7 @@ extern "C"
             b->dt.push_back(dt);
             b->nt.push_back(nt);
             b->c0.push_back(0.5 * dt * K(omegas[u], 0.0));
-            st = ensure_states(w);
+            st = ensure_period(w);
             const size_t nd = (size_t)w->ndof;
             cudaError_t e = cudaSuccess;
             if (st == WDG_OK)
@@ -413,6 +573,18 @@ extern "C"
             if (gr.st)
                 cudaStreamDestroy(gr.st);
         }
+        for (size_t k = 0; k < b->rs.size(); ++k)
+        {
+            for (double *p : {b->d_fscale[k], b->d_cfilter[k], b->d_end[k]})
+                if (p)
+                    cudaFree(p);
+            if (b->rdone[k])
+                cudaEventDestroy(b->rdone[k]);
+            if (b->rs[k])
+                cudaStreamDestroy(b->rs[k]);
+        }
+        if (b->h_err)
+            cudaFreeHost(b->h_err);
         if (b->fork)
             cudaEventDestroy(b->fork);
         if (b->cs)
@@ -436,6 +608,7 @@ extern "C"
         if (!b || rounds < 1 || rounds > 16 || ring < 2 || ring > 6)
             return fail(WDG_ERR_ARG, "wdg_whbatch_set_launch: rounds 1..16, ring 2..6");
         Dev g(b->device);
+        b->explicit_launch = true;
         return shape(b, rounds, ring);
     }
 
@@ -500,7 +673,11 @@ extern "C"
             b->h_state[s] = fresh_state(b, s, ws, tol, maxit, stall_limit, known);
         }
         WDG_CUDA(cudaMemcpyAsync(b->d_state, b->h_state, sizeof(WhbState) * b->n, cudaMemcpyHostToDevice, b->cs));
-        if (!b->graph)
+        WDG_TRY(resident_solves(b));
+        bool running = false;
+        for (int s = 0; s < b->n; ++s)
+            running = running || b->h_state[s].active;
+        if (running && !b->graph)
             WDG_TRY(record(b));
         // replay blocks of steps until no solve is running; bounded by the longest possible
         // run (maxit + 1 periods of the longest period)
@@ -508,7 +685,6 @@ extern "C"
         for (int s = 0; s < b->n; ++s)
             limit = std::max<long long>(limit, (long long)(maxit + 1) * b->nt[s]);
         long long steps = 0;
-        bool running = true;
         while (running && steps <= limit + b->graph_steps)
         {
             WDG_CUDA(cudaGraphLaunch(b->graph, b->cs));

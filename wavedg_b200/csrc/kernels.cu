@@ -803,6 +803,7 @@ namespace wdg
 } // namespace wdg
 
 #include "stage_ws.cuh"
+#include "stage_line.cuh"
 #include "stage_ws_batch.cuh"
 
 namespace wdg
@@ -817,11 +818,11 @@ namespace wdg
     }
     int ws_warp_scratch_bytes(int n, bool fp32)
     {
-        return fp32 ? ws_layout<float>(n, 0, 0).warp_scratch : ws_layout<double>(n, 0, 0).warp_scratch;
+        return fp32 ? ws_layout<float>(n, stream_sums(n).el, 0, 0).warp_scratch : ws_layout<double>(n, stream_sums(n).el, 0, 0).warp_scratch;
     }
     size_t ws_smem_bytes(int n, bool fp32, int chunk, int ring)
     {
-        return fp32 ? (size_t)ws_layout<float>(n, chunk, ring).total : (size_t)ws_layout<double>(n, chunk, ring).total;
+        return fp32 ? (size_t)ws_layout<float>(n, stream_sums(n).el, chunk, ring).total : (size_t)ws_layout<double>(n, stream_sums(n).el, chunk, ring).total;
     }
     int ws_default_chunk(int n, bool fp32)
     {
@@ -895,8 +896,11 @@ namespace wdg
     {
         // a launch over part of the elements exists only in the warp-specialised family
         const bool partial = a.el_begin != 0 || (a.el_end > 0 && a.el_end != a.nel);
+        const bool line = rk && line_takes<Real>(a, grid_limit);
 #define WDG_CASE(NV)                                                                       \
     case NV:                                                                               \
+        if (line)                                                                          \
+            return launch_line<NV, Real>(a, s);                                            \
         if (a.family == 2 && rk && a.use_tma && a.tma_out && ws_fits<NV, Real>(a))         \
             return launch_ws_n<NV, Real>(a, grid_limit, s);                                \
         if (partial)                                                                       \

@@ -36,6 +36,11 @@ namespace wdg
             "l"(src), "r"(bytes), "r"(smem_u32(bar))
             : "memory");
     }
+    // the same piece of global memory into L2 only
+    __device__ __forceinline__ void bulk_prefetch(const void *src, uint32_t bytes)
+    {
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+    }
     __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
     {
         uint32_t ok;

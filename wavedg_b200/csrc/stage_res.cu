@@ -82,42 +82,6 @@ namespace wdg
             L.bytes = (L.code + ew * 4 + 15) & ~15;
             return L;
         }
-        // The column sums' strides (row j of an element, element): columns are written at 3 i, rows read at
-        // j * row, both with as few wavefronts as the 16 double-wide banks of a half-warp allow
-        struct ResStride
-        {
-            int row, el;
-        };
-        __host__ __device__ constexpr int res_waves(int n, int a, int e)
-        {
-            int waves = 0;
-            for (int h = 0; h < 2; ++h)
-            {
-                int cnt[16] = {}, most = 0;
-                for (int i = 16 * h; i < 16 * h + 16 && i < 32 / n * n; ++i)
-                    if (++cnt[(i / n * e + i % n * a) & 15] > most)
-                        most = cnt[(i / n * e + i % n * a) & 15];
-                waves += most;
-            }
-            return waves;
-        }
-        __host__ __device__ constexpr ResStride res_strides(int n)
-        {
-            ResStride b{3 * n, 3 * n * n};
-            int cost = 1 << 30;
-            for (int row = 3 * n; row < 3 * n + 8; ++row)
-                for (int el = row * n; el < row * n + 6; ++el)
-                {
-                    const int c = 32 * (res_waves(n, 3, el) + res_waves(n, row, el)) + (el - 3 * n * n) / 2;
-                    if (c < cost)
-                    {
-                        cost = c;
-                        b.row = row;
-                        b.el = el;
-                    }
-                }
-            return b;
-        }
         // FP32 stepping adds the forcing where the streaming kernel does, to the row's finished sums, so that
         // batches of either kind give the same bits; its values then need a place of their own.  FP64 adds it
         // to the column's sums and lets it share the scratch: that place would cost a warp or two.
@@ -130,7 +94,7 @@ namespace wdg
         // a warp's scratch: the forcing (FP64), then the column sums of a group
         __host__ __device__ constexpr int res_scratch(int n, int real)
         {
-            return ((32 / n) * res_strides(n).el * real + 15) & ~15;
+            return ((32 / n) * sum_strides(n).el * real + 15) & ~15;
         }
 
         __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p)
@@ -172,7 +136,7 @@ namespace wdg
             const int most = (a.ngroups + gridDim.x - 1) / gridDim.x;
             unsigned char *groups = rsm;
             constexpr int kScratch = res_scratch(N, sizeof(Real));
-            constexpr ResStride RS = res_strides(N);
+            constexpr SumStride RS = sum_strides(N);
             constexpr bool LATE = kLateForcing<Real>;
             const int scratch = kScratch + (a.F ? res_forcing(N, sizeof(Real)) : 0);
             Real *Rc = reinterpret_cast<Real *>(groups + (size_t)most * L.bytes + (size_t)warp * scratch);

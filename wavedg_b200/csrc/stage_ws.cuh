@@ -24,8 +24,8 @@
 //                             contraction, the face nodes of sides 3 and 1,
 //                             then per node the column pass's sums, M^{-1}
 //                             and the RK update, in place.  The row pass works
-//                             on contiguous 3 n-value runs, so its shared
-//                             memory accesses are free of bank conflicts.
+//                             on contiguous 3 n-value runs: free of bank
+//                             conflicts for odd n, in wide pieces for even n.
 //              Warps sync only with __syncwarp; a chunk is released when all
 //              consumer warps have arrived on its `done` barrier.
 //
@@ -34,8 +34,10 @@
 // in place, so the slot's copy of u cannot serve another warp.  The gather
 // runs on the producer's lanes ahead of time, so no consumer waits on L2.
 //
-// Used for RK launches whose arrays are 16-byte aligned; every other launch
-// takes the tiled kernel.
+// Used for RK launches whose arrays are 16-byte aligned where the caller chose a launch shape or a CTA
+// limit, and for FP32 launches with forcing or filter; the batch's streaming launches run its roles
+// (stage_ws_batch.cuh).  Other RK launches take the kernel of one warp per CTA (stage_line.cuh),
+// launches with unaligned arrays the tiled one.
 
 namespace wdg
 {
@@ -46,6 +48,9 @@ namespace wdg
         static constexpr int EW = 32 / N; // elements per warp-round, one lane per line
     };
     constexpr int kWsThreads = 32 * (kWsConsumers + 1);
+    // the column sums' strides: dense for odd n, whose strides are odd as they are (n = 5: padding saves 5
+    // of 90 wavefronts an element and costs 1 KB a warp; 147 -> 160 us a stage of 512 x 512)
+    __host__ __device__ constexpr SumStride stream_sums(int n) { return n % 2 ? SumStride{3 * n, 3 * n * n} : sum_strides(n); }
 
     int ws_epw(int n) { return 32 / n; }
 
@@ -58,7 +63,7 @@ namespace wdg
         int slot, tab, slots, scratch, warp_scratch, total;
     };
     template <typename Real>
-    __host__ __device__ inline WsLayout ws_layout(int n, int chunk, int stages, bool staged = false);
+    __host__ __device__ inline WsLayout ws_layout(int n, int sum_el, int chunk, int stages, bool staged = false);
 
     __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
     {
@@ -71,18 +76,18 @@ namespace wdg
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
     }
 
-    // Face node k of side SIDE, subtracted into r; own trace `own`, the neighbour's in the slot's halo
+    // A face node of side SIDE, subtracted into r: own values `own`, the neighbour's `nb`
     template <int N, typename Real, int SIDE>
     __device__ __forceinline__ void ws_face(uint32_t codes, int flags, const double2 c01, const double2 c23,
-                                            const double2 c45, const double2 c67, Real wk, int k,
-                                            const Real *own, const Real *halo_e, Real &r0, Real &r1, Real &r2)
+                                            const double2 c45, const double2 c67, Real wk,
+                                            const Real *own, const Real *nb, Real &r0, Real &r1, Real &r2)
     {
         const uint32_t byte = (codes >> (8 * SIDE)) & 0xffu;
         if ((byte & 0x80u) ? !(flags & F_BND) : !(flags & F_INT))
             return;
         Real nx, ny, hm;
         line_side<Real, SIDE>(c01, c23, c45, c67, nx, ny, hm);
-        line_face<Real>(byte, nx, ny, wk * hm, own, halo_e + 3 * (SIDE * N + k), r0, r1, r2);
+        line_face<Real>(byte, nx, ny, wk * hm, own, nb, r0, r1, r2);
     }
 
     // One chunk of one RK stage as both roles see it (the single-solve kernel fills it from
@@ -277,27 +282,69 @@ namespace wdg
         }
     }
 
+    // A grid row of a state (3 n values, contiguous) is read and written in pieces of V values, the widest
+    // (to 16 bytes) that its length and place allow.  V = 1 where n is odd: rows then lie an odd number of
+    // values apart, which is free of bank conflicts; even n would have 2 to 8 lanes on a bank (us a stage,
+    // value by value -> in pieces: 512 x 512, n = 4: 109 -> 103 in FP64, 63 -> 59 in FP32; n = 8: 193 -> 184, 108 -> 96).
+    template <int N, typename Real>
+    struct RowPiece
+    {
+        static constexpr int V = sizeof(Real) == 8 ? (N % 2 == 0 ? 2 : 1) : N % 4 == 0 ? 4 : N % 2 == 0 ? 2 : 1;
+        struct alignas(V * sizeof(Real)) T
+        {
+            Real v[V];
+        };
+    };
+    // the values of V nodes, from the first one's place
+    template <int N, typename Real>
+    __device__ __forceinline__ void row_get(const Real *p, Real (&v)[3 * RowPiece<N, Real>::V])
+    {
+        constexpr int V = RowPiece<N, Real>::V;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            const typename RowPiece<N, Real>::T x = reinterpret_cast<const typename RowPiece<N, Real>::T *>(p)[k];
+#pragma unroll
+            for (int q = 0; q < V; ++q)
+                v[V * k + q] = x.v[q];
+        }
+    }
+    template <int N, typename Real>
+    __device__ __forceinline__ void row_put(Real *p, const Real (&v)[3 * RowPiece<N, Real>::V])
+    {
+        constexpr int V = RowPiece<N, Real>::V;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            typename RowPiece<N, Real>::T x;
+#pragma unroll
+            for (int q = 0; q < V; ++q)
+                x.v[q] = v[V * k + q];
+            reinterpret_cast<typename RowPiece<N, Real>::T *>(p)[k] = x;
+        }
+    }
+
     // ---------------------------------------------------------------- consumer: one chunk
-    // Warp `cw` takes rounds of EW whole elements; Rc is its scratch for the column sums.
+    // Warp `cw` takes R rounds of EW whole elements, whose parts lie at base + o; Rc is its scratch for
+    // the column sums, xm and wm the node and weight of its lane's line.
     template <int N, typename Real, bool EXTRA, bool BATCH>
-    __device__ __forceinline__ void ws_consume(const WsChunk<Real> &c, unsigned char *base, Real *Rc,
-                                               const Real *xtab, const Real *wtab, int cw, int lane)
+    __device__ __forceinline__ void ws_consume(const WsChunk<Real> &c, unsigned char *base, const WsSlot &o,
+                                               int R, Real *Rc, Real xm, Real wm, int cw, int lane)
     {
         using Sh = WsShape<N>;
-        constexpr int NN = Sh::NN, ND = Sh::ND, NF = Sh::NF, EW = Sh::EW;
+        constexpr int ND = Sh::ND, NF = Sh::NF, EW = Sh::EW;
         constexpr bool STG = WsStage<Real, EXTRA>::value;
-        const WsSlot o = ws_slot<Real>(N, c.chunk, STG);
+        constexpr SumStride RS = stream_sums(N);
+        constexpr int V = RowPiece<N, Real>::V;
         const int flags = c.flags;
         // forcing and filter: staged in the slot (chunk-local index) or read in place
         const Real *Fx = STG ? reinterpret_cast<const Real *>(base + o.fb) - (size_t)c.el0 * ND : c.F;
         double *Ax = STG ? reinterpret_cast<double *>(base + o.ab) - (size_t)c.el0 * ND : c.acc;
         const bool has_du = (flags & F_READ_DU) != 0;
-        const int R = c.chunk / (kWsConsumers * EW); // warp-rounds per chunk
         const int el_l = lane / N, ln = lane - el_l * N; // element of the round, grid line
         const bool lane_on = lane < EW * N;
-        const Real xm = lane_on ? xtab[ln] : Real(0), wm = lane_on ? wtab[ln] : Real(0);
         Real *us = reinterpret_cast<Real *>(base);
-        Real *dus = us + c.chunk * ND;
+        Real *dus = reinterpret_cast<Real *>(base + o.ub);
         const Real *halo = reinterpret_cast<const Real *>(base + o.hb);
         const double *cs = reinterpret_cast<const double *>(base + o.cb);
         const uint32_t *fks = reinterpret_cast<const uint32_t *>(base + o.kb);
@@ -311,7 +358,7 @@ namespace wdg
                 uint32_t codes = 0;
                 const Real *halo_e = halo + le * NF * 3;
                 Real *ue = us + le * ND;
-                Real *rc = Rc + el_l * NN * 3; // this element's column-pass sums, (node, field)
+                Real *rc = Rc + el_l * RS.el; // this element's column-pass sums, (node, field)
                 if (act)
                 {
                     const double2 *c2 = reinterpret_cast<const double2 *>(cs + 8 * le);
@@ -331,13 +378,13 @@ namespace wdg
                     if (flags & F_VOL)
                         line_column<N, Real>(c01, c23, c45, c67, ue, i, wi, sp, su, sv);
                     // face nodes of the column: (i, 0) on side 0, (i, n-1) on side 2, face-node index i
-                    ws_face<N, Real, 0>(codes, flags, c01, c23, c45, c67, wi, i, ue + 3 * i, halo_e, sp[0], su[0], sv[0]);
-                    ws_face<N, Real, 2>(codes, flags, c01, c23, c45, c67, wi, i, ue + 3 * (i + N * (N - 1)), halo_e,
+                    ws_face<N, Real, 0>(codes, flags, c01, c23, c45, c67, wi, ue + 3 * i, halo_e + 3 * (N * 0 + i), sp[0], su[0], sv[0]);
+                    ws_face<N, Real, 2>(codes, flags, c01, c23, c45, c67, wi, ue + 3 * (i + N * (N - 1)), halo_e + 3 * (N * 2 + i),
                                         sp[N - 1], su[N - 1], sv[N - 1]);
 #pragma unroll
                     for (int j = 0; j < N; ++j)
                     {
-                        Real *o = rc + 3 * (i + N * j);
+                        Real *o = rc + 3 * i + RS.row * j;
                         o[0] = sp[j];
                         o[1] = su[j];
                         o[2] = sv[j];
@@ -353,80 +400,84 @@ namespace wdg
                     Real q0[N], q1[N], q2[N], mv[N];
                     Real ap[N], au[N], av[N];
 #pragma unroll
-                    for (int l = 0; l < N; ++l)
+                    for (int l0 = 0; l0 < N; l0 += V)
                     {
-                        q0[l] = row[3 * l];
-                        q1[l] = row[3 * l + 1];
-                        q2[l] = row[3 * l + 2];
-                        ap[l] = au[l] = av[l] = 0;
+                        Real v[3 * V];
+                        row_get<N, Real>(row + 3 * l0, v);
+#pragma unroll
+                        for (int l = 0; l < V; ++l)
+                        {
+                            q0[l0 + l] = v[3 * l];
+                            q1[l0 + l] = v[3 * l + 1];
+                            q2[l0 + l] = v[3 * l + 2];
+                            ap[l0 + l] = au[l0 + l] = av[l0 + l] = 0;
+                        }
                     }
                     line_row<N, Real, true>(c01, c23, c45, c67, xm, wj, (flags & F_VOL) != 0, q0, q1, q2, ap, au, av, mv);
                     // face nodes of the row: (0, j) on side 3, (n-1, j) on side 1, face-node index j
-                    ws_face<N, Real, 3>(codes, flags, c01, c23, c45, c67, wj, j, row, halo_e, ap[0], au[0], av[0]);
-                    ws_face<N, Real, 1>(codes, flags, c01, c23, c45, c67, wj, j, row + 3 * (N - 1), halo_e,
+                    ws_face<N, Real, 3>(codes, flags, c01, c23, c45, c67, wj, row, halo_e + 3 * (N * 3 + j), ap[0], au[0], av[0]);
+                    ws_face<N, Real, 1>(codes, flags, c01, c23, c45, c67, wj, row + 3 * (N - 1), halo_e + 3 * (N * 1 + j),
                                         ap[N - 1], au[N - 1], av[N - 1]);
 
                     // ---- epilogue per node of the row: + column-pass sums, forcing, M^{-1}, RK
                     // update in place (wavedg/ode.hpp:66-93); the row is this lane's alone
                     Real *drow = dus + le * ND + 3 * N * j;
 #pragma unroll
-                    for (int i = 0; i < N; ++i)
+                    for (int i0 = 0; i0 < N; i0 += V)
                     {
-                        const Real *cr = rc + 3 * (i + N * j);
-                        Real r0 = ap[i] + cr[0], r1 = au[i] + cr[1], r2 = av[i] + cr[2];
-                        const size_t g = (size_t)(c.el0 + le) * ND + 3 * (i + N * j);
-                        if (EXTRA && (flags & F_FORCE))
+                        Real d[3 * V], uo[3 * V];
+                        if (has_du)
+                            row_get<N, Real>(drow + 3 * i0, d);
+#pragma unroll
+                        for (int l = 0; l < V; ++l)
                         {
-                            r0 += c.fscale * Fx[g];
-                            r1 += c.fscale * Fx[g + 1];
-                            r2 += c.fscale * Fx[g + 2];
-                        }
-                        if (flags & F_MINV)
-                        {
-                            r0 *= mv[i];
-                            r1 *= mv[i];
-                            r2 *= mv[i];
-                        }
-                        Real *dn = drow + 3 * i;
-                        const Real d0 = rk_register(has_du, c.rk_a, dn[0], c.dt, r0);
-                        const Real d1 = rk_register(has_du, c.rk_a, dn[1], c.dt, r1);
-                        const Real d2 = rk_register(has_du, c.rk_a, dn[2], c.dt, r2);
-                        Real uo[3] = {rk_state(q0[i], c.rk_b, d0), rk_state(q1[i], c.rk_b, d1), rk_state(q2[i], c.rk_b, d2)};
-                        dn[0] = d0;
-                        dn[1] = d1;
-                        dn[2] = d2;
-                        if (BATCH && c.pend)
-                        {
-                            // last step of a period: the filter's last term completes the period's
-                            // result; the state and the filter restart from the new iterate
+                            const int i = i0 + l;
+                            const Real *cr = rc + 3 * i + RS.row * j;
+                            Real r[3] = {ap[i] + cr[0], au[i] + cr[1], av[i] + cr[2]};
+                            const Real q[3] = {q0[i], q1[i], q2[i]};
+                            const size_t g = (size_t)(c.el0 + le) * ND + 3 * (i + N * j);
 #pragma unroll
                             for (int f = 0; f < 3; ++f)
                             {
-                                const double fin = Ax[g + f] + c.acc_c * (double)uo[f];
-                                nsum += fin * fin;
-                                double w0;
-                                if (c.pend == 1)
+                                if (EXTRA && (flags & F_FORCE))
+                                    r[f] += c.fscale * Fx[g + f];
+                                if (flags & F_MINV)
+                                    r[f] *= mv[i];
+                                d[3 * l + f] = rk_register(has_du, c.rk_a, d[3 * l + f], c.dt, r[f]);
+                                uo[3 * l + f] = rk_state(q[f], c.rk_b, d[3 * l + f]);
+                            }
+                            if (BATCH && c.pend)
+                            {
+                                // last step of a period: the filter's last term completes the period's
+                                // result; the state and the filter restart from the new iterate
+#pragma unroll
+                                for (int f = 0; f < 3; ++f)
                                 {
-                                    const double dw = fin - c.W[g + f];
-                                    dsum += dw * dw;
-                                    c.W[g + f] = fin;
-                                    w0 = fin;
+                                    const double fin = Ax[g + f] + c.acc_c * (double)uo[3 * l + f];
+                                    nsum += fin * fin;
+                                    double w0;
+                                    if (c.pend == 1)
+                                    {
+                                        const double dw = fin - c.W[g + f];
+                                        dsum += dw * dw;
+                                        c.W[g + f] = fin;
+                                        w0 = fin;
+                                    }
+                                    else
+                                        w0 = c.W[g + f];
+                                    Ax[g + f] = c.c0 * w0;
+                                    uo[3 * l + f] = (Real)w0;
                                 }
-                                else
-                                    w0 = c.W[g + f];
-                                Ax[g + f] = c.c0 * w0;
-                                uo[f] = (Real)w0;
+                            }
+                            else if (EXTRA && (flags & F_FILTER))
+                            {
+#pragma unroll
+                                for (int f = 0; f < 3; ++f)
+                                    Ax[g + f] += c.acc_c * (double)uo[3 * l + f];
                             }
                         }
-                        else if (EXTRA && (flags & F_FILTER))
-                        {
-                            Ax[g] += c.acc_c * (double)uo[0];
-                            Ax[g + 1] += c.acc_c * (double)uo[1];
-                            Ax[g + 2] += c.acc_c * (double)uo[2];
-                        }
-                        row[3 * i] = uo[0];
-                        row[3 * i + 1] = uo[1];
-                        row[3 * i + 2] = uo[2];
+                        row_put<N, Real>(drow + 3 * i0, d);
+                        row_put<N, Real>(row + 3 * i0, uo);
                     }
                 }
                 __syncwarp(); // the scratch is reused by the next round
@@ -448,15 +499,15 @@ namespace wdg
     }
 
     template <typename Real>
-    __host__ __device__ inline WsLayout ws_layout(int n, int chunk, int stages, bool staged)
+    __host__ __device__ inline WsLayout ws_layout(int n, int sum_el, int chunk, int stages, bool staged)
     {
         WsLayout L;
-        const int nn = n * n, ew = 32 / n;
+        const int ew = 32 / n;
         L.slot = ws_slot<Real>(n, chunk, staged).bytes;
         L.tab = 128;
         L.slots = (L.tab + 2 * n * (int)sizeof(Real) + 127) & ~127;
         L.scratch = L.slots + stages * L.slot;
-        L.warp_scratch = ((ew * 3 * nn * (int)sizeof(Real)) + 15) & ~15;
+        L.warp_scratch = ((ew * sum_el * (int)sizeof(Real)) + 15) & ~15;
         L.total = L.scratch + kWsConsumers * L.warp_scratch;
         return L;
     }
@@ -467,7 +518,8 @@ namespace wdg
         const int C = a.chunk, S = a.ring, G = gridDim.x;
         const int e0 = a.el_begin, e1 = a.el_end > 0 ? a.el_end : a.nel; // this launch's elements
         const int nchunks = (e1 - e0 + C - 1) / C;
-        const WsLayout L = ws_layout<Real>(N, C, S, WsStage<Real, EXTRA>::value);
+        constexpr SumStride RS = stream_sums(N); // a constant: not searched for in the kernel
+        const WsLayout L = ws_layout<Real>(N, RS.el, C, S, WsStage<Real, EXTRA>::value);
 
         extern __shared__ __align__(128) unsigned char smem[];
         uint64_t *full = reinterpret_cast<uint64_t *>(smem);
@@ -563,7 +615,10 @@ namespace wdg
         }
 
         // ---------------------------------------------------------------- consumers
-        Real *Rc = reinterpret_cast<Real *>(smem + L.scratch + warp * L.warp_scratch); // [EW][NN][3] column sums
+        Real *Rc = reinterpret_cast<Real *>(smem + L.scratch + warp * L.warp_scratch); // column sums
+        const WsSlot o = ws_slot<Real>(N, C, WsStage<Real, EXTRA>::value);
+        const int rounds = C / (kWsConsumers * (32 / N));
+        const Real xm = xt[lane % N], wm = wt[lane % N];
         for (int m = 0; m < M; ++m)
         {
             const int q = m % S;
@@ -574,7 +629,7 @@ namespace wdg
                 break;
             }
             at(m);
-            ws_consume<N, Real, EXTRA, false>(c, slots + q * L.slot, Rc, xt, wt, warp, lane);
+            ws_consume<N, Real, EXTRA, false>(c, slots + q * L.slot, o, rounds, Rc, xm, wm, warp, lane);
             // results are in the slot: hand them to the async proxy, then release the slot
             fence_async_smem();
             __syncwarp();
@@ -588,7 +643,7 @@ namespace wdg
     static bool ws_fits(const StageArgs<Real> &a)
     {
         const bool extra = (a.flags & (F_FORCE | F_FILTER)) != 0;
-        const size_t smem = (size_t)ws_layout<Real>(N, a.chunk, a.ring, extra && WsStage<Real, true>::value).total;
+        const size_t smem = (size_t)ws_layout<Real>(N, stream_sums(N).el, a.chunk, a.ring, extra && WsStage<Real, true>::value).total;
         return smem <= 227 * 1024;
     }
 
@@ -597,8 +652,8 @@ namespace wdg
     {
         const bool extra = (a.flags & (F_FORCE | F_FILTER)) != 0;
         auto kern = extra ? ws_stage_kernel<N, Real, true> : ws_stage_kernel<N, Real, false>;
-        const size_t smem = (size_t)(extra ? ws_layout<Real>(N, a.chunk, a.ring, WsStage<Real, true>::value).total
-                                           : ws_layout<Real>(N, a.chunk, a.ring).total);
+        const size_t smem = (size_t)(extra ? ws_layout<Real>(N, stream_sums(N).el, a.chunk, a.ring, WsStage<Real, true>::value).total
+                                           : ws_layout<Real>(N, stream_sums(N).el, a.chunk, a.ring).total);
 
         int dev = 0;
         cudaGetDevice(&dev);

@@ -167,6 +167,7 @@ namespace wdg
         a.ring = w->ws_ring;
         a.err = w->d_err;
         a.nread = w->halo ? (int)(w->ndof + w->halo) : 0;
+        a.line = w->explicit_launch ? 0 : 1;
         a.wait_ns = w->wait_ns;
         return a;
     }
@@ -808,10 +809,10 @@ extern "C"
             int family, a, b;
         };
         std::vector<Cand> cands;
-        // family 3 stands for family 2 with the elements resident, where they fit
+        // family 3 stands for family 2 without a launch shape of the caller's: the elements resident where
+        // they fit, the kernel of one warp per CTA elsewhere
         const bool save_explicit = w->explicit_launch;
-        if (w->d_flags && res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, w->max_ctas, false).fits)
-            cands.push_back({3, 0, 0});
+        cands.push_back({3, 0, 0});
         cands.push_back({0, save_tile, save_stages});
         for (int st = 2; st <= 4; ++st)
             for (int tile = 4; tile <= max_tile(w->n); tile += 4)

@@ -74,6 +74,43 @@ namespace wdg
         static __device__ __forceinline__ float D(int n, int k) { return c_tab[n].Df[k]; }
     };
 
+    // The column sums' strides (row j of an element, element): columns are written at 3 i, rows read at
+    // j * row, both with as few wavefronts as the 16 double-wide banks of a half-warp allow
+    struct SumStride
+    {
+        int row, el;
+    };
+    __host__ __device__ constexpr int sum_waves(int n, int a, int e)
+    {
+        int waves = 0;
+        for (int h = 0; h < 2; ++h)
+        {
+            int cnt[16] = {}, most = 0;
+            for (int i = 16 * h; i < 16 * h + 16 && i < 32 / n * n; ++i)
+                if (++cnt[(i / n * e + i % n * a) & 15] > most)
+                    most = cnt[(i / n * e + i % n * a) & 15];
+            waves += most;
+        }
+        return waves;
+    }
+    __host__ __device__ constexpr SumStride sum_strides(int n)
+    {
+        SumStride b{3 * n, 3 * n * n};
+        int cost = 1 << 30;
+        for (int row = 3 * n; row < 3 * n + 8; ++row)
+            for (int el = row * n; el < row * n + 6; ++el)
+            {
+                const int c = 32 * (sum_waves(n, 3, el) + sum_waves(n, row, el)) + (el - 3 * n * n) / 2;
+                if (c < cost)
+                {
+                    cost = c;
+                    b.row = row;
+                    b.el = el;
+                }
+            }
+        return b;
+    }
+
     template <int N>
     __device__ __forceinline__ int partner_stride(uint32_t byte)
     {

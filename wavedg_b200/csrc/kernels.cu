@@ -896,11 +896,12 @@ namespace wdg
     {
         // a launch over part of the elements exists only in the warp-specialised family
         const bool partial = a.el_begin != 0 || (a.el_end > 0 && a.el_end != a.nel);
-        const bool line = rk && line_takes<Real>(a, grid_limit);
+        const StageArgs<Real> la = rk ? a : line_operator(a);
+        const bool line = line_takes<Real>(la, grid_limit);
 #define WDG_CASE(NV)                                                                       \
     case NV:                                                                               \
         if (line)                                                                          \
-            return launch_line<NV, Real>(a, s);                                            \
+            return launch_line<NV, Real>(la, s);                                           \
         if (a.family == 2 && rk && a.use_tma && a.tma_out && ws_fits<NV, Real>(a))         \
             return launch_ws_n<NV, Real>(a, grid_limit, s);                                \
         if (partial)                                                                       \

@@ -58,31 +58,27 @@ namespace wdg
         return WDG_OK;
     }
 
-    // what resident launches need beside the state, where the mesh fits: flags and the two trace buffers (two
-    // allocations: the driver carves those below a megabyte out of what it has)
+    // what resident launches need beside the state, where the mesh fits: flags and the two trace buffers, in one
+    // allocation (each new piece of device memory costs a third of a millisecond, whatever its size)
     int ensure_resident(wdg_wave *w)
     {
         if (w->d_flags || w->halo || !res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, 0, false).fits)
             return WDG_OK;
         const size_t flags = (sizeof(unsigned long long) * res_flag_count(w->n, w->nel) + 255) & ~size_t(255);
-        const size_t trace = w->real_size() * 16 * (size_t)w->n * w->nel;
-        unsigned char *p = nullptr, *q = nullptr;
-        cudaError_t e = cudaMalloc((void **)&p, flags + trace);
-        if (e == cudaSuccess)
-            e = cudaMalloc((void **)&q, trace);
+        const size_t trace = (w->real_size() * 16 * (size_t)w->n * w->nel + 255) & ~size_t(255);
+        unsigned char *p = nullptr;
+        cudaError_t e = cudaMalloc((void **)&p, flags + 2 * trace);
         if (e == cudaSuccess)
             e = cudaMemsetAsync(p, 0, flags, w->stream);
         if (e != cudaSuccess)
         {
             if (p)
                 cudaFree(p);
-            if (q)
-                cudaFree(q);
             return cuda_fail(e, "cudaMalloc(trace buffers)");
         }
         w->d_flags = reinterpret_cast<unsigned long long *>(p);
         w->d_trace[0] = p + flags;
-        w->d_trace[1] = q;
+        w->d_trace[1] = p + flags + trace;
         return WDG_OK;
     }
 
@@ -635,7 +631,7 @@ extern "C"
         void *ptrs[] = {w->d_corners, w->d_nbr, w->d_finfo, w->d_face_edge, w->d_fbase, w->d_fcode, w->d_edgesI,
                         w->d_edgesB, w->d_codes,
                         w->d_state[0], w->d_state[1], w->d_state[2], w->d_du, w->d_stage[0], w->d_stage[1],
-                        w->d_stage[2], w->d_scratch, w->d_result, w->d_err, w->d_src, w->d_flags, w->d_trace[1]};
+                        w->d_stage[2], w->d_scratch, w->d_result, w->d_err, w->d_src, w->d_flags};
         for (void *p : ptrs)
             if (p)
                 cudaFree(p);

@@ -46,7 +46,7 @@ struct wdg_wave
     // resident launches, on handles whose mesh fits: a flag per element group, the value they count on
     // from, and two trace buffers (with the states)
     unsigned long long *d_flags = nullptr, flag_base = 0;
-    void *d_trace[2] = {nullptr, nullptr}; // (the first is part of d_flags' allocation)
+    void *d_trace[2] = {nullptr, nullptr}; // (parts of d_flags' allocation)
     unsigned long long wait_ns = 0; // limit of the stage kernels' bounded waits (0: kWaitLimitNs)
     int test_skip = 0;              // test hook: 1 + chunk the next RK launch leaves unloaded
     double *d_src = nullptr;    // gaussian source table

@@ -135,7 +135,7 @@ int wdg_wave_node_coords(wdg_wave *wave, double *xy);
 int wdg_wave_set_wait_limit(wdg_wave *wave, double seconds);
 /* Test hooks (no counterpart in the reference) that exercise that failure detection without
  * faulting the GPU.  wdg_test_skip_chunk: in the first stage launch of the next RK4 call that
- * takes the warp-specialised kernel, every CTA leaves its chunk number `chunk` unloaded (-1:
+ * streams (and takes the warp-specialised kernel for it), every CTA leaves its chunk number `chunk` unloaded (-1:
  * none), so the waits on that chunk run out.  wdg_test_set_partner: overwrites the fused
  * kernels' partner offset of (elem, side) (returns the previous value in *previous); an offset
  * outside the state makes the kernels skip that trace and report WDG_ERR_ARG ("neighbour
@@ -237,7 +237,7 @@ int wdg_euler_create(const wdg_mesh *mesh, int n_colloc, int device, wdg_claw **
 /* The same system with approx_quad = false, as examples/cl2d.cpp ships: DivF2D<false>
  * (wavedg/DivF.hpp:262-394) and EdgeFluxF2D<false> (wavedg/EdgeFluxF.hpp:182-254) on their
  * default 2n-point Gauss-Legendre rules (source/DivF.cpp:59, source/EdgeFluxF.cpp:55), the
- * face traces interpolated to the face rule, and MassMatrix<false>'s dense inverse.  The
+ * face traces interpolated to the face rule, and MassMatrix<false>'s exact inverse.  The
  * entry points below serve both kinds of handle. */
 int wdg_euler_create_exact(const wdg_mesh *mesh, int n_colloc, int device, wdg_claw **out);
 void wdg_claw_destroy(wdg_claw *claw);

@@ -21,6 +21,18 @@ extern "C" {
 int wdg_fno_gemm(const void *A, const void *B, float *C, int M, int N, int K, long long lda, long long ldb,
                  long long ldc, long long strideA, long long strideB, long long strideC, int batch, int transA,
                  int transB, float alpha, float beta, int ksplit, void *stream);
+/* Batch products op(A[b]) op(B[b]) with an epilogue instead of alpha and beta.  mode 1: v = product +
+ * bias[row], out = v, y = BF16 act(v).  mode 2: v = product times GELU'(z) (act) or the product,
+ * out = v, y = BF16 v.  out or y may be null; out, z and y have C's shape (M, ldc) per batch. */
+int wdg_fno_gemm_act(const void *A, const void *B, float *out, int M, int N, int K, long long lda, long long ldb,
+                     long long ldc, long long strideA, long long strideB, long long strideC, int batch, int transA,
+                     int transB, int mode, const float *bias, const float *z, void *y, int act, void *stream);
+/* A Fourier layer's output in one pass.  back = 0: z = W V + U X (U: the mixed spectrum after the inverse
+ * DFT along y, per channel and row, K1 wide; X: the inverse DFT along x) plus bias to out, BF16 GELU(z) (act)
+ * or z to y.  back = 1: W^T V + U X times GELU'(z) (act), to out and in BF16 to y.  out may be null.  C and
+ * K1 are multiples of 8 up to 32, G a multiple of 8, every array 16-byte aligned. */
+int wdg_fno_layer(const void *U, const void *X, const void *W, const void *V, const float *bias, const float *z,
+                  float *out, void *y, int B, int C, int K1, int G, int act, int back, void *stream);
 /* DFT along y on the retained wavenumbers ky(k) = k (k < K/2), k - K (k >= K/2):
  * forward (inverse = 0): out[bc, k, kx] = sum_y e^{sign i 2 pi ky y / G} in[bc, y, kx];
  * inverse (inverse = 1): out[bc, y, kx] = sum_k e^{sign i 2 pi ky y / G} in[bc, k, kx]

@@ -366,7 +366,7 @@ namespace
         return (size_t)h->n * 3 * 2 * (type == 0 ? h->w->nI : h->w->nB);
     }
 
-    int qfused_launch(wdg_waveq *h, const XArgs &a)
+    int exact_launch(wdg_waveq *h, const XArgs &a)
     {
         WDG_CUDA(xline_launch<WaveX>(h->n, a, h->w->stream));
         return WDG_OK;
@@ -375,7 +375,7 @@ namespace
     // nsteps of ode::RungeKutta4 on device array u (not a rotation buffer), one fused launch per
     // stage: the rotation u -> B -> C -> B -> C -> u of the wave handle's buffers; with F, the
     // forcing F s(t) at the stage times; with acc, acc += c_filter[step] u after each step
-    int qfused_rk4(wdg_waveq *h, double *u, double dt, double t, int nsteps, const double *F, double omega,
+    int exact_rk4(wdg_waveq *h, double *u, double dt, double t, int nsteps, const double *F, double omega,
                    double *acc, const double *c_filter)
     {
         wdg_wave *w = h->w;
@@ -400,7 +400,7 @@ namespace
                 a.fs = F ? -std::sin(omega * (t + rk4c[st] * dt)) / omega : 0.0;
                 a.acc = (st == 4) ? acc : nullptr;
                 a.acc_c = (st == 4 && acc) ? c_filter[step] : 0.0;
-                WDG_TRY(qfused_launch(h, a));
+                WDG_TRY(exact_launch(h, a));
                 src = dst;
             }
             t += dt;
@@ -467,7 +467,7 @@ namespace
         a.c.mode = CLAW_RHS;
         a.F = F;
         a.fs = s;
-        return qfused_launch(h, a);
+        return exact_launch(h, a);
     }
 
     typedef int (*Unary)(wdg_waveq *, const double *, double *);
@@ -502,7 +502,7 @@ namespace wdg
     int waveq_period(wdg_waveq *h, double *u, double dt, int nt, const double *F, double omega, double *acc,
                      const double *c_filter)
     {
-        return qfused_rk4(h, u, dt, 0.0, nt, F, omega, acc, c_filter);
+        return exact_rk4(h, u, dt, 0.0, nt, F, omega, acc, c_filter);
     }
 
     // P = M^{-1}(A + B) W on the exact operators (WaveHoltz::postprocess's RHS)
@@ -740,7 +740,7 @@ extern "C"
         wdg_wave *w = h->w;
         HostArg a;
         WDG_TRY(bind_arg(w, 0, u, w->ndof, true, true, a));
-        WDG_TRY(qfused_rk4(h, a.dev, dt, *t, nsteps, nullptr, 0.0, nullptr, nullptr));
+        WDG_TRY(exact_rk4(h, a.dev, dt, *t, nsteps, nullptr, 0.0, nullptr, nullptr));
         for (int s = 0; s < nsteps; ++s)
             *t += dt; // ode::RungeKutta4::step advances t once per step
         return finish_args(w, &a, 1);

@@ -1,6 +1,7 @@
 // Device kernels of libwdg_b200 (sm_100a).
 //
-// The hot kernel is `stage_kernel`: one pass over the state per RK stage that
+// A stage kernel is one pass over the state per RK stage (streaming kernels for aligned arrays:
+// stage_line.cuh, stage_ws.cuh; here `stage_kernel`, the tiled one, which takes any array) that
 // fuses what the reference does in eight separate loops per time derivative
 // and two per RK stage (Div::action, FaceProlongator::action, EdgeFlux::action,
 // FaceProlongator::t for interior and boundary faces, apply_bc_2d, the forcing

@@ -41,7 +41,8 @@ namespace wdg
         int tma_out;          // 1: full tiles of u' and du' are stored with cp.async.bulk (RK mode)
         int stages;           // pipeline depth (2..4): tiles whose bulk loads are in flight + 1
         int family;           // 0: warp-per-element kernel, 1: tiled TMA-pipeline kernel,
-                              // 2: warp-specialised kernel (RK launches on aligned arrays; else tiled)
+                              // 2: the streaming kernels (RK and operator launches on aligned arrays: one
+                              // warp per CTA, or warp-specialised; else tiled)
         int chunk;            // family 2: elements per chunk (a multiple of 8 x elements per warp-round)
         int ring;             // family 2: chunk slots in the shared-memory ring (2..6)
         Real rk_a, rk_b, dt, fscale;
@@ -73,7 +74,7 @@ namespace wdg
     int upload_basis_tables(int device);   // once per device
     bool degree_supported(int n);
     int default_tile(int n, bool fp32, int stages);
-    // the warp-specialised kernel for RK launches (operator launches take the tiled one)
+    // the streaming kernels
     inline int default_family(int) { return 2; }
     constexpr int kDefaultStages = 3;
     int max_tile(int n);

@@ -15,7 +15,7 @@
 // An FP32 group need not be a whole number of 16-byte units: it is loaded with the few bytes around it,
 // and stored in its whole units by bulk copies, the values beside them one by one.
 //
-// What bounds it: per element the shared-memory pipe (about 75 wavefronts at n = 5), the passes' dependent
+// What bounds it: per element the shared-memory pipe (90 wavefronts at n = 5, three quarters busy), the passes' dependent
 // FP64 chains with three warps per scheduler, and in FP32 the issue slots; HBM follows (512 x 512, n = 5:
 // 90 us a stage in FP64 and 46 in FP32 at the copy rate).  us a stage, against the warp-specialised kernel as
 // it was: FP64: 600 x 600, n = 3: 102 -> 81; 512 x 512, n = 4: 141 -> 96, n = 5: 139 -> 113; 400 x 400,

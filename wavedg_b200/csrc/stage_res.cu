@@ -22,9 +22,9 @@
 //
 // What bounds it: the latency of a group's chain (column sums, flags, traces, row sums, update) with
 // ten warps per SM, and the shared-memory pipe behind it (about 480 wavefronts per group and stage);
-// with one group per warp, the chain alone.  Per stage, FP64: 128 x 128, N = 5: 17.4 -> 9.1 us (forced
-// and unforced periods of WaveHoltz together), 32 x 32, N = 4: 8.2 -> 2.8 us against stage launches.
-// Tried: flags released late, after the next group's column sums (9.5 us); traces read in the state's
+// with one group per warp, the chain alone.  Per stage, FP64: 128 x 128, N = 5: 17.4 -> 7.7 us (forced
+// and unforced periods of WaveHoltz together), 32 x 32, N = 4: 8.2 -> 2.7 us against stage launches.
+// Tried, when the first stood at 9.1 us: flags released late, after the next group's column sums (9.5 us); traces read in the state's
 // layout (12.2 us), staged through shared memory (11.0 us), in 16-byte pieces (10.4 us).
 #include <cuda_runtime.h>
 

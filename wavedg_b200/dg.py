@@ -256,7 +256,7 @@ class Discretisation:
 
     def set_kernel(self, family: int) -> None:
         """0: warp per element, 1: tiled TMA pipeline, 2: warp-specialised TMA ring,
-        -1: default for this degree."""
+        -1: default (resident steps where the mesh fits the chip, else one warp per CTA)."""
         check(lib().wdg_wave_set_kernel(self._h, int(family)), "set_kernel")
 
     def launch_config(self) -> dict:
@@ -940,7 +940,7 @@ class EulerSystem:
     with the example's flux, EdgeFluxF2D with its local Lax-Friedrichs flux (exterior boundary
     state = interior state) and MassMatrix on GLL nodes, with the example's approx_quad switch:
     True for the collocation rule, False (as the example ships) for the 2n-point Gauss-Legendre
-    rules and the dense inverse mass matrix.  FP64."""
+    rules and the exact inverse mass matrix.  FP64."""
 
     n_var = 4
 

@@ -350,6 +350,7 @@ namespace wdg
                         ok = false;
                         break;
                     }
+                    __syncwarp(); // a side's traces are read by other lanes than the one that acquired its flag
                     // this line's four face nodes in the neighbours' traces, all in flight together
                     Real x[4][3];
 #pragma unroll

@@ -421,6 +421,9 @@ int wdg_whbatch_autotune(wdg_whbatch *batch, int steps, float *best_ms_per_step)
 int wdg_whbatch_solve(wdg_whbatch *batch, const double *const *F, double tol, int maxit, int stall_limit,
                       double *const *W, const int *warm, double *pi0_norm, int *iters, double *residuals,
                       int *status);
+/* Test hook: the call-th allocation (or stream, or event) that the batch's solves make for their
+ * resident periods from now on fails once, as an exhausted device's would (0: none). */
+int wdg_test_whbatch_fail(wdg_whbatch *batch, int call);
 
 #ifdef __cplusplus
 }

@@ -523,6 +523,8 @@ namespace wdg
     int res_rk4(wdg_wave *w, const ResPlan &p, Real *A, double dt, int nsteps, const RKExtras &x, bool &ran, cudaStream_t stream)
     {
         ran = false;
+        if ((x.F && !x.d_fscale) || (x.acc && !x.d_cfilter))
+            return fail(WDG_ERR_ARG, "resident steps: forcing or filter without its table");
         ResArgs<Real> a{};
         a.A = A;
         a.T[0] = static_cast<Real *>(w->d_trace[0]);

@@ -55,8 +55,10 @@ struct wdg_whbatch
     WhbState *h_state = nullptr; // pinned
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
-    // resident periods: per solve its tables, partial sums and stream (made on first use)
-    bool explicit_launch = false;
+    // resident periods: per solve its tables, partial sums and stream (made on first use; `ready` once
+    // all of them are)
+    bool explicit_launch = false, ready = false;
+    int test_fail = 0; // test hook: the set-up call that fails, counting from 1 (0: none)
     std::vector<double *> d_fscale, d_cfilter, d_end;
     std::vector<cudaStream_t> rs;
     std::vector<cudaEvent_t> rdone;
@@ -316,25 +318,40 @@ namespace
         return lo;
     }
 
+    // What resident periods need.  A call that fails leaves what was made before it for the next solve
+    // to go on from.
     int resident_prepare(wdg_whbatch *b)
     {
-        if (!b->rs.empty())
+        if (b->ready)
             return WDG_OK;
-        b->d_fscale.assign(b->n, nullptr);
-        b->d_cfilter.assign(b->n, nullptr);
-        b->d_end.assign(b->n, nullptr);
-        b->rs.assign(b->n, nullptr);
-        b->rdone.assign(b->n, nullptr);
-        WDG_CUDA(cudaMallocHost(&b->h_err, sizeof(unsigned) * b->n));
+        b->d_fscale.resize(b->n, nullptr);
+        b->d_cfilter.resize(b->n, nullptr);
+        b->d_end.resize(b->n, nullptr);
+        b->rs.resize(b->n, nullptr);
+        b->rdone.resize(b->n, nullptr);
+        auto make = [&](auto &p, auto call) -> int
+        {
+            if (p)
+                return WDG_OK;
+            const bool fails = b->test_fail > 0 && --b->test_fail == 0;
+            const cudaError_t e = fails ? cudaErrorMemoryAllocation : call(&p);
+            if (e == cudaSuccess)
+                return WDG_OK;
+            p = nullptr;
+            return cuda_fail(e, "batched WaveHoltz: set-up of the resident periods");
+        };
+        auto doubles = [](size_t count) { return [count](double **p) { return cudaMalloc((void **)p, sizeof(double) * count); }; };
+        WDG_TRY(make(b->h_err, [&](unsigned **p) { return cudaMallocHost((void **)p, sizeof(unsigned) * b->n); }));
         for (int s = 0; s < b->n; ++s)
         {
-            WDG_CUDA(cudaMalloc(&b->d_fscale[s], sizeof(double) * 5 * b->nt[s]));
-            WDG_CUDA(cudaMalloc(&b->d_cfilter[s], sizeof(double) * b->nt[s]));
-            WDG_CUDA(cudaMalloc(&b->d_end[s], sizeof(double) * 2 * kWhbEndBlocks));
-            WDG_CUDA(cudaStreamCreateWithFlags(&b->rs[s], cudaStreamNonBlocking));
-            WDG_CUDA(cudaEventCreateWithFlags(&b->rdone[s], cudaEventDisableTiming));
+            WDG_TRY(make(b->d_fscale[s], doubles(5 * (size_t)b->nt[s])));
+            WDG_TRY(make(b->d_cfilter[s], doubles((size_t)b->nt[s])));
+            WDG_TRY(make(b->d_end[s], doubles(2 * kWhbEndBlocks)));
+            WDG_TRY(make(b->rs[s], [](cudaStream_t *p) { return cudaStreamCreateWithFlags(p, cudaStreamNonBlocking); }));
+            WDG_TRY(make(b->rdone[s], [](cudaEvent_t *p) { return cudaEventCreateWithFlags(p, cudaEventDisableTiming); }));
             WDG_CUDA(launch_whb_tables(b->omega[s], b->dt[s], b->nt[s], b->d_fscale[s], b->d_cfilter[s], b->cs));
         }
+        b->ready = true;
         return WDG_OK;
     }
 
@@ -610,6 +627,14 @@ extern "C"
         Dev g(b->device);
         b->explicit_launch = true;
         return shape(b, rounds, ring);
+    }
+
+    int wdg_test_whbatch_fail(wdg_whbatch *b, int call)
+    {
+        if (!b || call < 0)
+            return fail(WDG_ERR_ARG, "wdg_test_whbatch_fail: call must be >= 1 (or 0: none)");
+        b->test_fail = call;
+        return WDG_OK;
     }
 
     int wdg_whbatch_get_launch(const wdg_whbatch *b, int *rounds, int *ring, int *grid)

@@ -554,8 +554,9 @@ namespace wdg
             a.fscale = x.d_fscale ? x.d_fscale + 5 * s0 : nullptr;
             a.cfilter = x.d_cfilter ? x.d_cfilter + s0 : nullptr;
             // A replayed graph repeats this launch with the same base, so its flags start below it again;
-            // launches outside a graph count on from a base no replay has reached
-            if (cap == cudaStreamCaptureStatusActive)
+            // launches outside a graph count on from a base no replay has reached, the first from zero
+            const bool captured = cap == cudaStreamCaptureStatusActive;
+            if (captured || !w->flags_set)
                 WDG_CUDA(cudaMemsetAsync(w->d_flags, 0, sizeof(unsigned long long) * kFlagStride * p.ngroups, stream));
             a.base = w->flag_base;
             cudaError_t e = cudaErrorInvalidValue;
@@ -579,6 +580,7 @@ namespace wdg
             if (e != cudaSuccess)
                 return cuda_fail(e, "resident stage kernel launch");
             w->flag_base += 5ull * a.nsteps + 1;
+            w->flags_set = w->flags_set || !captured;
             ran = true;
         }
         return WDG_OK;

@@ -58,71 +58,42 @@ namespace wdg
         return WDG_OK;
     }
 
-    // what resident launches need beside the state, where the mesh fits: flags and the two trace buffers, in one
-    // allocation (each new piece of device memory costs a third of a millisecond, whatever its size)
-    int ensure_resident(wdg_wave *w)
-    {
-        if (w->d_flags || w->halo || !res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, 0, false).fits)
-            return WDG_OK;
-        const size_t flags = (sizeof(unsigned long long) * res_flag_count(w->n, w->nel) + 255) & ~size_t(255);
-        const size_t trace = (w->real_size() * 16 * (size_t)w->n * w->nel + 255) & ~size_t(255);
-        unsigned char *p = nullptr;
-        cudaError_t e = cudaMalloc((void **)&p, flags + 2 * trace);
-        if (e == cudaSuccess)
-            e = cudaMemsetAsync(p, 0, flags, w->stream);
-        if (e != cudaSuccess)
-        {
-            if (p)
-                cudaFree(p);
-            return cuda_fail(e, "cudaMalloc(trace buffers)");
-        }
-        w->d_flags = reinterpret_cast<unsigned long long *>(p);
-        w->d_trace[0] = p + flags;
-        w->d_trace[1] = p + flags + trace;
-        return WDG_OK;
-    }
-
-    // the three state buffers and the RK register, allocated on first use so
+    // The three state buffers and the RK register, allocated on first use so
     // that operator-only handles (WaveEquation, WaveBC, MassMatrix drop-ins)
-    // hold geometry only
-    static int ensure_state(wdg_wave *w, int k)
-    {
-        if (!w->d_state[k])
-        {
-            cudaError_t e = cudaMalloc(&w->d_state[k], w->real_size() * (size_t)(w->ndof + w->halo) + 64);
-            if (e != cudaSuccess)
-            {
-                w->d_state[k] = nullptr;
-                return cuda_fail(e, "cudaMalloc(state)");
-            }
-        }
-        return WDG_OK;
-    }
+    // hold geometry only.  Where the mesh may be resident, the rotation buffers are also
+    // large enough to serve as its trace buffers and the register is followed by its flags: a step is
+    // resident or streams, never both, and after this neither allocates, in a capture or out of one.
     int ensure_states(wdg_wave *w)
     {
+        if (w->d_du)
+            return WDG_OK; // the last of them
+        const bool res = !w->halo && res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, 0, false).fits;
+        const size_t trace = res ? w->real_size() * 16 * (size_t)w->n * w->nel : 0;
         for (int k = 0; k < 3; ++k)
-            WDG_TRY(ensure_state(w, k));
-        if (!w->d_du)
-        {
-            cudaError_t e = cudaMalloc(&w->d_du, w->real_size() * (size_t)w->ndof + 64);
-            if (e != cudaSuccess)
+            if (!w->d_state[k])
             {
-                w->d_du = nullptr;
-                return cuda_fail(e, "cudaMalloc(du)");
+                const size_t state = w->real_size() * (size_t)(w->ndof + w->halo);
+                cudaError_t e = cudaMalloc(&w->d_state[k], (k > 0 ? std::max(state, trace) : state) + 64);
+                if (e != cudaSuccess)
+                {
+                    w->d_state[k] = nullptr;
+                    return cuda_fail(e, "cudaMalloc(state)");
+                }
             }
+        const size_t du = (w->real_size() * (size_t)w->ndof + 64 + 255) & ~size_t(255);
+        cudaError_t e = cudaMalloc(&w->d_du, du + (res ? sizeof(unsigned long long) * res_flag_count(w->n, w->nel) : 0));
+        if (e != cudaSuccess)
+        {
+            w->d_du = nullptr;
+            return cuda_fail(e, "cudaMalloc(du)");
+        }
+        if (res)
+        {
+            w->d_flags = reinterpret_cast<unsigned long long *>(static_cast<unsigned char *>(w->d_du) + du);
+            w->d_trace[0] = w->d_state[1];
+            w->d_trace[1] = w->d_state[2];
         }
         return WDG_OK;
-    }
-    // what WaveHoltz periods need before one is captured: the rotation buffers and the register only where
-    // they will not be resident
-    int ensure_period(wdg_wave *w)
-    {
-        auto fits = [&](bool forced)
-        { return res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, w->max_ctas, forced).fits; };
-        if (w->family != 2 || w->explicit_launch || w->halo || !fits(true) || !fits(false))
-            return ensure_states(w);
-        WDG_TRY(ensure_state(w, 0));
-        return ensure_resident(w);
     }
 
     int check_device_error(wdg_wave *w)
@@ -173,14 +144,14 @@ namespace wdg
     {
         if (A && (A == w->d_state[1] || A == w->d_state[2]))
             return fail(WDG_ERR_ARG, "rk4: state buffer aliases the rotation buffers");
+        WDG_TRY(ensure_states(w));
         // a mesh that fits the chip stays there for all steps (unless the caller chose a kernel, or the
         // skipped-chunk test asks for the streaming one)
         if (w->family == 2 && !w->explicit_launch && !w->test_skip && nsteps > 0 && (!x.F || x.d_fscale) &&
-            (!x.acc || x.d_cfilter))
+            (!x.acc || x.d_cfilter) && w->d_flags)
         {
-            WDG_TRY(ensure_resident(w));
             const ResPlan p = res_plan(w->n, sizeof(Real) == 4, w->nel, w->sms, w->max_ctas, x.F != nullptr);
-            if (p.fits && w->d_flags)
+            if (p.fits)
             {
                 bool ran = false;
                 WDG_TRY(res_rk4<Real>(w, p, A, dt, nsteps, x, ran, w->stream));
@@ -192,7 +163,6 @@ namespace wdg
                 }
             }
         }
-        WDG_TRY(ensure_states(w));
         Real *B = static_cast<Real *>(w->d_state[1]);
         Real *Cb = static_cast<Real *>(w->d_state[2]);
         Real *du = static_cast<Real *>(w->d_du);
@@ -631,7 +601,7 @@ extern "C"
         void *ptrs[] = {w->d_corners, w->d_nbr, w->d_finfo, w->d_face_edge, w->d_fbase, w->d_fcode, w->d_edgesI,
                         w->d_edgesB, w->d_codes,
                         w->d_state[0], w->d_state[1], w->d_state[2], w->d_du, w->d_stage[0], w->d_stage[1],
-                        w->d_stage[2], w->d_scratch, w->d_result, w->d_err, w->d_src, w->d_flags};
+                        w->d_stage[2], w->d_scratch, w->d_result, w->d_err, w->d_src};
         for (void *p : ptrs)
             if (p)
                 cudaFree(p);
@@ -789,7 +759,6 @@ extern "C"
             return fail(WDG_ERR_ARG, "wdg_wave_autotune: bad arguments");
         DeviceGuard g(w->device);
         WDG_TRY(ensure_states(w));
-        WDG_TRY(ensure_resident(w));
         cudaEvent_t e0, e1;
         WDG_CUDA(cudaEventCreate(&e0));
         WDG_CUDA(cudaEventCreate(&e1));

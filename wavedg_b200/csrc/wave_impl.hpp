@@ -43,10 +43,11 @@ struct wdg_wave
     double *d_result = nullptr; // 8 doubles
     double *h_result = nullptr; // pinned, 8 doubles
     unsigned *d_err = nullptr;
-    // resident launches, on handles whose mesh fits: a flag per element group, the value they count on
-    // from, and two trace buffers (with the states)
+    // resident launches, on handles whose mesh fits: a flag per element group (behind d_du), the value they
+    // count on from, whether they are set, and two trace buffers (the rotation buffers)
     unsigned long long *d_flags = nullptr, flag_base = 0;
-    void *d_trace[2] = {nullptr, nullptr}; // (parts of d_flags' allocation)
+    bool flags_set = false;
+    void *d_trace[2] = {nullptr, nullptr};
     unsigned long long wait_ns = 0; // limit of the stage kernels' bounded waits (0: kWaitLimitNs)
     int test_skip = 0;              // test hook: 1 + chunk the next RK launch leaves unloaded
     double *d_src = nullptr;    // gaussian source table
@@ -61,8 +62,6 @@ namespace wdg
     int is_device_ptr(const wdg_wave *w, const void *p, bool &dev);
     int ensure_stage(wdg_wave *w, int k);
     int ensure_states(wdg_wave *w);
-    int ensure_resident(wdg_wave *w);
-    int ensure_period(wdg_wave *w);
     int check_device_error(wdg_wave *w);
     int sync(wdg_wave *w);
 

@@ -82,8 +82,6 @@ namespace
     {
         wdg_wave *w = h->w;
         const bool fp32 = w->precision == WDG_FP32;
-        if (!h->q)
-            WDG_TRY(ensure_period(w)); // the launch settings may have changed since
         WDG_CUDA(cudaStreamBeginCapture(h->cs, cudaStreamCaptureModeThreadLocal));
         int s = WDG_OK;
         cudaError_t e = cudaSuccess;
@@ -197,7 +195,7 @@ extern "C"
         cudaGetDevice(&dev_prev);
         cudaSetDevice(w->device);
         // state buffers must exist before a period is captured into a graph
-        int s = ensure_period(w);
+        int s = ensure_states(w);
         cudaError_t e = (s == WDG_OK) ? cudaStreamCreateWithFlags(&h->cs, cudaStreamNonBlocking) : cudaSuccess;
         if (e == cudaSuccess)
             e = cudaEventCreateWithFlags(&h->ev_in, cudaEventDisableTiming);

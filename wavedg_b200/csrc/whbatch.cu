@@ -204,8 +204,6 @@ namespace
     {
         const bool fp32 = b->precision == WDG_FP32;
         const bool fork = b->groups.size() > 1;
-        for (wdg_wave *w : b->w)
-            WDG_TRY(ensure_states(w));
         WDG_CUDA(cudaStreamBeginCapture(b->cs, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = cudaSuccess;
         for (int k = 0; k < kGraphSteps && e == cudaSuccess; ++k)
@@ -516,7 +514,7 @@ extern "C"
             b->dt.push_back(dt);
             b->nt.push_back(nt);
             b->c0.push_back(0.5 * dt * K(omegas[u], 0.0));
-            st = ensure_period(w);
+            st = ensure_states(w);
             const size_t nd = (size_t)w->ndof;
             cudaError_t e = cudaSuccess;
             if (st == WDG_OK)

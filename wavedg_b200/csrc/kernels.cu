@@ -819,11 +819,13 @@ namespace wdg
     }
     int ws_warp_scratch_bytes(int n, bool fp32)
     {
-        return fp32 ? ws_layout<float>(n, stream_sums(n).el, 0, 0).warp_scratch : ws_layout<double>(n, stream_sums(n).el, 0, 0).warp_scratch;
+        const int el = stream_sums_el(n);
+        return fp32 ? ws_layout<float>(n, el, 0, 0).warp_scratch : ws_layout<double>(n, el, 0, 0).warp_scratch;
     }
     size_t ws_smem_bytes(int n, bool fp32, int chunk, int ring)
     {
-        return fp32 ? (size_t)ws_layout<float>(n, stream_sums(n).el, chunk, ring).total : (size_t)ws_layout<double>(n, stream_sums(n).el, chunk, ring).total;
+        const int el = stream_sums_el(n);
+        return fp32 ? (size_t)ws_layout<float>(n, el, chunk, ring).total : (size_t)ws_layout<double>(n, el, chunk, ring).total;
     }
     int ws_default_chunk(int n, bool fp32)
     {

@@ -92,9 +92,9 @@ namespace wdg
             return real == 4 ? ((32 / n) * 3 * n * n * real + 15) & ~15 : 0;
         }
         // a warp's scratch: the forcing (FP64), then the column sums of a group
-        __host__ __device__ constexpr int res_scratch(int n, int real)
+        __host__ __device__ constexpr int res_scratch(int n, SumStride sums, int real)
         {
-            return ((32 / n) * sum_strides(n).el * real + 15) & ~15;
+            return ((32 / n) * sums.el * real + 15) & ~15;
         }
 
         __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p)
@@ -135,8 +135,8 @@ namespace wdg
             const int ng = (int)((long long)(blockIdx.x + 1) * a.ngroups / gridDim.x) - g_lo; // this CTA's groups
             const int most = (a.ngroups + gridDim.x - 1) / gridDim.x;
             unsigned char *groups = rsm;
-            constexpr int kScratch = res_scratch(N, sizeof(Real));
             constexpr SumStride RS = sum_strides(N);
+            constexpr int kScratch = res_scratch(N, RS, sizeof(Real));
             constexpr bool LATE = kLateForcing<Real>;
             const int scratch = kScratch + (a.F ? res_forcing(N, sizeof(Real)) : 0);
             Real *Rc = reinterpret_cast<Real *>(groups + (size_t)most * L.bytes + (size_t)warp * scratch);
@@ -502,7 +502,7 @@ namespace wdg
             return p;
         const int most = (p.ngroups + p.ctas - 1) / p.ctas;
         const size_t gb = (size_t)(fp32 ? res_layout<float>(n).bytes : res_layout<double>(n).bytes);
-        const size_t sc = (size_t)res_scratch(n, fp32 ? 4 : 8) + (forced ? res_forcing(n, fp32 ? 4 : 8) : 0);
+        const size_t sc = (size_t)res_scratch(n, sum_strides_at(n), fp32 ? 4 : 8) + (forced ? res_forcing(n, fp32 ? 4 : 8) : 0);
         // as few rounds of groups per warp as twelve warps allow, the warps evened out over them; fewer
         // warps where their scratch is what does not fit
         for (int rounds = (most + kResMaxWarps - 1) / kResMaxWarps; rounds <= most && rounds <= 4 * kResMaxWarps; ++rounds)

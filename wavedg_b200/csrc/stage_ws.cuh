@@ -51,6 +51,7 @@ namespace wdg
     // the column sums' strides: dense for odd n, whose strides are odd as they are (n = 5: padding saves 5
     // of 90 wavefronts an element and costs 1 KB a warp; 147 -> 160 us a stage of 512 x 512)
     __host__ __device__ constexpr SumStride stream_sums(int n) { return n % 2 ? SumStride{3 * n, 3 * n * n} : sum_strides(n); }
+    inline int stream_sums_el(int n) { return n % 2 ? 3 * n * n : sum_strides_at(n).el; }
 
     int ws_epw(int n) { return 32 / n; }
 
@@ -643,7 +644,8 @@ namespace wdg
     static bool ws_fits(const StageArgs<Real> &a)
     {
         const bool extra = (a.flags & (F_FORCE | F_FILTER)) != 0;
-        const size_t smem = (size_t)ws_layout<Real>(N, stream_sums(N).el, a.chunk, a.ring, extra && WsStage<Real, true>::value).total;
+        constexpr int el = stream_sums(N).el;
+        const size_t smem = (size_t)ws_layout<Real>(N, el, a.chunk, a.ring, extra && WsStage<Real, true>::value).total;
         return smem <= 227 * 1024;
     }
 
@@ -652,8 +654,9 @@ namespace wdg
     {
         const bool extra = (a.flags & (F_FORCE | F_FILTER)) != 0;
         auto kern = extra ? ws_stage_kernel<N, Real, true> : ws_stage_kernel<N, Real, false>;
-        const size_t smem = (size_t)(extra ? ws_layout<Real>(N, stream_sums(N).el, a.chunk, a.ring, WsStage<Real, true>::value).total
-                                           : ws_layout<Real>(N, stream_sums(N).el, a.chunk, a.ring).total);
+        constexpr int el = stream_sums(N).el;
+        const size_t smem = (size_t)(extra ? ws_layout<Real>(N, el, a.chunk, a.ring, WsStage<Real, true>::value).total
+                                           : ws_layout<Real>(N, el, a.chunk, a.ring).total);
 
         int dev = 0;
         cudaGetDevice(&dev);

@@ -110,6 +110,23 @@ namespace wdg
             }
         return b;
     }
+    // the same where the host has n at run time: a table made by the compiler, for the search takes a host
+    // core 10 us
+    inline SumStride sum_strides_at(int n)
+    {
+        struct Table
+        {
+            SumStride s[kMaxN + 1];
+        };
+        static constexpr Table t = []
+        {
+            Table m{};
+            for (int k = kMinN; k <= kMaxN; ++k)
+                m.s[k] = sum_strides(k);
+            return m;
+        }();
+        return t.s[n];
+    }
 
     template <int N>
     __device__ __forceinline__ int partner_stride(uint32_t byte)

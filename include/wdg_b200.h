@@ -141,6 +141,9 @@ int wdg_wave_set_wait_limit(wdg_wave *wave, double seconds);
  * outside the state makes the kernels skip that trace and report WDG_ERR_ARG ("neighbour
  * index outside the mesh") instead of reading out of bounds. */
 int wdg_test_skip_chunk(wdg_wave *wave, int chunk);
+/* *ctas: the CTAs on which the handle's next steps (forced: with forcing) run with the mesh resident on
+ * the chip; 0: they stream */
+int wdg_test_resident(wdg_wave *wave, int forced, int *ctas);
 int wdg_test_set_partner(wdg_wave *wave, int elem, int side, int offset, int *previous);
 
 /* ---- Operator::action drop-ins, FP64, accumulate (y += A x) ---- */

@@ -139,18 +139,24 @@ namespace wdg
         return a;
     }
 
+    // (the skipped-chunk test asks for the streaming kernel)
+    ResPlan res_plan_of(const wdg_wave *w, bool forced, int max_ctas)
+    {
+        if (w->family != 2 || w->explicit_launch || w->test_skip || !w->d_flags)
+            return ResPlan{};
+        return res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, max_ctas, forced);
+    }
+
     template <typename Real>
     int rk4_run(wdg_wave *w, Real *A, double dt, double &t, int nsteps, const RKExtras &x)
     {
         if (A && (A == w->d_state[1] || A == w->d_state[2]))
             return fail(WDG_ERR_ARG, "rk4: state buffer aliases the rotation buffers");
         WDG_TRY(ensure_states(w));
-        // a mesh that fits the chip stays there for all steps (unless the caller chose a kernel, or the
-        // skipped-chunk test asks for the streaming one)
-        if (w->family == 2 && !w->explicit_launch && !w->test_skip && nsteps > 0 && (!x.F || x.d_fscale) &&
-            (!x.acc || x.d_cfilter) && w->d_flags)
+        // a mesh that fits the chip stays there for all steps, unless the caller chose a kernel
+        if (nsteps > 0 && (!x.F || x.d_fscale) && (!x.acc || x.d_cfilter))
         {
-            const ResPlan p = res_plan(w->n, sizeof(Real) == 4, w->nel, w->sms, w->max_ctas, x.F != nullptr);
+            const ResPlan p = res_plan_of(w, x.F != nullptr, w->max_ctas);
             if (p.fits)
             {
                 bool ran = false;
@@ -637,7 +643,8 @@ extern "C"
         return sync(w);
     }
 
-    static int ws_set(wdg_wave *w, int chunk, int ring)
+    // chose: the choice (kChoseTile or kChoseStages) this call makes, or takes back with `def`
+    static int ws_set(wdg_wave *w, int chunk, int ring, int chose, bool def)
     {
         const bool fp32 = w->precision == WDG_FP32;
         if (chunk == 0)
@@ -653,7 +660,7 @@ extern "C"
             return fail(WDG_ERR_ARG, "warp-specialised kernel: chunk x ring too large for shared memory");
         w->ws_chunk = chunk;
         w->ws_ring = ring;
-        w->explicit_launch = true;
+        w->explicit_launch = def ? w->explicit_launch & ~chose : w->explicit_launch | chose;
         return WDG_OK;
     }
 
@@ -662,7 +669,7 @@ extern "C"
         if (!w)
             return fail(WDG_ERR_ARG, "null discretisation");
         if (w->family == 2)
-            return ws_set(w, tile, w->ws_ring);
+            return ws_set(w, tile, w->ws_ring, kChoseTile, tile == 0);
         if (tile == 0)
             tile = default_tile(w->n, w->precision == WDG_FP32, w->stages);
         if (tile < 4 || (tile & 3) || tile > max_tile(w->n))
@@ -682,7 +689,7 @@ extern "C"
             const int unit = ws_chunk_unit(w->n), ring = stages ? stages : kWsDefaultRing;
             while (chunk > unit && ws_smem_bytes(w->n, w->precision == WDG_FP32, chunk, ring) > kMaxSmem)
                 chunk -= unit;
-            return ws_set(w, chunk, ring);
+            return ws_set(w, chunk, ring, kChoseStages, stages == 0);
         }
         if (!w || stages < 0 || stages == 1 || stages > 4)
             return fail(WDG_ERR_ARG, "wdg_wave_set_stages: stages must be 2, 3 or 4 (0 = default)");
@@ -714,6 +721,17 @@ extern "C"
         return WDG_OK;
     }
 
+    int wdg_test_resident(wdg_wave *w, int forced, int *ctas)
+    {
+        if (!w || !ctas)
+            return fail(WDG_ERR_ARG, "wdg_test_resident: bad arguments");
+        DeviceGuard g(w->device);
+        WDG_TRY(ensure_states(w));
+        const ResPlan p = res_plan_of(w, forced != 0, w->max_ctas);
+        *ctas = p.fits ? p.ctas : 0;
+        return WDG_OK;
+    }
+
     int wdg_test_set_partner(wdg_wave *w, int elem, int side, int offset, int *previous)
     {
         if (!w || elem < 0 || elem >= w->nel || side < 0 || side > 3)
@@ -736,7 +754,7 @@ extern "C"
             return fail(WDG_ERR_ARG,
                         "wdg_wave_set_kernel: 0 (warp per element), 1 (tiled), 2 (warp-specialised) or -1 (default)");
         w->family = (family < 0) ? default_family(w->n) : family;
-        w->explicit_launch = family >= 0;
+        w->explicit_launch = (family < 0) ? 0 : w->explicit_launch | kChoseKernel;
         return WDG_OK;
     }
 
@@ -776,7 +794,7 @@ extern "C"
         std::vector<Cand> cands;
         // family 3 stands for family 2 without a launch shape of the caller's: the elements resident where
         // they fit, the kernel of one warp per CTA elsewhere
-        const bool save_explicit = w->explicit_launch;
+        const int save_explicit = w->explicit_launch;
         cands.push_back({3, 0, 0});
         cands.push_back({0, save_tile, save_stages});
         for (int st = 2; st <= 4; ++st)
@@ -791,7 +809,7 @@ extern "C"
             {
                 const Cand &cd = cands[ci];
                 w->family = std::min(cd.family, 2);
-                w->explicit_launch = cd.family != 3;
+                w->explicit_launch = (cd.family != 3) ? kChoseKernel : 0;
                 w->tile = (cd.family == 1) ? cd.a : save_tile;
                 w->stages = (cd.family == 1) ? cd.b : save_stages;
                 w->ws_chunk = (cd.family == 2) ? cd.a : save_chunk;
@@ -834,7 +852,7 @@ extern "C"
         w->tile = (s == WDG_OK) ? bt : save_tile;
         w->stages = (s == WDG_OK) ? bs : save_stages;
         w->family = (s == WDG_OK) ? std::min(bf, 2) : save_family;
-        w->explicit_launch = (s == WDG_OK) ? bf != 3 : save_explicit;
+        w->explicit_launch = (s != WDG_OK) ? save_explicit : (bf != 3) ? kChoseKernel : 0;
         w->ws_chunk = (s == WDG_OK) ? bc : save_chunk;
         w->ws_ring = (s == WDG_OK) ? br : save_ring;
         if (s == WDG_OK)

@@ -15,7 +15,7 @@ struct wdg_wave
     int n = 0, nel = 0, precision = WDG_FP64, tile = 0, max_ctas = 0, stages = wdg::kDefaultStages;
     int family = 0; // fused-kernel family: 0 warp-per-element, 1 tiled TMA pipeline, 2 warp-specialised
     int ws_chunk = 0, ws_ring = wdg::kWsDefaultRing; // family 2 launch shape
-    bool explicit_launch = false; // the caller chose a kernel or its shape: no resident launches
+    int explicit_launch = 0; // what the caller chose (wdg::kChose*): no resident launches, no kernel of one warp per CTA
     int sms = 0;
     long long ndof = 0;
     long long halo = 0; // values of neighbour traces appended after the elements in each state
@@ -61,6 +61,13 @@ namespace wdg
     // which memory an argument lives in
     int is_device_ptr(const wdg_wave *w, const void *p, bool &dev);
     int ensure_stage(wdg_wave *w, int k);
+    // wdg_wave::explicit_launch: the kernel, its elements per block, its pipeline depth
+    enum : int
+    {
+        kChoseKernel = 1,
+        kChoseTile = 2,
+        kChoseStages = 4
+    };
     int ensure_states(wdg_wave *w);
     int check_device_error(wdg_wave *w);
     int sync(wdg_wave *w);
@@ -88,6 +95,9 @@ namespace wdg
         size_t smem = 0;
     };
     ResPlan res_plan(int n, bool fp32, int nel, int sms, int max_ctas, bool forced);
+    // the plan of a handle's next resident launch, on at most max_ctas (0: all) SMs; fits = false where
+    // its steps stream
+    ResPlan res_plan_of(const wdg_wave *w, bool forced, int max_ctas);
     size_t res_flag_count(int n, int nel);
     int upload_res_tables(int device); // once per device
     // nsteps of RK4 on A, on `stream`; ran = false (and nothing done) where the device cannot hold the launch

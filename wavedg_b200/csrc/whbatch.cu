@@ -295,9 +295,7 @@ namespace
     int least_ctas(const wdg_whbatch *b, int s)
     {
         const wdg_wave *w = b->w[s];
-        if (!w->d_flags || w->family != 2 || w->explicit_launch)
-            return 0;
-        auto fits = [&](int c) { return res_plan(w->n, b->precision == WDG_FP32, w->nel, w->sms, c, true).fits; };
+        auto fits = [&](int c) { return res_plan_of(w, true, c).fits; };
         const int most = w->max_ctas > 0 ? std::min(w->sms, w->max_ctas) : w->sms;
         if (!fits(most))
             return 0;

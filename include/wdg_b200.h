@@ -427,6 +427,8 @@ int wdg_whbatch_solve(wdg_whbatch *batch, const double *const *F, double tol, in
 /* Test hook: the call-th allocation (or stream, or event) that the batch's solves make for their
  * resident periods from now on fails once, as an exhausted device's would (0: none). */
 int wdg_test_whbatch_fail(wdg_whbatch *batch, int call);
+/* ctas[s]: the CTAs on which solve s runs in a solve's first round of resident periods (0: not in it) */
+int wdg_test_whbatch_shares(const wdg_whbatch *batch, int *ctas);
 
 #ifdef __cplusplus
 }

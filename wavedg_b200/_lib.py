@@ -158,6 +158,7 @@ SIGNATURES = {
     "wdg_whbatch_destroy": ([_v], None),
     "wdg_whbatch_params": ([_v, _i, _dp, _dp, _ip], _i),
     "wdg_test_resident": ([_v, _i, C.POINTER(_i)], _i),
+    "wdg_test_whbatch_shares": ([_v, _v], _i),
     "wdg_test_whbatch_fail": ([_v, _i], _i),
     "wdg_whbatch_set_launch": ([_v, _i, _i], _i),
     "wdg_whbatch_get_launch": ([_v, _ip, _ip, _ip], _i),

@@ -362,7 +362,7 @@ namespace
         x.acc = b->d_acc[s];
         x.d_fscale = b->d_fscale[s];
         x.d_cfilter = b->d_cfilter[s];
-        const ResPlan p = res_plan(w->n, sizeof(Real) == 4, w->nel, w->sms, ctas, true);
+        const ResPlan p = res_plan_of(w, true, ctas);
         Real *u = static_cast<Real *>(w->d_state[0]);
         WDG_TRY(res_rk4<Real>(w, p, u, b->dt[s], b->nt[s], x, ran, b->rs[s]));
         if (ran)
@@ -371,71 +371,85 @@ namespace
         return WDG_OK;
     }
 
-    // Every solve that can be resident, to its end; the others' records stay as they are.  A round holds as
-    // many running solves as the SMs do, each on at least its least share and on two rounds of groups per warp
-    // where it has them; what is left of the SMs goes by the work of a period.
-    int resident_solves(wdg_whbatch *b)
+    // least_ctas of every solve; all 0 where the caller chose the batch's launch shape
+    std::vector<int> least_shares(const wdg_whbatch *b)
     {
         std::vector<int> least(b->n, 0);
-        bool any = false;
-        int sms = b->w[0]->sms;
+        for (int s = 0; s < b->n && !b->explicit_launch; ++s)
+            least[s] = least_ctas(b, s);
+        return least;
+    }
+
+    // The CTAs of each solve in the next round (0: not in it).  A round holds as many running solves as the
+    // SMs do, each on at least its least share and on two rounds of groups per warp where it has them; what
+    // is left of the SMs goes by the work of a period.  No share exceeds its handle's CTA limit.
+    std::vector<int> round_shares(const wdg_whbatch *b, const std::vector<int> &least, const std::vector<char> &running)
+    {
+        const int sms = b->w[0]->sms;
+        std::vector<int> share(b->n, 0), cap(b->n);
+        int used = 0;
         for (int s = 0; s < b->n; ++s)
-            any = (least[s] = b->explicit_launch ? 0 : least_ctas(b, s)) > 0 || any;
-        if (!any)
-            return WDG_OK;
-        WDG_TRY(resident_prepare(b));
-        std::vector<double> work(b->n);
-        for (int s = 0; s < b->n; ++s)
-            work[s] = (double)b->w[s]->ndof * b->nt[s];
-        for (;;)
         {
-            std::vector<int> in, share;
-            int used = 0;
+            const wdg_wave *w = b->w[s];
+            const int ngroups = (w->nel + 32 / w->n - 1) / (32 / w->n);
+            cap[s] = std::min(w->max_ctas > 0 ? std::min(sms, w->max_ctas) : sms, ngroups);
+            if (!least[s] || !running[s])
+                continue;
+            const int want = std::max(least[s], std::min(cap[s], (ngroups + 23) / 24));
+            if (used > 0 && used + want > sms)
+                continue;
+            share[s] = want;
+            used += want;
+        }
+        // the SMs left over, to the solve with the longest period so far
+        for (int left = sms - used; left > 0; --left)
+        {
+            int at = -1;
+            double longest = 0.0;
             for (int s = 0; s < b->n; ++s)
             {
-                if (!least[s] || !b->h_state[s].active)
-                    continue;
-                const ResPlan p = res_plan(b->w[s]->n, b->precision == WDG_FP32, b->w[s]->nel, sms, least[s], true);
-                const int want = std::max(least[s], std::min(sms, (p.ngroups + 23) / 24));
-                if (!in.empty() && used + want > sms)
-                    continue;
-                in.push_back(s);
-                share.push_back(want);
-                used += want;
-            }
-            if (in.empty())
-                return WDG_OK;
-            // the SMs left over, to the solve with the longest period so far
-            for (int left = sms - used; left > 0; --left)
-            {
-                int at = -1;
-                double longest = 0.0;
-                for (size_t k = 0; k < in.size(); ++k)
+                const double work = (double)b->w[s]->ndof * b->nt[s];
+                if (share[s] > 0 && share[s] < cap[s] && work / share[s] > longest)
                 {
-                    const wdg_wave *w = b->w[in[k]];
-                    const int cap = std::min(w->max_ctas > 0 ? std::min(sms, w->max_ctas) : sms, (w->nel + 32 / w->n - 1) / (32 / w->n));
-                    if (share[k] < cap && work[in[k]] / share[k] > longest)
-                    {
-                        longest = work[in[k]] / share[k];
-                        at = (int)k;
-                    }
+                    longest = work / share[s];
+                    at = s;
                 }
-                if (at < 0)
-                    break;
-                ++share[at];
             }
+            if (at < 0)
+                break;
+            ++share[at];
+        }
+        // a share between two that fit may not: the next smaller one that does
+        for (int s = 0; s < b->n; ++s)
+            while (share[s] > least[s] && !res_plan_of(b->w[s], true, share[s]).fits)
+                --share[s];
+        return share;
+    }
+
+    // Every solve that can be resident, to its end; the others' records stay as they are.
+    int resident_solves(wdg_whbatch *b)
+    {
+        std::vector<int> least = least_shares(b);
+        if (std::all_of(least.begin(), least.end(), [](int c) { return c == 0; }))
+            return WDG_OK;
+        WDG_TRY(resident_prepare(b));
+        for (;;)
+        {
+            std::vector<char> running(b->n);
+            for (int s = 0; s < b->n; ++s)
+                running[s] = b->h_state[s].active != 0;
+            const std::vector<int> share = round_shares(b, least, running);
+            if (std::all_of(share.begin(), share.end(), [](int c) { return c == 0; }))
+                return WDG_OK;
             WDG_CUDA(cudaEventRecord(b->fork, b->cs));
-            for (size_t k = 0; k < in.size(); ++k)
+            for (int s = 0; s < b->n; ++s)
             {
-                const int s = in[k];
-                // a share between two that fit may not: the next smaller one that does
-                while (share[k] > least[s] &&
-                       !res_plan(b->w[s]->n, b->precision == WDG_FP32, b->w[s]->nel, sms, share[k], true).fits)
-                    --share[k];
+                if (!share[s])
+                    continue;
                 WDG_CUDA(cudaStreamWaitEvent(b->rs[s], b->fork, 0));
                 bool ran = false;
-                WDG_TRY(b->precision == WDG_FP32 ? resident_period<float>(b, s, share[k], ran)
-                                                 : resident_period<double>(b, s, share[k], ran));
+                WDG_TRY(b->precision == WDG_FP32 ? resident_period<float>(b, s, share[s], ran)
+                                                 : resident_period<double>(b, s, share[s], ran));
                 if (!ran)
                     least[s] = 0; // the device cannot hold it: left to the streaming launches
                 WDG_CUDA(cudaMemcpyAsync(b->h_err + s, b->w[s]->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, b->rs[s]));
@@ -444,8 +458,8 @@ namespace
             }
             WDG_CUDA(cudaMemcpyAsync(b->h_state, b->d_state, sizeof(WhbState) * b->n, cudaMemcpyDeviceToHost, b->cs));
             WDG_CUDA(cudaStreamSynchronize(b->cs));
-            for (int s : in)
-                if (b->h_err[s])
+            for (int s = 0; s < b->n; ++s)
+                if (share[s] && b->h_err[s])
                     WDG_TRY(check_device_error(b->w[s]));
         }
     }
@@ -623,6 +637,16 @@ extern "C"
         Dev g(b->device);
         b->explicit_launch = true;
         return shape(b, rounds, ring);
+    }
+
+    int wdg_test_whbatch_shares(const wdg_whbatch *b, int *ctas)
+    {
+        if (!b || !ctas)
+            return fail(WDG_ERR_ARG, "wdg_test_whbatch_shares: bad arguments");
+        const std::vector<int> share = round_shares(b, least_shares(b), std::vector<char>(b->n, 1));
+        for (int s = 0; s < b->n; ++s)
+            ctas[b->perm[s]] = share[s];
+        return WDG_OK;
     }
 
     int wdg_test_whbatch_fail(wdg_whbatch *b, int call)

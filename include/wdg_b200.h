@@ -129,14 +129,15 @@ int wdg_wave_autotune(wdg_wave *wave, int steps, float *best_ms_per_step);
 /* Mesh2D::element_metrics(basis).physical_coordinates(): xy (2, n, n, n_elem) */
 int wdg_wave_node_coords(wdg_wave *wave, double *xy);
 /* Failure detection (no counterpart in the reference, which has no device-side waits): every
- * wait of the fused stage kernels on a copy completion gives up after `seconds` (default 2),
+ * wait of the wave stage kernels on a copy or on a neighbour's flag gives up after `seconds` (default 2),
  * records it in the handle's device error word and lets the kernel finish; the next
  * synchronising call returns WDG_ERR_TIMEOUT and clears the word, and the handle stays usable. */
 int wdg_wave_set_wait_limit(wdg_wave *wave, double seconds);
 /* Test hooks (no counterpart in the reference) that exercise that failure detection without
- * faulting the GPU.  wdg_test_skip_chunk: in the first stage launch of the next RK4 call that
- * streams (and takes the warp-specialised kernel for it), every CTA leaves its chunk number `chunk` unloaded (-1:
- * none), so the waits on that chunk run out.  wdg_test_set_partner: overwrites the fused
+ * faulting the GPU.  wdg_test_skip_chunk: in the first stage launch of the handle's next RK4 call
+ * every CTA leaves its chunk (its group of elements, with one warp per CTA) number `chunk` unloaded, or,
+ * where the mesh is resident, the warp of group number `chunk` leaves before the first stage (-1: none),
+ * so the waits on that chunk or group run out.  wdg_test_set_partner: overwrites the fused
  * kernels' partner offset of (elem, side) (returns the previous value in *previous); an offset
  * outside the state makes the kernels skip that trace and report WDG_ERR_ARG ("neighbour
  * index outside the mesh") instead of reading out of bounds. */

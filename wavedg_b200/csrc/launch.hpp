@@ -51,7 +51,7 @@ namespace wdg
         int nread;            // values of u neighbour traces may come from (0: nel * 3 n^2; a domain
                               // of a decomposed mesh appends its halo traces after its elements)
         unsigned long long wait_ns; // limit of every bounded device-side wait (0: kWaitLimitNs)
-        int test_skip;        // test hook (family 2): 1 + the number of the chunk every CTA leaves
+        int test_skip;        // test hook (family 2): 1 + the number of the chunk or group every CTA leaves
                               // unloaded, so the waits on it run out; 0 (none) in every other launch
         int line;             // family 2: whether the launch may take the kernel of one warp per CTA
         int el_begin, el_end; // family 2: the launch updates elements [el_begin, el_end) only

@@ -106,6 +106,9 @@ namespace wdg
         asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
     }
 
+    // every cp.async of this thread, committed to a group or not
+    __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
     __device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes)
     {
         asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)),

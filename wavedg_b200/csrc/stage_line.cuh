@@ -234,7 +234,8 @@ namespace wdg
         int g = first(blockIdx.x), next = g;
         if (g >= ngroups)
             return;
-        load(g);
+        if (a.test_skip != 1) // test hook: group test_skip - 1 of every warp stays unloaded
+            load(g);
         gather();
         for (int m = 0; g < ngroups; ++m, g = next)
         {
@@ -271,9 +272,11 @@ namespace wdg
                 if (lane == 0)
                     bulk_wait_read();
                 __syncwarp();
-                load(next);
+                if (a.test_skip != m + 2)
+                    load(next);
             }
         }
+        cp_async_wait_all(); // after a wait that ran out, the gathered traces
         if (lane == 0)
             bulk_wait_all();
     }
@@ -316,7 +319,7 @@ namespace wdg
     template <typename Real>
     static bool line_takes(const StageArgs<Real> &a, int grid_limit)
     {
-        if (!a.line || a.family != 2 || !a.use_tma || !a.tma_out || grid_limit > 0 || a.test_skip)
+        if (!a.line || a.family != 2 || !a.use_tma || !a.tma_out || grid_limit > 0)
             return false;
         if (!a.out) // operators, FP64; the sum with a forcing has its own rounding: tiled kernel
             return sizeof(Real) == 8 && !(a.flags & F_FORCE);

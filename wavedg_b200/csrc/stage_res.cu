@@ -59,6 +59,7 @@ namespace wdg
             double *acc;           // FP64 filter (nullable): += cfilter[step] u after each step
             const double *cfilter;
             unsigned long long wait_ns;
+            int test_skip; // test hook: the group whose warp leaves before the first stage (-1: none)
         };
 
         // one group's shared memory (bytes)
@@ -278,6 +279,10 @@ namespace wdg
                 if (lane == 0)
                     st_release(a.flags + (size_t)kFlagStride * g, a.base + 1);
             }
+
+            // test hook: no flag of this warp's groups goes on, so their neighbours' waits run out
+            if (a.test_skip >= g_lo && a.test_skip < g_lo + ng && (a.test_skip - g_lo) % W == warp)
+                return;
 
             // ---- the stages
             const int nst = 5 * a.nsteps;
@@ -545,6 +550,7 @@ namespace wdg
         a.F = static_cast<const Real *>(x.F);
         a.acc = x.acc;
         a.wait_ns = w->wait_ns;
+        a.test_skip = w->test_skip - 1;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         WDG_CUDA(cudaStreamIsCapturing(stream, &cap));
         constexpr int kSteps = 4096; // per launch
@@ -581,6 +587,8 @@ namespace wdg
                 return cuda_fail(e, "resident stage kernel launch");
             w->flag_base += 5ull * a.nsteps + 1;
             w->flags_set = w->flags_set || !captured;
+            w->test_skip = 0; // this launch only
+            a.test_skip = -1;
             ran = true;
         }
         return WDG_OK;

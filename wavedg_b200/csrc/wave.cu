@@ -105,7 +105,7 @@ namespace wdg
         {
             WDG_CUDA(cudaMemsetAsync(w->d_err, 0, sizeof(unsigned), w->stream));
             if (err & 1u)
-                return fail(WDG_ERR_TIMEOUT, "a bounded device-side wait expired (TMA copy did not complete)");
+                return fail(WDG_ERR_TIMEOUT, "a bounded device-side wait expired (a copy or a neighbour's flag did not come)");
             return fail(WDG_ERR_ARG, "device kernel met a neighbour index outside the mesh");
         }
         return WDG_OK;
@@ -139,10 +139,9 @@ namespace wdg
         return a;
     }
 
-    // (the skipped-chunk test asks for the streaming kernel)
     ResPlan res_plan_of(const wdg_wave *w, bool forced, int max_ctas)
     {
-        if (w->family != 2 || w->explicit_launch || w->test_skip || !w->d_flags)
+        if (w->family != 2 || w->explicit_launch || !w->d_flags)
             return ResPlan{};
         return res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, max_ctas, forced);
     }

@@ -56,3 +56,24 @@ def test_wait_runs_out(gpu_lib, nx, n, precision, explicit, resident, skip):
         u = u0.copy()
         s.rk4_steps(u, dt, 0.0, 2)
         np.testing.assert_array_equal(u, want)
+
+
+def test_batch_reports_a_solve_whose_wait_ran_out(gpu_lib):
+    import wavedg_b200 as W
+
+    L = W.lib()
+    systems = [_system(m, n, "fp64") for m, n in ((20, 5), (16, 4), (9, 7))]
+    b = W.WaveHoltzBatch(systems, [5.0, 6.0, 7.0])
+    F = [np.random.default_rng(k).standard_normal(s.ndof) for k, s in enumerate(systems)]
+    want = b.solve(F, tol=1e-12, maxit=2)[0]
+    for s in systems[:2]:
+        assert L.wdg_wave_set_wait_limit(s._h, 0.005) == 0
+        assert L.wdg_test_skip_chunk(s._h, 1) == 0
+    with pytest.raises(W.WdgError) as e:
+        b.solve(F, tol=1e-12, maxit=2)
+    assert e.value.code == W._lib.WDG_ERR_TIMEOUT
+    for s in systems:
+        assert L.wdg_wave_set_wait_limit(s._h, 2.0) == 0
+    got = b.solve(F, tol=1e-12, maxit=2)[0]  # nothing of either solve's error is left
+    for x, y in zip(got, want):
+        assert np.array_equal(x, y)

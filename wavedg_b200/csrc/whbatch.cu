@@ -441,11 +441,9 @@ namespace
             const std::vector<int> share = round_shares(b, least, running);
             if (std::all_of(share.begin(), share.end(), [](int c) { return c == 0; }))
                 return WDG_OK;
-            WDG_CUDA(cudaEventRecord(b->fork, b->cs));
-            for (int s = 0; s < b->n; ++s)
+            // each solve's period on its stream, behind b->cs and before what follows there
+            auto launch = [&](int s) -> int
             {
-                if (!share[s])
-                    continue;
                 WDG_CUDA(cudaStreamWaitEvent(b->rs[s], b->fork, 0));
                 bool ran = false;
                 WDG_TRY(b->precision == WDG_FP32 ? resident_period<float>(b, s, share[s], ran)
@@ -455,12 +453,37 @@ namespace
                 WDG_CUDA(cudaMemcpyAsync(b->h_err + s, b->w[s]->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, b->rs[s]));
                 WDG_CUDA(cudaEventRecord(b->rdone[s], b->rs[s]));
                 WDG_CUDA(cudaStreamWaitEvent(b->cs, b->rdone[s], 0));
+                return WDG_OK;
+            };
+            WDG_CUDA(cudaEventRecord(b->fork, b->cs));
+            int st = WDG_OK;
+            for (int s = 0; s < b->n && st == WDG_OK; ++s)
+                if (share[s])
+                    st = launch(s);
+            if (st != WDG_OK)
+            {
+                // the solves already launched must not run into the next call's
+                const std::string msg = wdg_last_error();
+                for (int s = 0; s < b->n; ++s)
+                    cudaStreamSynchronize(b->rs[s]);
+                return fail(st, msg);
             }
             WDG_CUDA(cudaMemcpyAsync(b->h_state, b->d_state, sizeof(WhbState) * b->n, cudaMemcpyDeviceToHost, b->cs));
             WDG_CUDA(cudaStreamSynchronize(b->cs));
+            // the first error is reported, every solve's is cleared
+            std::string msg;
             for (int s = 0; s < b->n; ++s)
                 if (share[s] && b->h_err[s])
-                    WDG_TRY(check_device_error(b->w[s]));
+                {
+                    const int e = check_device_error(b->w[s]);
+                    if (st == WDG_OK && e != WDG_OK)
+                    {
+                        st = e;
+                        msg = wdg_last_error();
+                    }
+                }
+            if (st != WDG_OK)
+                return fail(st, msg);
         }
     }
 } // namespace

@@ -43,3 +43,19 @@ def test_defaults_are_not_choices(gpu_lib):
     assert _ctas(s) == default
     s.set_max_ctas(9)
     assert 0 < _ctas(s) <= 9
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_state_steps_need_a_state(gpu_lib, precision):
+    import numpy as np
+
+    import wavedg_b200 as W
+
+    s = W.WaveSystem(W.Mesh2D.uniform_rect(6, -1.0, 1.0, 5, -1.0, 1.0), 4, None, precision=precision)
+    assert s.step_state(1e-3, 0.5, 0) == 0.5
+    with pytest.raises(W.WdgError) as e:
+        s.step_state(1e-3, 0.0, 1)
+    assert e.value.code == W._lib.WDG_ERR_ARG
+    s.upload(np.ones(s.ndof))
+    s.step_state(1e-3, 0.0, 1)
+    assert np.isfinite(s.download()).all()

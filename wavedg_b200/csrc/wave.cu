@@ -1066,7 +1066,9 @@ extern "C"
         WDG_TRY(whole_mesh_only(w, "wdg_state_rk4_steps"));
         if (!w || !t || nsteps < 0)
             return fail(WDG_ERR_ARG, "wdg_state_rk4_steps: bad arguments");
-        if (nsteps > 0 && !w->d_state[0])
+        if (nsteps == 0)
+            return WDG_OK;
+        if (!w->d_state[0])
             return fail(WDG_ERR_ARG, "wdg_state_rk4_steps: no state was uploaded");
         DeviceGuard g(w->device);
         RKExtras none;

@@ -428,9 +428,12 @@ namespace
     // ky(k) = k for k < K/2, k - K otherwise; complex values as (re, im) pairs.  A CTA takes one plane bc
     // and kDftThreads pairs of outputs (k, kx) and (k + K/2, kx), so that a value read from shared memory
     // serves two sums; y runs in order, whatever the chunking.  The twiddles and a chunk of `chunk` rows
-    // sit in shared memory (the twiddles of a grid too large for it stay in global memory: TAB false).
+    // sit in shared memory (the twiddles of a grid too large for it stay in global memory: TAB false; so do
+    // rows of which not one fits: ROWS false).  Pairs are read and written whole where `vec`, their
+    // alignment, allows it.
     constexpr int kDftThreads = 128, kDftRows = 128;
     constexpr size_t kDftSmem = 96 * 1024;
+    constexpr long long kGridY = 65535; // blocks of a grid along y
     __device__ __forceinline__ void dft_add(float2 x, float2 cs, float sign, float &re, float &im)
     {
         const float c = cs.x, s = sign * cs.y;
@@ -438,49 +441,67 @@ namespace
         re += __fmaf_rn(c, x.x, -__fmul_rn(s, x.y));
         im += __fmaf_rn(s, x.x, __fmul_rn(c, x.y));
     }
-    template <bool TAB>
+    __device__ __forceinline__ float2 pair_get(const float *p, long long i, bool vec)
+    {
+        return vec ? __ldg(reinterpret_cast<const float2 *>(p) + i) : make_float2(__ldg(p + 2 * i), __ldg(p + 2 * i + 1));
+    }
+    __device__ __forceinline__ void pair_put(float *p, long long i, float re, float im, bool vec)
+    {
+        if (vec)
+            reinterpret_cast<float2 *>(p)[i] = make_float2(re, im);
+        else
+        {
+            p[2 * i] = re;
+            p[2 * i + 1] = im;
+        }
+    }
+    template <bool TAB, bool ROWS>
     __global__ void __launch_bounds__(kDftThreads) dft_y_fwd_kernel(const float *in, float *out, const float *cs,
                                                                     const float *sn, int G, int K, int KX, float sign,
-                                                                    int chunk)
+                                                                    int chunk, bool vec)
     {
         extern __shared__ float2 dsm[];
         float2 *tab = dsm, *xs = dsm + (TAB ? G : 0); // (cos, sin) of 2 pi m / G; a chunk of rows
         auto twiddle = [&](int m) { return TAB ? tab[m] : make_float2(__ldg(cs + m), __ldg(sn + m)); };
         const int t = threadIdx.x, half = K / 2;
         const long long bc = blockIdx.x;
-        const int q = blockIdx.y * kDftThreads + t, kx = q % KX, k = q / KX;
-        const bool on = k < half;
         for (int m = t; TAB && m < G; m += kDftThreads)
             tab[m] = make_float2(cs[m], sn[m]);
-        const float2 *src = reinterpret_cast<const float2 *>(in) + bc * (long long)G * KX;
-        const int step0 = k % G, step1 = ((k - half) % G + G) % G; // ky of k, of k + K/2: k + K/2 - K
-        float re0 = 0.f, im0 = 0.f, re1 = 0.f, im1 = 0.f;
-        int p0 = 0, p1 = 0;
-        for (int y0 = 0; y0 < G; y0 += chunk)
+        const float *src = in + 2 * bc * (long long)G * KX;
+        for (long long q0 = blockIdx.y * (long long)kDftThreads; q0 < (long long)half * KX; q0 += gridDim.y * (long long)kDftThreads)
         {
-            const int rows = min(chunk, G - y0);
-            __syncthreads();
-            for (int i = t; i < rows * KX; i += kDftThreads)
-                xs[i] = src[(long long)y0 * KX + i];
-            __syncthreads();
-            if (on)
+            const long long q = q0 + t;
+            const int kx = (int)(q % KX), k = (int)(q / KX);
+            const bool on = k < half;
+            const int step0 = k % G, step1 = ((k - half) % G + G) % G; // ky of k, of k + K/2: k + K/2 - K
+            float re0 = 0.f, im0 = 0.f, re1 = 0.f, im1 = 0.f;
+            int p0 = 0, p1 = 0;
+            for (int y0 = 0; y0 < G; y0 += chunk)
+            {
+                const int rows = min(chunk, G - y0);
+                __syncthreads();
+                for (int i = t; ROWS && i < rows * KX; i += kDftThreads)
+                    xs[i] = pair_get(src, (long long)y0 * KX + i, vec);
+                __syncthreads();
+                if (on)
 #pragma unroll 4
-                for (int y = 0; y < rows; ++y)
-                {
-                    const float2 x = xs[y * KX + kx];
-                    dft_add(x, twiddle(p0), sign, re0, im0);
-                    dft_add(x, twiddle(p1), sign, re1, im1);
-                    p0 += step0;
-                    p0 -= p0 >= G ? G : 0;
-                    p1 += step1;
-                    p1 -= p1 >= G ? G : 0;
-                }
-        }
-        if (on)
-        {
-            float2 *o = reinterpret_cast<float2 *>(out) + bc * (long long)K * KX;
-            o[k * KX + kx] = make_float2(re0, im0);
-            o[(k + half) * KX + kx] = make_float2(re1, im1);
+                    for (int y = 0; y < rows; ++y)
+                    {
+                        const float2 x = ROWS ? xs[y * KX + kx] : pair_get(src, (long long)(y0 + y) * KX + kx, vec);
+                        dft_add(x, twiddle(p0), sign, re0, im0);
+                        dft_add(x, twiddle(p1), sign, re1, im1);
+                        p0 += step0;
+                        p0 -= p0 >= G ? G : 0;
+                        p1 += step1;
+                        p1 -= p1 >= G ? G : 0;
+                    }
+            }
+            if (on)
+            {
+                float *o = out + 2 * bc * (long long)K * KX;
+                pair_put(o, (long long)k * KX + kx, re0, im0, vec);
+                pair_put(o, (long long)(k + half) * KX + kx, re1, im1, vec);
+            }
         }
     }
 
@@ -490,44 +511,53 @@ namespace
     constexpr int kInvRows = 32;
     template <bool TAB>
     __global__ void __launch_bounds__(kDftThreads) dft_y_inv_kernel(const float *in, float *out, bf16 *outb, const float *cs,
-                                                                    const float *sn, int G, int K, int KX, float sign)
+                                                                    const float *sn, int G, int K, int KX, float sign,
+                                                                    bool vec, bool vecb)
     {
         extern __shared__ float2 dsm[];
         float2 *tab = dsm, *xs = dsm + G;
         const int t = threadIdx.x, half = K / 2;
         const long long bc = blockIdx.x;
-        const float2 *src = reinterpret_cast<const float2 *>(in) + bc * (long long)K * KX;
+        const float *src = in + 2 * bc * (long long)K * KX;
         auto twiddle = [&](int m) { return TAB ? tab[m] : make_float2(__ldg(cs + m), __ldg(sn + m)); };
-        auto mode = [&](int m) { return TAB ? xs[m] : __ldg(src + m); };
-        const int y0 = blockIdx.y * kInvRows, rows = min(kInvRows, G - y0);
+        auto mode = [&](int k, int kx) { return TAB ? xs[k * KX + kx] : pair_get(src, (long long)k * KX + kx, vec); };
         for (int m = t; TAB && m < G; m += kDftThreads)
             tab[m] = make_float2(cs[m], sn[m]);
         for (int i = t; TAB && i < K * KX; i += kDftThreads)
-            xs[i] = src[i];
+            xs[i] = pair_get(src, i, vec);
         __syncthreads();
-        for (int i = t; i < rows * KX; i += kDftThreads)
+        for (long long y0 = blockIdx.y * (long long)kInvRows; y0 < G; y0 += gridDim.y * (long long)kInvRows)
         {
-            const int kx = i % KX, y = y0 + i / KX;
-            float re = 0.f, im = 0.f;
-            int p = 0;
-            for (int k = 0; k < half; ++k)
+            const int rows = (int)min((long long)kInvRows, G - y0);
+            for (long long i = t; i < (long long)rows * KX; i += kDftThreads)
             {
-                dft_add(mode(k * KX + kx), twiddle(p), sign, re, im);
-                p += y;
-                p -= p >= G ? G : 0;
+                const int kx = (int)(i % KX), y = (int)(y0 + i / KX);
+                float re = 0.f, im = 0.f;
+                int p = 0;
+                for (int k = 0; k < half; ++k)
+                {
+                    dft_add(mode(k, kx), twiddle(p), sign, re, im);
+                    p += y;
+                    p -= p >= G ? G : 0;
+                }
+                p = (G - (int)((long long)half * y % G)) % G; // ky = -K/2
+                for (int k = half; k < K; ++k)
+                {
+                    dft_add(mode(k, kx), twiddle(p), sign, re, im);
+                    p += y;
+                    p -= p >= G ? G : 0;
+                }
+                const long long o = (bc * G + y) * KX + kx;
+                if (out)
+                    pair_put(out, o, re, im, vec);
+                if (outb && vecb)
+                    reinterpret_cast<__nv_bfloat162 *>(outb)[o] = __floats2bfloat162_rn(re, im);
+                else if (outb)
+                {
+                    outb[2 * o] = __float2bfloat16(re);
+                    outb[2 * o + 1] = __float2bfloat16(im);
+                }
             }
-            p = (G - (int)((long long)half * y % G)) % G; // ky = -K/2
-            for (int k = half; k < K; ++k)
-            {
-                dft_add(mode(k * KX + kx), twiddle(p), sign, re, im);
-                p += y;
-                p -= p >= G ? G : 0;
-            }
-            const long long o = (bc * G + y) * KX + kx;
-            if (out)
-                reinterpret_cast<float2 *>(out)[o] = make_float2(re, im);
-            if (outb)
-                reinterpret_cast<__nv_bfloat162 *>(outb)[o] = __floats2bfloat162_rn(re, im);
         }
     }
 
@@ -937,31 +967,33 @@ extern "C"
     {
         if (!in || !cos_tab || !sin_tab || BC < 1 || G < 2 || K < 2 || (K & 1) || KX < 1 || (!out && !out_bf16))
             return wdg::fail(WDG_ERR_ARG, "wdg_fno_dft_y: bad arguments");
+        const bool vec = (((uintptr_t)in | (uintptr_t)out) & 7u) == 0;
         if (!inverse)
         {
             if (!out)
                 return wdg::fail(WDG_ERR_ARG, "wdg_fno_dft_y: the forward transform writes FP32");
             const bool tab = sizeof(float2) * ((size_t)G + KX) <= kDftSmem;
             const size_t left = kDftSmem / sizeof(float2) - (tab ? G : 0);
-            const int chunk = (int)std::min<size_t>(kDftRows, left / KX);
-            if (chunk < 1)
-                return wdg::fail(WDG_ERR_ARG, "wdg_fno_dft_y: more than 12288 modes along x");
-            const size_t smem = sizeof(float2) * ((tab ? (size_t)G : 0) + (size_t)chunk * KX);
-            auto kern = tab ? dft_y_fwd_kernel<true> : dft_y_fwd_kernel<false>;
+            const bool rows = left >= (size_t)KX;
+            const int chunk = rows ? (int)std::min<size_t>(kDftRows, left / KX) : G;
+            const size_t smem = sizeof(float2) * ((tab ? (size_t)G : 0) + (rows ? (size_t)chunk * KX : 0));
+            auto kern = tab ? dft_y_fwd_kernel<true, true> : rows ? dft_y_fwd_kernel<false, true> : dft_y_fwd_kernel<false, false>;
             if (smem > 48 * 1024)
                 cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDftSmem);
-            kern<<<dim3(BC, (K / 2 * KX + kDftThreads - 1) / kDftThreads), kDftThreads, smem, st(stream)>>>(
-                in, out, cos_tab, sin_tab, G, K, KX, sign, chunk);
+            const long long q = ((long long)(K / 2) * KX + kDftThreads - 1) / kDftThreads;
+            kern<<<dim3(BC, (unsigned)std::min(kGridY, q)), kDftThreads, smem, st(stream)>>>(in, out, cos_tab, sin_tab, G, K,
+                                                                                            KX, sign, chunk, vec);
         }
         else
         {
             const size_t want = sizeof(float2) * ((size_t)G + (size_t)K * KX);
-            const bool tab = want <= kDftSmem;
+            const bool tab = want <= kDftSmem, vecb = ((uintptr_t)out_bf16 & 3u) == 0;
             auto kern = tab ? dft_y_inv_kernel<true> : dft_y_inv_kernel<false>;
             if (tab && want > 48 * 1024)
                 cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDftSmem);
-            kern<<<dim3(BC, (G + kInvRows - 1) / kInvRows), kDftThreads, tab ? want : 0, st(stream)>>>(
-                in, out, static_cast<bf16 *>(out_bf16), cos_tab, sin_tab, G, K, KX, sign);
+            const long long q = ((long long)G + kInvRows - 1) / kInvRows;
+            kern<<<dim3(BC, (unsigned)std::min(kGridY, q)), kDftThreads, tab ? want : 0, st(stream)>>>(
+                in, out, static_cast<bf16 *>(out_bf16), cos_tab, sin_tab, G, K, KX, sign, vec, vecb);
         }
         return done("wdg_fno_dft_y");
     }

@@ -167,21 +167,19 @@ namespace wdg
         return WDG_OK;
     }
 
-    // x <- M x or M^{-1} x of one element by one warp, n and the variable count at run time (the
-    // operator entry points and the table-driven advection kernel): A (row-major n x n) is T = psi_m(x_k)
-    // for the inverse, B = phi_k(g_m) for the action; tmp holds nv n^2 values
-    __device__ inline void x_mass(int n, int nv, bool inverse, const double *A, const double *xg, const double *wg,
-                                  const double *c, double *x, double *tmp, int lane)
+    // r <- M^{-1} r of one element by one warp, n and the variable count at run time (the table-driven
+    // advection kernel): T (row-major n x n) holds psi_m(x_k), c the corners, tmp holds nv n^2 values
+    __device__ inline void x_mass_inv(int n, int nv, const double *T, const double *xg, const double *wg, const double *c,
+                                      double *r, double *tmp, int lane)
     {
         const int m = nv * n * n;
-        // (A x A)^T for the inverse's projection on psi, A x A for the action's values at the points
-        const int rs = inverse ? 1 : n, cs = inverse ? n : 1;
+        // (T x T)^T r at the Gauss points
         for (int o = lane; o < m; o += 32)
         {
             const int d = o % nv, i = (o / nv) % n, l = o / (nv * n);
             double s = 0.0;
             for (int k = 0; k < n; ++k)
-                s += __ldg(A + rs * i + cs * k) * x[d + nv * (k + n * l)];
+                s += __ldg(T + i + n * k) * r[d + nv * (k + n * l)];
             tmp[o] = s;
         }
         __syncwarp();
@@ -190,10 +188,9 @@ namespace wdg
             const int d = o % nv, i = (o / nv) % n, j = o / (nv * n);
             double s = 0.0, J[4];
             for (int k = 0; k < n; ++k)
-                s += __ldg(A + rs * j + cs * k) * tmp[d + nv * (i + n * k)];
+                s += __ldg(T + j + n * k) * tmp[d + nv * (i + n * k)];
             quad_jacobian(c, __ldg(xg + i), __ldg(xg + j), J);
-            const double w = __ldg(wg + i) * __ldg(wg + j) * (J[0] * J[3] - J[2] * J[1]);
-            x[o] = inverse ? s / w : s * w;
+            r[o] = s / (__ldg(wg + i) * __ldg(wg + j) * (J[0] * J[3] - J[2] * J[1]));
         }
         __syncwarp();
         for (int o = lane; o < m; o += 32)
@@ -201,7 +198,7 @@ namespace wdg
             const int d = o % nv, i = (o / nv) % n, l = o / (nv * n);
             double s = 0.0;
             for (int k = 0; k < n; ++k)
-                s += __ldg(A + cs * i + rs * k) * x[d + nv * (k + n * l)];
+                s += __ldg(T + n * i + k) * r[d + nv * (k + n * l)];
             tmp[o] = s;
         }
         __syncwarp();
@@ -210,8 +207,8 @@ namespace wdg
             const int d = o % nv, i = (o / nv) % n, j = o / (nv * n);
             double s = 0.0;
             for (int k = 0; k < n; ++k)
-                s += __ldg(A + cs * j + rs * k) * tmp[d + nv * (i + n * k)];
-            x[o] = s;
+                s += __ldg(T + n * j + k) * tmp[d + nv * (i + n * k)];
+            r[o] = s;
         }
         __syncwarp();
     }
@@ -219,13 +216,22 @@ namespace wdg
     // A device copy of what x_mass reads for a basis with nodes x
     struct MassTables
     {
-        double *T = nullptr, *B = nullptr, *xg = nullptr, *wg = nullptr;
+        double *T = nullptr, *xg = nullptr, *wg = nullptr;
     };
     int mass_tables(int n, const double *x, MassTables &t);
     void mass_tables_free(MassTables &t);
-    // y <- M x or M^{-1} x with nv interleaved variables (x and y may be the same array)
-    int mass_launch(const MassTables &t, int n, int nel, int nv, bool inverse, const double *corners, const double *x,
-                    double *y, cudaStream_t s);
+
+    // The operators M and M^{-1} on arrays of nv interleaved variables, for a basis with nodes x: the
+    // matrices go with each launch
+    struct MassOp
+    {
+        int n = 0;
+        double T[kMaxN * kMaxN], B[kMaxN * kMaxN], xg[kMaxN], wg[kMaxN]; // psi_m(x_k), phi_k(g_m) (row-major), the Gauss rule
+    };
+    MassOp mass_op(int n, const double *x);
+    // y <- M x or M^{-1} x (x and y may be the same array)
+    int mass_launch(const MassOp &t, int nel, int nv, bool inverse, const double *corners, const double *x, double *y,
+                    cudaStream_t s);
 
     struct XArgs
     {

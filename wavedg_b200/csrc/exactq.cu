@@ -18,7 +18,7 @@
 // matrix as two one-dimensional contractions around a diagonal, the stage update); the operator
 // entry points (Div, EdgeFlux, the mass matrix and its inverse) keep component kernels in the
 // reference layouts: one CTA per element for the volume term, one thread per edge for the face
-// term, one warp per element for the mass matrix.
+// term, a lane per grid line for the mass matrix.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -39,7 +39,7 @@ struct wdg_waveq
     double *d_xd = nullptr, *d_wd = nullptr, *d_Pd = nullptr, *d_Dd = nullptr; // Div rule, P(i,k), D(i,k)
     double *d_wf = nullptr, *d_Pf = nullptr;                                   // face rule, P(i,k)
     double *d_nI = nullptr, *d_nB = nullptr; // per edge (n_x, n_y, |E| / 2)
-    MassTables mass;
+    MassOp mass;
     double *d_uf = nullptr, *d_uB = nullptr; // face traces
 };
 
@@ -92,66 +92,201 @@ namespace wdg
             }
     }
 
-    // a warp per element, wpb warps of 2 nv n^2 doubles
-    __global__ void x_mass_kernel(int n, int nel, int nv, int inverse, const double *__restrict__ A,
-                                  const double *__restrict__ xg, const double *__restrict__ wg,
-                                  const double *__restrict__ corners, const double *x, double *y)
+    template <int N>
+    struct MassArgs
+    {
+        double A[N][N], xg[N], wg[N]; // psi_m(x_k) at [k][m] (inverse), phi_k(g_m) at [m][k] (action)
+        const double *corners, *x;
+        double *y;
+        int nel, nv, ew, rs;
+    };
+    // M = (B x B)^T D (B x B) and its inverse (T x T) D^{-1} (T x T)^T.  A warp owns ew whole elements, a lane
+    // a grid line of one of them, one variable after the other, in place: rows, columns (to the Gauss points,
+    // D, and back: the column is this lane's alone), rows.  The staged rows are rs (odd) doubles apart, so
+    // that neither pass has two lanes on a bank; the matrices are constant-bank operands.  Bound by memory: 16 bytes a value.
+    // 128 x 128, inverse, one and three variables: n = 2: 18 and 18 -> 4.5 and 5.5 us, n = 5: 21 and 49 -> 6.5
+    // and 10 us against a warp per element with generic loops (dense inverses: 6.2 and 6.2, 22 and 42 us).
+    template <int N, bool INV>
+    __global__ void __launch_bounds__(128) mass_kernel(const __grid_constant__ MassArgs<N> a)
     {
         extern __shared__ double sx[];
-        const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5, m = nv * n * n;
-        double *xs = sx + (size_t)wib * 2 * m;
-        for (int el = blockIdx.x * wpb + wib; el < nel; el += gridDim.x * wpb)
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nv = a.nv, rs = a.rs, m = nv * N;
+        const int e0 = (blockIdx.x * (int)(blockDim.x >> 5) + warp) * a.ew, ne = min(a.ew, a.nel - e0);
+        if (ne <= 0)
+            return;
+        double *E = sx + (size_t)warp * a.ew * N * rs;
+        const size_t first = (size_t)e0 * N * m;
+        for (int o = lane; o < ne * N * m; o += 32)
+            E[(o / m) * rs + o % m] = a.x[first + o];
+        const int le = lane / N, ln = lane - le * N;
+        const bool on = le < ne;
+        double *R = E + (le * N + ln) * rs, *C = E + le * N * rs + ln * nv;
+        double w[N];
+        if (on)
         {
-            for (int o = lane; o < m; o += 32)
-                xs[o] = x[(size_t)m * el + o];
-            __syncwarp();
-            x_mass(n, nv, inverse != 0, A, xg, wg, corners + 8 * (size_t)el, xs, xs + m, lane);
-            for (int o = lane; o < m; o += 32)
-                y[(size_t)m * el + o] = xs[o];
-            __syncwarp();
+            double c[8], J[4];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                c[k] = __ldg(a.corners + 8 * (size_t)(e0 + le) + k);
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+            {
+                quad_jacobian(c, a.xg[ln], a.xg[j], J);
+                w[j] = a.wg[ln] * a.wg[j] * (J[0] * J[3] - J[2] * J[1]);
+                if (INV)
+                    w[j] = 1.0 / w[j];
+            }
+        }
+        // v -> to the points along a line (`to`), or back
+        auto line = [&](double (&v)[N], bool to)
+        {
+            double s[N];
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+            {
+                s[i] = 0.0;
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    s[i] += (to != INV ? a.A[i][k] : a.A[k][i]) * v[k];
+            }
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+                v[i] = s[i];
+        };
+        __syncwarp();
+        if (on)
+            for (int d = 0; d < nv; ++d)
+            {
+                double v[N];
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    v[k] = R[k * nv + d];
+                line(v, true);
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    R[k * nv + d] = v[k];
+            }
+        __syncwarp();
+        if (on)
+            for (int d = 0; d < nv; ++d)
+            {
+                double v[N];
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    v[k] = C[k * rs + d];
+                line(v, true);
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    v[k] *= w[k];
+                line(v, false);
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    C[k * rs + d] = v[k];
+            }
+        __syncwarp();
+        if (on)
+            for (int d = 0; d < nv; ++d)
+            {
+                double v[N];
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    v[k] = R[k * nv + d];
+                line(v, false);
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    R[k * nv + d] = v[k];
+            }
+        __syncwarp();
+        for (int o = lane; o < ne * N * m; o += 32)
+            a.y[first + o] = E[(o / m) * rs + o % m];
+    }
+
+    template <int N>
+    int mass_launch_n(const MassOp &t, int nel, int nv, bool inverse, const double *corners, const double *x, double *y,
+                      cudaStream_t s)
+    {
+        MassArgs<N> a;
+        for (int i = 0; i < N; ++i)
+        {
+            for (int k = 0; k < N; ++k)
+                a.A[i][k] = inverse ? t.T[i * N + k] : t.B[i * N + k];
+            a.xg[i] = t.xg[i];
+            a.wg[i] = t.wg[i];
+        }
+        a.corners = corners;
+        a.x = x;
+        a.y = y;
+        a.nel = nel;
+        a.nv = nv;
+        a.rs = (nv * N) | 1;
+        // 48 KB: one element at least (callers bound nv), then a lane per line, then warps
+        const size_t element = sizeof(double) * N * a.rs, room = 48 * 1024;
+        a.ew = (int)std::max<size_t>(1, std::min<size_t>(32 / N, room / element));
+        const int wpb = (int)std::max<size_t>(1, std::min<size_t>(4, room / (element * a.ew)));
+        const unsigned blocks = (unsigned)(((nel + a.ew - 1) / a.ew + wpb - 1) / wpb);
+        const size_t smem = element * a.ew * wpb;
+        if (inverse)
+            mass_kernel<N, true><<<blocks, 32 * wpb, smem, s>>>(a);
+        else
+            mass_kernel<N, false><<<blocks, 32 * wpb, smem, s>>>(a);
+        WDG_CUDA(cudaGetLastError());
+        return WDG_OK;
+    }
+    int mass_launch(const MassOp &t, int nel, int nv, bool inverse, const double *corners, const double *x, double *y,
+                    cudaStream_t s)
+    {
+        switch (t.n)
+        {
+        case 2: return mass_launch_n<2>(t, nel, nv, inverse, corners, x, y, s);
+        case 3: return mass_launch_n<3>(t, nel, nv, inverse, corners, x, y, s);
+        case 4: return mass_launch_n<4>(t, nel, nv, inverse, corners, x, y, s);
+        case 5: return mass_launch_n<5>(t, nel, nv, inverse, corners, x, y, s);
+        case 6: return mass_launch_n<6>(t, nel, nv, inverse, corners, x, y, s);
+        case 7: return mass_launch_n<7>(t, nel, nv, inverse, corners, x, y, s);
+        case 8: return mass_launch_n<8>(t, nel, nv, inverse, corners, x, y, s);
+        case 9: return mass_launch_n<9>(t, nel, nv, inverse, corners, x, y, s);
+        default: return fail(WDG_ERR_UNSUPPORTED, "mass matrix: n_colloc must be 2..9");
         }
     }
 
-    int mass_tables(int n, const double *x, MassTables &t)
+    MassOp mass_op(int n, const double *x)
     {
-        std::vector<double> g(n), w(n), C((size_t)n * n), R((size_t)n * n);
-        gauss_legendre(n, g.data(), w.data());
-        auto put = [&](double **d, const std::vector<double> &v) -> int
-        {
-            WDG_TRY(device_alloc(d, v.size()));
-            return device_put(*d, v);
-        };
-        auto rows = [&]() // column-major -> row-major
+        MassOp t;
+        std::vector<double> C((size_t)n * n);
+        t.n = n;
+        gauss_legendre(n, t.xg, t.wg);
+        auto rows = [&](double *R) // column-major -> row-major
         {
             for (int r = 0; r < n; ++r)
                 for (int c = 0; c < n; ++c)
                     R[r * n + c] = C[r + (size_t)n * c];
         };
-        interp_matrix(n, g.data(), n, x, C.data());
-        rows();
-        WDG_TRY(put(&t.T, R));
-        interp_matrix(n, x, n, g.data(), C.data());
-        rows();
-        WDG_TRY(put(&t.B, R));
-        WDG_TRY(put(&t.xg, g));
-        return put(&t.wg, w);
+        interp_matrix(n, t.xg, n, x, C.data());
+        rows(t.T);
+        interp_matrix(n, x, n, t.xg, C.data());
+        rows(t.B);
+        return t;
+    }
+
+    int mass_tables(int n, const double *x, MassTables &t)
+    {
+        const MassOp m = mass_op(n, x);
+        auto put = [](double **d, const double *v, size_t count) -> int
+        {
+            WDG_TRY(device_alloc(d, count));
+            WDG_CUDA(cudaMemcpy(*d, v, sizeof(double) * count, cudaMemcpyHostToDevice));
+            return WDG_OK;
+        };
+        WDG_TRY(put(&t.T, m.T, (size_t)n * n));
+        WDG_TRY(put(&t.xg, m.xg, (size_t)n));
+        return put(&t.wg, m.wg, (size_t)n);
     }
     void mass_tables_free(MassTables &t)
     {
-        for (double *p : {t.T, t.B, t.xg, t.wg})
+        for (double *p : {t.T, t.xg, t.wg})
             if (p)
                 cudaFree(p);
         t = MassTables{};
-    }
-    int mass_launch(const MassTables &t, int n, int nel, int nv, bool inverse, const double *corners, const double *x,
-                    double *y, cudaStream_t s)
-    {
-        const size_t per = sizeof(double) * 2 * nv * n * n; // at most 20.3 KB (nv <= 16, n <= 9)
-        const int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (48 * 1024) / per));
-        x_mass_kernel<<<(unsigned)std::max(1, std::min((nel + wpb - 1) / wpb, 148 * 32)), 32 * wpb, per * wpb, s>>>(
-            n, nel, nv, inverse ? 1 : 0, inverse ? t.T : t.B, t.xg, t.wg, corners, x, y);
-        WDG_CUDA(cudaGetLastError());
-        return WDG_OK;
     }
 } // namespace wdg
 
@@ -432,7 +567,7 @@ namespace
     }
     int mass_dev(wdg_waveq *h, int nv, const double *x, double *y, bool inverse)
     {
-        return mass_launch(h->mass, h->n, h->w->nel, nv, inverse, h->w->d_corners, x, y, h->w->stream);
+        return mass_launch(h->mass, h->w->nel, nv, inverse, h->w->d_corners, x, y, h->w->stream);
     }
     // du += Div u + Prol_I^T Flux_I Prol_I u
     int wave_dev(wdg_waveq *h, const double *u, double *du)
@@ -607,7 +742,7 @@ extern "C"
             chk(device_put(h->d_Pf, Pf));
             chk(device_put(h->d_nI, nI));
             chk(device_put(h->d_nB, nB));
-            chk(mass_tables(n, x.data(), h->mass));
+            h->mass = mass_op(n, x.data());
         }
         if (st == WDG_OK)
         {
@@ -637,7 +772,6 @@ extern "C"
             for (double *p : {h->d_xd, h->d_wd, h->d_Pd, h->d_Dd, h->d_wf, h->d_Pf, h->d_nI, h->d_nB, h->d_uf, h->d_uB})
                 if (p)
                     cudaFree(p);
-            mass_tables_free(h->mass);
         }
         if (h->w)
             wdg_wave_destroy(h->w);

@@ -7,7 +7,7 @@
 //   approx_quad = true    M = diag(w_i w_j det J) at the basis nodes (MassMatrix<true>)
 //   approx_quad = false   the element matrices of the (n + 1)-point Gauss-Legendre rule and their
 //                         inverses (MassMatrix<false>) in factored form (exact_line.cuh: one-
-//                         dimensional contractions around a diagonal), one warp per element
+//                         dimensional contractions around a diagonal), a lane per grid line
 //   load                  (f, phi) from f's values at the default n-point Gauss-Legendre points:
 //                         f w_k w_l det J there, projected along y, then along x
 //                         (LinearFunctional<2>::action), on the host, once per call
@@ -31,7 +31,7 @@ struct wdg_massmatrix
     std::vector<double> corners;                 // (8, nel), for the load vector's geometry
     std::vector<double> xq, wq, B;               // the load vector's n-point rule, B(q, basis node)
     double *d_m = nullptr;                       // approx: w_i w_j det J per node
-    MassTables mass;                             // exact: the factors' matrices
+    MassOp mass;                                 // exact: the factors' matrices
 };
 
 namespace
@@ -62,7 +62,7 @@ namespace
         {
             if (sizeof(double) * 4 * (size_t)nv * c > 48 * 1024)
                 return fail(WDG_ERR_UNSUPPORTED, "mass matrix: n_var too large for one element in shared memory");
-            return mass_launch(h->mass, h->n, h->nel, nv, inverse, h->w->d_corners, x, y, h->w->stream);
+            return mass_launch(h->mass, h->nel, nv, inverse, h->w->d_corners, x, y, h->w->stream);
         }
         WDG_CUDA(cudaGetLastError());
         return WDG_OK;
@@ -120,7 +120,7 @@ extern "C"
             {
                 st = exact_mass_check(*mesh, n);
                 if (st == WDG_OK)
-                    st = mass_tables(n, xb.data(), h->mass);
+                    h->mass = mass_op(n, xb.data());
             }
         }
         if (st != WDG_OK)
@@ -141,7 +141,6 @@ extern "C"
             DeviceScope g(h->w->device);
             if (h->d_m)
                 cudaFree(h->d_m);
-            mass_tables_free(h->mass);
             wdg_wave_destroy(h->w);
         }
         delete h;

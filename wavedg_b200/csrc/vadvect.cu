@@ -403,7 +403,7 @@ namespace
             // M^{-1} and the output: lane per node.  The volume term's half contractions are done with
             // Df, which holds at least nv n^2 values (Q >= n)
             if (ex)
-                x_mass(n, nv, true, A.mass.T, A.mass.xg, A.mass.wg, a.corners + 8 * (size_t)el, r, Df, lane);
+                x_mass_inv(n, nv, A.mass.T, A.mass.xg, A.mass.wg, c, r, Df, lane);
             for (int row = lane; row < nn; row += 32)
             {
                 double y[kJacobiMax];

@@ -173,6 +173,32 @@ namespace wdg
                                       double *r, double *tmp, int lane)
     {
         const int m = nv * n * n;
+        if (n <= 3)
+        {
+            // both directions at once: at most nine terms, and two passes fewer
+            for (int o = lane; o < m; o += 32)
+            {
+                const int d = o % nv, i = (o / nv) % n, j = o / (nv * n);
+                double s = 0.0, J[4];
+                for (int l = 0; l < n; ++l)
+                    for (int k = 0; k < n; ++k)
+                        s += __ldg(T + i + n * k) * __ldg(T + j + n * l) * r[d + nv * (k + n * l)];
+                quad_jacobian(c, __ldg(xg + i), __ldg(xg + j), J);
+                tmp[o] = s / (__ldg(wg + i) * __ldg(wg + j) * (J[0] * J[3] - J[2] * J[1]));
+            }
+            __syncwarp();
+            for (int o = lane; o < m; o += 32)
+            {
+                const int d = o % nv, i = (o / nv) % n, j = o / (nv * n);
+                double s = 0.0;
+                for (int l = 0; l < n; ++l)
+                    for (int k = 0; k < n; ++k)
+                        s += __ldg(T + n * i + k) * __ldg(T + n * j + l) * tmp[d + nv * (k + n * l)];
+                r[o] = s;
+            }
+            __syncwarp();
+            return;
+        }
         // (T x T)^T r at the Gauss points
         for (int o = lane; o < m; o += 32)
         {

@@ -68,7 +68,7 @@ namespace
         const double *op, *G, *Pv, *Dv, *Pf, *xg, *wg, *e;
         MassTables mass;
         const int *nb;
-        int n, nv, Q, Qf, approx, legendre;
+        int n, nv, Q, Qf;
     };
 
     // one variable, approx_quad = false: exact_line.cuh's model on the handle's tables
@@ -134,18 +134,17 @@ namespace
         return x + n * y;
     }
 
+    template <bool ex, bool leg, bool MASS>
     __global__ void vadv_kernel(const VArgs A, int warps)
     {
         extern __shared__ double vsm[];
         const ClawArgs &a = A.c;
         const int n = A.n, nv = A.nv, Q = A.Q, Qf = A.Qf, nn = n * n, QQ = Q * Q, v2 = nv * nv;
-        const bool ex = !A.approx;
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         double *su = vsm + (size_t)warp * va_warp_doubles(n, nv, Q, Qf);
         double *r = su + nv * nn, *Pu = r + nv * nn, *Uq = Pu + nv * n * Q, *Fq = Uq + nv * QQ;
         double *Df = Fq + 2 * nv * QQ, *Pg = Df + nv * Q * n, *T0 = Pg + nv * Q * n, *T1 = T0 + 4 * n * nv;
         double *UF = T1 + 4 * n * nv;
-        const bool leg = A.legendre != 0;
         const long long limit = (long long)nn * a.nel;
         const bool vol = a.mode != VA_BC;
         for (int el = blockIdx.x * warps + warp; el < a.nel; el += gridDim.x * warps)
@@ -402,12 +401,12 @@ namespace
             }
             // M^{-1} and the output: lane per node.  The volume term's half contractions are done with
             // Df, which holds at least nv n^2 values (Q >= n)
-            if (ex)
+            if constexpr (MASS)
                 x_mass_inv(n, nv, A.mass.T, A.mass.xg, A.mass.wg, c, r, Df, lane);
             for (int row = lane; row < nn; row += 32)
             {
                 double y[kJacobiMax];
-                if (ex)
+                if constexpr (MASS)
                     for (int d = 0; d < nv; ++d)
                         y[d] = r[nv * row + d];
                 else
@@ -454,6 +453,15 @@ namespace
             __syncwarp();
         }
     }
+
+    // By quadrature (collocation; exact, an action; exact, ending with M^{-1}) and basis (Lobatto, Legendre):
+    // a kernel of its own each, so that no call's loops are compiled around another's.  64 x 64, n_var 2,
+    // against one kernel for all: exact action, n = 9, Legendre: 176 -> 162 us; collocated RHS, n = 9: 59 -> 55;
+    // exact SSPRK3 step, n = 2: 52 -> 49 (n = 3 and below take the mass factors in two passes instead of four).
+    using VadvKernel = void (*)(const VArgs, int);
+    const VadvKernel kVadvKernels[3][2] = {{vadv_kernel<false, false, false>, vadv_kernel<false, true, false>},
+                                           {vadv_kernel<true, false, false>, vadv_kernel<true, true, false>},
+                                           {vadv_kernel<true, false, true>, vadv_kernel<true, true, true>}};
 
     // _ComputeFlux::flux with a = -1, b = -1/2 (source/EdgeFlux.cpp:31-88): Fs(c, d) for side
     // s of n.A; one variable in the closed form, else from the symmetric eigen-decomposition
@@ -712,12 +720,11 @@ namespace
         A.nv = h->nv;
         A.Q = h->Q;
         A.Qf = h->Qf;
-        A.approx = h->approx ? 1 : 0;
-        A.legendre = h->legendre ? 1 : 0;
         const int warps = va_warps(h);
         const size_t smem = sizeof(double) * (size_t)va_warp_doubles(h->n, h->nv, h->Q, h->Qf) * warps;
         const unsigned blocks = (unsigned)std::max(1, std::min((c.nel + warps - 1) / warps, 148 * 16));
-        vadv_kernel<<<blocks, 32 * warps, smem, h->w->stream>>>(A, warps);
+        const bool mass = !h->approx && c.mode != VA_ACT && c.mode != VA_BC;
+        kVadvKernels[h->approx ? 0 : mass ? 2 : 1][h->legendre ? 1 : 0]<<<blocks, 32 * warps, smem, h->w->stream>>>(A, warps);
         WDG_CUDA(cudaGetLastError());
         return WDG_OK;
     }
@@ -841,8 +848,11 @@ extern "C"
             const int dev = h->w->device & 63;
             if (!(set & (1ull << dev)))
             {
-                cudaError_t e =
-                    cudaFuncSetAttribute(vadv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+                cudaError_t e = cudaSuccess;
+                for (const auto &row : kVadvKernels)
+                    for (const auto kern : row)
+                        if (e == cudaSuccess)
+                            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
                 std::vector<XTabs<AdvectX<false>>> t0(1);
                 std::vector<XTabs<AdvectX<true>>> t1(1);
                 xtabs_fill(t0[0], false);

@@ -262,7 +262,7 @@ namespace wdg
             const WsSlot o{L::ub, L::hb - sh, L::cb - sh, L::kb - sh, 0, 0, 0};
             c.F = reinterpret_cast<const Real *>(Fs + sh) - (size_t)c.el0 * ND;
             c.acc = reinterpret_cast<double *>(As + sh) - (size_t)c.el0 * ND;
-            ws_consume<N, Real, EXTRA, false>(c, smem + sh, o, 1, sums, xm, wm, 0, lane);
+            ws_consume<N, Real, EXTRA, false, false>(c, smem + sh, o, 1, sums, xm, wm, 0, lane);
             fence_async_smem();
             __syncwarp();
             store(c.el0, c.ne);

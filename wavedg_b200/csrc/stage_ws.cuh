@@ -328,7 +328,13 @@ namespace wdg
     // ---------------------------------------------------------------- consumer: one chunk
     // Warp `cw` takes R rounds of EW whole elements, whose parts lie at base + o; Rc is its scratch for
     // the column sums, xm and wm the node and weight of its lane's line.
-    template <int N, typename Real, bool EXTRA, bool BATCH>
+    // SLOT: a chunk in a slot of a CTA's ring.  Those kernels hold their ring's state beside the passes: from n = 5
+    // on FP64 spills and FP32 loses a CTA per SM, so the row is read again for the update instead of kept,
+    // and the update's tests stand once per node (FP64, 220 x 220, us a step: n = 5: 692 -> 653, n = 9: 3057 -> 2514;
+    // batches, us a stage: n = 5: 39.9 -> 32.9, n = 7: 51 -> 48, n = 9: 61 -> 49.5; FP32 n = 7: 737 -> 657; but n = 4, FP64:
+    // 499 -> 565).  The kernel of one warp per CTA spills nothing, and its shared-memory pipe is what the second
+    // reading would load.
+    template <int N, typename Real, bool EXTRA, bool BATCH, bool SLOT>
     __device__ __forceinline__ void ws_consume(const WsChunk<Real> &c, unsigned char *base, const WsSlot &o,
                                                int R, Real *Rc, Real xm, Real wm, int cw, int lane)
     {
@@ -337,6 +343,7 @@ namespace wdg
         constexpr bool STG = WsStage<Real, EXTRA>::value;
         constexpr SumStride RS = stream_sums(N);
         constexpr int V = RowPiece<N, Real>::V;
+        constexpr bool AGAIN = SLOT && N >= 5;
         const int flags = c.flags;
         // forcing and filter: staged in the slot (chunk-local index) or read in place
         const Real *Fx = STG ? reinterpret_cast<const Real *>(base + o.fb) - (size_t)c.el0 * ND : c.F;
@@ -435,14 +442,28 @@ namespace wdg
                             const int i = i0 + l;
                             const Real *cr = rc + 3 * i + RS.row * j;
                             Real r[3] = {ap[i] + cr[0], au[i] + cr[1], av[i] + cr[2]};
-                            const Real q[3] = {q0[i], q1[i], q2[i]};
+                            const Real q[3] = {AGAIN ? row[3 * i] : q0[i], AGAIN ? row[3 * i + 1] : q1[i],
+                                               AGAIN ? row[3 * i + 2] : q2[i]};
                             const size_t g = (size_t)(c.el0 + le) * ND + 3 * (i + N * j);
+                            auto force = [&](int f) { r[f] += c.fscale * Fx[g + f]; };
+                            if (AGAIN && EXTRA && (flags & F_FORCE))
+                            {
+                                force(0);
+                                force(1);
+                                force(2);
+                            }
+                            if (AGAIN && (flags & F_MINV))
+                            {
+                                r[0] *= mv[i];
+                                r[1] *= mv[i];
+                                r[2] *= mv[i];
+                            }
 #pragma unroll
                             for (int f = 0; f < 3; ++f)
                             {
-                                if (EXTRA && (flags & F_FORCE))
-                                    r[f] += c.fscale * Fx[g + f];
-                                if (flags & F_MINV)
+                                if (!AGAIN && EXTRA && (flags & F_FORCE))
+                                    force(f);
+                                if (!AGAIN && (flags & F_MINV))
                                     r[f] *= mv[i];
                                 d[3 * l + f] = rk_register(has_du, c.rk_a, d[3 * l + f], c.dt, r[f]);
                                 uo[3 * l + f] = rk_state(q[f], c.rk_b, d[3 * l + f]);
@@ -497,6 +518,16 @@ namespace wdg
                 c.part[2 * cw + 1] = nsum;
             }
         }
+    }
+
+    // the same for a slot of a CTA's ring
+    template <int N, typename Real, bool EXTRA, bool BATCH>
+    __device__ __forceinline__ void ws_consume_slot(const WsChunk<Real> &c, unsigned char *base, Real *Rc, const Real *xtab,
+                                                    const Real *wtab, int cw, int lane)
+    {
+        const WsSlot o = ws_slot<Real>(N, c.chunk, WsStage<Real, EXTRA>::value);
+        ws_consume<N, Real, EXTRA, BATCH, true>(c, base, o, c.chunk / (kWsConsumers * (32 / N)), Rc, xtab[lane % N],
+                                                wtab[lane % N], cw, lane);
     }
 
     template <typename Real>
@@ -617,9 +648,6 @@ namespace wdg
 
         // ---------------------------------------------------------------- consumers
         Real *Rc = reinterpret_cast<Real *>(smem + L.scratch + warp * L.warp_scratch); // column sums
-        const WsSlot o = ws_slot<Real>(N, C, WsStage<Real, EXTRA>::value);
-        const int rounds = C / (kWsConsumers * (32 / N));
-        const Real xm = xt[lane % N], wm = wt[lane % N];
         for (int m = 0; m < M; ++m)
         {
             const int q = m % S;
@@ -630,7 +658,7 @@ namespace wdg
                 break;
             }
             at(m);
-            ws_consume<N, Real, EXTRA, false>(c, slots + q * L.slot, o, rounds, Rc, xm, wm, warp, lane);
+            ws_consume_slot<N, Real, EXTRA, false>(c, slots + q * L.slot, Rc, xt, wt, warp, lane);
             // results are in the slot: hand them to the async proxy, then release the slot
             fence_async_smem();
             __syncwarp();

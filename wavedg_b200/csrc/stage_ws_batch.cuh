@@ -204,8 +204,7 @@ namespace wdg
                 break;
             }
             build(kc);
-            ws_consume<N, Real, true, LAST>(c, slots + q * a.slot_bytes, ws_slot<Real>(N, c.chunk, WsStage<Real, true>::value),
-                                            c.chunk / (kWsConsumers * (32 / N)), Rc, xt[lane % N], wt[lane % N], warp, lane);
+            ws_consume_slot<N, Real, true, LAST>(c, slots + q * a.slot_bytes, Rc, xt, wt, warp, lane);
             // results are in the slot: hand them to the async proxy, then release the slot
             fence_async_smem();
             __syncwarp();

@@ -21,7 +21,8 @@
 //   row pass     lane (element, row j): xi-fluxes likewise, sides 3 and 1, + the column sums, M^{-1},
 //                the update in place
 // State and register come and go by cp.async.bulk, one copy per element (padded element strides keep
-// the passes off each other's banks); the neighbour traces of the next group are gathered with
+// the passes off each other's banks), where an element is a whole number of 16-byte units and the arrays are
+// aligned, else by 8-byte copies and plain stores (one and three variables at odd n); the neighbour traces of the next group are gathered with
 // cp.async as soon as the current group is done with its own, their table entries loaded a group
 // ahead.  A warp never waits for another one.
 //
@@ -146,7 +147,9 @@ namespace wdg
             static constexpr size_t smem = sizeof(double) * (size_t)total;
             static_assert(smem <= 227 * 1024, "a warp's elements fit shared memory");
             static constexpr int FIT = (int)(227 * 1024 / (smem + 1024));
-            // the registers a line's sums and state want, so that they do not spill
+            // the warps that the registers a line's sums and state want leave room for; an SM's quarters hold
+            // them, so that 13 warps get those of 16 (128 a thread) and 9 those of 12 (168), and some shapes spill
+            // (n = 5, n_var 2: 100 bytes; n = 2, n_var 7: 700)
             static constexpr int REGS = 65536 / 32 / (4 * N * NV + 110 < 255 ? 4 * N * NV + 110 : 255);
             static constexpr int MINB = FIT < 1 ? 1 : FIT > REGS ? REGS : FIT;
             static constexpr bool BULK = ND % 2 == 0; // whole 16-byte units per element
@@ -246,7 +249,7 @@ namespace wdg
             constexpr int IT = (EW * 4 * N + 31) / 32; // face nodes per lane
             uint32_t byte[IT];
             int off[IT];
-            // side codes and partner offsets of this lane's face nodes of group g
+            // side codes and partner offsets of this lane's face nodes of group g (the volume term alone wants none)
             auto tables = [&](int g)
             {
 #pragma unroll
@@ -255,7 +258,7 @@ namespace wdg
                     const int o = lane + 32 * t, el = g * EW + o / (4 * N), s = (o / N) & 3;
                     byte[t] = 0x80u;
                     off[t] = -1;
-                    if (g < ngroups && o < EW * 4 * N && el < a.nel)
+                    if ((M::LINEAR || a.mode != CLAW_DIV) && g < ngroups && o < EW * 4 * N && el < a.nel)
                     {
                         byte[t] = (__ldg(a.fcode + el) >> (8 * s)) & 0xffu;
                         off[t] = __ldg(reinterpret_cast<const int *>(a.fbase + el) + s);

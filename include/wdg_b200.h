@@ -393,7 +393,9 @@ int wdg_waveholtz_solve(wdg_waveholtz *wh, const double *F, double tol, int maxi
 
 /* ------------------------------------------------------ batched WaveHoltz */
 /* Up to 64 independent WaveHoltz solves, each on its own discretisation (mesh, degree) with
- * its own omega, advanced together: per RK stage one persistent kernel launch per degree
+ * its own omega, advanced together.  Solves whose elements fit the chip beside others' run whole periods
+ * resident, each on its share of the SMs; the others, and all solves of a batch with a chosen launch
+ * shape, stream: per RK stage one persistent kernel launch per degree
  * over a work list of (solve, chunk of elements), the degrees' launches concurrent, blocks
  * of steps replayed as a CUDA graph.  Per solve,
  * T, dt and nt follow WaveHoltz::WaveHoltz (source/WaveHoltz.cpp:24-29), and the iteration is
@@ -406,11 +408,14 @@ typedef struct wdg_whbatch wdg_whbatch;
 int wdg_whbatch_create(int n_solves, wdg_wave *const *waves, const double *omegas, wdg_whbatch **out);
 void wdg_whbatch_destroy(wdg_whbatch *batch);
 int wdg_whbatch_params(const wdg_whbatch *batch, int solve, double *T, double *dt, int *nt);
-/* chunk = rounds x (4 warps x floor(32 / n) elements) per solve; ring = chunk slots (2..6) */
+/* chunk = rounds x (4 warps x floor(32 / n) elements) per solve; ring = chunk slots (2..6).  From then on
+ * every solve of the batch streams. */
 int wdg_whbatch_set_launch(wdg_whbatch *batch, int rounds, int ring);
 /* grid: CTAs of one launch of an RK stage without the filter, summed over the degree groups */
 int wdg_whbatch_get_launch(const wdg_whbatch *batch, int *rounds, int *ring, int *grid);
-/* times `steps` batch steps of every launch shape that fits and keeps the fastest */
+/* times `steps` batch steps of every launch shape that fits, over the solves that stream, and keeps the
+ * fastest; where every solve's periods run resident there is no shape to choose, and a step of their
+ * first round is timed */
 int wdg_whbatch_autotune(wdg_whbatch *batch, int steps, float *best_ms_per_step);
 /* F[s], W[s]: FP64 arrays (host or device) of solve s.  warm (nullable): warm[s] != 0 starts
  * solve s from W[s] (one extra period from zero then gives |pi0|), else from zero.

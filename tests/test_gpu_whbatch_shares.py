@@ -42,3 +42,27 @@ def test_free_solves_fill_the_chip(gpu_lib):
 
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert _shares([(64, 4, 0), (48, 5, 0)]).sum() == sms
+
+
+def test_autotune_times_what_the_solves_run(gpu_lib):
+    """Where every solve is resident the launch shape stays and the time is the resident steps', several times
+    below the streaming launches'; a mixed batch tunes for the solve that streams."""
+    import wavedg_b200 as W
+
+    def batch(shapes):
+        systems = [W.WaveSystem(W.Mesh2D.uniform_rect(m, -1.0, 1.0, m, -1.0, 1.0), n, None, precision="fp32")
+                   for m, n in shapes]
+        return systems, W.WaveHoltzBatch(systems, np.full(len(shapes), 9.0))
+
+    _, a = batch([(32, 4), (24, 5)])
+    before = a.launch_config()
+    ms = a.autotune(64)
+    assert a.launch_config() == before
+    _, b = batch([(32, 4), (24, 5)])
+    b.set_launch(1, 2)
+    assert 0.0 < ms < 0.7 * b.autotune(64)
+    _, c = batch([(330, 3), (20, 4)])  # the first is too large for the chip
+    shares = np.zeros(2, dtype=np.int32)
+    assert W.lib().wdg_test_whbatch_shares(c._h, shares.ctypes.data) == 0
+    assert shares[0] == 0 and shares[1] > 0
+    assert c.autotune(32) > 0.0

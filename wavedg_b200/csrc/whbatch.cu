@@ -351,9 +351,9 @@ namespace
         return WDG_OK;
     }
 
-    // one period of solve s on `ctas` CTAs, on its own stream
+    // nsteps of the period of solve s on `ctas` CTAs, on its own stream
     template <typename Real>
-    int resident_period(wdg_whbatch *b, int s, int ctas, bool &ran)
+    int resident_steps(wdg_whbatch *b, int s, int ctas, int nsteps, bool &ran)
     {
         wdg_wave *w = b->w[s];
         RKExtras x;
@@ -362,12 +362,17 @@ namespace
         x.acc = b->d_acc[s];
         x.d_fscale = b->d_fscale[s];
         x.d_cfilter = b->d_cfilter[s];
-        const ResPlan p = res_plan_of(w, true, ctas);
-        Real *u = static_cast<Real *>(w->d_state[0]);
-        WDG_TRY(res_rk4<Real>(w, p, u, b->dt[s], b->nt[s], x, ran, b->rs[s]));
+        return res_rk4<Real>(w, res_plan_of(w, true, ctas), static_cast<Real *>(w->d_state[0]), b->dt[s], nsteps, x, ran,
+                             b->rs[s]);
+    }
+    // one period of it
+    template <typename Real>
+    int resident_period(wdg_whbatch *b, int s, int ctas, bool &ran)
+    {
+        WDG_TRY(resident_steps<Real>(b, s, ctas, b->nt[s], ran));
         if (ran)
-            WDG_CUDA(launch_whb_period_end<Real>(b->d_state + s, u, b->d_acc[s], b->d_W[s], b->c0[s], w->ndof, b->d_end[s],
-                                                 b->rs[s]));
+            WDG_CUDA(launch_whb_period_end<Real>(b->d_state + s, static_cast<Real *>(b->w[s]->d_state[0]), b->d_acc[s],
+                                                 b->d_W[s], b->c0[s], b->w[s]->ndof, b->d_end[s], b->rs[s]));
         return WDG_OK;
     }
 
@@ -485,6 +490,48 @@ namespace
             if (st != WDG_OK)
                 return fail(st, msg);
         }
+    }
+
+    // ms per step of a first round of resident periods, over `steps` (at most a period's) after as many
+    int time_resident(wdg_whbatch *b, const std::vector<int> &least, int steps, cudaEvent_t e0, cudaEvent_t e1, float &ms)
+    {
+        WDG_TRY(resident_prepare(b));
+        const std::vector<int> share = round_shares(b, least, std::vector<char>(b->n, 1));
+        for (int s = 0; s < b->n; ++s)
+            if (share[s])
+                steps = std::min(steps, b->nt[s]);
+        auto round = [&]() -> int
+        {
+            WDG_CUDA(cudaEventRecord(b->fork, b->cs));
+            for (int s = 0; s < b->n; ++s)
+            {
+                if (!share[s])
+                    continue;
+                WDG_CUDA(cudaStreamWaitEvent(b->rs[s], b->fork, 0));
+                bool ran = false;
+                WDG_TRY(b->precision == WDG_FP32 ? resident_steps<float>(b, s, share[s], steps, ran)
+                                                 : resident_steps<double>(b, s, share[s], steps, ran));
+                WDG_CUDA(cudaEventRecord(b->rdone[s], b->rs[s]));
+                WDG_CUDA(cudaStreamWaitEvent(b->cs, b->rdone[s], 0));
+            }
+            return WDG_OK;
+        };
+        int st = round();
+        cudaError_t e = cudaEventRecord(e0, b->cs);
+        if (st == WDG_OK)
+            st = round();
+        if (e == cudaSuccess)
+            e = cudaEventRecord(e1, b->cs);
+        for (cudaStream_t r : b->rs) // also behind a launch that failed
+            cudaStreamSynchronize(r);
+        WDG_TRY(st);
+        if (e == cudaSuccess)
+            e = cudaEventSynchronize(e1);
+        if (e == cudaSuccess)
+            e = cudaEventElapsedTime(&ms, e0, e1);
+        WDG_CUDA(e);
+        ms /= (float)steps;
+        return WDG_OK;
     }
 } // namespace
 
@@ -783,7 +830,8 @@ extern "C"
         return WDG_OK;
     }
 
-    // time `steps` batch steps of every (rounds, ring) that fits and keep the fastest
+    // time `steps` batch steps of every (rounds, ring) that fits and keep the fastest; solves whose periods run
+    // resident take no shape and no part, and where all do, a step of their first round is timed
     int wdg_whbatch_autotune(wdg_whbatch *b, int steps, float *best_ms_per_step)
     {
         if (!b || steps < 1)
@@ -795,12 +843,16 @@ extern "C"
             WDG_CUDA(cudaMemsetAsync(b->d_W[s], 0, sizeof(double) * (size_t)b->w[s]->ndof, b->cs));
             WDG_TRY(zero_period(b, s));
         }
+        const std::vector<int> least = least_shares(b);
+        const bool resident = std::all_of(least.begin(), least.end(), [](int c) { return c > 0; });
         cudaEvent_t e0, e1;
         WDG_CUDA(cudaEventCreate(&e0));
         WDG_CUDA(cudaEventCreate(&e1));
         float best = 1e30f;
         int br = b->rounds, bg = b->ring, st = WDG_OK;
-        for (int rounds = 1; rounds <= 4 && st == WDG_OK; ++rounds)
+        if (resident)
+            st = time_resident(b, least, steps, e0, e1, best);
+        for (int rounds = 1; rounds <= 4 && st == WDG_OK && !resident; ++rounds)
             for (int ring = 2; ring <= 4 && st == WDG_OK; ++ring)
             {
                 if (shape(b, rounds, ring) != WDG_OK)
@@ -809,6 +861,7 @@ extern "C"
                 {
                     b->h_state[s] = fresh_state(b, s, false, 0.0, 1, 0);
                     b->h_state[s].nt = 1 << 30; // no period ends while timing
+                    b->h_state[s].active = least[s] ? 0 : 1;
                 }
                 cudaError_t e = cudaMemcpyAsync(b->d_state, b->h_state, sizeof(WhbState) * b->n,
                                                 cudaMemcpyHostToDevice, b->cs);
@@ -842,10 +895,10 @@ extern "C"
             }
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        if (st == WDG_OK)
+        if (st == WDG_OK && !resident)
             st = shape(b, br, bg);
-        if (st == WDG_OK)
-            st = check_device_error(b->w[0]);
+        for (int s = 0; s < b->n && st == WDG_OK; ++s)
+            st = check_device_error(b->w[s]);
         if (best_ms_per_step)
             *best_ms_per_step = best;
         return st;

@@ -752,8 +752,9 @@ class WaveHoltz:
 
 class WaveHoltzBatch:
     """Many independent WaveHoltz solves advanced together (wdg_whbatch_*): each solve has its
-    own WaveSystem (mesh, degree; all of one precision and device) and its own omega.  One
-    persistent kernel launch per RK stage covers every running solve."""
+    own WaveSystem (mesh, degree; all of one precision and device) and its own omega.  Solves that
+    fit the chip run whole periods resident, each on its share of the SMs; the others, and every solve
+    after set_launch, stream: one persistent kernel launch per RK stage and degree covers them."""
 
     STATUS = {0: "converged", 1: "iteration limit", 2: "stalled", -1: "running"}
 

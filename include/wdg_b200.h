@@ -122,6 +122,9 @@ int wdg_wave_set_stages(wdg_wave *wave, int stages);
  * 1 tiled (element tiles staged in shared memory by a TMA bulk-copy pipeline), -1 default */
 int wdg_wave_set_kernel(wdg_wave *wave, int family);
 int wdg_wave_get_launch(const wdg_wave *wave, int *family, int *elems_per_block, int *stages, int *max_ctas);
+/* the kernel that RK steps on the handle's own state take now: 0 warp per element, 1 tiled, 2 warp-
+ * specialised, 3 one warp per CTA, 4 the mesh resident on the chip for all of a call's steps */
+int wdg_wave_step_kernel(wdg_wave *wave, int *kernel);
 /* the project's autotuner: times `steps` RK4 steps (dt = 0, state unchanged) for the warp
  * kernel and every (elements per block, pipeline depth) of the tiled kernel that fits, and
  * keeps the fastest for this handle */

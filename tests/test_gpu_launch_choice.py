@@ -59,3 +59,20 @@ def test_state_steps_need_a_state(gpu_lib, precision):
     s.upload(np.ones(s.ndof))
     s.step_state(1e-3, 0.0, 1)
     assert np.isfinite(s.download()).all()
+
+
+def test_step_kernel(gpu_lib):
+    import wavedg_b200 as W
+
+    small, large = (W.WaveSystem(W.Mesh2D.uniform_rect(k, -1.0, 1.0, k, -1.0, 1.0), 5, None) for k in (20, 180))
+    assert (small.step_kernel(), large.step_kernel()) == ("resident", "line")
+    for s in (small, large):
+        s.set_kernel(2)
+        assert s.step_kernel() == "ws"
+        s.set_kernel(1)
+        assert s.step_kernel() == "tiled"
+        s.set_kernel(0)
+        assert s.step_kernel() == "warp"
+        s.set_kernel(-1)
+    large.set_max_ctas(40)
+    assert large.step_kernel() == "ws"

@@ -120,6 +120,7 @@ SIGNATURES = {
     "wdg_wave_set_stages": ([_v, _i], _i),
     "wdg_wave_set_kernel": ([_v, _i], _i),
     "wdg_wave_get_launch": ([_v, _ip, _ip, _ip, _ip], _i),
+    "wdg_wave_step_kernel": ([_v, C.POINTER(_i)], _i),
     "wdg_wave_autotune": ([_v, _i, C.POINTER(C.c_float)], _i),
     "wdg_wave_node_coords": ([_v, _v], _i),
     "wdg_wave_set_wait_limit": ([_v, _d], _i),

@@ -720,6 +720,19 @@ extern "C"
         return WDG_OK;
     }
 
+    int wdg_wave_step_kernel(wdg_wave *w, int *kernel)
+    {
+        if (!w || !kernel)
+            return fail(WDG_ERR_ARG, "wdg_wave_step_kernel: bad arguments");
+        DeviceGuard g(w->device);
+        WDG_TRY(ensure_states(w));
+        *kernel = (w->family != 2)                                ? w->family
+                  : res_plan_of(w, false, w->max_ctas).fits       ? 4
+                  : (w->explicit_launch || w->max_ctas > 0)       ? 2
+                                                                  : 3;
+        return WDG_OK;
+    }
+
     int wdg_test_resident(wdg_wave *w, int forced, int *ctas)
     {
         if (!w || !ctas)

@@ -264,6 +264,12 @@ class Discretisation:
         check(lib().wdg_wave_get_launch(self._h, C.byref(f), C.byref(t), C.byref(st), C.byref(mc)))
         return {"kernel": ("warp", "tiled", "ws")[f.value], "tile": t.value, "stages": st.value, "max_ctas": mc.value}
 
+    def step_kernel(self) -> str:
+        """The kernel that RK steps on the handle's own state take now."""
+        k = C.c_int()
+        check(lib().wdg_wave_step_kernel(self._h, C.byref(k)))
+        return ("warp", "tiled", "ws", "line", "resident")[k.value]
+
     def autotune(self, steps: int = 5) -> float:
         """Pick elements-per-block and pipeline depth by timing; returns the best ms per RK4 step."""
         ms = C.c_float()

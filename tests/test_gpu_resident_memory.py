@@ -86,3 +86,23 @@ def test_steps_do_not_allocate(gpu_lib):
     s.step_state(1e-4, 0.0, 2)
     s.sync()
     assert torch.cuda.mem_get_info()[0] == free
+
+
+@pytest.mark.parametrize("precision,nx", [("fp64", 32), ("fp64", 200)])
+def test_array_steps_hold_no_state(gpu_lib, precision, nx):
+    """Steps on the caller's array allocate what steps work in and no state; the state comes with its upload,
+    and both then give the same."""
+    import torch
+
+    import wavedg_b200 as W
+
+    s = _system(nx, 4, precision)
+    u = torch.randn(s.ndof, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    x = u.clone()
+    dt = 0.1 * s.mesh.min_h() / 16
+    s.rk4_steps(x, dt, 0.0, 2)
+    with pytest.raises(W.WdgError):
+        s.step_state(dt, 0.0, 1)
+    s.upload(u)
+    s.step_state(dt, 0.0, 2)
+    assert np.array_equal(s.download(), x.cpu().numpy())

@@ -58,26 +58,27 @@ namespace wdg
         return WDG_OK;
     }
 
-    // The three state buffers and the RK register, allocated on first use so
-    // that operator-only handles (WaveEquation, WaveBC, MassMatrix drop-ins)
-    // hold geometry only.  Where the mesh may be resident, the rotation buffers are also
-    // large enough to serve as its trace buffers and the register is followed by its flags: a step is
-    // resident or streams, never both, and after this neither allocates, in a capture or out of one.
-    int ensure_states(wdg_wave *w)
+    // The state and what steps work in (two rotation buffers, the RK register), allocated on first use so
+    // that operator-only handles (WaveEquation, WaveBC, MassMatrix drop-ins) hold geometry only.
+    // Where the mesh may be resident, the rotation buffers are also large enough to serve as its trace
+    // buffers and the register is followed by its flags: a step is resident or streams, never both, and
+    // after this neither allocates, in a capture or out of one.  Steps on the caller's array need no state
+    // of the handle's.
+    int ensure_work(wdg_wave *w)
     {
         if (w->d_du)
             return WDG_OK; // the last of them
         const bool res = !w->halo && res_plan(w->n, w->precision == WDG_FP32, w->nel, w->sms, 0, false).fits;
         const size_t trace = res ? w->real_size() * 16 * (size_t)w->n * w->nel : 0;
-        for (int k = 0; k < 3; ++k)
+        const size_t state = w->real_size() * (size_t)(w->ndof + w->halo) + 64;
+        for (int k = 1; k < 3; ++k)
             if (!w->d_state[k])
             {
-                const size_t state = w->real_size() * (size_t)(w->ndof + w->halo);
-                cudaError_t e = cudaMalloc(&w->d_state[k], (k > 0 ? std::max(state, trace) : state) + 64);
+                cudaError_t e = cudaMalloc(&w->d_state[k], std::max(state, trace));
                 if (e != cudaSuccess)
                 {
                     w->d_state[k] = nullptr;
-                    return cuda_fail(e, "cudaMalloc(state)");
+                    return cuda_fail(e, "cudaMalloc(rotation buffer)");
                 }
             }
         const size_t du = (w->real_size() * (size_t)w->ndof + 64 + 255) & ~size_t(255);
@@ -94,6 +95,19 @@ namespace wdg
             w->d_trace[1] = w->d_state[2];
         }
         return WDG_OK;
+    }
+    int ensure_states(wdg_wave *w)
+    {
+        if (!w->d_state[0])
+        {
+            cudaError_t e = cudaMalloc(&w->d_state[0], w->real_size() * (size_t)(w->ndof + w->halo) + 64);
+            if (e != cudaSuccess)
+            {
+                w->d_state[0] = nullptr;
+                return cuda_fail(e, "cudaMalloc(state)");
+            }
+        }
+        return ensure_work(w);
     }
 
     int check_device_error(wdg_wave *w)
@@ -151,7 +165,7 @@ namespace wdg
     {
         if (A && (A == w->d_state[1] || A == w->d_state[2]))
             return fail(WDG_ERR_ARG, "rk4: state buffer aliases the rotation buffers");
-        WDG_TRY(ensure_states(w));
+        WDG_TRY(ensure_work(w));
         // a mesh that fits the chip stays there for all steps, unless the caller chose a kernel
         if (nsteps > 0 && (!x.F || x.d_fscale) && (!x.acc || x.d_cfilter))
         {
@@ -725,7 +739,7 @@ extern "C"
         if (!w || !kernel)
             return fail(WDG_ERR_ARG, "wdg_wave_step_kernel: bad arguments");
         DeviceGuard g(w->device);
-        WDG_TRY(ensure_states(w));
+        WDG_TRY(ensure_work(w));
         *kernel = (w->family != 2)                                ? w->family
                   : res_plan_of(w, false, w->max_ctas).fits       ? 4
                   : (w->explicit_launch || w->max_ctas > 0)       ? 2
@@ -738,7 +752,7 @@ extern "C"
         if (!w || !ctas)
             return fail(WDG_ERR_ARG, "wdg_test_resident: bad arguments");
         DeviceGuard g(w->device);
-        WDG_TRY(ensure_states(w));
+        WDG_TRY(ensure_work(w));
         const ResPlan p = res_plan_of(w, forced != 0, w->max_ctas);
         *ctas = p.fits ? p.ctas : 0;
         return WDG_OK;

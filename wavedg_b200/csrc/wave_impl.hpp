@@ -68,7 +68,8 @@ namespace wdg
         kChoseTile = 2,
         kChoseStages = 4
     };
-    int ensure_states(wdg_wave *w);
+    int ensure_work(wdg_wave *w);   // rotation buffers, register, what resident launches need
+    int ensure_states(wdg_wave *w); // and the state
     int check_device_error(wdg_wave *w);
     int sync(wdg_wave *w);
 

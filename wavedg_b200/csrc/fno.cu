@@ -22,7 +22,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstdint>
+#include <type_traits>
 
 #include "common.hpp"
 
@@ -429,11 +431,11 @@ namespace
     // and kDftThreads pairs of outputs (k, kx) and (k + K/2, kx), so that a value read from shared memory
     // serves two sums; y runs in order, whatever the chunking.  The twiddles and a chunk of `chunk` rows
     // sit in shared memory (the twiddles of a grid too large for it stay in global memory: TAB false; so do
-    // rows of which not one fits: ROWS false).  Pairs are read and written whole where `vec`, their
-    // alignment, allows it.
+    // rows of which not one fits: ROWS false).  Pairs are read and written whole (VEC), or value by value, and
+    // then from global memory, where an array does not lie on their boundary.
     constexpr int kDftThreads = 128, kDftRows = 128;
     constexpr size_t kDftSmem = 96 * 1024;
-    constexpr long long kGridY = 65535; // blocks of a grid along y
+    constexpr long long kGridY = 65535; // blocks of a grid along y; longer work goes in several launches (`off`)
     __device__ __forceinline__ void dft_add(float2 x, float2 cs, float sign, float &re, float &im)
     {
         const float c = cs.x, s = sign * cs.y;
@@ -441,13 +443,18 @@ namespace
         re += __fmaf_rn(c, x.x, -__fmul_rn(s, x.y));
         im += __fmaf_rn(s, x.x, __fmul_rn(c, x.y));
     }
-    __device__ __forceinline__ float2 pair_get(const float *p, long long i, bool vec)
+    template <bool VEC>
+    __device__ __forceinline__ float2 pair_get(const float *p, long long i)
     {
-        return vec ? __ldg(reinterpret_cast<const float2 *>(p) + i) : make_float2(__ldg(p + 2 * i), __ldg(p + 2 * i + 1));
+        if constexpr (VEC)
+            return reinterpret_cast<const float2 *>(p)[i];
+        else
+            return make_float2(p[2 * i], p[2 * i + 1]);
     }
-    __device__ __forceinline__ void pair_put(float *p, long long i, float re, float im, bool vec)
+    template <bool VEC>
+    __device__ __forceinline__ void pair_put(float *p, long long i, float re, float im)
     {
-        if (vec)
+        if constexpr (VEC)
             reinterpret_cast<float2 *>(p)[i] = make_float2(re, im);
         else
         {
@@ -455,64 +462,62 @@ namespace
             p[2 * i + 1] = im;
         }
     }
-    template <bool TAB, bool ROWS>
+    template <bool TAB, bool ROWS, bool VEC>
     __global__ void __launch_bounds__(kDftThreads) dft_y_fwd_kernel(const float *in, float *out, const float *cs,
                                                                     const float *sn, int G, int K, int KX, float sign,
-                                                                    int chunk, bool vec)
+                                                                    int chunk, unsigned off)
     {
         extern __shared__ float2 dsm[];
         float2 *tab = dsm, *xs = dsm + (TAB ? G : 0); // (cos, sin) of 2 pi m / G; a chunk of rows
         auto twiddle = [&](int m) { return TAB ? tab[m] : make_float2(__ldg(cs + m), __ldg(sn + m)); };
+        using index = std::conditional_t<ROWS, int, long long>; // of an output pair (the host's choice of ROWS: it fits)
         const int t = threadIdx.x, half = K / 2;
         const long long bc = blockIdx.x;
+        const index q = (index)(off + blockIdx.y) * kDftThreads + t;
+        const int kx = (int)(q % KX), k = (int)(q / KX);
+        const bool on = k < half;
         for (int m = t; TAB && m < G; m += kDftThreads)
             tab[m] = make_float2(cs[m], sn[m]);
         const float *src = in + 2 * bc * (long long)G * KX;
-        for (long long q0 = blockIdx.y * (long long)kDftThreads; q0 < (long long)half * KX; q0 += gridDim.y * (long long)kDftThreads)
+        const int step0 = k % G, step1 = ((k - half) % G + G) % G; // ky of k, of k + K/2: k + K/2 - K
+        float re0 = 0.f, im0 = 0.f, re1 = 0.f, im1 = 0.f;
+        int p0 = 0, p1 = 0;
+        for (int y0 = 0; y0 < G; y0 += chunk)
         {
-            const long long q = q0 + t;
-            const int kx = (int)(q % KX), k = (int)(q / KX);
-            const bool on = k < half;
-            const int step0 = k % G, step1 = ((k - half) % G + G) % G; // ky of k, of k + K/2: k + K/2 - K
-            float re0 = 0.f, im0 = 0.f, re1 = 0.f, im1 = 0.f;
-            int p0 = 0, p1 = 0;
-            for (int y0 = 0; y0 < G; y0 += chunk)
-            {
-                const int rows = min(chunk, G - y0);
-                __syncthreads();
-                for (int i = t; ROWS && i < rows * KX; i += kDftThreads)
-                    xs[i] = pair_get(src, (long long)y0 * KX + i, vec);
-                __syncthreads();
-                if (on)
-#pragma unroll 4
-                    for (int y = 0; y < rows; ++y)
-                    {
-                        const float2 x = ROWS ? xs[y * KX + kx] : pair_get(src, (long long)(y0 + y) * KX + kx, vec);
-                        dft_add(x, twiddle(p0), sign, re0, im0);
-                        dft_add(x, twiddle(p1), sign, re1, im1);
-                        p0 += step0;
-                        p0 -= p0 >= G ? G : 0;
-                        p1 += step1;
-                        p1 -= p1 >= G ? G : 0;
-                    }
-            }
+            const int rows = min(chunk, G - y0);
+            __syncthreads();
+            for (int i = t; ROWS && i < rows * KX; i += kDftThreads)
+                xs[i] = pair_get<VEC>(src, (long long)y0 * KX + i);
+            __syncthreads();
             if (on)
-            {
-                float *o = out + 2 * bc * (long long)K * KX;
-                pair_put(o, (long long)k * KX + kx, re0, im0, vec);
-                pair_put(o, (long long)(k + half) * KX + kx, re1, im1, vec);
-            }
+#pragma unroll 4
+                for (int y = 0; y < rows; ++y)
+                {
+                    const float2 x = ROWS ? xs[y * KX + kx] : pair_get<VEC>(src, (long long)(y0 + y) * KX + kx);
+                    dft_add(x, twiddle(p0), sign, re0, im0);
+                    dft_add(x, twiddle(p1), sign, re1, im1);
+                    p0 += step0;
+                    p0 -= p0 >= G ? G : 0;
+                    p1 += step1;
+                    p1 -= p1 >= G ? G : 0;
+                }
+        }
+        if (on)
+        {
+            float *o = out + 2 * bc * (long long)K * KX;
+            pair_put<VEC>(o, (long long)k * KX + kx, re0, im0);
+            pair_put<VEC>(o, (long long)(k + half) * KX + kx, re1, im1);
         }
     }
 
     // out[bc, y, kx] = sum_k e^{s i 2 pi ky(k) y / G} in[bc, k, kx]; FP32 and/or BF16 output.  A CTA takes one
-    // plane and kInvRows rows; the plane's modes and the twiddles sit in shared memory (TAB) where
+    // plane and `per` rows, kInvRows of usual length; the plane's modes and the twiddles sit in shared memory (TAB) where
     // they fit, k runs in order.
     constexpr int kInvRows = 32;
-    template <bool TAB>
+    template <bool TAB, bool VEC>
     __global__ void __launch_bounds__(kDftThreads) dft_y_inv_kernel(const float *in, float *out, bf16 *outb, const float *cs,
                                                                     const float *sn, int G, int K, int KX, float sign,
-                                                                    bool vec, bool vecb)
+                                                                    int per, unsigned off)
     {
         extern __shared__ float2 dsm[];
         float2 *tab = dsm, *xs = dsm + G;
@@ -520,39 +525,39 @@ namespace
         const long long bc = blockIdx.x;
         const float *src = in + 2 * bc * (long long)K * KX;
         auto twiddle = [&](int m) { return TAB ? tab[m] : make_float2(__ldg(cs + m), __ldg(sn + m)); };
-        auto mode = [&](int k, int kx) { return TAB ? xs[k * KX + kx] : pair_get(src, (long long)k * KX + kx, vec); };
+        auto mode = [&](int k, int kx) { return TAB ? xs[k * KX + kx] : pair_get<VEC>(src, (long long)k * KX + kx); };
         for (int m = t; TAB && m < G; m += kDftThreads)
             tab[m] = make_float2(cs[m], sn[m]);
         for (int i = t; TAB && i < K * KX; i += kDftThreads)
-            xs[i] = pair_get(src, i, vec);
+            xs[i] = pair_get<VEC>(src, i);
         __syncthreads();
-        for (long long y0 = blockIdx.y * (long long)kInvRows; y0 < G; y0 += gridDim.y * (long long)kInvRows)
+        const int y0 = (int)((off + blockIdx.y) * per), rows = min(per, G - y0);
+        for (int i = t; i < rows * KX; i += kDftThreads)
         {
-            const int rows = (int)min((long long)kInvRows, G - y0);
-            for (long long i = t; i < (long long)rows * KX; i += kDftThreads)
+            const int kx = i % KX, y = y0 + i / KX;
+            float re = 0.f, im = 0.f;
+            int p = 0;
+            for (int k = 0; k < half; ++k)
             {
-                const int kx = (int)(i % KX), y = (int)(y0 + i / KX);
-                float re = 0.f, im = 0.f;
-                int p = 0;
-                for (int k = 0; k < half; ++k)
-                {
-                    dft_add(mode(k, kx), twiddle(p), sign, re, im);
-                    p += y;
-                    p -= p >= G ? G : 0;
-                }
-                p = (G - (int)((long long)half * y % G)) % G; // ky = -K/2
-                for (int k = half; k < K; ++k)
-                {
-                    dft_add(mode(k, kx), twiddle(p), sign, re, im);
-                    p += y;
-                    p -= p >= G ? G : 0;
-                }
-                const long long o = (bc * G + y) * KX + kx;
-                if (out)
-                    pair_put(out, o, re, im, vec);
-                if (outb && vecb)
+                dft_add(mode(k, kx), twiddle(p), sign, re, im);
+                p += y;
+                p -= p >= G ? G : 0;
+            }
+            p = (G - (int)((long long)half * y % G)) % G; // ky = -K/2
+            for (int k = half; k < K; ++k)
+            {
+                dft_add(mode(k, kx), twiddle(p), sign, re, im);
+                p += y;
+                p -= p >= G ? G : 0;
+            }
+            const long long o = (bc * G + y) * KX + kx;
+            if (out)
+                pair_put<VEC>(out, o, re, im);
+            if (outb)
+            {
+                if constexpr (VEC)
                     reinterpret_cast<__nv_bfloat162 *>(outb)[o] = __floats2bfloat162_rn(re, im);
-                else if (outb)
+                else
                 {
                     outb[2 * o] = __float2bfloat16(re);
                     outb[2 * o + 1] = __float2bfloat16(im);
@@ -967,33 +972,41 @@ extern "C"
     {
         if (!in || !cos_tab || !sin_tab || BC < 1 || G < 2 || K < 2 || (K & 1) || KX < 1 || (!out && !out_bf16))
             return wdg::fail(WDG_ERR_ARG, "wdg_fno_dft_y: bad arguments");
-        const bool vec = (((uintptr_t)in | (uintptr_t)out) & 7u) == 0;
+        const bool vec = (((uintptr_t)in | (uintptr_t)out) & 7u) == 0 && ((uintptr_t)out_bf16 & 3u) == 0;
         if (!inverse)
         {
             if (!out)
                 return wdg::fail(WDG_ERR_ARG, "wdg_fno_dft_y: the forward transform writes FP32");
-            const bool tab = sizeof(float2) * ((size_t)G + KX) <= kDftSmem;
+            const long long pairs = (long long)(K / 2) * KX;
+            const bool fits = vec && pairs <= INT_MAX - kDftThreads; // the outputs are counted in an int
+            const bool tab = fits && sizeof(float2) * ((size_t)G + KX) <= kDftSmem;
             const size_t left = kDftSmem / sizeof(float2) - (tab ? G : 0);
-            const bool rows = left >= (size_t)KX;
+            const bool rows = fits && left >= (size_t)KX;
             const int chunk = rows ? (int)std::min<size_t>(kDftRows, left / KX) : G;
             const size_t smem = sizeof(float2) * ((tab ? (size_t)G : 0) + (rows ? (size_t)chunk * KX : 0));
-            auto kern = tab ? dft_y_fwd_kernel<true, true> : rows ? dft_y_fwd_kernel<false, true> : dft_y_fwd_kernel<false, false>;
+            auto kern = tab    ? dft_y_fwd_kernel<true, true, true>
+                        : rows ? dft_y_fwd_kernel<false, true, true>
+                        : vec  ? dft_y_fwd_kernel<false, false, true>
+                               : dft_y_fwd_kernel<false, false, false>;
             if (smem > 48 * 1024)
                 cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDftSmem);
-            const long long q = ((long long)(K / 2) * KX + kDftThreads - 1) / kDftThreads;
-            kern<<<dim3(BC, (unsigned)std::min(kGridY, q)), kDftThreads, smem, st(stream)>>>(in, out, cos_tab, sin_tab, G, K,
-                                                                                            KX, sign, chunk, vec);
+            const long long q = (pairs + kDftThreads - 1) / kDftThreads;
+            for (long long q0 = 0; q0 < q; q0 += kGridY)
+                kern<<<dim3(BC, (unsigned)std::min(kGridY, q - q0)), kDftThreads, smem, st(stream)>>>(
+                    in, out, cos_tab, sin_tab, G, K, KX, sign, chunk, (unsigned)q0);
         }
         else
         {
             const size_t want = sizeof(float2) * ((size_t)G + (size_t)K * KX);
-            const bool tab = want <= kDftSmem, vecb = ((uintptr_t)out_bf16 & 3u) == 0;
-            auto kern = tab ? dft_y_inv_kernel<true> : dft_y_inv_kernel<false>;
+            const bool tab = vec && want <= kDftSmem;
+            const int per = std::max(1, std::min(kInvRows, (INT_MAX - kDftThreads) / KX)); // their values are counted in an int
+            auto kern = tab ? dft_y_inv_kernel<true, true> : vec ? dft_y_inv_kernel<false, true> : dft_y_inv_kernel<false, false>;
             if (tab && want > 48 * 1024)
                 cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDftSmem);
-            const long long q = ((long long)G + kInvRows - 1) / kInvRows;
-            kern<<<dim3(BC, (unsigned)std::min(kGridY, q)), kDftThreads, tab ? want : 0, st(stream)>>>(
-                in, out, static_cast<bf16 *>(out_bf16), cos_tab, sin_tab, G, K, KX, sign, vec, vecb);
+            const long long q = ((long long)G + per - 1) / per;
+            for (long long q0 = 0; q0 < q; q0 += kGridY)
+                kern<<<dim3(BC, (unsigned)std::min(kGridY, q - q0)), kDftThreads, tab ? want : 0, st(stream)>>>(
+                    in, out, static_cast<bf16 *>(out_bf16), cos_tab, sin_tab, G, K, KX, sign, per, (unsigned)q0);
         }
         return done("wdg_fno_dft_y");
     }

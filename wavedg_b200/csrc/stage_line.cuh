@@ -234,7 +234,7 @@ namespace wdg
         int g = first(blockIdx.x), next = g;
         if (g >= ngroups)
             return;
-        if (a.test_skip != 1) // test hook: group test_skip - 1 of every warp stays unloaded
+        if (OP || a.test_skip != 1) // test hook: group test_skip - 1 of every warp stays unloaded
             load(g);
         gather();
         for (int m = 0; g < ngroups; ++m, g = next)
@@ -253,6 +253,7 @@ namespace wdg
             {
                 if (lane == 0)
                     atomicOr(a.err, 1u);
+                cp_async_wait_all(); // the gathered traces
                 break;
             }
             c.el0 = e0 + g * G;
@@ -272,11 +273,10 @@ namespace wdg
                 if (lane == 0)
                     bulk_wait_read();
                 __syncwarp();
-                if (a.test_skip != m + 2)
+                if (OP || a.test_skip != m + 2)
                     load(next);
             }
         }
-        cp_async_wait_all(); // after a wait that ran out, the gathered traces
         if (lane == 0)
             bulk_wait_all();
     }
